@@ -22,31 +22,31 @@ MODELS = ("llama-3-8b", "llama-3.2-1b", "gemma-2-9b", "gemma-2-2b")
 def listed():
     return [
         # one user, one token: the query / key / value product of the small model, the smallest call there is
-        {"name": "qkv 1b, 1 row", "kind": "linear", "model": "llama-3.2-1b", "part": "qkv", "rows": 1},
+        {"name": "qkv 1b 1 row", "kind": "linear", "model": "llama-3.2-1b", "part": "qkv", "rows": 1},
         # the common serving batch of about a hundred sequences: the product with the longest reduction
-        {"name": "down 8b, 100 rows", "kind": "linear", "model": "llama-3-8b", "part": "down", "rows": 100},
+        {"name": "down 8b 100 rows", "kind": "linear", "model": "llama-3-8b", "part": "down", "rows": 100},
         # steady state of the offline batch job (4608 sequences in flight): the feed-forward of a decode step
-        {"name": "mlp 8b, 4608 rows", "kind": "mlp", "model": "llama-3-8b", "rows": 4608},
+        {"name": "mlp 8b 4608 rows", "kind": "mlp", "model": "llama-3-8b", "rows": 4608},
         # the number of sequences that the reference's production scripts set, on the translation model
-        {"name": "mlp gemma 9b, 750 rows", "kind": "mlp", "model": "gemma-2-9b", "rows": 750},
+        {"name": "mlp gemma 9b 750 rows", "kind": "mlp", "model": "gemma-2-9b", "rows": 750},
         # the same steady state, 128 tokens in and 128 out: contexts between 129 and 256
-        {"name": "decode 8b, 4608 seqs", "kind": "decode", "model": "llama-3-8b", "seqs": 4608, "lo": 129, "hi": 256},
+        {"name": "decode 8b 4608 seqs", "kind": "decode", "model": "llama-3-8b", "seqs": 4608, "lo": 129, "hi": 256},
         # a handful of users with long documents on the small model
-        {"name": "decode 1b, 6 long seqs", "kind": "decode", "model": "llama-3.2-1b", "seqs": 6, "lo": 3000, "hi": 8100},
+        {"name": "decode 1b 6 long seqs", "kind": "decode", "model": "llama-3.2-1b", "seqs": 6, "lo": 3000, "hi": 8100},
         # mixed lengths on the model with the large heads, soft cap and sliding window
-        {"name": "decode gemma 9b, 100 seqs", "kind": "decode", "model": "gemma-2-9b", "seqs": 100, "lo": 33, "hi": 2560},
+        {"name": "decode gemma 9b 100 seqs", "kind": "decode", "model": "gemma-2-9b", "seqs": 100, "lo": 33, "hi": 2560},
         # prompts of the offline batch job: a full step of 36 prompts of 128 tokens
-        {"name": "prompts 8b, 36 x 128", "kind": "portion", "model": "llama-3-8b", "prompts": 36, "lo": 128, "hi": 128, "past": 0},
+        {"name": "prompts 8b 36 x 128", "kind": "portion", "model": "llama-3-8b", "prompts": 36, "lo": 128, "hi": 128, "past": 0},
         # long and ragged prompts on the model with the large heads, soft cap and sliding window
-        {"name": "prompts gemma 9b, 3 long", "kind": "portion", "model": "gemma-2-9b", "prompts": 3, "lo": 333, "hi": 2048, "past": 0},
+        {"name": "prompts gemma 9b 3 long", "kind": "portion", "model": "gemma-2-9b", "prompts": 3, "lo": 333, "hi": 2048, "past": 0},
         # the end of a decode step: last norm, rows, vocabulary product, sampling at the default temperature
-        {"name": "head 8b, 128 rows", "kind": "head", "model": "llama-3-8b", "rows": 128, "temperature": 0.7},
+        {"name": "head 8b 128 rows", "kind": "head", "model": "llama-3-8b", "rows": 128, "temperature": 0.7},
         # a whole decode step at the small model's widths, replayed from a graph as the engine does (four layers: behind more of them two
         # correct orders of the same sums are further apart than a comparison could allow)
-        {"name": "step 1b, 48 seqs", "kind": "step", "model": "llama-3.2-1b", "layers": 4, "seqs": 48, "lo": 100, "hi": 900, "prompts": 0,
+        {"name": "step 1b 48 seqs", "kind": "step", "model": "llama-3.2-1b", "layers": 4, "seqs": 48, "lo": 100, "hi": 900, "prompts": 0,
          "prompt": 0},
         # the routed feed-forward of a decode step
-        {"name": "experts, 128 rows", "kind": "experts", "width": 2048, "ff": 1024, "experts": 16, "top": 4, "groups": 4, "keep": 2,
+        {"name": "experts 128 rows", "kind": "experts", "width": 2048, "ff": 1024, "experts": 16, "top": 4, "groups": 4, "keep": 2,
          "rows": 128},
     ]
 
