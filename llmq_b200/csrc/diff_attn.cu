@@ -19,6 +19,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "layered_common.cuh"
 
@@ -793,10 +794,21 @@ __global__ void __launch_bounds__(128) diff_attn_decode_kernel(DiffAttn a) {
 // one flag in mapped host memory for the process: a kernel whose wait ran out sets it, the host reads it without a copy
 int* wait_flag(int** dev) {
   static int *host = nullptr, *device = nullptr;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
   if (!host) {
-    if (cudaHostAlloc((void**)&host, 64, cudaHostAllocMapped) != cudaSuccess) return nullptr;
-    *host = 0;
-    if (cudaHostGetDevicePointer((void**)&device, host, 0) != cudaSuccess) return nullptr;
+    // (the first call may come while the caller captures a graph: a host allocation is no part of it)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    int *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc((void**)&h, 64, cudaHostAllocMapped) == cudaSuccess &&
+        cudaHostGetDevicePointer((void**)&d, h, 0) == cudaSuccess) {
+      *h = 0;
+      device = d;
+      host = h;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!host) return nullptr;
   }
   if (dev) *dev = device;
   return host;

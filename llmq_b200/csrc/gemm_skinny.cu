@@ -1,0 +1,348 @@
+// gemm_skinny.cu — C[M,N] = A[M,K] . W[N,K]^T for up to 128 rows of A (decode steps), bf16 operands, fp32 accumulation.
+//
+// Bound: the weight stream from HBM (2 N K bytes); everything else has to stay out of its way.
+//   * the weights are the tensor core's M side (128 or 256 rows of W per CTA), the rows of A its N side, padded to 16 and not
+//     to 128: a step of few rows pays for few;
+//   * the reduction is split over a cluster of up to 8 CTAs so that every shape puts enough CTAs on the stream; the fp32
+//     partial tiles meet in distributed shared memory, are added in the order of the splits (deterministic) and stored once:
+//     no scratch round trip and no second launch;
+//   * no tile loop: a CTA works one tile, and where the ring takes half of an SM's memory the second CTA of the SM covers its
+//     start and its end.
+// A gated unit (SwiGLU, GeGLU, clamped) works on gate rows in the first 128 rows of a 256-row tile and up rows in the other.
+#include "tcgen05.cuh"
+
+namespace b200q {
+
+constexpr int SK_THREADS = 192;
+constexpr int SK_BK = 64;
+constexpr int SK_TILE_BYTES = 128 * SK_BK * 2;  // 128 weight rows of one k-block
+constexpr int SK_MAX_STAGES = 8;
+constexpr int SK_MAX_SPLITS = 8;
+
+struct SkinnyArgs {
+  bf16* C;
+  float* parts;  // != NULL: the fp32 partial tiles go here ([splits][M][N]) and the caller adds them
+  const float* bias;
+  int* failed;
+  long long ldc;
+  float limit;
+  int M, N, K, mp, stages, a_bytes, cols, chunk;  // mp: M padded to 16; chunk: columns (rows of A) per exchange
+};
+
+// WT: 128-row weight tiles per CTA
+template <int WT, int kAct>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+    gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const SkinnyArgs a) {
+  constexpr int NT = WT * 128;
+  static_assert(kAct == ACT_NONE || WT == 2, "a gated unit needs both halves");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], done;
+  __shared__ uint32_t tmem_slot;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = blockIdx.x, splits = gridDim.x, tile = blockIdx.y;
+  const int kb_all = a.K / SK_BK, kb0 = split * kb_all / splits, kb1 = (split + 1) * kb_all / splits;
+  const int stage_bytes = WT * SK_TILE_BYTES + a.mp * (SK_BK * 2);
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_a);
+    for (int s = 0; s < a.stages; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    mbar_init(&done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&tmem_slot, a.cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
+      int kb = kb0 + (kb1 > kb0 ? tile * 5 % (kb1 - kb0) : 0);
+      for (int i = kb0; i < kb1; ++i, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
+        if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, a.failed)) break;
+        uint8_t* sw = smem + stage * stage_bytes;
+        mbar_expect_tx(full + stage, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
+        tma_load_2d(sw, &tmap_w, kb * SK_BK, tile * NT, full + stage);
+        tma_load_2d(sw + WT * SK_TILE_BYTES, &tmap_a, kb * SK_BK, 0, full + stage);
+        if (++stage == a.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.mp >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int i = kb0; i < kb1; ++i) {
+        if (!mbar_wait_or_fail(full + stage, phase, a.failed)) break;
+        tc_fence_after();
+        const uint32_t sw = smem_u32(smem + stage * stage_bytes), sa = sw + WT * SK_TILE_BYTES;
+#pragma unroll
+        for (int h = 0; h < WT; ++h)
+#pragma unroll
+          for (int k = 0; k < SK_BK / 16; ++k)
+            umma_bf16(tmem + (uint32_t)(h * a.mp), make_smem_desc(sw + h * SK_TILE_BYTES + k * 32), make_smem_desc(sa + k * 32), idesc,
+                      (i > kb0 || k > 0) ? 1u : 0u);
+        umma_commit(empty + stage);
+        if (++stage == a.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      umma_commit(&done);
+    }
+    __syncwarp();
+  }
+
+  // ---- the accumulators: lane = weight row, column = row of A ----
+  float* red = reinterpret_cast<float*>(smem);  // [chunk][NT]; the ring is free once every product has been made
+  const bool epi = warp >= 2;
+  const int quarter = warp & 3, row = quarter * 32 + lane;
+  if (epi) {
+    mbar_wait_or_fail(&done, 0, a.failed);
+    __syncwarp();
+    tc_fence_after();
+  }
+  if (a.parts) {
+    if (epi) {
+      float* dst = a.parts + (long long)split * a.M * a.N + (long long)tile * NT + row;
+#pragma unroll 1
+      for (int h = 0; h < WT; ++h)
+#pragma unroll 1
+        for (int c = 0; c < a.mp; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * a.mp + c), v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < a.M) dst[(long long)(c + j) * a.N + h * 128] = __uint_as_float(v[j]);
+        }
+    }
+  } else {
+    for (int c0 = 0; c0 < a.M; c0 += a.chunk) {
+      if (epi) {
+        const int cn = min(a.chunk, a.mp - c0);
+#pragma unroll 1
+        for (int h = 0; h < WT; ++h)
+#pragma unroll 1
+          for (int c = 0; c < cn; c += 16) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * a.mp + c0 + c), v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) red[(c + j) * NT + h * 128 + row] = __uint_as_float(v[j]);
+          }
+      }
+      if (splits > 1)
+        cluster_sync_all();
+      else
+        __syncthreads();
+      // rows split, split + splits, ... of the chunk are this CTA's to add and store, four columns of C per thread
+      constexpr int OUT = kAct != ACT_NONE ? 128 : NT, GR = OUT / 4;
+      const int rows = min(a.chunk, a.M - c0), mine = rows > split ? (rows - split + splits - 1) / splits : 0;
+      for (int i = threadIdx.x; i < mine * GR; i += SK_THREADS) {
+        const int r = (i / GR) * splits + split, n = (i % GR) * 4;
+        const float* src = red + r * NT + n;
+        // (all partial sums are asked for before the first is added: a remote read takes about 200 cycles)
+        float4 p[SK_MAX_SPLITS], q[kAct != ACT_NONE ? SK_MAX_SPLITS : 1];
+        if (splits > 1) {
+#pragma unroll
+          for (int s = 0; s < SK_MAX_SPLITS; ++s)
+            if (s < splits) {
+              const uint32_t at = mapa_shared(src, s);
+              p[s] = ld_cluster_v4(at);
+              if constexpr (kAct != ACT_NONE) q[s] = ld_cluster_v4(at + 512);
+            }
+        } else {
+          p[0] = *reinterpret_cast<const float4*>(src);
+          if constexpr (kAct != ACT_NONE) q[0] = *reinterpret_cast<const float4*>(src + 128);
+        }
+        float4 x = p[0], y = x;
+        if constexpr (kAct != ACT_NONE) y = q[0];
+#pragma unroll
+        for (int s = 1; s < SK_MAX_SPLITS; ++s)
+          if (s < splits) {
+            x.x += p[s].x; x.y += p[s].y; x.z += p[s].z; x.w += p[s].w;
+            if constexpr (kAct != ACT_NONE) { y.x += q[s].x; y.y += q[s].y; y.z += q[s].z; y.w += q[s].w; }
+          }
+        float o[4] = {x.x, x.y, x.z, x.w};
+        if constexpr (kAct != ACT_NONE) {
+          const float u[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if constexpr (kAct == ACT_CLAMPED) {
+              const float* b = a.bias + (long long)tile * NT + n + j;
+              o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), a.bias ? __ldg(b) : 0.f, a.bias ? __ldg(b + 128) : 0.f,
+                                  a.limit);
+            } else {
+              o[j] = gated_unit<kAct>(__float_as_uint(o[j]), __float_as_uint(u[j]));
+            }
+          }
+        }
+        *reinterpret_cast<uint2*>(a.C + (long long)(c0 + r) * a.ldc + (long long)tile * OUT + n) =
+            make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+      }
+      if (splits > 1)  // nobody writes over, or leaves with, what a peer still reads
+        cluster_sync_all();
+      else if (c0 + a.chunk < a.M)
+        __syncthreads();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, a.cols);
+  }
+}
+
+constexpr int SK_RING_ALONE = 208 * 1024, SK_RING_SHARED = 108 * 1024;  // ring bytes with one and with two CTAs per SM
+
+// How many clusters of `splits` CTAs fit at once, one CTA per SM (asked for once per size).  The occupancy query knows one CTA per SM
+// for kernels that hold tensor memory; the hardware keeps two of them (256 columns or less each) where shared memory allows.
+template <int WT, int kAct>
+static int resident_clusters(int splits) {
+  static int known[SK_MAX_SPLITS + 1];
+  int& n = known[splits];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, 148);
+    cfg.blockDim = dim3(SK_THREADS);
+    cfg.dynamicSmemBytes = SK_RING_ALONE + 1024;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int v = 0;
+    if (cudaOccupancyMaxActiveClusters(&v, gemm_skinny_kernel<WT, kAct>, &cfg) != cudaSuccess || v <= 0) {
+      cudaGetLastError();
+      v = 1;
+    }
+    n = v;
+  }
+  return n;
+}
+
+struct SkinnyPlan {
+  bool alone;
+  int splits;
+};
+// Measured on B200, weights from HBM, back to back in a graph, us (new kernel / the kernels of gemm_tcgen05.cu before it):
+//   rows                        1            64           100
+//   4096 x 4096            10.6 / 12.5  12.3 / 13.7  13.3 / 14.5
+//   4096 x 14336           24.1 / 26.5  26.1 / 29.4  28.1 / 29.9
+//   16384 x 2048 gated     15.6 / 45.8  19.6 / 46.1  22.1 / 45.9
+//   28672 x 4096 gated     41.5 / 70.5  48.4 / 72.9  53.1 / 72.5
+//   3072 x 2048             6.8 /  8.3   8.7 / 10.9   9.4 / 12.1   (the launch itself is most of it)
+// Splits: up to 64 rows two CTAs per SM with three or more stages each are best; with more rows a stage grows and one CTA per SM
+// with the whole memory as its ring is (28.7 against 29.7 us at 4096 x 14336, 100 rows), unless the tiles alone would leave half
+// of the SMs idle.  All clusters have to be resident at once: a cluster lies within a processing cluster of the chip, and one
+// that does not fit doubles the time (2048 x 8192, 100 rows: 23.8 us with 16 clusters of 8, 14.8 with 16 of 6).
+template <int WT, int kAct>
+static SkinnyPlan skinny_plan(int M, int N, int K) {
+  const int kb = K / SK_BK, tiles = N / (128 * WT);
+  SkinnyPlan p{((M + 15) & ~15) > 64 && tiles <= 74, 1};
+  for (int s = 2; s <= SK_MAX_SPLITS && kb / s >= 4; ++s)
+    if (tiles <= resident_clusters<WT, kAct>(s) * (p.alone ? 1 : 2)) p.splits = s;
+  return p;
+}
+
+template <int WT, int kAct>
+static int prepare_kernel() {
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200Q_CUDA(cudaFuncSetAttribute(gemm_skinny_kernel<WT, kAct>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_RING_ALONE + 1024));
+    attr_set = true;
+  }
+  return B200Q_OK;
+}
+
+template <int WT, int kAct>
+static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_t st) {
+  int rc = prepare_kernel<WT, kAct>();
+  if (rc) return rc;
+  const SkinnyPlan p = skinny_plan<WT, kAct>(a.M, a.N, a.K);
+  const int a_rows = (a.M + 7) & ~7;  // only the rows that exist travel; the rest of the padded tile is never stored
+  a.mp = (a.M + 15) & ~15;
+  a.a_bytes = a_rows * SK_BK * 2;
+  a.cols = 32;
+  while (a.cols < WT * a.mp) a.cols *= 2;
+  const int stage = WT * SK_TILE_BYTES + a.mp * SK_BK * 2;
+  a.stages = (p.alone ? SK_RING_ALONE : SK_RING_SHARED) / stage;
+  if (a.stages > SK_MAX_STAGES) a.stages = SK_MAX_STAGES;
+  a.chunk = a.stages * stage / (WT * 512) & ~15;
+  if (a.chunk > a.mp) a.chunk = a.mp;
+  CUtensorMap tw, ta;
+  rc = get_tmap(W, a.N, a.K, WT * 128, &tw);
+  if (rc) return rc;
+  rc = get_tmap(A, a.M, a.K, a_rows, &ta);
+  if (rc) return rc;
+  if (!wait_flag(&a.failed)) {
+    set_error("gemm: no host-visible flag for bounded waits");
+    return B200Q_ECUDA;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.splits, a.N / (WT * 128));
+  cfg.blockDim = dim3(SK_THREADS);
+  cfg.dynamicSmemBytes = a.stages * stage + 1024;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = a.parts ? 1 : p.splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  B200Q_CUDA(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<WT, kAct>, tw, ta, a));
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+// Tiles of 256 rows halve what a CTA re-reads of A, tiles of 128 give twice the CTAs: 256 only where 128 would give more than
+// two for every SM (and for gated units, which need both halves).
+static bool wide_tiles(int N) { return N % 256 == 0 && N / 256 >= 148; }
+
+// Which products the kernel above takes.  With 113 to 128 rows and tiles enough for most SMs the persistent kernel of
+// gemm_tcgen05.cu is as good or better, because its next tile's loads run during a tile's end (128256 x 4096: 180.7 us there,
+// 184.7 here; 178 here against 180 at 100 rows).
+bool gemm_skinny_ok(int M, int N, int K, bool gated) {
+  if (M < 1 || M > 128 || K % SK_BK != 0 || N % (gated ? 256 : 128) != 0 || N / 128 > 65535) return false;
+  return M <= 112 || (gated ? N / 256 <= 74 : !wide_tiles(N));
+}
+
+int gemm_skinny_splits(int M, int N, int K) {
+  if (wide_tiles(N)) return prepare_kernel<2, ACT_NONE>() ? 1 : skinny_plan<2, ACT_NONE>(M, N, K).splits;
+  return prepare_kernel<1, ACT_NONE>() ? 1 : skinny_plan<1, ACT_NONE>(M, N, K).splits;
+}
+
+// C (or, `parts`: the fp32 partial tiles [splits][M][N]) of up to 128 rows; `act`: ACT_*
+int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int act, long long ldc, const float* bias, float limit,
+                float* parts, cudaStream_t st) {
+  SkinnyArgs a{};
+  a.C = (bf16*)C;
+  a.parts = parts;
+  a.bias = bias;
+  a.limit = limit;
+  a.ldc = ldc;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  if (act == ACT_SWIGLU) return launch_skinny<2, ACT_SWIGLU>(A, W, a, st);
+  if (act == ACT_GEGLU) return launch_skinny<2, ACT_GEGLU>(A, W, a, st);
+  if (act == ACT_CLAMPED) return launch_skinny<2, ACT_CLAMPED>(A, W, a, st);
+  return wide_tiles(N) ? launch_skinny<2, ACT_NONE>(A, W, a, st) : launch_skinny<1, ACT_NONE>(A, W, a, st);
+}
+
+}  // namespace b200q

@@ -15,13 +15,12 @@
 //
 // Roofline: decode-sized M is HBM-bound on the weight stream (N*K*2 bytes), M >= ~256 is
 // tensor-bound (2*M*N*K flops against the measured bf16 peak).
-#include <cuda.h>
 #include <stdlib.h>
 
 #include <mutex>
 #include <unordered_map>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace b200q {
 
@@ -39,71 +38,6 @@ struct GemmCfg {
   static constexpr int TMEM_COLS = 2 * BN;  // 128 / 256 / 512: powers of two >= 32
   static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 4 * 4096 /*epilogue*/;
 };
-
-// ---- tcgen05 PTX wrappers ------------------------------------------------------------------
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(smem_dst)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]; kind::f16 covers bf16 inputs with fp32 accumulate
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrive on an mbarrier once all previously issued tcgen05.mma of this thread have completed
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// UMMA shared-memory descriptor, K-major operand, SWIZZLE_128B, 8-row groups 1024 B apart
-// (cute/arch/mma_sm100_desc.hpp SmemDescriptor: start[0,14) lbo[16,30) sbo[32,46) version[46,48)
-//  layout_type[61,64)).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);        // start address, 16 B units
-  d |= (uint64_t)1 << 16;                              // LBO (ignored for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                    // SBO: 8 rows * 128 B
-  d |= (uint64_t)1 << 46;                              // descriptor version (sm_100)
-  d |= (uint64_t)2 << 61;                              // SWIZZLE_128B
-  return d;
-}
 
 // instruction descriptor for kind::f16: D=f32, A=B=bf16, both K-major, M=128, N=BN
 __host__ __device__ constexpr uint32_t make_idesc(int n) {
@@ -123,32 +57,12 @@ __host__ __device__ constexpr uint32_t make_idesc(int n) {
 // [T, 2I] intermediate never touches HBM.
 constexpr int EPI_SMEM_PER_WARP = 32 * 128;  // 32 rows x 64 bf16
 
-// kAct: 0 = plain GEMM, 1 = SwiGLU (Llama), 2 = GeGLU with the tanh approximation (Gemma-2):
-// out = bf16(bf16(gelu_tanh(bf16(g))) * bf16(u)), gelu_tanh evaluated in fp32 like torch's kernel:
-// 0.5 * g * (1 + tanh(sqrt(2/pi) * (g + 0.044715 g^3)))
-// 3 = clamped unit (Lipedra: with biases; Fimilorn: without): g' sigmoid(1.702 g') (u' + 1), g' = min(g + bg, limit), u' = clamp(u + bu,
-// -limit, limit), in fp32 from the accumulators (one rounding); bias: fp32, this tile's [gate (BN/2) | up (BN/2)], or NULL
-constexpr int ACT_NONE = 0, ACT_SWIGLU = 1, ACT_GEGLU = 2, ACT_CLAMPED = 3;
-struct GateArgs {
-  const float* bias;
-  float limit;
-};
-
 template <int BN, int kAct>
 __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long long ldc,
                                               int row0, int M, uint8_t* patch, int lane,
                                               const float* gate_bias = nullptr, float limit = 0.f) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;  // gated epilogue: tile = [gate (BN/2) | up (BN/2)]
   constexpr int OUT_BN = kSwiGLU ? BN / 2 : BN;
-  auto act = [](uint32_t gb, uint32_t ub) -> float {
-    const float g = round_bf16(__uint_as_float(gb)), u = round_bf16(__uint_as_float(ub));
-    if constexpr (kAct == ACT_GEGLU) {
-      const float inner = 0.7978845608028654f * (g + 0.044715f * (g * g * g));
-      return round_bf16(0.5f * g * (1.f + tanhf(inner))) * u;
-    } else {
-      return round_bf16(g / (1.f + __expf(-g))) * u;
-    }
-  };
   const uint32_t patch_s = smem_u32(patch);
 #pragma unroll 1
   for (int c0 = 0; c0 < OUT_BN; c0 += 64) {
@@ -174,19 +88,14 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
         if constexpr (kAct == ACT_CLAMPED) {
           const float4* bg = reinterpret_cast<const float4*>(gate_bias + c0 + 32 * h);
           const float4* bu = reinterpret_cast<const float4*>(gate_bias + BN / 2 + c0 + 32 * h);
-          auto unit = [&](uint32_t gb, uint32_t ub, float b0, float b1) -> uint32_t {
-            const float g = fminf(__uint_as_float(gb) + b0, limit);
-            const float w = fminf(fmaxf(__uint_as_float(ub) + b1, -limit), limit);
-            return __float_as_uint(g / (1.f + __expf(-1.702f * g)) * (w + 1.f));
-          };
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             const float4 x = gate_bias ? __ldg(bg + j) : zero, y = gate_bias ? __ldg(bu + j) : zero;
-            v[4 * j + 0] = unit(v[4 * j + 0], u[4 * j + 0], x.x, y.x);
-            v[4 * j + 1] = unit(v[4 * j + 1], u[4 * j + 1], x.y, y.y);
-            v[4 * j + 2] = unit(v[4 * j + 2], u[4 * j + 2], x.z, y.z);
-            v[4 * j + 3] = unit(v[4 * j + 3], u[4 * j + 3], x.w, y.w);
+            v[4 * j + 0] = __float_as_uint(clamped_unit(v[4 * j + 0], u[4 * j + 0], x.x, y.x, limit));
+            v[4 * j + 1] = __float_as_uint(clamped_unit(v[4 * j + 1], u[4 * j + 1], x.y, y.y, limit));
+            v[4 * j + 2] = __float_as_uint(clamped_unit(v[4 * j + 2], u[4 * j + 2], x.z, y.z, limit));
+            v[4 * j + 3] = __float_as_uint(clamped_unit(v[4 * j + 3], u[4 * j + 3], x.w, y.w, limit));
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -198,10 +107,10 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
         } else
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          o[j].x = pack_bf16x2(act(v[8 * j + 0], u[8 * j + 0]), act(v[8 * j + 1], u[8 * j + 1]));
-          o[j].y = pack_bf16x2(act(v[8 * j + 2], u[8 * j + 2]), act(v[8 * j + 3], u[8 * j + 3]));
-          o[j].z = pack_bf16x2(act(v[8 * j + 4], u[8 * j + 4]), act(v[8 * j + 5], u[8 * j + 5]));
-          o[j].w = pack_bf16x2(act(v[8 * j + 6], u[8 * j + 6]), act(v[8 * j + 7], u[8 * j + 7]));
+          o[j].x = pack_bf16x2(gated_unit<kAct>(v[8 * j + 0], u[8 * j + 0]), gated_unit<kAct>(v[8 * j + 1], u[8 * j + 1]));
+          o[j].y = pack_bf16x2(gated_unit<kAct>(v[8 * j + 2], u[8 * j + 2]), gated_unit<kAct>(v[8 * j + 3], u[8 * j + 3]));
+          o[j].z = pack_bf16x2(gated_unit<kAct>(v[8 * j + 4], u[8 * j + 4]), gated_unit<kAct>(v[8 * j + 5], u[8 * j + 5]));
+          o[j].w = pack_bf16x2(gated_unit<kAct>(v[8 * j + 6], u[8 * j + 6]), gated_unit<kAct>(v[8 * j + 7], u[8 * j + 7]));
         }
       }
 #pragma unroll
@@ -427,21 +336,6 @@ struct Gemm2Cfg {
   static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + 4 * 4096;
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of `p` (a shared-memory object of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t mapa_shared(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster_addr, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(
                    bar_cluster_addr),
@@ -674,8 +568,7 @@ struct TmapKeyHash {
 
 // bf16 row-major [rows, cols] -> tiled map with box {64 cols, box_rows rows}, 128B swizzle
 // (ld: elements between rows, 0 = dense)
-static int get_tmap(const void* ptr, long long rows, long long cols, int box_rows,
-                    CUtensorMap* out, long long ld = 0) {
+int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out, long long ld) {
   static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
   static std::mutex mu;
   if (ld == 0) ld = cols;
@@ -726,8 +619,17 @@ static int num_sms() {
   return n;
 }
 
-static float* g_splitk_ws = nullptr;
-static size_t g_splitk_ws_bytes = 0;
+// fixed-size scratch of partial tiles (8 splits x 256 rows x 8192 cols fp32 = 64 MiB), allocated once and never moved: CUDA
+// graphs captured by the engine bake this pointer into their kernel nodes
+static int splitk_scratch(int splits, int M, int N, float** out) {
+  static float* ws = nullptr;
+  const size_t need = (size_t)splits * M * N * sizeof(float);
+  const size_t cap = (size_t)8 * 256 * 8192 * sizeof(float);
+  B200Q_CHECK_ARG(need <= cap, "split-K scratch too small for M=%d N=%d splits=%d", M, N, splits);
+  if (!ws) B200Q_CUDA(cudaMalloc(&ws, cap));
+  *out = ws;
+  return B200Q_OK;
+}
 
 template <int BN, int kAct = ACT_NONE>
 static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int K,
@@ -751,16 +653,8 @@ static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int 
   const int grid = tiles < num_sms() ? tiles : num_sms();
   float* ws = nullptr;
   if (splits > 1) {
-    // fixed-size scratch (8 splits x 256 rows x 8192 cols fp32 = 64 MiB), allocated once and never
-    // moved: CUDA graphs captured by the engine bake this pointer into their kernel nodes
-    const size_t need = (size_t)splits * M * N * sizeof(float);
-    const size_t cap = (size_t)8 * 256 * 8192 * sizeof(float);
-    B200Q_CHECK_ARG(need <= cap, "split-K scratch too small for M=%d N=%d splits=%d", M, N, splits);
-    if (!g_splitk_ws) {
-      B200Q_CUDA(cudaMalloc(&g_splitk_ws, cap));
-      g_splitk_ws_bytes = cap;
-    }
-    ws = g_splitk_ws;
+    rc = splitk_scratch(splits, M, N, &ws);
+    if (rc) return rc;
   }
   kern<<<grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st>>>(ta, tb, (bf16*)C, M, N, K, splits, ws,
                                                     a_rows * GEMM_BK * 2,
@@ -927,6 +821,12 @@ static int choose_splits(int M, int N, int K, bool invariant, int forced_bn) {
   return (splits > 1 && splits <= 8 && kb % splits == 0) ? splits : 1;
 }
 int g_gemm_mode = 0;      // 0 = auto, 1 = force 1-CTA kernels, 2 = force the 2-CTA kernel
+
+// Up to 128 rows go to gemm_skinny.cu unless a hook asks for one of the kernels here, or results must not depend on the number of
+// rows (its splits depend on it, and the kernels here that larger steps use add in another order).
+static bool use_skinny(int M, int N, int K, bool gated) {
+  return g_gemm_mode == 0 && g_gemm_force_bn == 0 && g_gemm_splitk == 0 && !batch_invariant_env() && gemm_skinny_ok(M, N, K, gated);
+}
 
 
 // ------------------------------------------------------------------------------------------------
@@ -1136,6 +1036,8 @@ static int gemm_gated(const char* what, const void* A, const void* W, void* C, i
                   "%s: operands must be 16-byte aligned", what);
   if (M == 0) return B200Q_OK;
   cudaStream_t st = as_stream(stream);
+  if (use_skinny(M, N, K, true))
+    return gemm_skinny(A, W, C, M, N, K, kAct, ldc > 0 ? ldc : N / 2, gate.bias, gate.limit, nullptr, st);
   if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && prefer_2cta(M, N)))
     return launch_gemm2<256, kAct>(A, W, C, M, N, K, st, ldc, gate);
   return launch_gemm<256, kAct>(A, W, C, M, N, K, st, 1, nullptr, ldc, gate);
@@ -1240,6 +1142,7 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
                   "gemm: operands must be 16-byte aligned");
   if (M == 0) return B200Q_OK;
   cudaStream_t st = as_stream(stream);
+  if (use_skinny(M, N, K, false)) return gemm_skinny(A, W, C, M, N, K, ACT_NONE, N, nullptr, 0.f, nullptr, st);
   int bn = g_gemm_force_bn;
   if (g_gemm_mode == 2 && M > GEMM_BM) {
     if ((bn == 0 || bn == 256) && N % 256 == 0) return launch_gemm2<256>(A, W, C, M, N, K, st);
@@ -1299,6 +1202,17 @@ int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, vo
                   "gemm: operands must be 16-byte aligned");
   if (M == 0 || g_gemm_mode == 2 || g_gemm_force_bn != 0 || (g_gemm_mode == 0 && prefer_2cta(M, N)))
     return B200Q_OK;
+  if (use_skinny(M, N, K, false)) {
+    const int n = gemm_skinny_splits(M, N, K);
+    if (n <= 1 || N > 8192) return B200Q_OK;
+    float* ws = nullptr;
+    int rc = splitk_scratch(n, M, N, &ws);
+    if (!rc) rc = gemm_skinny(A, W, nullptr, M, N, K, ACT_NONE, N, nullptr, 0.f, ws, as_stream(stream));
+    if (rc) return rc;
+    *partials_out = ws;
+    *splits_out = n;
+    return B200Q_OK;
+  }
   const int splits = choose_splits(M, N, K, batch_invariant_env(), 0);
   if (splits <= 1) return B200Q_OK;
   int rc = launch_gemm<128>(A, W, nullptr, M, N, K, as_stream(stream), splits, partials_out);

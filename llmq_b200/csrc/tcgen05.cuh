@@ -1,0 +1,151 @@
+// tcgen05.cuh — tensor-core pieces shared by the kernels that issue tcgen05.mma (gemm_tcgen05.cu, gemm_skinny.cu, ...): PTX
+// wrappers, the shared-memory descriptor, bounded barrier waits, the gated units of the feed-forwards, the tensor-map cache.
+#pragma once
+#include <cuda.h>
+
+#include "layered_common.cuh"
+
+namespace b200q {
+
+// ---- tcgen05 PTX wrappers ------------------------------------------------------------------
+__device__ __forceinline__ void tc_fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tc_fence_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                   smem_u32(smem_dst)),
+               "r"(ncols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
+               : "memory");
+}
+// D[tmem] (+)= A[smem desc] * B[smem desc]; kind::f16 covers bf16 inputs with fp32 accumulate
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                          uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrive on an mbarrier once all previously issued tcgen05.mma of this thread have completed
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait() {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+
+// wait with a limit: false when it ran out, and then *failed is set (the engine reports it)
+__device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, int* failed) {
+  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_wait_limited(bar, parity)) return true;
+  *(volatile int*)failed = 1;
+  return false;
+}
+
+// ---- thread-block clusters ------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of `p` (a shared-memory object of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa_shared(const void* p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// UMMA shared-memory descriptor, K-major operand, SWIZZLE_128B, 8-row groups 1024 B apart
+// (cute/arch/mma_sm100_desc.hpp SmemDescriptor: start[0,14) lbo[16,30) sbo[32,46) version[46,48)
+//  layout_type[61,64)).
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);        // start address, 16 B units
+  d |= (uint64_t)1 << 16;                              // LBO (ignored for swizzled K-major)
+  d |= (uint64_t)(1024 >> 4) << 32;                    // SBO: 8 rows * 128 B
+  d |= (uint64_t)1 << 46;                              // descriptor version (sm_100)
+  d |= (uint64_t)2 << 61;                              // SWIZZLE_128B
+  return d;
+}
+
+// kAct: 0 = plain GEMM, 1 = SwiGLU (Llama), 2 = GeGLU with the tanh approximation (Gemma-2):
+// out = bf16(bf16(gelu_tanh(bf16(g))) * bf16(u)), gelu_tanh evaluated in fp32 like torch's kernel:
+// 0.5 * g * (1 + tanh(sqrt(2/pi) * (g + 0.044715 g^3)))
+// 3 = clamped unit (Lipedra: with biases; Fimilorn: without): g' sigmoid(1.702 g') (u' + 1), g' = min(g + bg, limit), u' = clamp(u + bu,
+// -limit, limit), in fp32 from the accumulators (one rounding); bias: fp32, this tile's [gate (BN/2) | up (BN/2)], or NULL
+constexpr int ACT_NONE = 0, ACT_SWIGLU = 1, ACT_GEGLU = 2, ACT_CLAMPED = 3;
+struct GateArgs {
+  const float* bias;
+  float limit;
+};
+
+template <int kAct>
+__device__ __forceinline__ float gated_unit(uint32_t gb, uint32_t ub) {
+  const float g = round_bf16(__uint_as_float(gb)), u = round_bf16(__uint_as_float(ub));
+  if constexpr (kAct == ACT_GEGLU) {
+    const float inner = 0.7978845608028654f * (g + 0.044715f * (g * g * g));
+    return round_bf16(0.5f * g * (1.f + tanhf(inner))) * u;
+  } else {
+    return round_bf16(g / (1.f + __expf(-g))) * u;
+  }
+}
+__device__ __forceinline__ float clamped_unit(uint32_t gb, uint32_t ub, float b0, float b1, float limit) {
+  const float g = fminf(__uint_as_float(gb) + b0, limit);
+  const float w = fminf(fmaxf(__uint_as_float(ub) + b1, -limit), limit);
+  return g / (1.f + __expf(-1.702f * g)) * (w + 1.f);
+}
+
+// bf16 row-major [rows, cols] -> tiled map with box {64 cols, box_rows rows}, 128B swizzle (ld: elements between rows, 0 = dense);
+// maps are cached by address and shape (gemm_tcgen05.cu)
+int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out, long long ld = 0);
+
+// products of up to 128 rows (gemm_skinny.cu)
+bool gemm_skinny_ok(int M, int N, int K, bool gated);
+int gemm_skinny_splits(int M, int N, int K);
+int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int act, long long ldc, const float* bias, float limit,
+                float* parts, cudaStream_t st);
+
+}  // namespace b200q
