@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
 }
 
 // ------------------------------------------------------------------------------------------
-// K6 prefill
+// K6 prefill, contexts too short for the kernel of prefill_attn.cu (its rule stands there)
 // ------------------------------------------------------------------------------------------
 template <int D, int BS>
 struct PfSmem {
@@ -616,7 +616,7 @@ struct PfCfg {
 
 template <int D, int BS, bool kCap>
 __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
-    prefill_attn_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out,
+    prefill_tile_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out,
                         const uint8_t* __restrict__ kv_layer,
                         const int32_t* __restrict__ block_table, int bt_stride,
                         const int4* __restrict__ tiles, int n_q, int n_kv, int G,
@@ -847,7 +847,7 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
                           int n_q, int n_kv, float scale, float softcap, int window,
                           cudaStream_t st) {
   using S_ = PfSmem<D, BS>;
-  auto kern = prefill_attn_kernel<D, BS, kCap>;
+  auto kern = prefill_tile_kernel<D, BS, kCap>;
   static bool attr_set = false;
   if (!attr_set) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
@@ -874,6 +874,11 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
     if (D == 128) return cap ? FN<128, 16, true>(__VA_ARGS__) : FN<128, 16, false>(__VA_ARGS__); \
     return cap ? FN<256, 16, true>(__VA_ARGS__) : FN<256, 16, false>(__VA_ARGS__);               \
   } while (0)
+
+int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
+                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, cudaStream_t st) {
+  B200Q_ATTN_DISPATCH(launch_prefill, q, q_stride, out, kv, bt, bt_stride, tiles, n_tiles, n_q, n_kv, scale, softcap, window, st);
+}
 
 }  // namespace b200q
 
@@ -918,30 +923,6 @@ int b200q_decode_attn(const void* q, int q_stride, void* out, const void* kv_lay
                       void* stream) {
   return b200q_decode_attn_ex(q, q_stride, out, kv_layer, block_table, bt_stride, ctx_lens, n_seqs,
                               n_q, n_kv, D, block_size, scale, 0.f, 0, stream);
-}
-
-int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv_layer,
-                          const int32_t* block_table, int bt_stride, const int32_t* tiles,
-                          int n_tiles, int n_q, int n_kv, int D, int block_size, float scale,
-                          float softcap, int window, void* stream) {
-  B200Q_CHECK_ARG(n_tiles >= 0 && n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 8,
-                  "prefill_attn: unsupported heads n_q=%d n_kv=%d (GQA group must be <= 8)", n_q,
-                  n_kv);
-  B200Q_CHECK_ARG(block_size == 16 && (D == 64 || D == 128 || D == 256),
-                  "prefill_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D,
-                  block_size);
-  if (n_tiles == 0) return B200Q_OK;
-  cudaStream_t st = as_stream(stream);
-  B200Q_ATTN_DISPATCH(launch_prefill, q, q_stride, out, kv_layer, block_table, bt_stride, tiles,
-                      n_tiles, n_q, n_kv, scale, softcap, window, st);
-}
-
-int b200q_prefill_attn(const void* q, int q_stride, void* out, const void* kv_layer,
-                       const int32_t* block_table, int bt_stride, const int32_t* tiles,
-                       int n_tiles, int n_q, int n_kv, int D, int block_size, float scale,
-                       void* stream) {
-  return b200q_prefill_attn_ex(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles,
-                               n_q, n_kv, D, block_size, scale, 0.f, 0, stream);
 }
 
 }  // extern "C"

@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
       int stage = 0;
       uint32_t phase = 0;
       // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
-      int kb = kb0 + (kb1 > kb0 ? tile * 5 % (kb1 - kb0) : 0);
+      // (short reductions keep the order that the kernels for larger steps add in)
+      int kb = kb0 + (kb1 - kb0 >= 16 ? tile * 5 % (kb1 - kb0) : 0);
       for (int i = kb0; i < kb1; ++i, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
         if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, a.failed)) break;
         uint8_t* sw = smem + stage * stage_bytes;
@@ -255,7 +256,7 @@ template <int WT, int kAct>
 static SkinnyPlan skinny_plan(int M, int N, int K) {
   const int kb = K / SK_BK, tiles = N / (128 * WT);
   SkinnyPlan p{((M + 15) & ~15) > 64 && tiles <= 74, 1};
-  for (int s = 2; s <= SK_MAX_SPLITS && kb / s >= 4; ++s)
+  for (int s = 2; s <= SK_MAX_SPLITS && kb / s >= 6; ++s)  // (fewer than 6 k-blocks each: no faster)
     if (tiles <= resident_clusters<WT, kAct>(s) * (p.alone ? 1 : 2)) p.splits = s;
   return p;
 }

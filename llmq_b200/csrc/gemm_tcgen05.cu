@@ -608,6 +608,39 @@ int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUte
   return B200Q_OK;
 }
 
+int get_page_tmap(const void* kv, int D, CUtensorMap* out) {
+  static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
+  static std::mutex mu;
+  const TmapKey key{kv, 0, D, 16};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return B200Q_OK;
+  }
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled entry point unavailable (driver too old / no driver)");
+    return B200Q_ECUDA;
+  }
+  cuuint64_t gdim[4] = {64, 8, (cuuint64_t)(D / 64), 0x0ffffffeull};
+  cuuint64_t gstride[3] = {(cuuint64_t)D * 2, 128, (cuuint64_t)D * 16};
+  cuuint32_t box[4] = {64, 8, (cuuint32_t)(D / 64), 2};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUtensorMap m;
+  CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(kv), gdim, gstride, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d) for a page pool at %p", (int)r, kv);
+    return B200Q_ECUDA;
+  }
+  if (cache.size() > 4096) cache.clear();
+  cache[key] = m;
+  *out = m;
+  return B200Q_OK;
+}
+
 static int num_sms() {
   static int n = 0;
   if (n == 0) {

@@ -1,0 +1,795 @@
+// prefill_attn.cu — softmax attention of prompt portions over the paged cache on the 5th-generation tensor cores (page layout: attn.cu).
+//
+// Bound: tensor pipe and exponentials (a 128 x 128 block of scores costs 1024 cycles of products at D = 128 and 1024 cycles of the
+// exponential unit); the cache is read once per 256 query rows.
+//   * A CTA works a block of consecutive q-tiles (<= 16 tokens each) for one kv head.  Neighbouring tiles of one portion form a run; the
+//     run's rows are (token, head of the group) pairs, 128 of them to a tensor-core tile: all heads of a group share what is fetched.
+//   * Pages arrive by tiled TMA copies, one each, without a swizzle of their own: the cache stores its 16-byte chunks permuted within
+//     eight rows as the tensor core's 128-byte swizzle does, so groups of eight rows cut into 64-column slices are operands as they are
+//     (keys K-major, values N-major).
+//   * Scores and outputs live in tensor memory; probabilities go back there as bf16 and are the A operand of the second product.
+//     D = 64, 128: two query tiles per CTA (four warps of softmax each), one's exponentials behind the other's products; 128 keys at a
+//     time.  D = 256: one query tile (its outputs take 256 columns), 64 keys at a time, scores double buffered, eight warps that halve
+//     the columns of every row.
+//   * The running maximum moves only when a row's grows by more than 2^8 (exponents stay far from overflow; at D = 256 the first 512
+//     keys follow it exactly, so that short contexts round as the plain form does); the outputs in tensor memory are scaled in place.
+//   * Persistent: one CTA per SM walks its blocks, last tiles (the longest ones of a prompt) first; the page ring runs on across them.
+#include "tcgen05.cuh"
+
+namespace b200q {
+
+template <int D>
+struct FaCfg {
+  static constexpr int NQ = D > 128 ? 1 : 2;       // query tiles of 128 rows per CTA
+  static constexpr int KT = D > 128 ? 64 : 128;    // keys per step
+  static constexpr int COLS = D > 128 ? 32 : 128;  // score columns per softmax thread
+  static constexpr int STG = D == 64 ? 3 : 2;      // ring stages of keys and of values
+  static constexpr int MAX_G = D > 128 ? 4 : 8;
+  static constexpr int CH = D / 64;                // 64-column slices of a row
+  static constexpr int Q_BYTES = 128 * D * 2, T_BYTES = KT * D * 2;
+  static constexpr int PATCH = D > 128 ? 32 : 64;    // columns that a warp turns at a time on their way out (in shared memory)
+  static constexpr int SMEM = NQ * Q_BYTES + 2 * STG * T_BYTES + 8 * 32 * PATCH * 2 + 1024;
+  static constexpr int O_COL = NQ == 2 ? 256 : 128;  // tensor memory: scores from column 0, outputs from here
+};
+constexpr int FA_THREADS = 384;  // 8 softmax warps, one that fetches pages, one that issues products, two that fetch queries
+
+struct FaArgs {
+  const bf16* q;
+  bf16* out;
+  const uint8_t* kv;
+  const int32_t* block_table;
+  const int4* tiles;
+  int* failed;
+  int q_stride, bt_stride, n_tiles, per_block, n_q, n_kv, G, window;
+  float c0, c1;  // of a score: plain s * c0 in base 2; capped c1 * tanh(s * c0); c0 > 0
+  uint32_t q_flip;  // the queries' sign bits turned (a negative scale)
+  int vec;          // rows of q and out are 16-byte aligned
+  uint32_t inv_g;   // 65536 / G + 1: f / G = f * inv_g >> 16 for the rows of a CTA
+};
+
+struct FaRun {
+  int bt_row, row0, n, pos0;
+};
+
+// Which units (block of tiles, kv head) a CTA works, and in which order: blocks by the number of their steps, longest first, dealt out
+// back and forth over the CTAs (0 .. n-1, n-1 .. 0, ...), so that every CTA gets long and short ones: three prompts of 333 to 2048
+// tokens, D = 256, 448 units: 89 us, 110 to 150 with blocks dealt out in the order of the list.
+constexpr int FA_SORTED = 512;  // more blocks than this keep the order of the list, last ones first
+struct FaOrder {
+  const uint16_t* sorted;
+  int n_blocks, units;
+  __device__ __forceinline__ int block(int rank) const { return sorted ? sorted[rank] : n_blocks - 1 - rank; }
+};
+struct FaUnit {  // a CTA's place: unit u, at x of its round
+  int u = blockIdx.x, x = blockIdx.x;
+  __device__ __forceinline__ void step() {
+    const int g = gridDim.x;
+    u += 2 * (g - x) - 1;
+    x = g - 1 - x;
+  }
+};
+
+// the runs of a block, seen by a whole warp: lane l holds tile l of the block
+struct FaBlock {
+  int4 t, ahead;
+  uint32_t starts;  // bit l: tile l begins a run
+  int count, ahead_count;
+  // the tiles of unit u are asked for one unit ahead
+  __device__ __forceinline__ void fetch(const FaArgs& a, const FaOrder& o, int u, int lane) {
+    const int first = u < o.units ? o.block(u / a.n_kv) * a.per_block : a.n_tiles;
+    ahead_count = min(a.per_block, a.n_tiles - first);
+    ahead = lane < ahead_count ? __ldg(a.tiles + first + lane) : make_int4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ void begin(const FaArgs& a, const FaOrder& o, FaUnit at, int lane) {
+    count = ahead_count;
+    t = ahead;
+    at.step();
+    fetch(a, o, at.u, lane);
+    t.z = min(max(t.z, 0), 16);
+    const int br = __shfl_up_sync(0xffffffffu, t.x, 1), r0 = __shfl_up_sync(0xffffffffu, t.y, 1), nn = __shfl_up_sync(0xffffffffu, t.z, 1),
+              p0 = __shfl_up_sync(0xffffffffu, t.w, 1);
+    const bool next = lane > 0 && lane < count && br == t.x && r0 + nn == t.y && p0 + nn == t.w;
+    starts = __ballot_sync(0xffffffffu, lane < count && !next);
+  }
+  // run that begins at tile `at`; returns the tile behind it
+  __device__ __forceinline__ int run(int at, FaRun& r) const {
+    const uint32_t later = at < 31 ? starts & (0xfffffffeu << at) : 0u;
+    const int end = later ? __ffs(later) - 1 : count;
+    r.bt_row = __shfl_sync(0xffffffffu, t.x, at);
+    r.row0 = __shfl_sync(0xffffffffu, t.y, at);
+    r.pos0 = __shfl_sync(0xffffffffu, t.w, at);
+    r.n = __shfl_sync(0xffffffffu, t.y, end - 1) + __shfl_sync(0xffffffffu, t.z, end - 1) - r.row0;
+    return end;
+  }
+};
+
+// a wait that gives up after about two seconds, or once another role of the CTA has
+__device__ __forceinline__ void fa_wait(uint64_t* bar, uint32_t parity, volatile int* dead, int* failed) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*dead) return;
+    if (clock64() - t0 > 4000000000ll) {
+      *dead = 1;
+      *(volatile int*)failed = 1;
+      return;
+    }
+  }
+}
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ float fa_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fa_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int D, bool kCap>
+__global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __grid_constant__ CUtensorMap kv_map, const FaArgs a) {
+  using C = FaCfg<D>;
+  constexpr int NQ = C::NQ, KT = C::KT, STG = C::STG, CH = C::CH, COLS = C::COLS, PAGES = KT / 16;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* q_s = smem;
+  uint8_t* k_s = smem + NQ * C::Q_BYTES;
+  uint8_t* v_s = k_s + STG * C::T_BYTES;
+  __shared__ __align__(8) uint64_t k_full[STG], k_empty[STG], v_full[STG], v_empty[STG], q_ready[2], q_empty[2], s_full[2], p_ready[2], o_full[2], pv_done;
+  uint8_t* patches = v_s + STG * C::T_BYTES;
+  __shared__ float part[2][2][NQ == 1 ? 128 : 1];  // D = 256: maxima / sums of a row's two halves, in turns
+  __shared__ uint32_t tmem_slot;
+  __shared__ int dead;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  __shared__ uint16_t sorted[FA_SORTED];
+  int* steps_in = reinterpret_cast<int*>(patches);  // (free until the first rows leave)
+  const int n_blocks = (a.n_tiles + a.per_block - 1) / a.per_block;
+  const bool sort = n_blocks <= FA_SORTED && n_blocks * a.n_kv > (int)gridDim.x;  // (one unit each: nothing to deal out)
+  const FaOrder order{sort ? sorted : nullptr, n_blocks, n_blocks * a.n_kv};
+
+  if (threadIdx.x == 0) {
+    dead = 0;
+    for (int s = 0; s < STG; ++s) {
+      mbar_init(k_full + s, 1);
+      mbar_init(k_empty + s, 1);
+      mbar_init(v_full + s, 1);
+      mbar_init(v_empty + s, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(q_ready + i, 2);
+      mbar_init(q_empty + i, 1);
+      mbar_init(s_full + i, 1);
+      mbar_init(p_ready + i, NQ == 2 ? 4 : 8);
+      mbar_init(o_full + i, 1);
+    }
+    mbar_init(&pv_done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 9) tmem_alloc(&tmem_slot, 512);
+  if (sort) {
+    for (int i = threadIdx.x; i < n_blocks; i += FA_THREADS) steps_in[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {  // the last token of a run sees most keys
+      const int4 t = __ldg(a.tiles + i), n = __ldg(a.tiles + min(i + 1, a.n_tiles - 1));
+      const bool ends = i + 1 == a.n_tiles || (i + 1) % a.per_block == 0 || n.x != t.x || n.y != t.y + t.z || n.w != t.w + t.z;
+      const int keys = a.window > 0 ? min(t.w + t.z, a.window) : t.w + t.z;
+      if (ends) atomicAdd(steps_in + i / a.per_block, max(keys, 0) / KT + 2);  // (its start and end: about one step more)
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_blocks; i += FA_THREADS) {
+      const int mine = steps_in[i];
+      int rank = 0;
+      for (int k = 0; k < n_blocks; ++k) rank += steps_in[k] > mine || (steps_in[k] == mine && k > i);
+      sorted[rank] = (uint16_t)i;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  auto wait = [&](uint64_t* bar, uint32_t parity) { fa_wait(bar, parity, &dead, a.failed); };
+  // steps of KT keys that query tile i of a run walks: from the page of the first token's first visible key to the tile's last token
+  auto first_key = [&](const FaRun& r) { return a.window > 0 && r.pos0 + 1 > a.window ? (r.pos0 + 1 - a.window) / 16 * 16 : 0; };
+  auto steps_of = [&](const FaRun& r, int i, int k0) {
+    const int rows = min(r.n * a.G, (i + 1) * 128);
+    return rows > i * 128 ? (r.pos0 + (int)((uint32_t)(rows - 1) * a.inv_g >> 16) + 1 - k0 + KT - 1) / KT : 0;
+  };
+
+  // (384 threads were launched with 168 registers each: 2 x 208 + 88 = 3 x 168)
+  if (warp >= 8) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+  if (warp == 8) {
+    // ===== pages =====
+    if (lane == 0) tma_prefetch_desc(&kv_map);
+    int n_loaded[2] = {0, 0};
+    FaBlock b;
+    b.fetch(a, order, blockIdx.x, lane);
+    for (FaUnit w; w.u < order.units; w.step()) {
+      b.begin(a, order, w, lane);
+      const int kvh = w.u % a.n_kv;
+      for (int at = 0; at < b.count;) {
+        FaRun r;
+        at = b.run(at, r);
+        if (r.n <= 0) continue;
+        const int k0 = first_key(r), total = r.pos0 + r.n, last = NQ - 1;
+        const int n0 = steps_of(r, 0, k0), n1 = steps_of(r, last, k0), steps = n1 > 0 ? n1 : n0;
+        const int32_t* bt = a.block_table + (long long)r.bt_row * a.bt_stride + k0 / 16;
+        const int n_pages = (total + 15) / 16 - k0 / 16;
+        auto page_of = [&](int j) {
+          const int at_page = j * PAGES + lane;
+          return lane < PAGES && at_page < n_pages && j < steps ? __ldg(bt + at_page) : 0;
+        };
+        // one step's keys or values; keys are asked for a step ahead of values, whose slot is free that much later
+        auto load = [&](int which, int j, int blk) {
+          const int valid = min(KT, total - (k0 + j * KT)), mine = min(16, valid - 16 * lane);
+          const int st = n_loaded[which] % STG;
+          const uint32_t par = (uint32_t)(n_loaded[which] / STG) & 1u;
+          ++n_loaded[which];
+          uint64_t* full = which ? v_full + st : k_full + st;
+          wait(which ? v_empty + st : k_empty + st, par ^ 1u);
+          __syncwarp();
+          uint8_t* dst = (which ? v_s : k_s) + st * C::T_BYTES;
+          if (which && valid < KT) {  // probabilities of keys that are not there are zero: their values must not be NaN
+            for (int i = lane; i < (KT - valid) * CH * 8; i += 32) {
+              const int row = valid + i / (CH * 8), c = i % (CH * 8);
+              *reinterpret_cast<uint4*>(dst + (row >> 3) * (CH * 1024) + (c >> 3) * 1024 + (row & 7) * 128 + (c & 7) * 16) =
+                  make_uint4(0, 0, 0, 0);
+            }
+            fence_async_shared();
+            __syncwarp();
+          }
+          if (lane == 0) mbar_expect_tx(full, (uint32_t)(valid * D * 2));
+          __syncwarp();
+          if (lane < PAGES && mine > 0) {
+            const long long page = ((long long)blk * 2 + which) * a.n_kv + kvh;
+            uint8_t* to = dst + lane * (CH * 2048);
+            if (mine == 16) {
+              tma_load_4d(to, &kv_map, 0, 0, 0, (int)(page * 2), full);
+            } else {  // the rows that exist, one by one
+              const uint8_t* src = a.kv + page * (16 * D * 2);
+              for (int row = 0; row < mine; ++row)
+#pragma unroll
+                for (int c = 0; c < CH; ++c)
+                  tma_bulk_g2s(to + (row >> 3) * (CH * 1024) + c * 1024 + (row & 7) * 128, src + row * (D * 2) + c * 128, 128, full);
+            }
+          }
+          __syncwarp();
+        };
+        int blk = page_of(0), blk1 = page_of(1);
+        load(0, 0, blk);
+        for (int j = 0; j < steps; ++j) {
+          const int blk2 = page_of(j + 2);
+          if (j + 1 < steps) load(0, j + 1, blk1);
+          load(1, j, blk);
+          blk = blk1;
+          blk1 = blk2;
+        }
+      }
+    }
+  } else if (warp == 9) {
+    // ===== products =====
+    constexpr uint32_t base_desc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 4) << 24);
+    constexpr uint32_t qk_desc = base_desc | ((uint32_t)(KT >> 3) << 17);
+    constexpr uint32_t pv_desc = base_desc | (1u << 16) | ((uint32_t)(D >> 3) << 17);  // values: N-major
+    auto issue_qk = [&](int i, int slot, int st) {
+      const uint32_t qa = smem_u32(q_s + i * C::Q_BYTES), kb = smem_u32(k_s + st * C::T_BYTES);
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k)
+        umma_bf16(tmem + (uint32_t)(slot * KT), make_smem_desc(qa + (k >> 2) * 16384 + (k & 3) * 32),
+                  make_smem_desc(kb + (k >> 2) * 1024 + (k & 3) * 32, CH * 1024), qk_desc, k > 0 ? 1u : 0u);
+    };
+    auto issue_pv = [&](int i, int slot, int st, bool add) {
+      const uint32_t vb = smem_u32(v_s + st * C::T_BYTES);
+#pragma unroll
+      for (int k = 0; k < KT / 16; ++k)
+        umma_bf16_ts(tmem + (uint32_t)(C::O_COL + i * D), tmem + (uint32_t)(slot * KT + k * 8),
+                     make_smem_desc(vb + k * (CH * 2048), CH * 1024, 1024), pv_desc, add || k > 0 ? 1u : 0u);
+    };
+    int n_k = 0, n_v = 0, n_p[2] = {0, 0}, n_s = 0;
+    uint32_t q_par[2] = {0, 0};
+    auto next_k = [&]() {
+      wait(k_full + n_k % STG, (uint32_t)(n_k / STG) & 1u);
+      __syncwarp();
+      tc_fence_after();
+    };
+    FaBlock b;
+    b.fetch(a, order, blockIdx.x, lane);
+    for (FaUnit w; w.u < order.units; w.step()) {
+      b.begin(a, order, w, lane);
+      for (int at = 0; at < b.count;) {
+        FaRun r;
+        at = b.run(at, r);
+        if (r.n <= 0) continue;
+        const int k0 = first_key(r);
+        // (from one lane: the compiler then knows that the warp agrees)
+        const int n0 = __shfl_sync(0xffffffffu, steps_of(r, 0, k0), 0);
+        const int n1 = NQ == 2 ? __shfl_sync(0xffffffffu, steps_of(r, 1, k0), 0) : 0, steps = n1 > 0 ? n1 : n0;
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)
+          if (i == 0 || n1 > 0) {
+            wait(q_ready + i, q_par[i]);
+            q_par[i] ^= 1u;
+          }
+        next_k();
+        if constexpr (NQ == 2) {
+          if (elect_one()) {
+            issue_qk(0, 0, n_k % STG);
+            umma_commit(s_full + 0);
+            if (n0 == 1) umma_commit(q_empty + 0);
+            if (n1 > 0) {
+              issue_qk(1, 1, n_k % STG);
+              umma_commit(s_full + 1);
+              if (n1 == 1) umma_commit(q_empty + 1);
+            }
+            umma_commit(k_empty + n_k % STG);
+          }
+          __syncwarp();
+          ++n_k;
+          for (int j = 0; j < steps; ++j) {
+            const bool more = j + 1 < steps;
+            if (more) next_k();
+            wait(v_full + n_v % STG, (uint32_t)(n_v / STG) & 1u);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int n = i ? n1 : n0;
+              if (j < n) {
+                wait(p_ready + i, (uint32_t)n_p[i] & 1u);
+                __syncwarp();
+                ++n_p[i];
+                tc_fence_after();
+                if (elect_one()) {
+                  issue_pv(i, i, n_v % STG, j > 0);
+                  if (j + 1 < n) {  // (products are made in order: the scores are written once the probabilities have been read)
+                    issue_qk(i, i, n_k % STG);
+                    umma_commit(s_full + i);
+                    if (j + 2 == n) umma_commit(q_empty + i);
+                  } else {
+                    umma_commit(o_full + i);
+                  }
+                }
+                __syncwarp();
+              }
+            }
+            if (elect_one()) {
+              umma_commit(v_empty + n_v % STG);
+              if (more) umma_commit(k_empty + n_k % STG);
+            }
+            __syncwarp();
+            ++n_v;
+            if (more) ++n_k;
+          }
+        } else {
+          if (elect_one()) {
+            issue_qk(0, n_s & 1, n_k % STG);
+            umma_commit(s_full + (n_s & 1));
+            if (steps == 1) umma_commit(q_empty + 0);
+            umma_commit(k_empty + n_k % STG);
+          }
+          __syncwarp();
+          ++n_k;
+          for (int j = 0; j < steps; ++j) {
+            const int slot = n_s & 1;
+            if (j + 1 < steps) {
+              next_k();
+              if (elect_one()) {
+                issue_qk(0, slot ^ 1, n_k % STG);
+                umma_commit(s_full + (slot ^ 1));
+                if (j + 2 == steps) umma_commit(q_empty + 0);
+                umma_commit(k_empty + n_k % STG);
+              }
+              __syncwarp();
+              ++n_k;
+            }
+            wait(v_full + n_v % STG, (uint32_t)(n_v / STG) & 1u);
+            wait(p_ready + slot, (uint32_t)(n_s >> 1) & 1u);
+            __syncwarp();
+            ++n_s;
+            tc_fence_after();
+            if (elect_one()) {
+              issue_pv(0, slot, n_v % STG, j > 0);
+              umma_commit(v_empty + n_v % STG);
+              umma_commit(&pv_done);
+              if (j + 1 == steps) umma_commit(o_full + 0);
+            }
+            __syncwarp();
+            ++n_v;
+          }
+        }
+      }
+    }
+  } else if (warp >= 10) {
+    // ===== queries into shared memory, as the tensor core reads them =====
+    constexpr int LPR = D / 8, RPP = 64 / LPR;  // lanes per row, rows per pass of the two warps
+    const int tid = threadIdx.x - 320, c = tid % LPR;
+    uint32_t par[2] = {1, 1};
+    FaBlock b;
+    b.fetch(a, order, blockIdx.x, lane);
+    for (FaUnit w; w.u < order.units; w.step()) {
+      b.begin(a, order, w, lane);
+      const int kvh = w.u % a.n_kv;
+      for (int at = 0; at < b.count;) {
+        FaRun r;
+        at = b.run(at, r);
+        if (r.n <= 0) continue;
+        const int rows = r.n * a.G;
+        const bf16* src0 = a.q + (long long)r.row0 * a.q_stride + (long long)kvh * a.G * D + c * 8;
+        auto source = [&](int f) {
+          const int t = (int)((uint32_t)f * a.inv_g >> 16);
+          return src0 + (long long)t * a.q_stride + (f - t * a.G) * D;
+        };
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          if (i * 128 >= rows) break;
+          wait(q_empty + i, par[i]);
+          __syncwarp();
+          par[i] ^= 1u;
+          uint8_t* dst = q_s + i * C::Q_BYTES + (c >> 3) * 16384;
+          if (a.vec && a.q_flip == 0) {
+#pragma unroll 4
+            for (int x = tid / LPR; x < 128; x += RPP) {
+              const int f = i * 128 + x;
+              const bool on = f < rows;
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + x * 128 + (((c & 7) ^ (x & 7)) << 4))),
+                           "l"(on ? source(f) : src0), "r"(on ? 16 : 0)
+                           : "memory");
+            }
+          } else {
+            for (int x = tid / LPR; x < 128; x += RPP) {
+              const int f = i * 128 + x;
+              uint4 v = make_uint4(0, 0, 0, 0);
+              if (f < rows) {
+                const uint32_t* s4 = reinterpret_cast<const uint32_t*>(source(f));
+                v = make_uint4(s4[0] ^ a.q_flip, s4[1] ^ a.q_flip, s4[2] ^ a.q_flip, s4[3] ^ a.q_flip);
+              }
+              *reinterpret_cast<uint4*>(dst + x * 128 + (((c & 7) ^ (x & 7)) << 4)) = v;
+            }
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          if (i * 128 >= rows) break;
+          if (i + 1 < NQ && (i + 1) * 128 < rows)
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+          else
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+          fence_async_shared();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(q_ready + i);
+        }
+      }
+    }
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    // ===== softmax: a row per thread =====
+    const int wg = warp >> 2, i_tile = NQ == 2 ? wg : 0;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    uint32_t s_count = 0, o_par = 0, turn = 0;
+    const float c0e = 2.8853900817779268f * a.c0;  // 2 log2 e c0
+    auto capped = [&](float v) {  // c1 tanh(c0 v) = c1 - 2 c1 / (1 + e^(2 c0 v))
+      return fmaf(-2.f * a.c1, fa_rcp(fa_ex2(v * c0e) + 1.f), a.c1);
+    };
+    auto exponent = [&](float v, float base) {
+      if constexpr (kCap) {
+        // c1 tanh(z) from the first terms of its series (|z| <= 0.3: the next one is below 6e-8 of the sum), on the FMA pipe beside
+        // the exponential unit
+        const float z = v * a.c0, w = z * z;
+        float t = fmaf(w, 62.f / 2835.f, -17.f / 315.f);
+        t = fmaf(w, t, 2.f / 15.f);
+        t = fmaf(w, t, -1.f / 3.f);
+        t = fmaf(w, t, 1.f);
+        return fmaf(z * a.c1, t, -base);
+      }
+      return fmaf(v, a.c0, -base);
+    };
+    auto both = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    FaBlock b;
+    b.fetch(a, order, blockIdx.x, lane);
+    for (FaUnit w; w.u < order.units; w.step()) {
+      b.begin(a, order, w, lane);
+      const int kvh = w.u % a.n_kv;
+      for (int at = 0; at < b.count;) {
+        FaRun r;
+        at = b.run(at, r);
+        if (r.n <= 0) continue;
+        const int k0 = first_key(r), steps = steps_of(r, i_tile, k0), rows = r.n * a.G;
+        if (steps == 0) continue;
+        const int f = min(i_tile * 128 + row, rows - 1);
+        const int tok = (int)((uint32_t)f * a.inv_g >> 16);
+        const int pos = r.pos0 + tok, lo = a.window > 0 ? pos + 1 - a.window : 0;
+        const int pos_lo = __shfl_sync(0xffffffffu, pos, 0), pos_hi = __shfl_sync(0xffffffffu, pos, 31);  // (rows of later tokens behind)
+        float m = -INFINITY, l = 0.f;
+        for (int j = 0; j < steps; ++j) {
+          const int slot = NQ == 2 ? i_tile : (int)(s_count & 1u);
+          wait(s_full + slot, NQ == 2 ? s_count & 1u : (s_count >> 1) & 1u);
+          __syncwarp();
+          ++s_count;
+          tc_fence_after();
+          const uint32_t s_at = tmem + lanes + (uint32_t)(slot * KT);
+          const int c_first = NQ == 2 ? 0 : wg * COLS;  // this thread's first column
+          const int key0 = k0 + j * KT + c_first;
+          // chunks of 32 columns: those that no row of the warp sees are left out, masks only where some row does not see all
+          auto used = [&](int x) { return key0 + 32 * x <= pos_hi && (a.window <= 0 || key0 + 32 * x + 31 > pos_lo - a.window); };
+          auto masked = [&](int x) { return key0 + 32 * x + 31 > pos_lo || (a.window > 0 && key0 + 32 * x <= pos_hi - a.window); };
+          uint32_t s[COLS / 32][32];
+#pragma unroll
+          for (int x = 0; x < COLS / 32; ++x)
+            if (used(x)) tmem_ld32(s_at + (uint32_t)(c_first + 32 * x), s[x]);
+          tmem_ld_wait();
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, big[2] = {0.f, 0.f};
+#pragma unroll
+          for (int x = 0; x < COLS / 32; ++x)
+            if (used(x)) {
+              if constexpr (kCap) {
+#pragma unroll
+                for (int y = 0; y < 32; ++y) big[y & 1] = fmaxf(big[y & 1], fabsf(__uint_as_float(s[x][y])));
+              }
+              if (masked(x)) {
+                const int hi_c = pos - key0 - 32 * x, lo_c = lo - key0 - 32 * x;
+#pragma unroll
+                for (int y = 0; y < 32; ++y)
+                  if (y > hi_c) s[x][y] = 0xff800000u;
+                if (a.window > 0) {
+#pragma unroll
+                  for (int y = 0; y < 32; ++y)
+                    if (y < lo_c) s[x][y] = 0xff800000u;
+                }
+              }
+#pragma unroll
+              for (int y = 0; y < 32; ++y) mx[y & 3] = fmaxf(mx[y & 3], __uint_as_float(s[x][y]));
+            }
+          const bool small = !kCap || __all_sync(0xffffffffu, fmaxf(big[0], big[1]) * a.c0 <= 0.3f);
+          float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+          if constexpr (NQ == 1) {
+            part[turn][wg][row] = top;
+            both();
+            top = fmaxf(top, part[turn][wg ^ 1][row]);
+            turn ^= 1u;
+          }
+          // (c0 > 0 and tanh grows: the largest product gives the largest score; -inf, no key seen, stays -inf)
+          if constexpr (kCap)
+            top = top == -INFINITY ? top : capped(top);
+          else
+            top *= a.c0;
+          const bool grew = top > m + (NQ == 1 && j < 8 ? 0.f : 8.f);
+          if (__any_sync(0xffffffffu, grew)) {
+            const float m_new = grew ? top : m;
+            const float alpha = grew ? fa_ex2(m - m_new) : 1.f;
+            m = m_new;
+            l *= alpha;
+            if (j > 0) {
+              if constexpr (NQ == 1) wait(&pv_done, (s_count & 1u));  // (the product of the step before, number s_count - 2)
+              __syncwarp();
+              tc_fence_after();
+              constexpr int OC = NQ == 2 ? D : D / 2;
+              const uint32_t o_at = tmem + lanes + (uint32_t)(C::O_COL + (NQ == 2 ? i_tile * D : wg * OC));
+              constexpr int AT_ONCE = NQ == 1 ? 2 : 1;
+#pragma unroll 1
+              for (int c = 0; c < OC; c += 32 * AT_ONCE) {
+                uint32_t o[AT_ONCE][32];
+#pragma unroll
+                for (int h = 0; h < AT_ONCE; ++h) tmem_ld32(o_at + (uint32_t)(c + 32 * h), o[h]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int h = 0; h < AT_ONCE; ++h) {
+#pragma unroll
+                  for (int y = 0; y < 32; ++y) o[h][y] = __float_as_uint(__uint_as_float(o[h][y]) * alpha);
+                  tmem_st32(o_at + (uint32_t)(c + 32 * h), o[h]);
+                }
+              }
+            }
+          }
+          const float base = m == -INFINITY ? 0.f : m;
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int x = 0; x < COLS / 32; ++x) {
+            if (used(x)) {
+              // (a hidden key's product is -inf; plain scores carry that through by themselves)
+              if (!small) {
+#pragma unroll
+                for (int y = 0; y < 32; ++y) {
+                  const float v = __uint_as_float(s[x][y]), p = fa_ex2(v == -INFINITY ? v : capped(v) - base);
+                  sum[y & 3] += p;
+                  s[x][y] = __float_as_uint(p);
+                }
+              } else if (kCap && masked(x)) {
+#pragma unroll
+                for (int y = 0; y < 32; ++y) {
+                  const float v = __uint_as_float(s[x][y]), p = fa_ex2(v == -INFINITY ? v : exponent(v, base));
+                  sum[y & 3] += p;
+                  s[x][y] = __float_as_uint(p);
+                }
+              } else {
+#pragma unroll
+                for (int y = 0; y < 32; ++y) {
+                  const float p = fa_ex2(exponent(__uint_as_float(s[x][y]), base));
+                  sum[y & 3] += p;
+                  s[x][y] = __float_as_uint(p);
+                }
+              }
+#pragma unroll
+              for (int y = 0; y < 16; ++y) s[x][y] = pack_bf16x2(__uint_as_float(s[x][2 * y]), __uint_as_float(s[x][2 * y + 1]));
+            } else {
+#pragma unroll
+              for (int y = 0; y < 16; ++y) s[x][y] = 0u;
+            }
+            tmem_st16(s_at + (uint32_t)(c_first / 2 + 16 * x), s[x]);
+          }
+          l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_ready + slot);
+        }
+        // ---- out = O / l ----
+        if constexpr (NQ == 1) {
+          part[turn][wg][row] = l;
+          both();
+          l += part[turn][wg ^ 1][row];
+          turn ^= 1u;
+        }
+        wait(o_full + i_tile, o_par);
+        __syncwarp();
+        o_par ^= 1u;
+        tc_fence_after();
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        constexpr int OC = NQ == 2 ? D : D / 2;
+        const int c_out = NQ == 2 ? 0 : wg * OC;
+        const uint32_t o_at = tmem + lanes + (uint32_t)(C::O_COL + (NQ == 2 ? i_tile * D : c_out));
+        // the warp's 32 rows x PATCH columns are turned in shared memory: full sectors leave for every row
+        constexpr int PC = C::PATCH / 8;  // 16-byte chunks per row
+        const uint32_t patch = smem_u32(patches + warp * (32 * C::PATCH * 2));
+        const int w0 = (warp & 3) * 32;
+#pragma unroll 1
+        for (int c = 0; c < OC; c += C::PATCH) {
+#pragma unroll
+          for (int h = 0; h < C::PATCH / 32; ++h) {
+            uint32_t o[32];
+            tmem_ld32(o_at + (uint32_t)(c + 32 * h), o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+              uint32_t w[4];
+#pragma unroll
+              for (int z = 0; z < 4; ++z)
+                w[z] = pack_bf16x2(__uint_as_float(o[8 * y + 2 * z]) * inv, __uint_as_float(o[8 * y + 2 * z + 1]) * inv);
+              const int k = 4 * h + y, sw = PC == 8 ? k ^ (lane & 7) : k ^ ((lane >> 1) & 3);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch + lane * (PC * 16) + sw * 16), "r"(w[0]), "r"(w[1]),
+                           "r"(w[2]), "r"(w[3])
+                           : "memory");
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int y = 0; y < PC; ++y) {
+            const int rr = y * (32 / PC) + lane / PC, k = lane % PC, sw = PC == 8 ? k ^ (rr & 7) : k ^ ((rr >> 1) & 3);
+            uint4 v;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                         : "r"(patch + rr * (PC * 16) + sw * 16));
+            const int g = i_tile * 128 + w0 + rr;
+            if (g < rows) {
+              const int t = (int)((uint32_t)g * a.inv_g >> 16);
+              bf16* dst = a.out + (long long)(r.row0 + t) * a.n_q * D + (long long)(kvh * a.G + g - t * a.G) * D + c_out + c + k * 8;
+              if (a.vec) {
+                st_v4(dst, v);
+              } else {
+                uint32_t* d4 = reinterpret_cast<uint32_t*>(dst);
+                d4[0] = v.x; d4[1] = v.y; d4[2] = v.z; d4[3] = v.w;
+              }
+            }
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+      }
+    }
+  }
+  __syncthreads();
+  if (dead) {  // (copies in flight end before the block's memory is given back)
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000ll) {
+    }
+    __syncthreads();
+  }
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+template <int D, bool kCap>
+static int launch_prefill(FaArgs a, cudaStream_t st) {
+  using C = FaCfg<D>;
+  B200Q_CHECK_ARG(a.G <= C::MAX_G, "prefill_attn: GQA group %d too large for D=%d (max %d)", a.G, D, C::MAX_G);
+  // as many q-tiles as fill the query tiles; fewer where the SMs would not all get a unit (27 prompts of 10 to 31 tokens at D = 256,
+  // 4 kv heads: 24.6 us with full blocks, whose CTAs walk several short runs one after the other)
+  a.per_block = C::NQ * 128 / (16 * a.G);
+  while (a.per_block > 1 && (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv < 148) a.per_block = (a.per_block + 1) / 2;
+  CUtensorMap map;
+  int rc = get_page_tmap(a.kv, D, &map);
+  if (rc) return rc;
+  if (!wait_flag(&a.failed)) {
+    set_error("prefill_attn: no host-visible flag for bounded waits");
+    return B200Q_ECUDA;
+  }
+  auto kern = prefill_attn_kernel<D, kCap>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    attr_set = true;
+  }
+  const long long units = (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv;
+  const int grid = units < 148 ? (int)units : 148;
+  kern<<<grid, FA_THREADS, C::SMEM, st>>>(map, a);
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+// The kernel above needs about 7 us for a run whatever its size (a chain of copies, products and waits), the kernel of 16-token tiles
+// (attn.cu) about 1 us per 16 keys.  What the host knows of the contexts is the width of the block table.  us, here / there:
+//   D = 128, 32 / 8 heads   18 x 256 tokens 40 / 71, 30 x 64-256 49 / 65, 8 x 100-380 26 / 40, 40 tokens behind 1500 33 / 47, one of 4400
+//                           198 / 778; but one of 200 10.9 / 8.4, 5 behind 300 12.2 / 11.5, 27 x 10-31 behind 42 21 / 11
+//   D = 64, 32 / 8 heads    one of 4400 186 / 533; but 30 x 64-256 42 / 38, one of 300 12.6 / 10.2, one of 512 18.9 / 18.1
+//   D = 256, 8 / 4 heads    one of 200 14.3 / 19.3, one of 300 17 / 27, 300 behind 900 33 / 99; but 27 x 10-31 behind 42 19.5 / 11.5
+static bool tensor_memory_pays(int n_kv, int D, long long keys, int n_tiles) {
+  if (D == 64) return keys > 512;
+  if (D == 128) return keys > 512 || (keys > 128 && (long long)n_tiles * n_kv >= 512);
+  return keys > 128;
+}
+
+}  // namespace b200q
+
+using namespace b200q;
+
+extern "C" {
+
+int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                          const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, float softcap,
+                          int window, void* stream) {
+  B200Q_CHECK_ARG(n_tiles >= 0 && n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 8,
+                  "prefill_attn: unsupported heads n_q=%d n_kv=%d (GQA group must be <= 8)", n_q, n_kv);
+  B200Q_CHECK_ARG(block_size == 16 && (D == 64 || D == 128 || D == 256),
+                  "prefill_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D, block_size);
+  if (n_tiles == 0 || n_q == 0) return B200Q_OK;
+  cudaStream_t st = as_stream(stream);
+  if (!tensor_memory_pays(n_kv, D, 16LL * bt_stride, n_tiles))
+    return prefill_tiles(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, scale, softcap, window, st);
+  const float log2e = 1.4426950408889634f;
+  FaArgs a{};
+  a.q = (const bf16*)q;
+  a.out = (bf16*)out;
+  a.kv = (const uint8_t*)kv_layer;
+  a.block_table = block_table;
+  a.tiles = (const int4*)tiles;
+  a.q_stride = q_stride;
+  a.bt_stride = bt_stride;
+  a.n_tiles = n_tiles;
+  a.n_q = n_q;
+  a.n_kv = n_kv;
+  a.G = n_q / n_kv;
+  a.window = window;
+  a.q_flip = scale < 0.f ? 0x80008000u : 0u;
+  const float s = scale < 0.f ? -scale : scale;
+  a.c0 = softcap > 0.f ? s / softcap : s * log2e;
+  a.inv_g = 65536u / (uint32_t)a.G + 1u;
+  if (!(a.c0 > 1e-37f)) a.c0 = a.c0 >= 0.f ? 1e-37f : a.c0;  // (0: all scores equal; times a hidden key's -inf it would be NaN)
+  a.c1 = softcap * log2e;
+  a.vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 && q_stride % 8 == 0;
+  const bool cap = softcap > 0.f;
+  if (D == 64) return cap ? launch_prefill<64, true>(a, st) : launch_prefill<64, false>(a, st);
+  if (D == 128) return cap ? launch_prefill<128, true>(a, st) : launch_prefill<128, false>(a, st);
+  return cap ? launch_prefill<256, true>(a, st) : launch_prefill<256, false>(a, st);
+}
+
+int b200q_prefill_attn(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                       const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, void* stream) {
+  return b200q_prefill_attn_ex(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, block_size, scale, 0.f,
+                               0, stream);
+}
+
+}  // extern "C"

@@ -68,6 +68,54 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr));
 }
 
+// One lane of a converged warp, the same one every time.  Products are issued behind this and not behind `lane == 0`: ptxas keeps the
+// operands of what follows in uniform registers, while behind a lane test every product moves its descriptors there one by one: 50
+// against 150 cycles per product on an SM whose other warps are busy (46 where they idle), more than a 128 x 128 x 16 product takes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(on));
+  return on != 0;
+}
+
+// 32 (16) columns of this warp's lanes, one value per lane and column
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"r"(v[0]),
+      "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+      "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]),
+      "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]),
+      "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(v[0]),
+      "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+      "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[tmem] (+)= A[tmem] * B[smem desc]
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // wait with a limit: false when it ran out, and then *failed is set (the engine reports it)
 __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, int* failed) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -101,11 +149,11 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
 // UMMA shared-memory descriptor, K-major operand, SWIZZLE_128B, 8-row groups 1024 B apart
 // (cute/arch/mma_sm100_desc.hpp SmemDescriptor: start[0,14) lbo[16,30) sbo[32,46) version[46,48)
 //  layout_type[61,64)).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t sbo = 1024, uint32_t lbo = 16) {
   uint64_t d = 0;
   d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);        // start address, 16 B units
-  d |= (uint64_t)1 << 16;                              // LBO (ignored for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                    // SBO: 8 rows * 128 B
+  d |= (uint64_t)(lbo >> 4) << 16;                     // LBO (N-major: from one 64-column slice to the next; else ignored)
+  d |= (uint64_t)(sbo >> 4) << 32;                     // SBO: from eight rows to the next eight, 1024 B where they are dense
   d |= (uint64_t)1 << 46;                              // descriptor version (sm_100)
   d |= (uint64_t)2 << 61;                              // SWIZZLE_128B
   return d;
@@ -141,6 +189,14 @@ __device__ __forceinline__ float clamped_unit(uint32_t gb, uint32_t ub, float b0
 // bf16 row-major [rows, cols] -> tiled map with box {64 cols, box_rows rows}, 128B swizzle (ld: elements between rows, 0 = dense);
 // maps are cached by address and shape (gemm_tcgen05.cu)
 int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out, long long ld = 0);
+
+// pages of 16 cached rows of D bf16 values, from `kv` on (as many as there are; the caller knows).  One box is a page, laid down as
+// [two groups of 8 rows][64-column slices][8 rows][128 bytes]; coordinates {0, 0, 0, page * 2}.
+int get_page_tmap(const void* kv, int D, CUtensorMap* out);
+
+// prompt portions over short contexts (attn.cu)
+int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
+                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, cudaStream_t st);
 
 // products of up to 128 rows (gemm_skinny.cu)
 bool gemm_skinny_ok(int M, int N, int K, bool gated);

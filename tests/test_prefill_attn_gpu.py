@@ -1,0 +1,113 @@
+"""Attention of prompt portions (csrc/prefill_attn.cu) against a plain fp64 form: portions at the edges of pages, of key steps and of
+query tiles, behind cached tokens, several of them to a block of tiles, every group size, windows, soft caps, unaligned rows, a negative
+and a zero scale; unused cache rows hold NaN."""
+import math
+
+import pytest
+import torch
+
+from oracle import ops as O
+from tests.util import bf16_close
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+BS = 16
+
+
+def make_cache(ctxs, n_kv, D, seed, wide):
+    g = torch.Generator().manual_seed(seed)
+    blocks = sum((c + BS - 1) // BS for c in ctxs) + 3
+    perm = torch.randperm(blocks, generator=g).tolist()
+    kv = torch.zeros(blocks, 2, n_kv, BS, D, dtype=BF)
+    kv.view(torch.int16)[:] = 0x7FC0
+    # (a table of 40 columns and more could hold contexts that the tensor-memory kernel takes at every head size)
+    bt = torch.zeros(len(ctxs), max((max(ctxs) + BS - 1) // BS + 1, 40 if wide else 0), dtype=torch.int32)
+    sw = O.kv_swizzle_index(BS, D)
+    rows = []
+    for i, c in enumerate(ctxs):
+        k, v = torch.randn(c, n_kv, D, generator=g).to(BF), torch.randn(c, n_kv, D, generator=g).to(BF)
+        rows.append((k, v))
+        for b in range((c + BS - 1) // BS):
+            blk = perm.pop()
+            bt[i, b] = blk
+            n = min(BS, c - b * BS)
+            for which, src in ((0, k), (1, v)):
+                page = src[b * BS: b * BS + n].transpose(0, 1)                      # [n_kv, n, D]
+                kv[blk, which, :, :n] = torch.zeros_like(page).scatter(2, sw[:n].expand(n_kv, n, D), page)
+    return kv, bt, rows
+
+
+def reference(q, k, v, pos, scale, cap, window):
+    G = q.shape[1] // k.shape[1]
+    kk, vv = k.double().repeat_interleave(G, 1), v.double().repeat_interleave(G, 1)
+    s = torch.einsum("qhd,khd->hqk", q.double(), kk) * scale
+    s = cap * torch.tanh(s / cap) if cap else s
+    j = torch.arange(k.shape[0])[None]
+    hide = j > pos[:, None]
+    hide = hide | (j <= pos[:, None] - window) if window else hide
+    return torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hide[None], -math.inf), -1), vv)
+
+
+def check(cuda, D, n_q, n_kv, portions, scale=None, cap=0.0, window=0, pad=0, order=None, seed=1, wide=True):
+    """portions: (cached tokens, tokens of this step) per sequence"""
+    from llmq_b200 import lib
+    scale = D ** -0.5 if scale is None else scale
+    kv, bt, rows = make_cache([a + n for a, n in portions], n_kv, D, seed, wide)
+    T = sum(n for _, n in portions)
+    g = torch.Generator().manual_seed(seed + 50)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * D + pad, generator=g).to(BF)
+    tiles, row = [], 0
+    for i, (a, n) in enumerate(portions):
+        tiles += [[i, row + j, min(16, n - j), a + j] for j in range(0, n, 16)]
+        row += n
+    if order is not None:
+        tiles = order(tiles)
+    t = torch.tensor(tiles, dtype=torch.int32, device=cuda)
+    out = torch.full((T + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
+    lib.prefill_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), t, n_q, n_kv, D, BS, scale, softcap=cap, window=window)
+    got = out.cpu()
+    assert torch.isnan(got[T].float()).all(), "rows behind the last one stay as they were"
+    assert lib.load().b200q_wait_failures() == 0
+    row = 0
+    for i, (a, n) in enumerate(portions):
+        q = qkv[row: row + n, : n_q * D].view(n, n_q, D)
+        ref = reference(q, *rows[i], torch.arange(a, a + n), scale, cap, window).to(BF)
+        # probabilities are rounded to bf16 before the value product: 2^-9 each, outputs agree to ~5e-3 or 2 ulps
+        bf16_close(got[row: row + n].view(n, n_q, D), ref, ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"portion {i} ({a} + {n})")
+        row += n
+
+
+MIX = [(0, 128), (0, 5), (16, 16), (100, 37), (3, 49), (0, 1), (0, 64), (250, 70), (0, 257), (127, 2), (0, 300)]
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 32, 8), (128, 32, 8), (256, 16, 8), (64, 2, 2), (128, 6, 2), (128, 10, 2), (64, 6, 1), (128, 7, 1),
+                                        (128, 8, 1), (256, 3, 3), (256, 3, 1), (256, 8, 2)])
+def test_head_layouts(cuda, D, n_q, n_kv):
+    check(cuda, D, n_q, n_kv, MIX)
+    check(cuda, D, n_q, n_kv, MIX, wide=False, window=30)
+    check(cuda, D, n_q, n_kv, MIX[:2] + [(60, 40)] * 40)          # many short runs to a block
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 4, 1), (128, 8, 2), (256, 4, 2)])
+@pytest.mark.parametrize("cap,window", [(0.0, 40), (20.0, 0), (20.0, 1), (5.0, 130), (50.0, 64)])
+def test_caps_and_windows(cuda, D, n_q, n_kv, cap, window):
+    check(cuda, D, n_q, n_kv, MIX + [(900, 150), (0, 700)], cap=cap, window=window, seed=3)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("kind", ["unaligned", "negative", "zero", "large", "shuffled", "reversed"])
+def test_forms(cuda, D, kind):
+    g = torch.Generator().manual_seed(9)
+    kw = {"unaligned": dict(pad=2), "negative": dict(scale=-0.3), "zero": dict(scale=0.0), "large": dict(scale=4.0),
+          "shuffled": dict(order=lambda t: [t[i] for i in torch.randperm(len(t), generator=g).tolist()]),
+          "reversed": dict(order=lambda t: t[::-1])}[kind]
+    check(cuda, D, 4, 1, MIX, **kw)
+    if kind in ("negative", "zero"):
+        check(cuda, D, 4, 1, MIX, cap=10.0, window=50, **kw)
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 127, 129, 255, 256, 511, 1500])
+def test_lengths(cuda, n):
+    for D in (64, 128, 256):
+        check(cuda, D, 8, 2, [(0, n)], seed=n)
+        check(cuda, D, 4, 2, [(n, 33)], seed=n + 1)
