@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], done;
   __shared__ uint32_t tmem_slot;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int split = blockIdx.x, splits = gridDim.x, tile = blockIdx.y;
   const int kb_all = a.K / SK_BK, kb0 = split * kb_all / splits, kb1 = (split + 1) * kb_all / splits;
   const int stage_bytes = WT * SK_TILE_BYTES + a.mp * (SK_BK * 2);
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -81,13 +81,13 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.mp >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int i = kb0; i < kb1; ++i) {
-        if (!mbar_wait_or_fail(full + stage, phase, a.failed)) break;
-        tc_fence_after();
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.mp >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = kb0; i < kb1; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait_or_fail(full + stage, phase, a.failed))) break;
+      tc_fence_after();
+      if (elect_one()) {
         const uint32_t sw = smem_u32(smem + stage * stage_bytes), sa = sw + WT * SK_TILE_BYTES;
 #pragma unroll
         for (int h = 0; h < WT; ++h)
@@ -96,13 +96,15 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
             umma_bf16(tmem + (uint32_t)(h * a.mp), make_smem_desc(sw + h * SK_TILE_BYTES + k * 32), make_smem_desc(sa + k * 32), idesc,
                       (i > kb0 || k > 0) ? 1u : 0u);
         umma_commit(empty + stage);
-        if (++stage == a.stages) {
-          stage = 0;
-          phase ^= 1u;
-        }
       }
-      umma_commit(&done);
+      __syncwarp();
+      if (++stage == a.stages) {
+        stage = 0;
+        phase ^= 1u;
+      }
     }
+    __syncwarp();
+    if (elect_one()) umma_commit(&done);
     __syncwarp();
   }
 

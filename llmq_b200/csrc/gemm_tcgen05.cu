@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;  // 4 warps x 4 KB transpose patches
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
   const int n_tiles = N / BN;
   const int num_tiles = m_tiles * n_tiles * splits;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ===== TMA producer =====
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       for (int kb = 0; kb < k_blocks; ++kb) {
         mbar_wait(full + stage, phase);
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
 #pragma unroll
@@ -407,7 +407,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;  // 4 warps x 4 KB transpose patches
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int m_tiles = (M + 255) / 256;
@@ -435,7 +435,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   __syncthreads();
   cluster_sync_all();  // peer barriers are initialised before anybody signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs): own A rows + own half of B, completion on the LEADER =====
@@ -474,7 +474,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         for (int kb = 0; kb < k_blocks; ++kb) {
           mbar_wait(full + stage, phase);
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
             const uint32_t sb = sa + Cfg::A_BYTES;
 #pragma unroll
@@ -897,7 +897,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int mt_per_group = (ga.M + GEMM_BM - 1) / GEMM_BM;
   const int m_tiles = ga.tab ? *ga.n_mt : mt_per_group * ga.groups;
   const int n_tiles = N / BN;
@@ -936,7 +936,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       for (int kb = 0; kb < k_blocks; ++kb) {
         mbar_wait(full + stage, phase);
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
 #pragma unroll
