@@ -22,7 +22,9 @@
 // their code: kCap = attention-logit soft-capping (score <- cap * tanh(score * scale / cap)), and a
 // runtime sliding window (query at position p sees keys p - window < j <= p; pages that lie entirely
 // before the window are never fetched).  D = 256 (Gemma-2 head size) uses 2-stage rings.
-#include "common.cuh"
+#include <stdlib.h>
+
+#include "tcgen05.cuh"
 
 namespace b200q {
 
@@ -184,8 +186,11 @@ struct DecSmem {
   static constexpr int TOTAL = RING_BYTES + MERGE_FLOATS * 4 + DEC_WARPS * STAGES * 8;
 };
 
-template <int D, int BS, bool kCap>
-__global__ void __launch_bounds__(DEC_WARPS * 32, 2)
+// A cluster of gridDim.x CTAs shares a sequence's pages where there are few sequences: warp w of CTA r takes pages r * DEC_WARPS + w,
+// + warps of the cluster, ...; the CTAs read each other's partial states through distributed shared memory and each adds up and stores
+// its share of the outputs.
+template <int D, int BS, bool kCap, bool kShared>
+__global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
     decode_attn_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out,
                        const uint8_t* __restrict__ kv_layer,
                        const int32_t* __restrict__ block_table, int bt_stride,
@@ -195,8 +200,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
   using S_ = DecSmem<D, BS>;
   constexpr int DEC_STAGES = S_::STAGES;
   extern __shared__ __align__(128) uint8_t smem[];
-  const int seq = blockIdx.x, kvh = blockIdx.y;
+  const int seq = blockIdx.y, kvh = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = kShared ? gridDim.x : 1, split = kShared ? blockIdx.x : 0;
+  const int wg = split * DEC_WARPS + warp, n_warps = splits * DEC_WARPS;  // this warp's place among the sequence's warps
   uint8_t* ring = smem + warp * DEC_STAGES * S_::STAGE_BYTES;
   float* merge = reinterpret_cast<float*>(smem + S_::RING_BYTES);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S_::RING_BYTES + S_::MERGE_FLOATS * 4) +
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
   const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
   const int page0 = lo / BS;
   const int n_pages = (ctx + BS - 1) / BS - page0;
-  const int my_n = n_pages > warp ? (n_pages - warp + DEC_WARPS - 1) / DEC_WARPS : 0;
+  const int my_n = n_pages > wg ? (n_pages - wg + n_warps - 1) / n_warps : 0;
 
   if (lane == 0) {
 #pragma unroll
@@ -220,15 +227,15 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
   const long long page_stride = (long long)G_::PAGE_BYTES;  // bytes per (block,kv,head) page
   // page address: ((blk*2 + kv) * n_kv + kvh) * PAGE_BYTES
   int ids_base = 0;
-  int ids = (lane < my_n) ? __ldg(bt + warp + DEC_WARPS * lane) : 0;
+  int ids = (lane < my_n) ? __ldg(bt + wg + n_warps * lane) : 0;
 
   auto issue = [&](int k) {  // whole warp calls; k = warp-local page index
     if (k - ids_base >= 32) {
       ids_base += 32;
-      ids = (ids_base + lane < my_n) ? __ldg(bt + warp + DEC_WARPS * (ids_base + lane)) : 0;
+      ids = (ids_base + lane < my_n) ? __ldg(bt + wg + n_warps * (ids_base + lane)) : 0;
     }
     const int blk = __shfl_sync(0xffffffffu, ids, k - ids_base);
-    const int p = page0 + warp + DEC_WARPS * k;
+    const int p = page0 + wg + n_warps * k;
     const int n_valid = min(BS, ctx - p * BS);
     const int st = k % DEC_STAGES;
     uint8_t* ks = ring + st * S_::STAGE_BYTES;
@@ -277,7 +284,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
     const int st = k % DEC_STAGES;
     const uint32_t phase = (uint32_t)(k / DEC_STAGES) & 1u;
     mbar_wait(bars + st, phase);
-    const int p = page0 + warp + DEC_WARPS * k;
+    const int p = page0 + wg + n_warps * k;
     const int n_valid = min(BS, ctx - p * BS);
     const int t_lo = lo - p * BS;  // first visible token of this page (<= 0 except on the window's first page)
     const uint32_t k_s = smem_u32(ring + st * S_::STAGE_BYTES);
@@ -361,23 +368,51 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
       mo[D + 1] = l;
     }
   }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < G * D; idx += DEC_WARPS * 32) {
+  if constexpr (!kShared) {
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < G * D; idx += DEC_WARPS * 32) {
+      const int r = idx / D, d = idx % D;
+      float M = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, merge[(w * 8 + r) * (D + 2) + D]);
+      float num = 0.f, den = 0.f;
+#pragma unroll
+      for (int w = 0; w < DEC_WARPS; ++w) {
+        const float* mo = merge + (w * 8 + r) * (D + 2);
+        const float wgt = (mo[D] == -INFINITY) ? 0.f : exp2f(mo[D] - M);
+        num += wgt * mo[d];
+        den += wgt * mo[D + 1];
+      }
+      const float v = den > 0.f ? num / den : 0.f;
+      out[(long long)seq * n_q * D + (long long)(kvh * G + r) * D + d] = __float2bfloat16_rn(v);
+    }
+    return;
+  }
+  cluster_sync_all();
+  for (int idx = split * DEC_WARPS * 32 + threadIdx.x; idx < G * D; idx += splits * DEC_WARPS * 32) {
     const int r = idx / D, d = idx % D;
-    float M = -INFINITY;
+    float M = -INFINITY, num = 0.f, den = 0.f;
+    // (warps of the cluster in order; two passes, so that the largest maximum is known before anything is added)
+    for (int s = 0; s < splits; ++s) {
+      const uint32_t base = mapa_shared(merge, s);
 #pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, merge[(w * 8 + r) * (D + 2) + D]);
-    float num = 0.f, den = 0.f;
+      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, ld_cluster_f32(base + ((w * 8 + r) * (D + 2) + D) * 4));
+    }
+    for (int s = 0; s < splits; ++s) {
+      const uint32_t base = mapa_shared(merge, s);
 #pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) {
-      const float* mo = merge + (w * 8 + r) * (D + 2);
-      const float wgt = (mo[D] == -INFINITY) ? 0.f : exp2f(mo[D] - M);
-      num += wgt * mo[d];
-      den += wgt * mo[D + 1];
+      for (int w = 0; w < DEC_WARPS; ++w) {
+        const uint32_t mo = base + (w * 8 + r) * (D + 2) * 4;
+        const float m_w = ld_cluster_f32(mo + D * 4), v_w = ld_cluster_f32(mo + d * 4), l_w = ld_cluster_f32(mo + (D + 1) * 4);
+        const float wgt = m_w == -INFINITY ? 0.f : exp2f(m_w - M);
+        num += wgt * v_w;
+        den += wgt * l_w;
+      }
     }
     const float v = den > 0.f ? num / den : 0.f;
     out[(long long)seq * n_q * D + (long long)(kvh * G + r) * D + d] = __float2bfloat16_rn(v);
   }
+  cluster_sync_all();  // nobody leaves while a peer still reads
 }
 
 // ------------------------------------------------------------------------------------------
@@ -782,27 +817,51 @@ static inline ScoreConsts score_consts(float scale, float softcap) {
   return {scale * log2e, 0.f};
 }
 
-template <int D, int BS, bool kCap>
-static int launch_decode(const void* q, int q_stride, void* out, const void* kv,
+int g_decode_variant = 0;  // test hook: 0 = auto, 1 = split kernel (v1), 2 = streaming kernel
+
+// How many CTAs share a sequence (and kv head): as many as keep two CTAs on every SM busy, but no fewer than four pages per warp of the
+// longest context that the block table could hold (shorter ones gain nothing: an exchange costs about 2 us).  6 sequences of 3000 to
+// 8100 tokens, D = 64, 8 kv heads: 22 us, 65 with one CTA each.  B200Q_BATCH_INVARIANT=1: always one, whatever the batch.
+static int decode_splits(int n_seqs, int n_kv, int bt_stride) {
+  static const bool invariant = [] {
+    const char* e = getenv("B200Q_BATCH_INVARIANT");
+    return e && e[0] == '1';
+  }();
+  if (invariant || g_decode_variant == 1) return 1;
+  const long long ctas = (long long)n_seqs * n_kv;
+  int splits = 1;
+  while (splits < 8 && ctas * (splits + 1) <= 296 && bt_stride / (DEC_WARPS * (splits + 1)) >= 4) ++splits;
+  return splits;
+}
+
+template <int D, int BS, bool kCap, bool kShared>
+static int launch_decode_form(int splits, const void* q, int q_stride, void* out, const void* kv,
                          const int32_t* bt, int bt_stride, const int32_t* ctx, int n_seqs, int n_q,
                          int n_kv, float scale, float softcap, int window, cudaStream_t st) {
   using S_ = DecSmem<D, BS>;
-  auto kern = decode_attn_kernel<D, BS, kCap>;
+  auto kern = decode_attn_kernel<D, BS, kCap, kShared>;
   static bool attr_set = false;
   if (!attr_set) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
     attr_set = true;
   }
   const ScoreConsts sc = score_consts(scale, softcap);
-  dim3 grid(n_seqs, n_kv);
-  kern<<<grid, DEC_WARPS * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out,
-                                                (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
-                                                n_q / n_kv, sc.c0, sc.c1, window);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits, n_seqs, n_kv);
+  cfg.blockDim = dim3(DEC_WARPS * 32);
+  cfg.dynamicSmemBytes = S_::TOTAL;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  B200Q_CUDA(cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
+                                n_q / n_kv, sc.c0, sc.c1, window));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
-
-int g_decode_variant = 0;  // test hook: 0 = auto, 1 = split kernel (v1), 2 = streaming kernel
 
 static int attn_num_sms() {
   static int n = 0;
@@ -813,6 +872,17 @@ static int attn_num_sms() {
     if (n <= 0) n = 148;
   }
   return n;
+}
+
+template <int D, int BS, bool kCap>
+static int launch_decode(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* ctx,
+                         int n_seqs, int n_q, int n_kv, float scale, float softcap, int window, cudaStream_t st) {
+  const int splits = decode_splits(n_seqs, n_kv, bt_stride);
+  if (splits > 1)
+    return launch_decode_form<D, BS, kCap, true>(splits, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap,
+                                                 window, st);
+  return launch_decode_form<D, BS, kCap, false>(1, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap, window,
+                                                st);
 }
 
 template <int D, int BS, bool kCap>
