@@ -5,7 +5,7 @@
 // vLLM's native op definitions / HF transformers' Llama.
 #include <stdarg.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace b200q {
 
@@ -492,39 +492,59 @@ __device__ __forceinline__ float gumbel_from_bits(uint32_t x) {
   return -logf(-logf(u));
 }
 
-__global__ void __launch_bounds__(1024)
+// A cluster of gridDim.x CTAs shares a row (a row per CTA left most SMs idle or one deep: 60 us for 128 rows of 128256 logits, 33 so).
+// Bound: integer work of the random numbers, 20 instructions per logit.  The two logarithms of a logit's noise are taken only where
+// the logit could still win: its value t + noise exceeds the best so far only if -log u < e^(t - best), and -log u >= 1 - u, which the
+// bits give directly.  The margin covers the roundings of t, best and the exponential (|best| * 1e-6 + 1.5e-3 in base 2, some ten times
+// what they are), so what is left out is smaller than the best, and the result is the one that all logarithms give.
+constexpr int SAMPLE_THREADS = 512;
+__global__ void __launch_bounds__(SAMPLE_THREADS, 3)
     sample_kernel(const bf16* __restrict__ logits, const int32_t* __restrict__ params,
                   int32_t* __restrict__ ids, int V) {
-  const bf16* row = logits + (long long)blockIdx.x * V;
-  const float temp = __int_as_float(params[4 * blockIdx.x + 0]);
-  const uint32_t k0 = (uint32_t)params[4 * blockIdx.x + 1], k1 = (uint32_t)params[4 * blockIdx.x + 2];
-  const uint32_t pos = (uint32_t)params[4 * blockIdx.x + 3];
+  const int split = blockIdx.x, splits = gridDim.x, r_ = blockIdx.y;
+  const bf16* row = logits + (long long)r_ * V;
+  const float temp = __int_as_float(params[4 * r_ + 0]);
+  const uint32_t k0 = (uint32_t)params[4 * r_ + 1], k1 = (uint32_t)params[4 * r_ + 2];
+  const uint32_t pos = (uint32_t)params[4 * r_ + 3];
   const bool greedy = !(temp > 0.f);
   const float inv_t = greedy ? 1.f : 1.f / temp;
+  const float log2e = 1.4426950408889634f;
   float best = -INFINITY;
   int bi = 0x7fffffff;
+  float bound = -INFINITY;  // (best of the warp) * log2 e - margin
   // groups of 4 consecutive elements share one Philox block: counter = (group, position, 0, 0)
-  const int n4 = V / 4;
-  for (int g = threadIdx.x; g < n4; g += blockDim.x) {
-    const uint2 a = *reinterpret_cast<const uint2*>(row + 4 * g);  // 4 bf16 (V*2 B rows are 8 B aligned)
-    float v[4] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y)};
-    if (!greedy) {
-      uint32_t r[4];
-      philox4x32_10((uint32_t)g, pos, 0u, 0u, k0, k1, r);
+  const int n4 = V / 4, step = splits * SAMPLE_THREADS;
+  for (int g0 = split * SAMPLE_THREADS; g0 < n4; g0 += step) {  // (whole warps go round together)
+    const int g = g0 + threadIdx.x;
+    if (g < n4) {
+      const uint2 a = *reinterpret_cast<const uint2*>(row + 4 * g);  // 4 bf16 (V*2 B rows are 8 B aligned)
+      float v[4] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y)};
+      if (greedy) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = v[k] * inv_t + gumbel_from_bits(r[k]);
-    }
+        for (int k = 0; k < 4; ++k) amax_update(v[k], 4 * g + k, best, bi);
+      } else {
+        uint32_t r[4];
+        philox4x32_10((uint32_t)g, pos, 0u, 0u, k0, k1, r);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) amax_update(v[k], 4 * g + k, best, bi);
-  }
-  for (int i = n4 * 4 + threadIdx.x; i < V; i += blockDim.x) {  // tail (V % 4 elements)
-    float v = __bfloat162float(row[i]);
-    if (!greedy) {
-      uint32_t r[4];
-      philox4x32_10((uint32_t)(i / 4), pos, 0u, 0u, k0, k1, r);
-      v = v * inv_t + gumbel_from_bits(r[i & 3]);
+        for (int k = 0; k < 4; ++k) {
+          const float t = v[k] * inv_t;
+          float least;  // e^(t - best), a little more
+          asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(least) : "f"(fmaf(t, log2e, -bound)));
+          // 1 - u >= 2 - f - 2^-23 with f = 1 + the upper 23 bits
+          const float one_less_u = (2.f - __uint_as_float(0x3f800000u | (r[k] >> 9))) - 1.1920929e-7f;
+          if (!(one_less_u > least)) amax_update(v[k] * inv_t + gumbel_from_bits(r[k]), 4 * g + k, best, bi);
+        }
+      }
     }
-    amax_update(v, i, best, bi);
+    if (!greedy) {
+      // the warp's best, through integers of the same order
+      int o = __float_as_int(best);
+      o ^= (o >> 31) & 0x7fffffff;
+      o = __reduce_max_sync(0xffffffffu, o);
+      o ^= (o >> 31) & 0x7fffffff;
+      const float top = __int_as_float(o);
+      bound = fmaf(top, log2e, -(1.5e-3f + fabsf(top) * 1e-6f));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -548,14 +568,19 @@ __global__ void __launch_bounds__(1024)
       int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       amax_update(ov, oi, best, bi);
     }
-    if (threadIdx.x == 0) ids[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
+    if (threadIdx.x == 0) {
+      sv[0] = best;
+      si[0] = bi;
+    }
   }
-}
-
-static inline int grid_for(long long items, int threads) {
-  long long b = (items + threads - 1) / threads;
-  const long long cap = 148LL * 16;  // 16 resident 256-thread CTAs per SM
-  return (int)(b < 1 ? 1 : (b > cap ? cap : b));
+  if (splits > 1) {
+    cluster_sync_all();
+    if (split == 0 && threadIdx.x == 0)
+      for (int s = 1; s < splits; ++s)
+        amax_update(ld_cluster_f32(mapa_shared(sv, s)), __float_as_int(ld_cluster_f32(mapa_shared(si, s))), best, bi);
+    cluster_sync_all();
+  }
+  if (split == 0 && threadIdx.x == 0) ids[r_] = bi == 0x7fffffff ? 0 : bi;
 }
 
 }  // namespace b200q
@@ -740,8 +765,22 @@ int b200q_sample_bf16(const void* logits, const int32_t* params, int32_t* ids, i
   B200Q_CHECK_ARG(B >= 0 && V > 0 && V % 4 == 0, "sample: bad shape B=%d V=%d (V %% 4 == 0)", B, V);
   B200Q_CHECK_ARG(params != nullptr, "sample: params is null");
   if (B == 0) return B200Q_OK;
-  sample_kernel<<<B, 1024, 0, as_stream(stream)>>>((const bf16*)logits, params, ids, V);
-  B200Q_LAUNCH_CHECK();
+  // (a grid's second dimension ends at 65535 rows)
+  for (int at = 0; at < B; at += 65535) {
+    const int rows = B - at < 65535 ? B - at : 65535;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = rows >= 444 ? 1 : (444 + rows - 1) / rows < 8 ? (444 + rows - 1) / rows : 8;  // three CTAs per SM
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(attr.val.clusterDim.x, rows);
+    cfg.blockDim = dim3(SAMPLE_THREADS);
+    cfg.stream = as_stream(stream);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    B200Q_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, (const bf16*)logits + (long long)at * V, params + 4 * (long long)at, ids + at, V));
+    B200Q_LAUNCH_CHECK();
+  }
   return B200Q_OK;
 }
 
