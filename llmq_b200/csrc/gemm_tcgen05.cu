@@ -752,18 +752,34 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
   return B200Q_OK;
 }
 
-// Measured on B200 (profiles/r1_gemm_2cta.md): at M >= 256 the CTA-pair kernel with a 256 x 256
-// tile is 0-8 % faster per unit of work than the 1-CTA 128 x 256 kernel (half the B traffic per
-// SM).  Use it when its coarser tiles do not cost an extra round of the persistent loop:
-// rounds(pair tiles over 74 pairs) <= rounds(1-CTA tiles over 148 SMs); a round costs the same
-// wall time in both kernels (every SM works one 128 x 256 tile per round).
-static bool prefer_2cta(int M, int N) {
-  if (M < 256 || N % 256) return false;
-  const long long sms = num_sms(), pairs = sms / 2;
-  const long long t2 = (long long)((M + 255) / 256) * (N / 256);
-  const long long t1 = (long long)((M + GEMM_BM - 1) / GEMM_BM) * (N / 256);
-  if (t2 < pairs) return false;  // not even one full round of pairs: finer 1-CTA tiles / split-K fill the chip better
-  return (t2 + pairs - 1) / pairs <= (t1 + sms - 1) / sms;
+// Which kernel and tile: the least (rounds of the persistent loop) x (time of a round).  Rounds: tiles over 148 SMs, or tiles of 256 rows
+// over 74 CTA pairs.  A round's time beside the 128 x 256 tile's (K 14336, one round, us: 85.5; pair 256 x 256 70-74, pair 256 x 128
+// 50.7, 128 x 128 55, 128 x 64 50; K 8192 the same shares, 49.5 / 41.5 / 29.8 / 32 / 29): the pair kernels fetch half the weight rows
+// per SM, narrow tiles are bound by what they fetch.  Before, the pair kernel was taken for whole rounds of 74 tiles only:
+// 768 x 3584 x 14336 86 -> 71 us, 512 x 4096 x 14336 58 -> 53, 1536 x 2048 x 8192 50 -> 43.
+struct TileChoice {
+  bool pair;
+  int bn;
+};
+static TileChoice choose_tile(int M, int N, bool gated) {
+  const struct {
+    bool pair;
+    int bn;
+    double cost;
+  } all[5] = {{true, 256, 0.84}, {false, 256, 1.0}, {true, 128, 0.595}, {false, 128, 0.645}, {false, 64, 0.585}};
+  TileChoice best{false, N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64};
+  double least = 1e30;
+  for (const auto& c : all) {
+    if (N % c.bn || (gated && c.bn != 256) || (c.pair && M <= GEMM_BM)) continue;
+    const long long rows = c.pair ? 256 : GEMM_BM, slots = c.pair ? num_sms() / 2 : num_sms();
+    const long long tiles = (M + rows - 1) / rows * (N / c.bn);
+    const double t = (double)((tiles + slots - 1) / slots) * c.cost;
+    if (t < least - 1e-9) {
+      least = t;
+      best = {c.pair, c.bn};
+    }
+  }
+  return best;
 }
 
 // ---- weight-stream probe (tools/gpu_probe.py stream_probe; not used by the product path) --------
@@ -841,6 +857,8 @@ static bool batch_invariant_env() {
 static int choose_splits(int M, int N, int K, bool invariant, int forced_bn) {
   const int want = invariant ? 1 : g_gemm_splitk;  // 0 = auto, 1 = off, >1 = forced (tests)
   if (want == 1 || forced_bn != 0 || M > 256 || N % 128 != 0 || N > 8192) return 1;
+  // (129 to 256 rows: with 2048 <= K < 4096 the partial tiles cost more than the idle SMs: 256 x 3072 x 2048 14.0 us split, 10.4 not)
+  if (want == 0 && M > GEMM_BM && K >= 2048 && K < 4096) return 1;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (N / 128);
   const int kb = K / GEMM_BK;
   int splits = want > 1 ? want : 1;
@@ -1071,7 +1089,7 @@ static int gemm_gated(const char* what, const void* A, const void* W, void* C, i
   cudaStream_t st = as_stream(stream);
   if (use_skinny(M, N, K, true))
     return gemm_skinny(A, W, C, M, N, K, kAct, ldc > 0 ? ldc : N / 2, gate.bias, gate.limit, nullptr, st);
-  if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && prefer_2cta(M, N)))
+  if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && choose_tile(M, N, true).pair))
     return launch_gemm2<256, kAct>(A, W, C, M, N, K, st, ldc, gate);
   return launch_gemm<256, kAct>(A, W, C, M, N, K, st, 1, nullptr, ldc, gate);
 }
@@ -1181,7 +1199,6 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
     if ((bn == 0 || bn == 256) && N % 256 == 0) return launch_gemm2<256>(A, W, C, M, N, K, st);
     if ((bn == 0 || bn == 128) && N % 128 == 0) return launch_gemm2<128>(A, W, C, M, N, K, st);
   }
-  if (g_gemm_mode == 0 && bn == 0 && prefer_2cta(M, N)) return launch_gemm2<256>(A, W, C, M, N, K, st);
   {
     // split-K for decode-sized batches: when a projection has too few 128-wide output tiles to
     // put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
@@ -1192,24 +1209,10 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
     if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits);
   }
   if (bn == 0) {
-    // Every CTA walks ceil(tiles / SMs) tiles; measured on B200 (profiles/r1_microbench.md) a
-    // 128-wide tile costs ~0.85x and a 64-wide tile ~0.8x the time of a 256-wide one (the kernel
-    // is bound by per-SM operand ingest, not by the MMA), so pick the candidate with the least
-    // (tiles per CTA) x (relative tile time); ties go to the wider tile.
-    const int m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
-    const int sms = num_sms();
-    const int cand[3] = {256, 128, 64};
-    const double cost[3] = {1.0, 0.85, 0.8};
-    double best = 1e30;
-    for (int i = 0; i < 3; ++i) {
-      if (N % cand[i]) continue;
-      const long long tiles = (long long)m_tiles * (N / cand[i]);
-      const double t = (double)((tiles + sms - 1) / sms) * cost[i];
-      if (t < best - 1e-9) {
-        best = t;
-        bn = cand[i];
-      }
-    }
+    const TileChoice t = choose_tile(M, N, false);
+    if (t.pair && g_gemm_mode == 0)
+      return t.bn == 256 ? launch_gemm2<256>(A, W, C, M, N, K, st) : launch_gemm2<128>(A, W, C, M, N, K, st);
+    bn = t.bn;
   }
   if (N % bn != 0) bn = (N % 128 == 0) ? 128 : 64;
   if (bn == 256) return launch_gemm<256>(A, W, C, M, N, K, st);
@@ -1233,8 +1236,7 @@ int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, vo
                   "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
   B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0,
                   "gemm: operands must be 16-byte aligned");
-  if (M == 0 || g_gemm_mode == 2 || g_gemm_force_bn != 0 || (g_gemm_mode == 0 && prefer_2cta(M, N)))
-    return B200Q_OK;
+  if (M == 0 || g_gemm_mode == 2 || g_gemm_force_bn != 0) return B200Q_OK;
   if (use_skinny(M, N, K, false)) {
     const int n = gemm_skinny_splits(M, N, K);
     if (n <= 1 || N > 8192) return B200Q_OK;
