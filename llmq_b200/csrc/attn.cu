@@ -119,7 +119,7 @@ constexpr bool kTransposedPV = D >= 256;
 // PV needs D/16 MMAs per page instead of D/8.  The S accumulators of qk_page<false> (rows = heads,
 // cols = tokens) are exactly the B fragments of P^T: b0 = tokens 0-7, b1 = tokens 8-15.  A = V^T
 // comes from the swizzled V page with ldmatrix.trans: matrix i of the x4 load covers tokens
-// 8*(i>>1).. and the 16-byte chunk 2*tile + (i&1).  (lane-accurate check: tools/emu/)
+// 8*(i>>1).. and the 16-byte chunk 2*tile + (i&1).
 template <int D, int BS>
 __device__ __forceinline__ void pv_page_t(uint32_t v_s, const float (&p)[BS / 8][4],
                                           float (&o)[D / 16][4], int lane) {

@@ -533,7 +533,7 @@ static int schedule_and_launch(b200q_engine* e, InFlightStep& step) {
     // policy 1 also reserves the blocks the RUNNING requests are expected to grow into (their
     // expected final length, see expected_growth_blocks): admitting on today's free blocks alone
     // over-commits the pool under a steady backlog, and every later preemption recomputes a whole
-    // sequence (3 % of all tokens at 4608 x 128-in/128-out on one B200, tools/sched_sim.py).
+    // sequence (3 % of all tokens at 4608 x 128-in/128-out on one B200, in a simulation).
     // Requests that outgrow the estimate are still handled by preempt-by-recompute.
     // The reservation only pays while there is a backlog to fill the batch from later: when every
     // waiting request fits the free slots (the queue is draining) a deferred request would run on
