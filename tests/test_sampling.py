@@ -76,3 +76,76 @@ def test_sample_kernel_matches_oracle_and_distribution(cuda, V):
     keep = p * n >= 5
     chi2 = (((counts - p * n) ** 2) / (p * n))[keep].sum()
     assert counts.sum() == n and chi2 < 2.0 * keep.sum() + 20, (chi2, keep.sum())
+
+
+def draw_on_gpu(cuda, rows, temps, seeds, positions):
+    from llmq_b200 import lib
+    params = torch.zeros(len(rows), 4, dtype=torch.int32)
+    for i, (t, s, p) in enumerate(zip(temps, seeds, positions)):
+        params[i, 0] = int(np.float32(t).view(np.int32))
+        params[i, 1], params[i, 3] = s, p
+    out = torch.full((len(rows),), -1, dtype=torch.int32, device=cuda)
+    lib.sample_bf16(rows.to(torch.bfloat16).to(cuda), params.to(cuda), out)
+    return out.cpu().tolist()
+
+
+def expect(got, rows, temps, seeds, positions):
+    """the oracle's ids; fp32 may decide a near-tie the other way: logarithms to about 1e-4 (as above), the product and the sum each to
+    half an ulp (2^-24) of values up to largest logit / temperature"""
+    for i, row in enumerate(rows.to(torch.bfloat16).double().numpy()):
+        ref = S.sample(row, temps[i], seeds[i], positions[i])
+        if got[i] != ref:
+            assert temps[i] > 0, (i, got[i], ref)
+            near = 1e-4 + 2.0 ** -22 * row.max() / temps[i]
+            assert S.sample_margin(row, temps[i], seeds[i], positions[i]) < near, (i, got[i], ref)
+
+
+# (seed 1: at these positions these tokens draw the largest bits there are)
+LARGEST = {26: 138, 65: 57555, 345: 112154}
+
+
+def test_largest_bits_are_where_the_kernel_test_has_them():
+    for pos, token in LARGEST.items():
+        g = S.gumbel_noise(128256, 1, pos)
+        assert int(g.argmax()) == token and abs(g[token] - 25 * np.log(2.0)) < 1e-6   # u = 1 - 2^-25
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("low", [-30.0, 0.0])
+def test_largest_bits_do_not_win_by_themselves(cuda, low):
+    positions = sorted(LARGEST)
+    rows = torch.randn(3, 128256, generator=torch.Generator().manual_seed(2)) * 2
+    for i, pos in enumerate(positions):
+        rows[i, LARGEST[pos]] = low
+    got = draw_on_gpu(cuda, rows, [0.7] * 3, [1] * 3, positions)
+    expect(got, rows, [0.7] * 3, [1] * 3, positions)
+    if low < 0:
+        assert all(t != LARGEST[p] for t, p in zip(got, positions))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 56, 64, 74, 89, 111, 148, 222, 444])   # rows of 8, 8, 7, 6, 5, 4, 3, 2 and 1 CTAs
+def test_masked_rows_and_ties(cuda, B):
+    V = 4 * 512 * 8 + 12   # (some CTAs of a row of eight take a second, short turn)
+    rows = torch.randn(B, V, generator=torch.Generator().manual_seed(B)) * 3
+    kind = [i % 6 for i in range(B)]
+    for i, k in enumerate(kind):
+        if k == 1:
+            rows[i, torch.randperm(V, generator=torch.Generator().manual_seed(i))[: V - 5]] = -float("inf")
+        elif k == 2:
+            rows[i] = -float("inf")
+        elif k == 3:
+            rows[i] = 1.5                          # only the noise decides, and all of the greedy row is equal
+        elif k == 4:
+            rows[i, 3::2048] = 50.0                # equal largest logits in every CTA of the row
+        elif k == 5:
+            rows[i, i % V] = float("nan")          # never drawn
+    temps = [(0.7, 0.0, 1.3, 0.7, 0.01)[i % 5] for i in range(B)]
+    seeds, positions = [100 + i for i in range(B)], [3 * i for i in range(B)]
+    got = draw_on_gpu(cuda, rows, temps, seeds, positions)
+    assert got == draw_on_gpu(cuda, rows, temps, seeds, positions)
+    ref = rows.clone()
+    ref[ref.isnan()] = -float("inf")
+    expect(got, ref, temps, seeds, positions)
+    for i, k in enumerate(kind):
+        assert k != 2 or got[i] == 0
