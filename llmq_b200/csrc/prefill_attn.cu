@@ -524,10 +524,6 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
 #pragma unroll
           for (int x = 0; x < COLS / 32; ++x)
             if (used(x)) {
-              if constexpr (kCap) {
-#pragma unroll
-                for (int y = 0; y < 32; ++y) big[y & 1] = fmaxf(big[y & 1], fabsf(__uint_as_float(s[x][y])));
-              }
               if (masked(x)) {
                 const int hi_c = pos - key0 - 32 * x, lo_c = lo - key0 - 32 * x;
 #pragma unroll
@@ -538,6 +534,15 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
                   for (int y = 0; y < 32; ++y)
                     if (y < lo_c) s[x][y] = 0xff800000u;
                 }
+                // (of visible keys only: rows behind the last key hold whatever was in shared memory before)
+                if constexpr (kCap) {
+#pragma unroll
+                  for (int y = 0; y < 32; ++y)
+                    big[y & 1] = fmaxf(big[y & 1], s[x][y] == 0xff800000u ? 0.f : fabsf(__uint_as_float(s[x][y])));
+                }
+              } else if constexpr (kCap) {
+#pragma unroll
+                for (int y = 0; y < 32; ++y) big[y & 1] = fmaxf(big[y & 1], fabsf(__uint_as_float(s[x][y])));
               }
 #pragma unroll
               for (int y = 0; y < 32; ++y) mx[y & 3] = fmaxf(mx[y & 3], __uint_as_float(s[x][y]));
