@@ -22,8 +22,6 @@
 // their code: kCap = attention-logit soft-capping (score <- cap * tanh(score * scale / cap)), and a
 // runtime sliding window (query at position p sees keys p - window < j <= p; pages that lie entirely
 // before the window are never fetched).  D = 256 (Gemma-2 head size) uses 2-stage rings.
-#include <stdlib.h>
-
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -200,7 +198,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   using S_ = DecSmem<D, BS>;
   constexpr int DEC_STAGES = S_::STAGES;
   extern __shared__ __align__(128) uint8_t smem[];
-  const int seq = blockIdx.y, kvh = blockIdx.z;
+  const int seq = kShared ? blockIdx.y : blockIdx.x, kvh = kShared ? blockIdx.z : blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = kShared ? gridDim.x : 1, split = kShared ? blockIdx.x : 0;
   const int wg = split * DEC_WARPS + warp, n_warps = splits * DEC_WARPS;  // this warp's place among the sequence's warps
@@ -823,11 +821,7 @@ int g_decode_variant = 0;  // test hook: 0 = auto, 1 = split kernel (v1), 2 = st
 // longest context that the block table could hold (shorter ones gain nothing: an exchange costs about 2 us).  6 sequences of 3000 to
 // 8100 tokens, D = 64, 8 kv heads: 22 us, 65 with one CTA each.  B200Q_BATCH_INVARIANT=1: always one, whatever the batch.
 static int decode_splits(int n_seqs, int n_kv, int bt_stride) {
-  static const bool invariant = [] {
-    const char* e = getenv("B200Q_BATCH_INVARIANT");
-    return e && e[0] == '1';
-  }();
-  if (invariant || g_decode_variant == 1) return 1;
+  if (batch_invariant() || g_decode_variant == 1) return 1;
   const long long ctas = (long long)n_seqs * n_kv;
   int splits = 1;
   while (splits < 8 && ctas * (splits + 1) <= 296 && bt_stride / (DEC_WARPS * (splits + 1)) >= 4) ++splits;
@@ -847,7 +841,7 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
   }
   const ScoreConsts sc = score_consts(scale, softcap);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, n_seqs, n_kv);
+  cfg.gridDim = kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
   cfg.blockDim = dim3(DEC_WARPS * 32);
   cfg.dynamicSmemBytes = S_::TOTAL;
   cfg.stream = st;
@@ -856,7 +850,7 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
   attr.val.clusterDim.x = splits;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = kShared ? 1 : 0;
   B200Q_CUDA(cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
                                 n_q / n_kv, sc.c0, sc.c1, window));
   B200Q_LAUNCH_CHECK();
@@ -976,10 +970,11 @@ int b200q_decode_attn_ex(const void* q, int q_stride, void* out, const void* kv_
                   block_size);
   if (n_seqs == 0) return B200Q_OK;
   cudaStream_t st = as_stream(stream);
-  // streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items
+  // streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
+  // another order of sums)
   const bool stream_variant =
       g_decode_variant >= 2 ||
-      (g_decode_variant == 0 && (long long)n_seqs * n_kv >= 16LL * attn_num_sms());
+      (g_decode_variant == 0 && !batch_invariant() && (long long)n_seqs * n_kv >= 16LL * attn_num_sms());
   if (stream_variant)
     B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
                         ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);

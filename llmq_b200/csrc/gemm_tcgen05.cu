@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(64)
 int g_gemm_force_bn = 0;  // test hook: 0 = heuristic
 int g_gemm_splitk = 0;    // 0 = auto, 1 = never, n > 1 = force n splits where legal (tests)
 
-static bool batch_invariant_env() {
+bool batch_invariant() {
   static const bool v = [] {
     const char* e = getenv("B200Q_BATCH_INVARIANT");
     return e && e[0] == '1';
@@ -876,7 +876,7 @@ int g_gemm_mode = 0;      // 0 = auto, 1 = force 1-CTA kernels, 2 = force the 2-
 // Up to 128 rows go to gemm_skinny.cu unless a hook asks for one of the kernels here, or results must not depend on the number of
 // rows (its splits depend on it, and the kernels here that larger steps use add in another order).
 static bool use_skinny(int M, int N, int K, bool gated) {
-  return g_gemm_mode == 0 && g_gemm_force_bn == 0 && g_gemm_splitk == 0 && !batch_invariant_env() && gemm_skinny_ok(M, N, K, gated);
+  return g_gemm_mode == 0 && g_gemm_force_bn == 0 && g_gemm_splitk == 0 && !batch_invariant() && gemm_skinny_ok(M, N, K, gated);
 }
 
 
@@ -1203,9 +1203,9 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
     // split-K for decode-sized batches: when a projection has too few 128-wide output tiles to
     // put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
     // B200Q_BATCH_INVARIANT=1 (read once): never split K, so every output element is reduced in
-    // one sequential pass and a request's tokens cannot depend on its batch-mates (like
+    // one sequential pass (the attention kernels do likewise) and a request's tokens cannot depend on its batch-mates (like
     // VLLM_BATCH_INVARIANT); costs decode-sized GEMMs up to 2x
-    const int splits = choose_splits(M, N, K, batch_invariant_env(), bn);
+    const int splits = choose_splits(M, N, K, batch_invariant(), bn);
     if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits);
   }
   if (bn == 0) {
@@ -1248,7 +1248,7 @@ int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, vo
     *splits_out = n;
     return B200Q_OK;
   }
-  const int splits = choose_splits(M, N, K, batch_invariant_env(), 0);
+  const int splits = choose_splits(M, N, K, batch_invariant(), 0);
   if (splits <= 1) return B200Q_OK;
   int rc = launch_gemm<128>(A, W, nullptr, M, N, K, as_stream(stream), splits, partials_out);
   if (rc) return rc;

@@ -741,7 +741,10 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
 //                           198 / 778; but one of 200 10.9 / 8.4, 5 behind 300 12.2 / 11.5, 27 x 10-31 behind 42 21 / 11
 //   D = 64, 32 / 8 heads    one of 4400 186 / 533; but 30 x 64-256 42 / 38, one of 300 12.6 / 10.2, one of 512 18.9 / 18.1
 //   D = 256, 8 / 4 heads    one of 200 14.3 / 19.3, one of 300 17 / 27, 300 behind 900 33 / 99; but 27 x 10-31 behind 42 19.5 / 11.5
+// B200Q_BATCH_INVARIANT=1: always the kernel of 16-token tiles, where a row's sums follow from its own sequence; here they depend on how
+// the tiles of all portions are cut into blocks.
 static bool tensor_memory_pays(int n_kv, int D, long long keys, int n_tiles) {
+  if (batch_invariant()) return false;
   if (D == 64) return keys > 512;
   if (D == 128) return keys > 512 || (keys > 128 && (long long)n_tiles * n_kv >= 512);
   return keys > 128;

@@ -191,6 +191,10 @@ __device__ __forceinline__ float clamped_unit(uint32_t gb, uint32_t ub, float b0
   return g / (1.f + __expf(-1.702f * g)) * (w + 1.f);
 }
 
+// B200Q_BATCH_INVARIANT=1 (read once): what a row of a step gives must not depend on the other rows, so every kernel is taken whose
+// order of sums would otherwise change with them (gemm_tcgen05.cu)
+bool batch_invariant();
+
 // bf16 row-major [rows, cols] -> tiled map with box {64 cols, box_rows rows}, 128B swizzle (ld: elements between rows, 0 = dense);
 // maps are cached by address and shape (gemm_tcgen05.cu)
 int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out, long long ld = 0);
