@@ -128,8 +128,80 @@ __device__ __forceinline__ float fa_rcp(float x) {
   return y;
 }
 
+// One query row of one head once more, by a whole warp: columns [c_out, c_out + OC) over the keys lo .. pos and no others.  In the
+// products of the kernel below a hidden key's probability is 0 and times a value that is not finite that is NaN, for every row of the
+// query tile that shares the step; such rows come here (a tile's row that sees the value itself comes here too, and gets what it sees).
+template <int D, int OC, bool kCap>
+__device__ __noinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, const bf16* q_row, bf16* out_row, int kvh, int lo, int pos,
+                                          int c_out) {
+  const int lane = threadIdx.x & 31;
+  constexpr int NW = OC / 64;  // 32-bit words of the output per lane
+  const long long page_bytes = 16 * D * 2;
+  const uint32_t* q4 = reinterpret_cast<const uint32_t*>(q_row);
+  float m = -INFINITY, l = 0.f, acc[NW][2];
+#pragma unroll
+  for (int w = 0; w < NW; ++w) acc[w][0] = acc[w][1] = 0.f;
+  lo = max(lo, 0);
+  for (int j0 = lo & ~31; j0 <= pos; j0 += 32) {
+    const int j = j0 + lane, t = j & 15;
+    const bool seen = j >= lo && j <= pos;
+    const int blk = seen ? __ldg(bt + (j >> 4)) : 0;
+    float s = -INFINITY;
+    if (seen) {
+      const uint8_t* row = a.kv + ((long long)blk * 2 * a.n_kv + kvh) * page_bytes + t * (D * 2);
+      float dot = 0.f;
+#pragma unroll 4
+      for (int c = 0; c < D / 8; ++c) {
+        const uint4 k = *reinterpret_cast<const uint4*>(row + ((c ^ (t & 7)) << 4));
+        const uint32_t kk[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const uint32_t q = q4[4 * c + x] ^ a.q_flip;
+          dot = fmaf(bf16_lo(q), bf16_lo(kk[x]), dot);
+          dot = fmaf(bf16_hi(q), bf16_hi(kk[x]), dot);
+        }
+      }
+      s = kCap ? a.c1 * tanhf(dot * a.c0) : dot * a.c0;
+    }
+    float top = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (top > m) {
+      const float alpha = fa_ex2(m - top);
+      m = top;
+      l *= alpha;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        acc[w][0] *= alpha;
+        acc[w][1] *= alpha;
+      }
+    }
+    const float p = seen ? fa_ex2(s - (m == -INFINITY ? 0.f : m)) : 0.f;
+    l += p;
+    const float p16 = round_bf16(p);
+    for (int i = max(lo - j0, 0); i < 32 && j0 + i <= pos; ++i) {  // (the warp agrees on i)
+      const float pi = __shfl_sync(0xffffffffu, p16, i);
+      const int bi = __shfl_sync(0xffffffffu, blk, i), ti = (j0 + i) & 15;
+      const uint8_t* row = a.kv + (((long long)bi * 2 + 1) * a.n_kv + kvh) * page_bytes + ti * (D * 2);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const int word = c_out / 2 + w * 32 + lane;
+        const uint32_t v = *reinterpret_cast<const uint32_t*>(row + (((word >> 2) ^ (ti & 7)) << 4) + (word & 3) * 4);
+        acc[w][0] = fmaf(pi, bf16_lo(v), acc[w][0]);
+        acc[w][1] = fmaf(pi, bf16_hi(v), acc[w][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+  for (int w = 0; w < NW; ++w)
+    reinterpret_cast<uint32_t*>(out_row + c_out)[w * 32 + lane] = pack_bf16x2(acc[w][0] * inv, acc[w][1] * inv);
+}
+
 template <int D, bool kCap>
-__global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __grid_constant__ CUtensorMap kv_map, const FaArgs a) {
+__global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ FaArgs a) {
   using C = FaCfg<D>;
   constexpr int NQ = C::NQ, KT = C::KT, STG = C::STG, CH = C::CH, COLS = C::COLS, PAGES = KT / 16;
   extern __shared__ uint8_t smem_raw[];
@@ -649,6 +721,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
         constexpr int PC = C::PATCH / 8;  // 16-byte chunks per row
         const uint32_t patch = smem_u32(patches + warp * (32 * C::PATCH * 2));
         const int w0 = (warp & 3) * 32;
+        float check = 0.f;  // NaN once a column of the row is not finite
 #pragma unroll 1
         for (int c = 0; c < OC; c += C::PATCH) {
 #pragma unroll
@@ -656,6 +729,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
             uint32_t o[32];
             tmem_ld32(o_at + (uint32_t)(c + 32 * h), o);
             tmem_ld_wait();
+#pragma unroll
+            for (int y = 0; y < 32; ++y) check = fmaf(__uint_as_float(o[y]), 0.f, check);
 #pragma unroll
             for (int y = 0; y < 4; ++y) {
               uint32_t w[4];
@@ -689,6 +764,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
             }
           }
           __syncwarp();
+        }
+        // (a sum that is not finite comes from the scores, which are the row's own)
+        uint32_t again = __ballot_sync(0xffffffffu, check != check && l < INFINITY && i_tile * 128 + row < rows);
+        while (again) {
+          const int g = i_tile * 128 + w0 + __ffs(again) - 1, t = (int)((uint32_t)g * a.inv_g >> 16), head = kvh * a.G + g - t * a.G;
+          again &= again - 1;
+          fa_row_again<D, OC, kCap>(a, a.block_table + (long long)r.bt_row * a.bt_stride,
+                                    a.q + (long long)(r.row0 + t) * a.q_stride + (long long)head * D,
+                                    a.out + (long long)(r.row0 + t) * a.n_q * D + (long long)head * D, kvh,
+                                    a.window > 0 ? r.pos0 + t + 1 - a.window : 0, r.pos0 + t, c_out);
         }
         tc_fence_before();
       }

@@ -146,3 +146,38 @@ def test_same_bits_whatever_ran_before(cuda, D, cap, window):
     second = small()
     assert torch.equal(first.view(torch.int16), second.view(torch.int16))
     assert torch.equal(first.view(torch.int16), small().view(torch.int16))
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 4, 2), (64, 2, 2), (128, 8, 2), (128, 2, 2), (256, 4, 2), (256, 2, 2)])
+@pytest.mark.parametrize("cap,window", [(0.0, 0), (20.0, 0), (0.0, 90)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), -float("inf")])
+def test_values_that_are_not_finite_stay_with_those_who_see_them(cuda, D, n_q, n_kv, cap, window, value):
+    """one element of a cached value row is not finite: tokens before it, and tokens whose window has passed it, get what they would"""
+    from llmq_b200 import lib
+    portions, bad = [(0, 1500), (300, 700), (0, 40)], {0: 1333, 1: 700}      # (sequence: token)
+    kv, bt, rows = make_cache([a + n for a, n in portions], n_kv, D, 31, True)
+    sw = O.kv_swizzle_index(BS, D)
+    for i, t in bad.items():
+        kv[bt[i, t // BS], 1, 0, t % BS, sw[t % BS, D // 3]] = value       # head 0, column D // 3
+    T = sum(n for _, n in portions)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * D, generator=torch.Generator().manual_seed(8)).to(BF)
+    tiles, row = [], 0
+    for i, (a, n) in enumerate(portions):
+        tiles += [[i, row + j, min(16, n - j), a + j] for j in range(0, n, 16)]
+        row += n
+    out = torch.full((T + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
+    lib.prefill_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), torch.tensor(tiles, dtype=torch.int32, device=cuda), n_q, n_kv, D, BS,
+                     D ** -0.5, softcap=cap, window=window)
+    got, row = out.cpu(), 0
+    assert torch.isnan(got[T].float()).all() and lib.load().b200q_wait_failures() == 0
+    for i, (a, n) in enumerate(portions):
+        q = qkv[row: row + n, : n_q * D].view(n, n_q, D)
+        ref = reference(q, *rows[i], torch.arange(a, a + n), D ** -0.5, cap, window)
+        mine, pos = got[row: row + n].view(n, n_q, D), torch.arange(a, a + n)
+        sees = (pos >= bad.get(i, 1 << 30)) & ((pos < bad.get(i, 0) + window) if window else True)
+        touched = torch.zeros(n, n_q, D, dtype=torch.bool)
+        touched[sees, : n_q // n_kv, D // 3] = True
+        # (head 0's column of the tokens that see it is value itself, or NaN; everything else is as it was without it)
+        assert not torch.isfinite(mine[touched].float()).any()
+        bf16_close(torch.where(touched, ref.to(BF), mine), ref.to(BF), ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"portion {i}")
+        row += n
