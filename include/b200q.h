@@ -177,6 +177,12 @@ int b200q_prefill_attn_ex(const void* q_dev, int q_stride, void* out_dev, const 
                           const int32_t* block_table_dev, int bt_stride, const int32_t* tiles_dev,
                           int n_tiles, int n_q, int n_kv, int D, int block_size, float scale,
                           float softcap, int window, void* stream);
+/* ... with the number of sequences that the tiles belong to at most (rows of the block table; 0 = unknown): where it shows whether the
+ *     portions are short or long, one kernel is launched instead of two that share them.  Any number gives the same results. */
+int b200q_prefill_attn_seqs(const void* q_dev, int q_stride, void* out_dev, const void* kv_layer_dev,
+                            const int32_t* block_table_dev, int bt_stride, int n_seqs, const int32_t* tiles_dev,
+                            int n_tiles, int n_q, int n_kv, int D, int block_size, float scale,
+                            float softcap, int window, void* stream);
 
 /* fused gate_up GEMM + GeGLU: out = bf16(bf16(gelu_tanh(g)) * u), weight rows interleaved exactly as
  *     for b200q_gemm_swiglu_bf16                          (vllm activation.py GeluAndMul, approximate="tanh") */

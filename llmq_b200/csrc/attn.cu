@@ -652,8 +652,8 @@ __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
     prefill_tile_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out,
                         const uint8_t* __restrict__ kv_layer,
                         const int32_t* __restrict__ block_table, int bt_stride,
-                        const int4* __restrict__ tiles, int n_q, int n_kv, int G,
-                        float c0, float c1, int window) {
+                        const int4* __restrict__ tiles, int n_tiles, int n_q, int n_kv, int G,
+                        float c0, float c1, int window, int long_keys) {
   using G_ = Geo<D, BS>;
   using S_ = PfSmem<D, BS>;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -661,6 +661,7 @@ __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
   uint64_t* empty = full + PF_STAGES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y;
+  if (long_keys > 0 && portion_keys(tiles, n_tiles, blockIdx.x, lane) >= long_keys) return;
   const int4 tile = __ldg(tiles + blockIdx.x);
   const int bt_row = tile.x, row0 = tile.y, n_rows = tile.z, pos0 = tile.w;
   const int total_kv = pos0 + n_rows;  // keys 0 .. pos0+n_rows-1 are visible to this tile
@@ -908,7 +909,7 @@ static int launch_decode_stream(const void* q, int q_stride, void* out, const vo
 template <int D, int BS, bool kCap>
 static int launch_prefill(const void* q, int q_stride, void* out, const void* kv,
                           const int32_t* bt, int bt_stride, const int32_t* tiles, int n_tiles,
-                          int n_q, int n_kv, float scale, float softcap, int window,
+                          int n_q, int n_kv, float scale, float softcap, int window, int long_keys,
                           cudaStream_t st) {
   using S_ = PfSmem<D, BS>;
   auto kern = prefill_tile_kernel<D, BS, kCap>;
@@ -924,7 +925,8 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
   dim3 grid(n_tiles, n_kv);
   kern<<<grid, (G + 1) * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out,
                                               (const uint8_t*)kv, bt, bt_stride,
-                                              (const int4*)tiles, n_q, n_kv, G, sc.c0, sc.c1, window);
+                                              (const int4*)tiles, n_tiles, n_q, n_kv, G, sc.c0, sc.c1, window,
+                                              long_keys);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -940,8 +942,9 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
   } while (0)
 
 int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
-                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, cudaStream_t st) {
-  B200Q_ATTN_DISPATCH(launch_prefill, q, q_stride, out, kv, bt, bt_stride, tiles, n_tiles, n_q, n_kv, scale, softcap, window, st);
+                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, int long_keys, cudaStream_t st) {
+  B200Q_ATTN_DISPATCH(launch_prefill, q, q_stride, out, kv, bt, bt_stride, tiles, n_tiles, n_q, n_kv, scale, softcap, window, long_keys,
+                      st);
 }
 
 }  // namespace b200q

@@ -14,6 +14,11 @@ void set_error(const char* fmt, ...);
 extern thread_local char g_err[512];
 void count_launch(int n = 1);
 // bumped by every test/tuning setter: cached CUDA graphs bake kernel choices in and must be rebuilt
+// prompt attention (prefill_attn.cu): which kernel takes a step's portions, and the call
+int prefill_attn_route(const int32_t* desc, int n_desc, int n_seqs, int n_tiles, int bt_stride, int n_q, int n_kv, int D, int window);
+int prefill_attn(int route, const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                 const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, float softcap, int window,
+                 cudaStream_t st);
 void bump_tuning_epoch();
 int tuning_epoch();
 

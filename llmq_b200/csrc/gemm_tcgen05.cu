@@ -849,7 +849,7 @@ bool batch_invariant() {
     const char* e = getenv("B200Q_BATCH_INVARIANT");
     return e && e[0] == '1';
   }();
-  return v;
+  return v || g_gemm_splitk == 1;  // (the hook without splits stands for the variable)
 }
 
 // split-K factor for a decode-sized projection (1 = do not split): when it has too few 128-wide

@@ -302,6 +302,12 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
     }
     return b200q_gemm_bf16(A, W, C, T, N, K, stream);
   };
+  // (a caller without a host copy of the portions: every sequence that ends a portion samples)
+  const int32_t* portions = b->h_seq_desc && b->n_rows >= b->n_dec ? b->h_seq_desc + 4 * (long long)b->n_dec : nullptr;
+  int prefill_route[2];
+  for (int w = 0; w < 2; ++w)
+    prefill_route[w] = prefill_attn_route(portions, b->n_rows - b->n_dec, b->n_sample > b->n_dec ? b->n_sample - b->n_dec : 0, b->n_tiles,
+                                          b->bt_stride, NQ, NKV, D, w ? c.sliding_window : 0);
   for (int li = 0; li < c.n_layers; ++li) {
     const b200q_layer& L = m->layers[li];
     uint8_t* kv_layer = m->kv + li * kv_layer_bytes;
@@ -330,9 +336,9 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
     B200Q_TRY(B200Q_PROF_DECODE_ATTN, (double)b->sum_ctx_dec * kv_tok_bytes, b200q_decode_attn_ex(m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
                                 b->ctx_lens, b->n_dec, NQ, NKV, D, c.block_size, c.attn_scale,
                                 c.attn_softcap, window, stream));
-    B200Q_TRY(B200Q_PROF_PREFILL_ATTN, (double)b->prefill_flops_per_layer, b200q_prefill_attn_ex(m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
+    B200Q_TRY(B200Q_PROF_PREFILL_ATTN, (double)b->prefill_flops_per_layer, prefill_attn(prefill_route[window > 0], m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
                                  b->tiles, b->n_tiles, NQ, NKV, D, c.block_size, c.attn_scale,
-                                 c.attn_softcap, window, stream));
+                                 c.attn_softcap, window, as_stream(stream)));
     B200Q_TRY(B200Q_PROF_GEMM, 2.0 * T * H * QD, gemm_maybe_split(m->attn, L.o, m->x, H, QD, &part, &splits));
     if (gemma) {
       B200Q_TRY(B200Q_PROF_ELEMENTWISE, 4.0 * T * H * 2, b200q_gemma_norm_add_norm(m->x, m->residual, L.post_attn_norm, L.pre_ffn_norm, T, H, c.rms_eps, stream));

@@ -14,6 +14,8 @@
 //   * The running maximum moves only when a row's grows by more than 2^8 (exponents stay far from overflow; at D = 256 the first 512
 //     keys follow it exactly, so that short contexts round as the plain form does); the outputs in tensor memory are scaled in place.
 //   * Persistent: one CTA per SM walks its blocks, last tiles (the longest ones of a prompt) first; the page ring runs on across them.
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -41,6 +43,7 @@ struct FaArgs {
   const int4* tiles;
   int* failed;
   int q_stride, bt_stride, n_tiles, per_block, n_q, n_kv, G, window;
+  int long_keys;    // (kSplit) portions of fewer keys are left to the kernel of 16-token tiles
   float c0, c1;  // of a score: plain s * c0 in base 2; capped c1 * tanh(s * c0); c0 > 0
   uint32_t q_flip;  // the queries' sign bits turned (a negative scale)
   int vec;          // rows of q and out are 16-byte aligned
@@ -69,23 +72,53 @@ struct FaUnit {  // a CTA's place: unit u, at x of its round
   }
 };
 
+// portion_keys of the tiles first .. first + 15, one per lane
+__device__ __forceinline__ int block_portion_keys(const FaArgs& a, int first, int lane) {
+  uint64_t ends = 0;  // bit p: tile first + p does not continue the one before it
+  int keys[2], x = 0, y = 0, w = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = first + 32 * h + lane;
+    const int4 t = __ldg(a.tiles + min(i, a.n_tiles - 1));
+    const int n = min(max(t.z, 0), 16);
+    keys[h] = t.w + n;
+    // (lane 0 compares with lane 31 of the half before)
+    const int px = __shfl_up_sync(0xffffffffu, t.x, 1);
+    const int x0 = __shfl_sync(0xffffffffu, x, 31), y0 = __shfl_sync(0xffffffffu, y, 31), w0 = __shfl_sync(0xffffffffu, w, 31);
+    const int py = __shfl_up_sync(0xffffffffu, t.y + n, 1), pw = __shfl_up_sync(0xffffffffu, t.w + n, 1);
+    const bool on = (lane ? px : x0) == t.x && (lane ? py : y0) == t.y && (lane ? pw : w0) == t.w && i < a.n_tiles;
+    ends |= (uint64_t)__ballot_sync(0xffffffffu, !on) << (32 * h);
+    x = t.x;
+    y = t.y + n;
+    w = t.w + n;
+  }
+  const uint64_t later = ends >> (lane + 1);
+  const int last = lane + min(later ? __ffsll((long long)later) - 1 : 31, 31);
+  const int k0 = __shfl_sync(0xffffffffu, keys[0], last & 31), k1 = __shfl_sync(0xffffffffu, keys[1], last & 31);
+  return last < 32 ? k0 : k1;
+}
+
 // the runs of a block, seen by a whole warp: lane l holds tile l of the block
 struct FaBlock {
   int4 t, ahead;
   uint32_t starts;  // bit l: tile l begins a run
-  int count, ahead_count;
+  int count, ahead_count, ahead_first;
   // the tiles of unit u are asked for one unit ahead
   __device__ __forceinline__ void fetch(const FaArgs& a, const FaOrder& o, int u, int lane) {
-    const int first = u < o.units ? o.block(u / a.n_kv) * a.per_block : a.n_tiles;
-    ahead_count = min(a.per_block, a.n_tiles - first);
-    ahead = lane < ahead_count ? __ldg(a.tiles + first + lane) : make_int4(0, 0, 0, 0);
+    ahead_first = u < o.units ? o.block(u / a.n_kv) * a.per_block : a.n_tiles;
+    ahead_count = min(a.per_block, a.n_tiles - ahead_first);
+    ahead = lane < ahead_count ? __ldg(a.tiles + ahead_first + lane) : make_int4(0, 0, 0, 0);
   }
+  template <bool kSplit>
   __device__ __forceinline__ void begin(const FaArgs& a, const FaOrder& o, FaUnit at, int lane) {
+    const int first = ahead_first;
     count = ahead_count;
     t = ahead;
     at.step();
     fetch(a, o, at.u, lane);
     t.z = min(max(t.z, 0), 16);
+    if constexpr (kSplit)
+      if (block_portion_keys(a, first, lane) < a.long_keys) t.z = 0;  // (no rows: no run)
     const int br = __shfl_up_sync(0xffffffffu, t.x, 1), r0 = __shfl_up_sync(0xffffffffu, t.y, 1), nn = __shfl_up_sync(0xffffffffu, t.z, 1),
               p0 = __shfl_up_sync(0xffffffffu, t.w, 1);
     const bool next = lane > 0 && lane < count && br == t.x && r0 + nn == t.y && p0 + nn == t.w;
@@ -200,7 +233,9 @@ __device__ __noinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, co
     reinterpret_cast<uint32_t*>(out_row + c_out)[w * 32 + lane] = pack_bf16x2(acc[w][0] * inv, acc[w][1] * inv);
 }
 
-template <int D, bool kCap>
+// kSplit: only the portions of long_keys keys and more (a variant of its own: the code to look at them costs the other one 1 to 2 % in
+// instruction fetches, where CTAs walk many short units)
+template <int D, bool kCap, bool kSplit>
 __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ FaArgs a) {
   using C = FaCfg<D>;
   constexpr int NQ = C::NQ, KT = C::KT, STG = C::STG, CH = C::CH, COLS = C::COLS, PAGES = KT / 16;
@@ -221,6 +256,14 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
   const bool sort = n_blocks <= FA_SORTED && n_blocks * a.n_kv > (int)gridDim.x;  // (one unit each: nothing to deal out)
   const FaOrder order{sort ? sorted : nullptr, n_blocks, n_blocks * a.n_kv};
 
+  if constexpr (kSplit) {  // no tile sees so many keys: nothing to do here
+    bool any = false;
+    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {
+      const int4 t = __ldg(a.tiles + i);
+      any |= t.w + min(max(t.z, 0), 16) >= a.long_keys;
+    }
+    if (!__syncthreads_or(any)) return;
+  }
   if (threadIdx.x == 0) {
     dead = 0;
     for (int s = 0; s < STG; ++s) {
@@ -246,8 +289,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {  // the last token of a run sees most keys
       const int4 t = __ldg(a.tiles + i), n = __ldg(a.tiles + min(i + 1, a.n_tiles - 1));
       const bool ends = i + 1 == a.n_tiles || (i + 1) % a.per_block == 0 || n.x != t.x || n.y != t.y + t.z || n.w != t.w + t.z;
-      const int keys = a.window > 0 ? min(t.w + t.z, a.window) : t.w + t.z;
-      if (ends) atomicAdd(steps_in + i / a.per_block, max(keys, 0) / KT + 2);  // (its start and end: about one step more)
+      const int all = t.w + t.z, keys = a.window > 0 ? min(all, a.window) : all;
+      if (ends && (!kSplit || all >= a.long_keys)) atomicAdd(steps_in + i / a.per_block, max(keys, 0) / KT + 2);  // (start and end: about one step)
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n_blocks; i += FA_THREADS) {
@@ -279,7 +322,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     FaBlock b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
-      b.begin(a, order, w, lane);
+      b.template begin<kSplit>(a, order, w, lane);
       const int kvh = w.u % a.n_kv;
       for (int at = 0; at < b.count;) {
         FaRun r;
@@ -369,7 +412,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     FaBlock b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
-      b.begin(a, order, w, lane);
+      b.template begin<kSplit>(a, order, w, lane);
       for (int at = 0; at < b.count;) {
         FaRun r;
         at = b.run(at, r);
@@ -479,7 +522,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     FaBlock b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
-      b.begin(a, order, w, lane);
+      b.template begin<kSplit>(a, order, w, lane);
       const int kvh = w.u % a.n_kv;
       for (int at = 0; at < b.count;) {
         FaRun r;
@@ -562,7 +605,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     FaBlock b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
-      b.begin(a, order, w, lane);
+      b.template begin<kSplit>(a, order, w, lane);
       const int kvh = w.u % a.n_kv;
       for (int at = 0; at < b.count;) {
         FaRun r;
@@ -792,14 +835,20 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
   }
 }
 
-template <int D, bool kCap>
+// q-tiles to a block: as many as fill the query tiles; fewer where the SMs would not all get a unit (27 prompts of 10 to 31 tokens at
+// D = 256, 4 kv heads: 24.6 us with full blocks, whose CTAs walk several short runs one after the other)
+constexpr int FA_SMS = 148;
+static int tiles_per_block(int n_tiles, int n_kv, int G, int D) {
+  int n = (D > 128 ? 128 : 256) / (16 * G);
+  while (n > 1 && (long long)((n_tiles + n - 1) / n) * n_kv < FA_SMS) n = (n + 1) / 2;
+  return n;
+}
+
+template <int D, bool kCap, bool kSplit>
 static int launch_prefill(FaArgs a, cudaStream_t st) {
   using C = FaCfg<D>;
   B200Q_CHECK_ARG(a.G <= C::MAX_G, "prefill_attn: GQA group %d too large for D=%d (max %d)", a.G, D, C::MAX_G);
-  // as many q-tiles as fill the query tiles; fewer where the SMs would not all get a unit (27 prompts of 10 to 31 tokens at D = 256,
-  // 4 kv heads: 24.6 us with full blocks, whose CTAs walk several short runs one after the other)
-  a.per_block = C::NQ * 128 / (16 * a.G);
-  while (a.per_block > 1 && (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv < 148) a.per_block = (a.per_block + 1) / 2;
+  a.per_block = tiles_per_block(a.n_tiles, a.n_kv, a.G, D);
   CUtensorMap map;
   int rc = get_page_tmap(a.kv, D, &map);
   if (rc) return rc;
@@ -807,51 +856,130 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
     set_error("prefill_attn: no host-visible flag for bounded waits");
     return B200Q_ECUDA;
   }
-  auto kern = prefill_attn_kernel<D, kCap>;
+  auto kern = prefill_attn_kernel<D, kCap, kSplit>;
   static bool attr_set = false;
   if (!attr_set) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     attr_set = true;
   }
   const long long units = (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv;
-  const int grid = units < 148 ? (int)units : 148;
+  const int grid = units < FA_SMS ? (int)units : FA_SMS;
   kern<<<grid, FA_THREADS, C::SMEM, st>>>(map, a);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
 
-// The kernel above needs about 7 us for a run whatever its size (a chain of copies, products and waits), the kernel of 16-token tiles
-// (attn.cu) about 1 us per 16 keys.  What the host knows of the contexts is the width of the block table.  us, here / there:
-//   D = 128, 32 / 8 heads   18 x 256 tokens 40 / 71, 30 x 64-256 49 / 65, 8 x 100-380 26 / 40, 40 tokens behind 1500 33 / 47, one of 4400
-//                           198 / 778; but one of 200 10.9 / 8.4, 5 behind 300 12.2 / 11.5, 27 x 10-31 behind 42 21 / 11
-//   D = 64, 32 / 8 heads    one of 4400 186 / 533; but 30 x 64-256 42 / 38, one of 300 12.6 / 10.2, one of 512 18.9 / 18.1
-//   D = 256, 8 / 4 heads    one of 200 14.3 / 19.3, one of 300 17 / 27, 300 behind 900 33 / 99; but 27 x 10-31 behind 42 19.5 / 11.5
-// B200Q_BATCH_INVARIANT=1: always the kernel of 16-token tiles, where a row's sums follow from its own sequence; here they depend on how
-// the tiles of all portions are cut into blocks.
-static bool tensor_memory_pays(int n_kv, int D, long long keys, int n_tiles) {
-  if (batch_invariant()) return false;
-  if (D == 64) return keys > 512;
-  if (D == 128) return keys > 512 || (keys > 128 && (long long)n_tiles * n_kv >= 512);
-  return keys > 128;
+// ---- which kernel -------------------------------------------------------------------------------
+// Times of both kernels from a step's portions, us.  The kernel of 16-token tiles (attn.cu): the tile with most pages, or all pages and
+// tiles over the SMs.  The kernel above: its longest unit, or all runs and steps over the SMs.  (The smaller of the two counts in part:
+// `less`.)  Fitted to 3300 measured pairs (1 to 200 portions of 2 to 3000 tokens, up to 2000 cached ones before them, groups of 1 to 8
+// heads; each kernel within 7 to 14 %): taking the faster one by these sums costs 0.2 to 0.8 % against always knowing it (at worst half as much again: 20 portions of 2 tokens
+// behind 1000, one head per group).  tiles / tensor
+// memory at D = 128, 32 / 8 heads: 36 x 128 tokens 50 / 33, 16 x 128 25 / 20, one of 512 25 / 23, one of 2000 191 / 56, 40 behind 1500
+// 48 / 35, but one of 200 9 / 12, 32 x 16 5 / 15, 200 x 8-40 42 / 82.
+struct PromptCosts {
+  double start, page, pages, pages_per_head, tile_per_head, less;
+  double fa_start, fa_run, fa_step, fa_less;
+};
+class PromptTimes {
+ public:
+  PromptTimes(int n_tiles, int n_q, int n_kv, int D, int window)
+      : c_(D == 64    ? PromptCosts{3.31, 0.33, 0.044, 0.041, 0.12, 0.74, 2.37, 3.67, 1.83, 0.42}
+           : D == 128 ? PromptCosts{3.85, 0.49, 0.049, 0.082, 0.33, 0.58, 2.74, 4.48, 2.16, 0.42}
+                      : PromptCosts{3.70, 1.19, 0.647, 0.081, 0.60, 0.44, 3.84, 6.17, 1.21, 0.47}),
+        n_kv_(n_kv),
+        G_(n_q / n_kv),
+        window_(window),
+        step_(D > 128 ? 64 : 128),
+        per_(tiles_per_block(n_tiles, n_kv, n_q / n_kv, D)) {}
+  void add(int n, int past) {
+    if (n <= 0) return;
+    const int t = (n + 15) / 16;
+    // pages of the first to the last tile, one more each, no more than the window holds
+    const long long a = (past + (n < 16 ? n : 16) + 15) / 16, b = a + t - 1, cap = window_ > 0 ? window_ / 16 + 2 : b;
+    const long long m = b < cap ? b : cap, below = m >= a ? m - a + 1 : 0;
+    pages_ += (double)(below * (a + m) / 2 + (t - below) * cap);
+    if (m > most_pages_) most_pages_ = m;
+    for (int at = 0; at < t;) {
+      const int block = (tile_ + at) / per_, left = per_ - (tile_ + at) % per_, len = left < t - at ? left : t - at;
+      const int begin = past + 16 * at, end = past + (16 * (at + len) < n ? 16 * (at + len) : n);
+      const int k0 = window_ > 0 && begin + 1 > window_ ? begin + 1 - window_ : 0;
+      const double us = c_.fa_run + c_.fa_step * ((end - k0 + step_ - 1) / step_);
+      unit_ = block == block_ ? unit_ + us : us;
+      block_ = block;
+      if (unit_ > longest_) longest_ = unit_;
+      all_ += us;
+      at += len;
+    }
+    tile_ += t;
+  }
+  double tiles_us() const {
+    return c_.start + both(c_.page * most_pages_,
+                           ((c_.pages + c_.pages_per_head * G_) * pages_ + c_.tile_per_head * G_ * tile_) * n_kv_ / FA_SMS, c_.less);
+  }
+  double tensor_us() const { return c_.fa_start + both(longest_, all_ * n_kv_ / FA_SMS, c_.fa_less); }
+
+ private:
+  static double both(double x, double y, double less) { return x > y ? x + less * y : y + less * x; }
+  PromptCosts c_;
+  int n_kv_, G_, window_, step_, per_, tile_ = 0, block_ = -1;
+  long long most_pages_ = 0;
+  double pages_ = 0, all_ = 0, unit_ = 0, longest_ = 0;
+};
+
+// keys from which a portion alone is faster above (us, tiles / tensor memory): D = 64 one of 512 tokens 18 / 19, D = 128 one of 300 14 / 15,
+// four of 300 28 / 23, D = 256 one of 128 12 / 12, one of 200 19 / 14
+static int long_portion(int D) { return D == 64 ? 512 : D == 128 ? 320 : 160; }
+
+// 0: the kernel of 16-token tiles, 1: the one above, 2: both, each for its portions (`long_keys` divides them).
+// desc: the portions as {.., tokens, cached tokens before them, ..}, or NULL where the caller does not know them.  Then n_seqs is how many
+// portions there are at most (0: unknown).  If that many like portions without cached tokens would go to the kernel above, they do (cached
+// tokens and longer portions favour it further, but for groups of one head).  If not, and they would go there behind what the block table
+// could hold, or as the few that it could hold, each portion is looked at on the GPU: the tile kernel's CTAs of long portions leave at
+// once, the kernel above passes over the short ones.  (About 2 us for the kernel that finds nothing to do.)
+// B200Q_BATCH_INVARIANT=1: always the tile kernel, where a row's sums follow from its own sequence; here they depend on how the tiles of
+// all portions are cut into blocks.
+static int g_route = -1;  // test hook: >= 0 forces one
+
+int prefill_attn_route(const int32_t* desc, int n_desc, int n_seqs, int n_tiles, int bt_stride, int n_q, int n_kv, int D, int window) {
+  if (g_route >= 0) return g_route;
+  if (batch_invariant() || n_tiles <= 0 || n_q / n_kv < 1) return 0;
+  auto tensor = [](const PromptTimes& t) { return t.tensor_us() < t.tiles_us(); };
+  if (desc) {
+    PromptTimes t(n_tiles, n_q, n_kv, D, window);
+    for (int i = 0; i < n_desc; ++i) t.add(desc[4 * i + 1], desc[4 * i + 2]);
+    return tensor(t) ? 1 : 0;
+  }
+  const long long width = bt_stride > 0 ? 16LL * bt_stride : 16;
+  const int many = n_seqs > 0 && n_seqs < n_tiles ? n_seqs : n_tiles;
+  auto even = [&](int k, bool cached) {  // the tiles in k like portions
+    PromptTimes t(n_tiles, n_q, n_kv, D, window);
+    for (int i = 0; i < k; ++i) {
+      const long long n = 16 * (n_tiles * (i + 1LL) / k - n_tiles * (long long)i / k);
+      t.add((int)n, cached && width > n ? (int)(width - n) : 0);
+    }
+    return tensor(t);
+  };
+  if (even(many, false)) return 1;
+  if (width < long_portion(D)) return 0;
+  // (a table four times as wide as the portions are on average holds other sequences too, or a few of the portions are long)
+  return even(many, true) || (width * many >= 64LL * n_tiles && even((int)((16LL * n_tiles + width - 1) / width), false)) ? 2 : 0;
 }
 
-}  // namespace b200q
-
-using namespace b200q;
-
-extern "C" {
-
-int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
-                          const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, float softcap,
-                          int window, void* stream) {
+int prefill_attn(int route, const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                 const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, float softcap, int window,
+                 cudaStream_t st) {
   B200Q_CHECK_ARG(n_tiles >= 0 && n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 8,
                   "prefill_attn: unsupported heads n_q=%d n_kv=%d (GQA group must be <= 8)", n_q, n_kv);
   B200Q_CHECK_ARG(block_size == 16 && (D == 64 || D == 128 || D == 256),
                   "prefill_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D, block_size);
   if (n_tiles == 0 || n_q == 0) return B200Q_OK;
-  cudaStream_t st = as_stream(stream);
-  if (!tensor_memory_pays(n_kv, D, 16LL * bt_stride, n_tiles))
-    return prefill_tiles(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, scale, softcap, window, st);
+  const int long_keys = route == 2 ? long_portion(D) : 0;
+  if (route != 1) {
+    const int rc = prefill_tiles(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, scale, softcap, window,
+                                 long_keys, st);
+    if (rc || route == 0) return rc;
+  }
   const float log2e = 1.4426950408889634f;
   FaArgs a{};
   a.q = (const bf16*)q;
@@ -866,6 +994,7 @@ int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv
   a.n_kv = n_kv;
   a.G = n_q / n_kv;
   a.window = window;
+  a.long_keys = long_keys;
   a.q_flip = scale < 0.f ? 0x80008000u : 0u;
   const float s = scale < 0.f ? -scale : scale;
   a.c0 = softcap > 0.f ? s / softcap : s * log2e;
@@ -873,16 +1002,54 @@ int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv
   if (!(a.c0 > 1e-37f)) a.c0 = a.c0 >= 0.f ? 1e-37f : a.c0;  // (0: all scores equal; times a hidden key's -inf it would be NaN)
   a.c1 = softcap * log2e;
   a.vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 && q_stride % 8 == 0;
-  const bool cap = softcap > 0.f;
-  if (D == 64) return cap ? launch_prefill<64, true>(a, st) : launch_prefill<64, false>(a, st);
-  if (D == 128) return cap ? launch_prefill<128, true>(a, st) : launch_prefill<128, false>(a, st);
-  return cap ? launch_prefill<256, true>(a, st) : launch_prefill<256, false>(a, st);
+  auto launch = [&](auto cap) {
+    constexpr bool c = decltype(cap)::value;
+    if (D == 64) return long_keys ? launch_prefill<64, c, true>(a, st) : launch_prefill<64, c, false>(a, st);
+    if (D == 128) return long_keys ? launch_prefill<128, c, true>(a, st) : launch_prefill<128, c, false>(a, st);
+    return long_keys ? launch_prefill<256, c, true>(a, st) : launch_prefill<256, c, false>(a, st);
+  };
+  return softcap > 0.f ? launch(std::true_type{}) : launch(std::false_type{});
+}
+
+}  // namespace b200q
+
+using namespace b200q;
+
+extern "C" {
+
+int b200q_prefill_attn_seqs(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                            int n_seqs, const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale,
+                            float softcap, int window, void* stream) {
+  const int route = n_kv > 0 && n_q >= n_kv ? prefill_attn_route(nullptr, 0, n_seqs, n_tiles, bt_stride, n_q, n_kv, D, window) : 0;
+  return prefill_attn(route, q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, block_size, scale, softcap,
+                      window, as_stream(stream));
+}
+
+int b200q_prefill_attn_ex(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                          const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, float softcap,
+                          int window, void* stream) {
+  return b200q_prefill_attn_seqs(q, q_stride, out, kv_layer, block_table, bt_stride, 0, tiles, n_tiles, n_q, n_kv, D, block_size, scale,
+                                 softcap, window, stream);
 }
 
 int b200q_prefill_attn(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
                        const int32_t* tiles, int n_tiles, int n_q, int n_kv, int D, int block_size, float scale, void* stream) {
-  return b200q_prefill_attn_ex(q, q_stride, out, kv_layer, block_table, bt_stride, tiles, n_tiles, n_q, n_kv, D, block_size, scale, 0.f,
-                               0, stream);
+  return b200q_prefill_attn_seqs(q, q_stride, out, kv_layer, block_table, bt_stride, 0, tiles, n_tiles, n_q, n_kv, D, block_size, scale,
+                                 0.f, 0, stream);
+}
+
+// test hooks: one route for all calls (-1: choose)
+int b200q_prefill_attn_set_route(int route) {
+  B200Q_CHECK_ARG(route >= -1 && route <= 2, "prefill route must be -1..2");
+  g_route = route;
+  bump_tuning_epoch();
+  return B200Q_OK;
+}
+
+// the route of a step (prefill_attn_route; desc is host memory, [n_desc][4], or NULL)
+int b200q_prefill_attn_route(const int32_t* desc, int n_desc, int n_seqs, int n_tiles, int bt_stride, int n_q, int n_kv, int D,
+                             int window) {
+  return prefill_attn_route(desc, n_desc, n_seqs, n_tiles, bt_stride, n_q, n_kv, D, window);
 }
 
 }  // extern "C"

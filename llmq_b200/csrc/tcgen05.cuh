@@ -124,6 +124,17 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// ---- q-tiles of prompt attention: {block table row, first row, rows, first position} -----------
+// keys that the last token of tile i's portion sees (a whole warp asks; neighbouring tiles of one sequence that continue each other are a
+// portion), as far as 31 tiles on: exact for a comparison with up to 512
+__device__ __forceinline__ int portion_keys(const int4* tiles, int n_tiles, int i, int lane) {
+  const int4 t = __ldg(tiles + min(i + lane, n_tiles - 1));
+  const int n = min(max(t.z, 0), 16);
+  const int x = __shfl_up_sync(0xffffffffu, t.x, 1), y = __shfl_up_sync(0xffffffffu, t.y + n, 1), w = __shfl_up_sync(0xffffffffu, t.w + n, 1);
+  const uint32_t ends = __ballot_sync(0xffffffffu, lane > 0 && (i + lane >= n_tiles || x != t.x || y != t.y || w != t.w));
+  return __shfl_sync(0xffffffffu, t.w + n, ends ? __ffs(ends) - 2 : 31);
+}
+
 // ---- thread-block clusters ------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -203,9 +214,9 @@ int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUte
 // [two groups of 8 rows][64-column slices][8 rows][128 bytes]; coordinates {0, 0, 0, page * 2}.
 int get_page_tmap(const void* kv, int D, CUtensorMap* out);
 
-// prompt portions over short contexts (attn.cu)
+// prompt portions over short contexts (attn.cu); long_keys > 0: portions of so many keys and more are left out
 int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
-                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, cudaStream_t st);
+                  int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, int long_keys, cudaStream_t st);
 
 // products of up to 128 rows (gemm_skinny.cu)
 bool gemm_skinny_ok(int M, int N, int K, bool gated);

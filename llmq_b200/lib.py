@@ -224,6 +224,9 @@ SIGNATURES = {
     "b200q_gemma_norm_add_norm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _f, _vp]),
     "b200q_decode_attn_ex": (_i, [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _vp]),
     "b200q_prefill_attn_ex": (_i, [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _vp]),
+    "b200q_prefill_attn_seqs": (_i, [_vp, _i, _vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _vp]),
+    "b200q_prefill_attn_set_route": (_i, [_i]),
+    "b200q_prefill_attn_route": (_i, [_vp, _i, _i, _i, _i, _i, _i, _i, _i]),
     "b200q_gemm_geglu_bf16": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "b200q_softcap_bf16": (_i, [_vp, _i64, _f, _vp]),
     # layered architectures
@@ -477,14 +480,9 @@ def decode_attn(qkv, out, kv_layer, block_table, ctx_lens, n_q, n_kv, D, block_s
 
 def prefill_attn(qkv, out, kv_layer, block_table, tiles, n_q, n_kv, D, block_size, scale, stream=None,
                  softcap: float = 0.0, window: int = 0):
-    if softcap or window:
-        check(load().b200q_prefill_attn_ex(_p(qkv), qkv.shape[1], _p(out), _p(kv_layer), _p(block_table),
-                                           block_table.shape[1], _p(tiles), tiles.shape[0], n_q, n_kv, D,
-                                           block_size, scale, softcap, window, _stream(stream)))
-        return
-    check(load().b200q_prefill_attn(_p(qkv), qkv.shape[1], _p(out), _p(kv_layer), _p(block_table),
-                                    block_table.shape[1], _p(tiles), tiles.shape[0], n_q, n_kv, D,
-                                    block_size, scale, _stream(stream)))
+    check(load().b200q_prefill_attn_seqs(_p(qkv), qkv.shape[1], _p(out), _p(kv_layer), _p(block_table),
+                                         block_table.shape[1], block_table.shape[0], _p(tiles), tiles.shape[0], n_q, n_kv, D,
+                                         block_size, scale, softcap, window, _stream(stream)))
 
 
 def embed_scaled(ids, table, out, scale, stream=None):

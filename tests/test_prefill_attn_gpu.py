@@ -48,11 +48,12 @@ def reference(q, k, v, pos, scale, cap, window):
     return torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hide[None], -math.inf), -1), vv)
 
 
-def check(cuda, D, n_q, n_kv, portions, scale=None, cap=0.0, window=0, pad=0, order=None, seed=1, wide=True):
-    """portions: (cached tokens, tokens of this step) per sequence"""
+def check(cuda, D, n_q, n_kv, portions, scale=None, cap=0.0, window=0, pad=0, order=None, seed=1, wide=True, more_rows=0, routes=None):
+    """portions: (cached tokens, tokens of this step) per sequence; more_rows: of other sequences in the block table"""
     from llmq_b200 import lib
     scale = D ** -0.5 if scale is None else scale
     kv, bt, rows = make_cache([a + n for a, n in portions], n_kv, D, seed, wide)
+    bt = torch.cat([bt, torch.zeros(more_rows, bt.shape[1], dtype=torch.int32)])
     T = sum(n for _, n in portions)
     g = torch.Generator().manual_seed(seed + 50)
     qkv = torch.randn(T, (n_q + 2 * n_kv) * D + pad, generator=g).to(BF)
@@ -63,18 +64,27 @@ def check(cuda, D, n_q, n_kv, portions, scale=None, cap=0.0, window=0, pad=0, or
     if order is not None:
         tiles = order(tiles)
     t = torch.tensor(tiles, dtype=torch.int32, device=cuda)
-    out = torch.full((T + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
-    lib.prefill_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), t, n_q, n_kv, D, BS, scale, softcap=cap, window=window)
-    got = out.cpu()
-    assert torch.isnan(got[T].float()).all(), "rows behind the last one stay as they were"
-    assert lib.load().b200q_wait_failures() == 0
-    row = 0
+    refs, row = [], 0
     for i, (a, n) in enumerate(portions):
         q = qkv[row: row + n, : n_q * D].view(n, n_q, D)
-        ref = reference(q, *rows[i], torch.arange(a, a + n), scale, cap, window).to(BF)
-        # probabilities are rounded to bf16 before the value product: 2^-9 each, outputs agree to ~5e-3 or 2 ulps
-        bf16_close(got[row: row + n].view(n, n_q, D), ref, ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"portion {i} ({a} + {n})")
+        refs.append(reference(q, *rows[i], torch.arange(a, a + n), scale, cap, window).to(BF))
         row += n
+    for route in routes or ((-1, 1) if wide else (-1,)):   # the one that is chosen, and the tensor-memory kernel
+        out = torch.full((T + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
+        lib.check(lib.load().b200q_prefill_attn_set_route(route))
+        try:
+            lib.prefill_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), t, n_q, n_kv, D, BS, scale, softcap=cap, window=window)
+        finally:
+            lib.check(lib.load().b200q_prefill_attn_set_route(-1))
+        got = out.cpu()
+        assert torch.isnan(got[T].float()).all(), "rows behind the last one stay as they were"
+        assert lib.load().b200q_wait_failures() == 0
+        row = 0
+        for i, (a, n) in enumerate(portions):
+            # probabilities are rounded to bf16 before the value product: 2^-9 each, outputs agree to ~5e-3 or 2 ulps
+            bf16_close(got[row: row + n].view(n, n_q, D), refs[i], ulps=2.0, atol=5e-3, max_mismatch_frac=0.6,
+                       what=f"portion {i} ({a} + {n}) route {route}")
+            row += n
 
 
 MIX = [(0, 128), (0, 5), (16, 16), (100, 37), (3, 49), (0, 1), (0, 64), (250, 70), (0, 257), (127, 2), (0, 300)]
@@ -128,7 +138,9 @@ def step(cuda, D, n_q, n_kv, portions, seed, scale, cap=0.0, window=0, wide=True
 
     def call():
         out = torch.empty(T, n_q * D, dtype=BF, device=cuda)
+        lib.check(lib.load().b200q_prefill_attn_set_route(1))
         lib.prefill_attn(dev[0], out, dev[1], dev[2], dev[3], n_q, n_kv, D, BS, scale, softcap=cap, window=window)
+        lib.check(lib.load().b200q_prefill_attn_set_route(-1))
         return out.cpu()
     return call
 
@@ -166,8 +178,10 @@ def test_values_that_are_not_finite_stay_with_those_who_see_them(cuda, D, n_q, n
         tiles += [[i, row + j, min(16, n - j), a + j] for j in range(0, n, 16)]
         row += n
     out = torch.full((T + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
+    lib.check(lib.load().b200q_prefill_attn_set_route(1))   # (the kernel of 16-token tiles passes on what its own 16 tokens see)
     lib.prefill_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), torch.tensor(tiles, dtype=torch.int32, device=cuda), n_q, n_kv, D, BS,
                      D ** -0.5, softcap=cap, window=window)
+    lib.check(lib.load().b200q_prefill_attn_set_route(-1))
     got, row = out.cpu(), 0
     assert torch.isnan(got[T].float()).all() and lib.load().b200q_wait_failures() == 0
     for i, (a, n) in enumerate(portions):
@@ -181,3 +195,22 @@ def test_values_that_are_not_finite_stay_with_those_who_see_them(cuda, D, n_q, n
         assert not torch.isfinite(mine[touched].float()).any()
         bf16_close(torch.where(touched, ref.to(BF), mine), ref.to(BF), ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"portion {i}")
         row += n
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 8, 2), (128, 8, 2), (128, 2, 2), (128, 8, 1), (256, 4, 2), (256, 3, 3)])
+@pytest.mark.parametrize("cap,window", [(0.0, 0), (20.0, 150)])
+@pytest.mark.parametrize("order", ["listed", "turned", "shuffled"])
+def test_portions_shared_by_both_kernels(cuda, D, n_q, n_kv, cap, window, order):
+    """where the table says nothing about the portions, each is looked at on the GPU.  Portions at the edge of what counts as
+    long (160, 320, 512 keys), longer than the 32 tiles that are looked at, and short ones between them"""
+    g = torch.Generator().manual_seed(4)
+    turn = {"listed": None, "turned": lambda t: t[::-1], "shuffled": lambda t: [t[i] for i in torch.randperm(len(t), generator=g).tolist()]}
+    portions = [(0, 159), (0, 160), (0, 161), (300, 19), (300, 20), (0, 511), (480, 32), (480, 33), (0, 7), (0, 700), (900, 2), (0, 30),
+                (0, 31), (3, 1100), (0, 16), (511, 1)]
+    check(cuda, D, n_q, n_kv, portions, cap=cap, window=window, order=turn[order], seed=17, more_rows=300, routes=(2,))
+
+
+def test_only_short_and_only_long_portions_of_a_wide_table(cuda):
+    for D in (64, 128, 256):
+        check(cuda, D, 8, 4, [(0, n) for n in (5, 16, 31, 40)] * 6, more_rows=300, seed=2, routes=(-1, 2))
+        check(cuda, D, 8, 4, [(0, 600), (1000, 40), (0, 900)], more_rows=300, seed=3, routes=(-1, 2))
