@@ -87,7 +87,7 @@ int b200q_decode_attn(const void* q_dev, int q_stride, void* out_dev, const void
                       int n_seqs, int n_q, int n_kv, int D, int block_size, float scale,
                       void* stream);
 
-/* K6  paged causal prefill attention over q-tiles of <=16 consecutive tokens of one sequence.
+/* K6  paged causal prefill attention over q-tiles of <=16 consecutive tokens of one sequence (bounded waits: b200q_wait_failures).
  *     tiles: int32[n_tiles][4] = {block_table_row, first_batch_row, n_rows, first_position}.
  *     (replaces flashinfer trtllm_batch_context_with_kv_cache, vllm flashinfer.py:1665) */
 int b200q_prefill_attn(const void* q_dev, int q_stride, void* out_dev, const void* kv_layer_dev,
@@ -96,7 +96,8 @@ int b200q_prefill_attn(const void* q_dev, int q_stride, void* out_dev, const voi
                        void* stream);
 
 /* K3/K8/K9/K11/K12  C[M,N] = A[M,K] * W[N,K]^T, bf16 in, fp32 accumulate in TMEM (tcgen05),
- *     bf16 out.  A, W, C row-major and contiguous; K % 64 == 0, N % 64 == 0.
+ *     bf16 out.  A, W, C row-major and contiguous; K % 64 == 0, N % 64 == 0.  Waits inside the kernel are bounded
+ *     (b200q_wait_failures).
  *     (replaces F.linear -> cuBLASLt, vllm/model_executor/layers/utils.py:92-98) */
 int b200q_gemm_bf16(const void* A_dev, const void* W_dev, void* C_dev,
                     int M, int N, int K, void* stream);
@@ -639,8 +640,9 @@ int b200q_sandwich_close(float* x_dev, const void* y_dev, int y_f32, int splits,
  * + eps) * w in the model dtype */
 int b200q_pass_begin(float* x_dev, const float* x0_dev, const float* step_dev, float* keep_dev, const float* w_dev,
                      void* out_dev, int T, int W, float eps, int dtype, void* stream);
-/* nonzero once a kernel's bounded wait has run out in this process (its outputs are then missing); engine steps report
- * it as B200Q_ECUDA */
+/* nonzero once a kernel's bounded wait has run out in this process (its outputs are then missing or wrong); engine steps report
+ * it as B200Q_ECUDA.  Calls return before their kernels run: who calls b200q_gemm_* (up to 128 rows), b200q_prefill_attn* or the
+ * layered attention directly asks here once the stream has been waited for. */
 int b200q_wait_failures(void);
 
 /* ------------------------------------------------------------------------------------

@@ -24,10 +24,19 @@ struct SkinnyArgs {
   float* parts;  // != NULL: the fp32 partial tiles go here ([splits][M][N]) and the caller adds them
   const float* bias;
   int* failed;
-  long long ldc;
+  long long ldc, patience;  // patience: cycles that the product warp waits for a stage
   float limit;
   int M, N, K, mp, stages, a_bytes, cols, chunk;  // mp: M padded to 16; chunk: columns (rows of A) per exchange
 };
+
+// After a wait ran out, before the block's memory is given back: what the first thread asked for has come, and what was issued has been
+// made (`done` is committed behind the last product in any case)
+__device__ __noinline__ void skinny_end_copies(uint64_t* full, uint64_t* done, int asked, int stages) {
+  if (threadIdx.x == 0)
+    for (int i = asked > stages ? asked - stages : 0; i < asked; ++i) mbar_wait_limited(full + i % stages, (uint32_t)(i / stages) & 1u);
+  mbar_wait_limited(done, 0);
+  __syncthreads();
+}
 
 // WT: 128-row weight tiles per CTA
 template <int WT, int kAct>
@@ -39,6 +48,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], done;
   __shared__ uint32_t tmem_slot;
+  __shared__ int dead;  // a wait ran out: the other roles stop as well
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int split = blockIdx.x, splits = gridDim.x, tile = blockIdx.y;
   const int kb_all = a.K / SK_BK, kb0 = split * kb_all / splits, kb1 = (split + 1) * kb_all / splits;
@@ -53,12 +63,14 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     }
     mbar_init(&done, 1);
     mbar_fence_init();
+    dead = 0;
   }
   if (warp == 1) tmem_alloc(&tmem_slot, a.cols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  int asked = 0;  // (of the fetching thread) stages asked for
 
   if (warp == 0) {
     if (lane == 0) {
@@ -67,8 +79,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
       // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
       // (short reductions keep the order that the kernels for larger steps add in)
       int kb = kb0 + (kb1 - kb0 >= 16 ? tile * 5 % (kb1 - kb0) : 0);
-      for (int i = kb0; i < kb1; ++i, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
-        if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, a.failed)) break;
+      for (; asked < kb1 - kb0; ++asked, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
+        if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, &dead, a.failed)) break;
         uint8_t* sw = smem + stage * stage_bytes;
         mbar_expect_tx(full + stage, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
         tma_load_2d(sw, &tmap_w, kb * SK_BK, tile * NT, full + stage);
@@ -85,7 +97,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     int stage = 0;
     uint32_t phase = 0;
     for (int i = kb0; i < kb1; ++i) {
-      if (!__all_sync(0xffffffffu, mbar_wait_or_fail(full + stage, phase, a.failed))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait_or_fail(full + stage, phase, &dead, a.failed, a.patience))) break;
       tc_fence_after();
       if (elect_one()) {
         const uint32_t sw = smem_u32(smem + stage * stage_bytes), sa = sw + WT * SK_TILE_BYTES;
@@ -113,10 +125,12 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   const bool epi = warp >= 2;
   const int quarter = warp & 3, row = quarter * 32 + lane;
   if (epi) {
-    mbar_wait_or_fail(&done, 0, a.failed);
+    mbar_wait_or_fail(&done, 0, &dead, a.failed);
     __syncwarp();
     tc_fence_after();
   }
+  // (products that stop early say so before `done`: copies may then still arrive in the ring, which is left alone)
+  const bool give = epi && *(volatile int*)&dead == 0;
   if (a.parts) {
     if (epi) {
       float* dst = a.parts + (long long)split * a.M * a.N + (long long)tile * NT + row;
@@ -134,7 +148,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     }
   } else {
     for (int c0 = 0; c0 < a.M; c0 += a.chunk) {
-      if (epi) {
+      if (give) {
         const int cn = min(a.chunk, a.mp - c0);
 #pragma unroll 1
         for (int h = 0; h < WT; ++h)
@@ -204,6 +218,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   }
   tc_fence_before();
   __syncthreads();
+  if (dead) skinny_end_copies(full, &done, asked, a.stages);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, a.cols);
@@ -238,6 +253,8 @@ static int resident_clusters(int splits) {
   }
   return n;
 }
+
+bool g_gemm_give_up = false;  // test hook: the product warp's first wait counts as run out
 
 struct SkinnyPlan {
   bool alone;
@@ -339,6 +356,7 @@ int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int 
   a.bias = bias;
   a.limit = limit;
   a.ldc = ldc;
+  a.patience = g_gemm_give_up ? -1 : WAIT_CYCLES;
   a.M = M;
   a.N = N;
   a.K = K;
@@ -349,3 +367,16 @@ int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int 
 }
 
 }  // namespace b200q
+
+using namespace b200q;
+
+extern "C" {
+
+// test hook: 1 = products of up to 128 rows give up at their first wait (wrong values, and b200q_wait_failures() says so), 0 = normal
+int b200q_gemm_set_give_up(int on) {
+  g_gemm_give_up = on != 0;
+  bump_tuning_epoch();
+  return B200Q_OK;
+}
+
+}  // extern "C"

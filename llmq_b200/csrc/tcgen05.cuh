@@ -116,10 +116,23 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       : "memory");
 }
 
-// wait with a limit: false when it ran out, and then *failed is set (the engine reports it)
-__device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, int* failed) {
-  if (mbar_try_wait(bar, parity)) return true;
-  if (mbar_wait_limited(bar, parity)) return true;
+// wait with a limit: false when it ran out, or once another role of the CTA has given up (*dead); then *failed is set, which the engine
+// and b200q_wait_failures report.  A limit below 0 counts as run out at once.  The flag and the clock are looked at after EVERY
+// tries (a try suspends the thread for a while by itself).
+constexpr long long WAIT_CYCLES = 4000000000ll;  // about two seconds
+template <int EVERY = 1>
+__device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* dead, int* failed,
+                                                  long long limit = WAIT_CYCLES) {
+  if (limit >= 0) {
+    if (EVERY == 1 && mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (int n = 1;; ++n) {
+      if (mbar_try_wait(bar, parity)) return true;
+      if (n % EVERY == 0 && (*dead || clock64() - t0 > limit)) break;
+    }
+  }
+  *dead = 1;
+  __threadfence_block();
   *(volatile int*)failed = 1;
   return false;
 }

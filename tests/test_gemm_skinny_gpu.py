@@ -67,3 +67,35 @@ def test_gated(cuda, M, N, K, act):
     tol = 3 * 2.0 ** -7 * ref.abs() + 2.0 ** -7 * (g * slope * u).abs().reshape(M, -1) + 2e-5
     off = (got - ref).abs()
     assert torch.isfinite(got).all() and (off <= tol).all(), f"{act} {M} x {N} x {K}: {float((off / tol).max())}"
+
+
+def give_up():
+    """in a process of its own (the flag stays set): every product gives up at its first wait with copies of the ring in flight, and the
+    next ones are right"""
+    from llmq_b200 import lib
+    L, dev = lib.load(), torch.device("cuda")
+    shapes = [(1, 128, 1024), (17, 512, 4096), (64, 2048, 8192), (100, 4096, 14336), (128, 2048, 8192), (100, 38144, 4096)]
+    for M, N, K in shapes:
+        a, w = rnd(dev, M, K, seed=M), rnd(dev, N, K, seed=N + K, scale=K ** -0.5)
+        c, ref = torch.zeros(M, N, dtype=BF, device=dev), (a.double() @ w.double().t()).to(BF)
+        L.b200q_gemm_set_give_up(1)
+        for _ in range(20):
+            lib.gemm_bf16(a, w, c)
+            if N % 256 == 0:
+                lib.gemm_swiglu_bf16(a, w, torch.empty(M, N // 2, dtype=BF, device=dev))
+        torch.cuda.synchronize()
+        assert L.b200q_wait_failures() != 0
+        L.b200q_gemm_set_give_up(0)
+        lib.gemm_bf16(a, w, c)
+        bf16_close(c.cpu(), ref.cpu(), ulps=1.0, atol=2e-5, what=f"{M} x {N} x {K}")
+    print("right again")
+
+
+def test_waits_that_run_out(cuda):
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", "from tests.test_gemm_skinny_gpu import give_up; give_up()"], cwd=root, capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "right again" in r.stdout, r.stdout + r.stderr
