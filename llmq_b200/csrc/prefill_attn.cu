@@ -161,14 +161,11 @@ __device__ __forceinline__ float fa_rcp(float x) {
   return y;
 }
 
-// One query row of one head once more, by a whole warp: columns [c_out, c_out + OC) over the keys lo .. pos and no others.  In the
-// products of the kernel below a hidden key's probability is 0 and times a value that is not finite that is NaN, for every row of the
-// query tile that shares the step; such rows come here (a tile's row that sees the value itself comes here too, and gets what it sees).
-template <int D, int OC, bool kCap>
-__device__ __noinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, const bf16* q_row, bf16* out_row, int kvh, int lo, int pos,
-                                          int c_out) {
+// One query row of one head once more, by a whole warp, over the keys lo .. pos and no others
+template <int D, bool kCap>
+__device__ __forceinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, const bf16* q_row, bf16* out_row, int kvh, int lo, int pos) {
   const int lane = threadIdx.x & 31;
-  constexpr int NW = OC / 64;  // 32-bit words of the output per lane
+  constexpr int NW = D / 64;  // 32-bit words of the output per lane
   const long long page_bytes = 16 * D * 2;
   const uint32_t* q4 = reinterpret_cast<const uint32_t*>(q_row);
   float m = -INFINITY, l = 0.f, acc[NW][2];
@@ -218,7 +215,7 @@ __device__ __noinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, co
       const uint8_t* row = a.kv + (((long long)bi * 2 + 1) * a.n_kv + kvh) * page_bytes + ti * (D * 2);
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        const int word = c_out / 2 + w * 32 + lane;
+        const int word = w * 32 + lane;
         const uint32_t v = *reinterpret_cast<const uint32_t*>(row + (((word >> 2) ^ (ti & 7)) << 4) + (word & 3) * 4);
         acc[w][0] = fmaf(pi, bf16_lo(v), acc[w][0]);
         acc[w][1] = fmaf(pi, bf16_hi(v), acc[w][1]);
@@ -230,7 +227,39 @@ __device__ __noinline__ void fa_row_again(const FaArgs& a, const int32_t* bt, co
   const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
   for (int w = 0; w < NW; ++w)
-    reinterpret_cast<uint32_t*>(out_row + c_out)[w * 32 + lane] = pack_bf16x2(acc[w][0] * inv, acc[w][1] * inv);
+    reinterpret_cast<uint32_t*>(out_row)[w * 32 + lane] = pack_bf16x2(acc[w][0] * inv, acc[w][1] * inv);
+}
+
+// The rows of this CTA's units whose outputs are NaN, once more, by its softmax warps behind their loops.  In the products of the kernel
+// below a hidden key's probability is 0, and times a value that is not finite that is NaN, for every row of the query tile that shares the
+// step.  (A row that sees such a value itself comes here too, and gets what it sees.)
+template <int D, bool kCap, bool kSplit>
+__device__ __noinline__ void fa_rows_again(const FaArgs& a, const FaOrder order) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (FaUnit w; w.u < order.units; w.step()) {
+    const int kvh = w.u % a.n_kv, first = order.block(w.u / a.n_kv) * a.per_block, count = min(a.per_block, a.n_tiles - first);
+    int keys = 0;
+    if constexpr (kSplit) keys = block_portion_keys(a, first, lane);
+    for (int i = 0; i < count; ++i) {
+      const int4 t = __ldg(a.tiles + first + i);
+      if (kSplit && __shfl_sync(0xffffffffu, keys, i) < a.long_keys) continue;
+      const int rows = min(max(t.z, 0), 16) * a.G;
+      for (int f = warp; f < rows; f += 8) {
+        const int tok = f / a.G, head = kvh * a.G + f - tok * a.G, pos = t.w + tok;
+        bf16* out_row = a.out + (long long)(t.y + tok) * a.n_q * D + (long long)head * D;
+        bool nan = false;
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) {
+          const uint32_t v = reinterpret_cast<const uint32_t*>(out_row)[c * 32 + lane];
+          nan |= bf16_lo(v) != bf16_lo(v) || bf16_hi(v) != bf16_hi(v);
+        }
+        if (__any_sync(0xffffffffu, nan))
+          fa_row_again<D, kCap>(a, a.block_table + (long long)t.x * a.bt_stride,
+                                a.q + (long long)(t.y + tok) * a.q_stride + (long long)head * D, out_row, kvh,
+                                a.window > 0 ? pos + 1 - a.window : 0, pos);
+      }
+    }
+  }
 }
 
 // kSplit: only the portions of long_keys keys and more (a variant of its own: the code to look at them costs the other one 1 to 2 % in
@@ -248,7 +277,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
   uint8_t* patches = v_s + STG * C::T_BYTES;
   __shared__ float part[2][2][NQ == 1 ? 128 : 1];  // D = 256: maxima / sums of a row's two halves, in turns
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ int dead, redo;  // a wait ran out; some output is NaN although its row's sum is finite
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   __shared__ uint16_t sorted[FA_SORTED];
   int* steps_in = reinterpret_cast<int*>(patches);  // (free until the first rows leave)
@@ -265,7 +294,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     if (!__syncthreads_or(any)) return;
   }
   if (threadIdx.x == 0) {
-    dead = 0;
+    dead = redo = 0;
     for (int s = 0; s < STG; ++s) {
       mbar_init(k_full + s, 1);
       mbar_init(k_empty + s, 1);
@@ -771,7 +800,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
         constexpr int PC = C::PATCH / 8;  // 16-byte chunks per row
         const uint32_t patch = smem_u32(patches + warp * (32 * C::PATCH * 2));
         const int w0 = (warp & 3) * 32;
-        float check = 0.f;  // NaN once a column of the row is not finite
+        __nv_bfloat162 check = __float2bfloat162_rn(0.f);  // NaN once a column of the row is not finite
 #pragma unroll 1
         for (int c = 0; c < OC; c += C::PATCH) {
 #pragma unroll
@@ -780,13 +809,13 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
             tmem_ld32(o_at + (uint32_t)(c + 32 * h), o);
             tmem_ld_wait();
 #pragma unroll
-            for (int y = 0; y < 32; ++y) check = fmaf(__uint_as_float(o[y]), 0.f, check);
-#pragma unroll
             for (int y = 0; y < 4; ++y) {
               uint32_t w[4];
 #pragma unroll
-              for (int z = 0; z < 4; ++z)
+              for (int z = 0; z < 4; ++z) {
                 w[z] = pack_bf16x2(__uint_as_float(o[8 * y + 2 * z]) * inv, __uint_as_float(o[8 * y + 2 * z + 1]) * inv);
+                check = __hfma2(*reinterpret_cast<__nv_bfloat162*>(&w[z]), __float2bfloat162_rn(0.f), check);
+              }
               const int k = 4 * h + y, sw = PC == 8 ? k ^ (lane & 7) : k ^ ((lane >> 1) & 3);
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch + lane * (PC * 16) + sw * 16), "r"(w[0]), "r"(w[1]),
                            "r"(w[2]), "r"(w[3])
@@ -816,18 +845,12 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
           __syncwarp();
         }
         // (a sum that is not finite comes from the scores, which are the row's own)
-        uint32_t again = __ballot_sync(0xffffffffu, check != check && l < INFINITY && i_tile * 128 + row < rows);
-        while (again) {
-          const int g = i_tile * 128 + w0 + __ffs(again) - 1, t = (int)((uint32_t)g * a.inv_g >> 16), head = kvh * a.G + g - t * a.G;
-          again &= again - 1;
-          fa_row_again<D, OC, kCap>(a, a.block_table + (long long)r.bt_row * a.bt_stride,
-                                    a.q + (long long)(r.row0 + t) * a.q_stride + (long long)head * D,
-                                    a.out + (long long)(r.row0 + t) * a.n_q * D + (long long)head * D, kvh,
-                                    a.window > 0 ? r.pos0 + t + 1 - a.window : 0, r.pos0 + t, c_out);
-        }
+        if ((__hisnan(check.x) || __hisnan(check.y)) && l < INFINITY && i_tile * 128 + row < rows) redo = 1;
         tc_fence_before();
       }
     }
+    both();  // (every row of the CTA has left)
+    if (*(volatile int*)&redo) fa_rows_again<D, kCap, kSplit>(a, order);
   }
   __syncthreads();
   if (dead) {  // (copies in flight end before the block's memory is given back)
