@@ -487,13 +487,13 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t
   out[3] = c3;
 }
 
-// -log(-log u), u = (n + 1/2) / 2^24 with n = the upper 24 bits.  n + 1/2 takes 25 bits from 2^23 on and would round (to u = 1 for the
-// largest n, whose noise is 17.3 and not infinite); 1 - u takes 24 there, so that log u is formed from it.
+// -log(-log u), u = (n + 1/2) / 2^24 with n = the upper 24 bits.  n + 1/2 takes 25 bits from 2^23 on and rounds half a step up or down (to
+// u = 1 for the largest n, whose noise is 17.3 and not infinite): what was rounded off, d = +-2^-25, comes back as log u = log u' + d / u',
+// 1 / u' = 2 - u' being near enough (off by 1.5e-8 of 0.69 at u' = 1/2).  Below 2^23, d = 0.
 __device__ __forceinline__ float gumbel_from_bits(uint32_t x) {
-  const uint32_t n = x >> 8;
-  const float log_u = n < 0x800000u ? logf(((float)n + 0.5f) * (1.0f / 16777216.0f))
-                                    : log1pf(((float)(0xffffffu - n) + 0.5f) * (-1.0f / 16777216.0f));
-  return -logf(-log_u);
+  const float n = (float)(x >> 8), n5 = n + 0.5f, u = n5 * (1.0f / 16777216.0f);
+  const float d = ((n - n5) + 0.5f) * (1.0f / 16777216.0f);
+  return -logf(-fmaf(d, 2.f - u, logf(u)));
 }
 
 // A cluster of gridDim.x CTAs shares a row (a row per CTA left most SMs idle or one deep: 60 us for 128 rows of 128256 logits, 33 so).
