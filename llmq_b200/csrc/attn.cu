@@ -818,46 +818,6 @@ static inline ScoreConsts score_consts(float scale, float softcap) {
 
 int g_decode_variant = 0;  // test hook: 0 = auto, 1 = split kernel (v1), 2 = streaming kernel
 
-// How many CTAs share a sequence (and kv head): as many as keep two CTAs on every SM busy, but no fewer than four pages per warp of the
-// longest context that the block table could hold (shorter ones gain nothing: an exchange costs about 2 us).  6 sequences of 3000 to
-// 8100 tokens, D = 64, 8 kv heads: 22 us, 65 with one CTA each.  B200Q_BATCH_INVARIANT=1: always one, whatever the batch.
-static int decode_splits(int n_seqs, int n_kv, int bt_stride) {
-  if (batch_invariant() || g_decode_variant == 1) return 1;
-  const long long ctas = (long long)n_seqs * n_kv;
-  int splits = 1;
-  while (splits < 8 && ctas * (splits + 1) <= 296 && bt_stride / (DEC_WARPS * (splits + 1)) >= 4) ++splits;
-  return splits;
-}
-
-template <int D, int BS, bool kCap, bool kShared>
-static int launch_decode_form(int splits, const void* q, int q_stride, void* out, const void* kv,
-                         const int32_t* bt, int bt_stride, const int32_t* ctx, int n_seqs, int n_q,
-                         int n_kv, float scale, float softcap, int window, cudaStream_t st) {
-  using S_ = DecSmem<D, BS>;
-  auto kern = decode_attn_kernel<D, BS, kCap, kShared>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
-    attr_set = true;
-  }
-  const ScoreConsts sc = score_consts(scale, softcap);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
-  cfg.blockDim = dim3(DEC_WARPS * 32);
-  cfg.dynamicSmemBytes = S_::TOTAL;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = kShared ? 1 : 0;
-  B200Q_CUDA(cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
-                                n_q / n_kv, sc.c0, sc.c1, window));
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
-}
-
 static int attn_num_sms() {
   static int n = 0;
   if (n == 0) {
@@ -869,10 +829,112 @@ static int attn_num_sms() {
   return n;
 }
 
+template <int D, int BS, bool kCap, bool kShared>
+static int prepare_decode() {
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200Q_CUDA(cudaFuncSetAttribute(decode_attn_kernel<D, BS, kCap, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    DecSmem<D, BS>::TOTAL));
+    attr_set = true;
+  }
+  return B200Q_OK;
+}
+
+template <int D, int BS, bool kShared>
+static cudaLaunchConfig_t decode_config(int splits, int n_seqs, int n_kv, cudaLaunchAttribute* attr, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
+  cfg.blockDim = dim3(DEC_WARPS * 32);
+  cfg.dynamicSmemBytes = DecSmem<D, BS>::TOTAL;
+  cfg.stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = splits;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = kShared ? 1 : 0;
+  return cfg;
+}
+
+// how many clusters of `splits` CTAs are resident at once (asked for once per size)
+template <int D, int BS, bool kCap>
+static int decode_resident(int splits) {
+  static int known[9];
+  int& n = known[splits];
+  if (n == 0) {
+    int v = 0;
+    cudaError_t e;
+    if (splits == 1) {
+      e = prepare_decode<D, BS, kCap, false>()
+              ? cudaErrorUnknown
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, decode_attn_kernel<D, BS, kCap, false>, DEC_WARPS * 32,
+                                                              DecSmem<D, BS>::TOTAL);
+      v *= attn_num_sms();
+    } else {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t cfg = decode_config<D, BS, true>(splits, attn_num_sms(), 1, &attr, nullptr);
+      e = prepare_decode<D, BS, kCap, true>() ? cudaErrorUnknown
+                                              : cudaOccupancyMaxActiveClusters(&v, decode_attn_kernel<D, BS, kCap, true>, &cfg);
+    }
+    if (e != cudaSuccess || v <= 0) {
+      cudaGetLastError();
+      v = 1;
+    }
+    n = v;
+  }
+  return n;
+}
+
+// How many CTAs share a sequence (and kv head): the number with the least time by what bounds each: rounds of resident clusters x (a
+// round's start and end, and the chain of a warp's pages, a little longer where several CTAs share an SM), or the bytes, and the
+// exchange.  Clusters lie within a processing cluster of the chip, so fewer fit than CTAs would (444, 296 and 148 of them at D = 64, 128,
+// 256; 384, 240 and 120 in threes), and a second round for the last of them costs more than sharing gives: 12 sequences of 700 tokens,
+// 8 kv heads, D = 256: 14 us with one CTA each, 26 with three, which 296 CTAs had been thought to have room for.  No fewer than four
+// pages per warp.  The contexts are taken to fill the block table.  Fitted to 1800 sizes (1 to 90 sequences of 256 to 8000 tokens), 1 to
+// 2.5 % slower than the best number of CTAs on average; against one CTA each 0.78 of the time, nowhere more than 1.09.  6 sequences of
+// 3000 to 8100 tokens, D = 64, 8 kv heads: 22 us, 65 with one CTA each.  B200Q_BATCH_INVARIANT=1: always one, whatever the batch.
+template <int D, int BS, bool kCap>
+static int decode_splits(int n_seqs, int n_kv, int bt_stride, int window) {
+  if (batch_invariant() || g_decode_variant == 1) return 1;
+  constexpr double ROUND = D > 128 ? 4 : 8, PAGE = D > 128 ? 0.83 : D > 64 ? 0.58 : 0.5, SHARE = D > 128 ? 2 : D > 64 ? 3 : 1.5;
+  const long long n = (long long)n_seqs * n_kv;
+  const int sms = attn_num_sms(), per_sm = decode_resident<D, BS, kCap>(1) / sms;
+  const int pages = window > 0 && (window + 15) / 16 + 1 < bt_stride ? (window + 15) / 16 + 1 : bt_stride;
+  int best = 1;
+  double least = 0;
+  for (int s = 1; s <= 8 && (s == 1 || pages >= 4 * DEC_WARPS * s); ++s) {
+    const long long resident = decode_resident<D, BS, kCap>(s), rounds = (n + resident - 1) / resident, deep = (n * s + sms - 1) / sms;
+    const double chain = (pages + DEC_WARPS * s - 1) / (DEC_WARPS * s) * PAGE * (1 + 0.15 * ((deep < per_sm ? deep : per_sm) - 1));
+    const double bytes_us = (double)n * pages * (2 * BS * D * 2) / 9e6;
+    const double work = rounds * (ROUND + chain);
+    const double t = 2 + (work > bytes_us ? work : bytes_us) + (s > 1 ? SHARE + (s & (s - 1) ? 0.5 : 0) : 0);
+    if (s == 1 || t < 0.97 * least) {
+      least = t;
+      best = s;
+    }
+  }
+  return best;
+}
+
+template <int D, int BS, bool kCap, bool kShared>
+static int launch_decode_form(int splits, const void* q, int q_stride, void* out, const void* kv,
+                         const int32_t* bt, int bt_stride, const int32_t* ctx, int n_seqs, int n_q,
+                         int n_kv, float scale, float softcap, int window, cudaStream_t st) {
+  auto kern = decode_attn_kernel<D, BS, kCap, kShared>;
+  const int rc = prepare_decode<D, BS, kCap, kShared>();
+  if (rc) return rc;
+  const ScoreConsts sc = score_consts(scale, softcap);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = decode_config<D, BS, kShared>(splits, n_seqs, n_kv, &attr, st);
+  B200Q_CUDA(cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
+                                n_q / n_kv, sc.c0, sc.c1, window));
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
 template <int D, int BS, bool kCap>
 static int launch_decode(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* ctx,
                          int n_seqs, int n_q, int n_kv, float scale, float softcap, int window, cudaStream_t st) {
-  const int splits = decode_splits(n_seqs, n_kv, bt_stride);
+  const int splits = decode_splits<D, BS, kCap>(n_seqs, n_kv, bt_stride, window);
   if (splits > 1)
     return launch_decode_form<D, BS, kCap, true>(splits, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap,
                                                  window, st);
