@@ -334,12 +334,28 @@ static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_
 // two for every SM (and for gated units, which need both halves).
 static bool wide_tiles(int N) { return N % 256 == 0 && N / 256 >= 148; }
 
-// Which products the kernel above takes.  With 113 to 128 rows and tiles enough for most SMs the persistent kernel of
-// gemm_tcgen05.cu is as good or better, because its next tile's loads run during a tile's end (128256 x 4096: 180.7 us there,
-// 184.7 here; 178 here against 180 at 100 rows).
+// Which products the kernel above takes; us, here / kernels of gemm_tcgen05.cu:
+//   * plain, K < 1024: few k-blocks leave no splits to share out the end of a tile, and the narrower tiles there are done sooner: K = 512
+//     5 / 4.5 at one row, 7.7 / 4.6 at 128, K = 64 6.1 / 3.2, for all N up to 8192; K = 768 even at 16 rows; 24576 x 512 8.8 / 9.4 at 32.
+//   * plain, up to 64 tiles of 128, so that at least two CTAs work on each: always (1024 x 1024 6-9 / 6.5-8.6, 2048 x 2048 6-9 / 8-10,
+//     5120 x 4096 0.7 of the time there).
+//   * plain, more tiles, a CTA to each: the longer the reduction, the less the start and the end of a tile count, which the persistent
+//     kernels hide.  Share of the time there, 12288 columns: K = 2048 0.99 at 16 rows, 1.07 at 48, 1.31 at 128; K = 4096 0.98 at 80, 1.06
+//     at 128; K = 8192 1.02 at 100; two CTAs per SM hide some of it: 24576 x 2048 0.97 at 64 rows, 1.08 at 128.
+//   * plain, tiles of 256 (vocabulary sizes): up to 32 rows (128256 x 2048 86 / 88); up to 112 where K >= 4096 and the tiles fill rounds
+//     of two CTAs per SM (128256 x 4096 177 / 179 at 100 rows, 1.7 rounds; but 50176 x 5120 98 / 89, 0.66).
+//   * gated: below 128 rows always: the kernels there spend 15 to 20 us on the division of rows that do not exist (28672 x 4096 54 / 73 at
+//     113, 2048 x 512 6 / 40 at one row).  At 128: 16384 x 2048 24 / 28, but 28672 x 3584 51 / 49, 2048 x 512 16 / 15.
 bool gemm_skinny_ok(int M, int N, int K, bool gated) {
   if (M < 1 || M > 128 || K % SK_BK != 0 || N % (gated ? 256 : 128) != 0 || N / 128 > 65535) return false;
-  return M <= 112 || (gated ? N / 256 <= 74 : !wide_tiles(N));
+  if (gated) return M < 128 || (K >= 1024 && N / 256 <= 74);
+  if (wide_tiles(N)) {
+    const int tiles = N / 256, rounds = (tiles + 295) / 296;
+    return M <= 32 || (M <= 112 && K >= 4096 && 5 * tiles >= 4 * 296 * rounds);
+  }
+  const int tiles = N / 128;
+  if (K < 1024) return M <= (tiles > 148 ? 32 : K >= 768 ? 16 : 0);
+  return M <= (tiles <= 64 ? 128 : K >= 8192 ? 112 : K >= 4096 ? 80 : tiles > 148 ? 64 : 16);
 }
 
 int gemm_skinny_splits(int M, int N, int K) {

@@ -63,6 +63,9 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
                                               const float* gate_bias = nullptr, float limit = 0.f) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;  // gated epilogue: tile = [gate (BN/2) | up (BN/2)]
   constexpr int OUT_BN = kSwiGLU ? BN / 2 : BN;
+  // (no row of this warp exists: its accumulators are sums of zeros, which the gated units' division treats as a special case: 384 rows
+  // x 2048 x 512 gated 29 us, 15 without)
+  if (row0 >= M) return;
   const uint32_t patch_s = smem_u32(patch);
 #pragma unroll 1
   for (int c0 = 0; c0 < OUT_BN; c0 += 64) {

@@ -69,6 +69,31 @@ def test_gated(cuda, M, N, K, act):
     assert torch.isfinite(got).all() and (off <= tol).all(), f"{act} {M} x {N} x {K}: {float((off / tol).max())}"
 
 
+@pytest.mark.parametrize("M", [1, 17, 33, 65, 113, 127, 128])
+@pytest.mark.parametrize("N,K", [(128, 1024), (384, 1088), (256, 768), (512, 512), (8320, 4096), (19072, 768), (37760, 1024), (38144, 1024),
+                                 (65536, 4096)])
+def test_plain_at_the_edges_of_the_choice(cuda, M, N, K):
+    test_plain(cuda, M, N, K)
+
+
+@pytest.mark.parametrize("act", ["swiglu", "clamped_bias"])
+@pytest.mark.parametrize("M,N,K", [(113, 28672, 256), (127, 19456, 128), (128, 16384, 1024), (128, 512, 512)])
+def test_gated_at_the_edges_of_the_choice(cuda, M, N, K, act):
+    test_gated(cuda, M, N, K, act)
+
+
+@pytest.mark.parametrize("M", [129, 161, 257, 384, 640])
+@pytest.mark.parametrize("N,K", [(2048, 512), (512, 64)])
+def test_warps_without_rows(cuda, M, N, K):
+    """more than 128 rows, the last tile's warps partly or all without any: rows behind the last one stay as they were"""
+    test_plain(cuda, M, N, K)
+    test_gated(cuda, M, N, K, "swiglu")
+    from llmq_b200 import lib
+    c = torch.full((M + 130, N // 2), 7.0, dtype=BF, device=cuda)
+    lib.gemm_swiglu_bf16(rnd(cuda, M, K, seed=M), rnd(cuda, N, K, seed=N + K, scale=1.5 * K ** -0.5), c[:M])
+    assert (c[M:] == 7.0).all()
+
+
 def give_up():
     """in a process of its own (the flag stays set): every product gives up at its first wait with copies of the ring in flight, and the
     next ones are right"""
