@@ -963,10 +963,12 @@ static int long_portion(int D) { return D == 64 ? 512 : D == 128 ? 320 : 160; }
 
 // 0: the kernel of 16-token tiles, 1: the one above, 2: both, each for its portions (`long_keys` divides them).
 // desc: the portions as {.., tokens, cached tokens before them, ..}, or NULL where the caller does not know them.  Then n_seqs is how many
-// portions there are at most (0: unknown).  If that many like portions without cached tokens would go to the kernel above, they do (cached
-// tokens and longer portions favour it further, but for groups of one head).  If not, and they would go there behind what the block table
-// could hold, or as the few that it could hold, each portion is looked at on the GPU: the tile kernel's CTAs of long portions leave at
-// once, the kernel above passes over the short ones.  (About 2 us for the kernel that finds nothing to do.)
+// portions there are at most (0: unknown), and three steps are looked at: that many like portions without cached tokens (if they go to the
+// kernel above, longer contexts do), as many behind what the block table could hold, and as few as it could hold.  If only the second or
+// third would go there: where little is lost if that is wrong, the portions are taken to be as long as the table is wide (a second launch
+// costs 2 to 4 us: 40 tokens behind 1500 35 us, 39 with it; 16 tokens of a table of 2048 that are all there is take 9 instead of 4);
+// otherwise each portion is looked at on the GPU: the tile kernel's CTAs of long portions leave at once, the kernel above passes over the
+// short ones (200 x 8-40 tokens, a table of 2048: 47 us, 82 above, 42 with a table of 64).
 // B200Q_BATCH_INVARIANT=1: always the tile kernel, where a row's sums follow from its own sequence; here they depend on how the tiles of
 // all portions are cut into blocks.
 static int g_route = -1;  // test hook: >= 0 forces one
@@ -988,12 +990,15 @@ int prefill_attn_route(const int32_t* desc, int n_desc, int n_seqs, int n_tiles,
       const long long n = 16 * (n_tiles * (i + 1LL) / k - n_tiles * (long long)i / k);
       t.add((int)n, cached && width > n ? (int)(width - n) : 0);
     }
-    return tensor(t);
+    return t;
   };
-  if (even(many, false)) return 1;
-  if (width < long_portion(D)) return 0;
+  const PromptTimes none = even(many, false);
+  if (tensor(none)) return 1;
+  if (2 * width < 3 * long_portion(D)) return 0;  // (near the line there is nothing to gain)
+  const bool full = tensor(even(many, true));
   // (a table four times as wide as the portions are on average holds other sequences too, or a few of the portions are long)
-  return even(many, true) || (width * many >= 64LL * n_tiles && even((int)((16LL * n_tiles + width - 1) / width), false)) ? 2 : 0;
+  if (!full && !(width * many >= 64LL * n_tiles && tensor(even((int)((16LL * n_tiles + width - 1) / width), false)))) return 0;
+  return full && none.tensor_us() < none.tiles_us() + 6 ? 1 : 2;
 }
 
 int prefill_attn(int route, const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,

@@ -44,6 +44,8 @@ def test_tiles_alone():
         assert route(D, n_seqs=3, n_tiles=240, columns=128) == 1          # at least 1280 tokens each on average
         assert route(D, n_seqs=200, n_tiles=300, columns=4) == 0
         assert route(D, n_seqs=500, n_tiles=300, columns=512) == 2
+        assert route(D, n_seqs=1, n_tiles=3, columns=96) == 1             # 40 tokens behind 1500
+    assert route(64, n_seqs=1, n_tiles=3, columns=32) == 0                # ... behind 400
     assert route(128, n_seqs=36, n_tiles=288, columns=8) == 1             # 36 prompts of 128 tokens
     assert route(128, n_seqs=0, n_tiles=0) == 0
 
