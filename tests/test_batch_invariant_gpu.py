@@ -1,6 +1,6 @@
 """B200Q_BATCH_INVARIANT=1: bit for bit, what a request gives does not depend on its batch-mates: prompt attention beside a long
 sequence (which makes the block table wide) and cut into blocks elsewhere, single tokens among enough others for the streaming kernel,
-products at every range of rows.  The variable is read once, so the checks run in a process of their own."""
+products at every range of rows, an engine's tokens beside a long sequence.  The variable is read once, so the checks run in a process of their own."""
 import os
 import subprocess
 import sys
@@ -11,7 +11,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("what", ["prompts", "tokens", "products"])
+@pytest.mark.parametrize("what", ["prompts", "tokens", "products", "engine"])
 def test_same_bits_whatever_the_batch(cuda, what):
     env = dict(os.environ, B200Q_BATCH_INVARIANT="1", PYTHONPATH=ROOT + os.pathsep + os.environ.get("PYTHONPATH", ""))
     r = subprocess.run([sys.executable, os.path.abspath(__file__), what], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
@@ -70,6 +70,37 @@ def tokens():
         assert torch.equal(run(0, 20, bt.shape[1]), full[:20])
 
 
+def engine():
+    """short prompts admitted beside a running sequence of 900 tokens and alone: the same tokens"""
+    import dataclasses
+
+    from llmq_b200.model import Engine
+    from tests.test_model_gpu import TINY, build
+    from tests.test_model_gpu import prompts as make
+    dims = dataclasses.replace(TINY["d128"], max_pos=1024)
+    model, _, _ = build(dims, max_tokens=1024)
+    reqs = make(dims.vocab, [900, 30, 7, 130, 64, 16, 250], seed=3)
+
+    def run(which):
+        eng = Engine(model, max_num_seqs=8, max_num_batched_tokens=1024, eos_token_id=None)
+        outs = {i: [] for i in which}
+        eng.add_request(which[0], reqs[which[0]], 20 + 10 * (which[0] == 0), ignore_eos=True)
+        for i in which[1:]:
+            ids, toks, _ = eng.step()
+            for r, t in zip(ids.tolist(), toks.tolist()):
+                outs[r].append(t)
+            eng.add_request(i, reqs[i], 20, ignore_eos=True)
+        while eng.has_work():
+            ids, toks, _ = eng.step()
+            for r, t in zip(ids.tolist(), toks.tolist()):
+                outs[r].append(t)
+        eng.close()
+        return outs
+    together = run(list(range(7)))
+    for i in range(7):
+        assert run([i])[i] == together[i], i
+
+
 def products():
     import torch
     from llmq_b200 import lib
@@ -89,5 +120,5 @@ def products():
 
 
 if __name__ == "__main__":
-    {"prompts": prompts, "tokens": tokens, "products": products}[sys.argv[1]]()
+    {"prompts": prompts, "tokens": tokens, "products": products, "engine": engine}[sys.argv[1]]()
     print("equal")
