@@ -1,12 +1,12 @@
 #!/usr/bin/env python
-"""bench.py — headline benchmark of the b200 worker's hot path (BASELINE.json metric).
+"""bench.py — headline benchmark of the b200 worker's hot path.
 
   python bench.py --gpus N --steps K --warmup W            # native arm
   python bench.py --impl reference --gpus N --steps K --warmup W   # CPU reference arm
 
-Workload (BASELINE.json `metric`): Llama-3-8B, random-init bf16, 128 prompt tokens in / 128
+Workload: Llama-3-8B, random-init bf16, 128 prompt tokens in / 128
 generated tokens out, queue-sharded data parallel — one worker process per GPU, job i of the
-canonical seeded job stream goes to rank i % N, no data-path collective (SURVEY.md §8e).
+canonical seeded job stream goes to rank i % N, no data-path collective.
 
 The engine runs in steady state: `--max-num-seqs` (4608) sequences in flight and a backlog behind
 them that never empties — the situation of a worker on a 100k-prompt queue.  A *step* is `--jobs`
@@ -47,7 +47,7 @@ UNIT = "tokens/s"
 
 
 def ensure_llmq_importable():
-    """the reference package (pip --target baseline/_ref, see DESIGN.md) + the aio_pika/semhash
+    """the reference package (pip --target baseline/_ref) + the aio_pika/semhash
     stand-ins this image lacks (tests/shims) — needed to instantiate the real BaseWorker slot"""
     try:
         import aio_pika  # noqa: F401
@@ -85,8 +85,7 @@ def ncu_traffic():
     the newest committed `ncu --set full` capture under profiles/, or None"""
     import csv
 
-    for fname, kernel in (("r2_ncu_full_targets.csv", "gemm2_bf16_kernel<256, 1>"),
-                          ("r1_ncu_full_targets.csv", "gemm_bf16_kernel<256, 1>")):
+    for fname, kernel in (("r2_ncu_full_targets.csv", "gemm2_bf16_kernel<256, 1>"),):
         try:
             rows = list(csv.reader(open(os.path.join(ROOT, "profiles", fname))))
             hdr, units = rows[0], rows[1]
@@ -830,7 +829,7 @@ def main():
     ap.add_argument("--impl", default="native", choices=["native", "reference"])
     ap.add_argument("--model", default="llama-3-8b")
     # 4608 = 36 x 128 rows: with 148 SMs every projection's tile count is within 3 % of a whole
-    # number of rounds of the persistent GEMM loop (DESIGN.md §5); the KV pool holds them all
+    # number of rounds of the persistent GEMM loop; the KV pool holds them all
     ap.add_argument("--jobs", type=int, default=1152,
                     help="completed jobs per step per GPU (a quarter of the 4608 concurrent sequences)")
     ap.add_argument("--e2e-steps", type=int, default=8, help="the e2e arm times min(--steps, this) steps")

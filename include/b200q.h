@@ -46,7 +46,7 @@ int b200q_device_check(void);
 
 /* ------------------------------------------------------------------------------------
  * Op-level entry points (used by the parity tests and by b200q_model_forward).
- * Each replaces one op vLLM dispatches for the reference worker (SURVEY.md §2.1 K1-K13).
+ * Each replaces one op vLLM dispatches for the reference worker.
  * ---------------------------------------------------------------------------------- */
 
 /* K1  embedding gather: out[t,:] = table[ids[t],:]            (vLLM VocabParallelEmbedding) */
@@ -148,7 +148,7 @@ int b200q_argmax_bf16(const void* logits_dev, int32_t* ids_dev, int B, int V, vo
 int b200q_sample_bf16(const void* logits_dev, const int32_t* params_dev, int32_t* ids_dev,
                       int B, int V, void* stream);
 
-/* ---- Gemma-2 family (SURVEY.md §8 f1; vllm/model_executor/models/gemma2.py) ----------------- */
+/* ---- Gemma-2 family (vllm/model_executor/models/gemma2.py) ----------------- */
 
 /* embedding gather with the Gemma normaliser: out[t,:] = bf16(table[ids[t],:] * scale), scale =
  *     bf16(sqrt(H))                                                    (gemma2.py embed_tokens * normalizer) */

@@ -1,4 +1,4 @@
-// attn.cu — paged-KV attention for the b200 worker (SURVEY.md §2.1 K6, K7).
+// attn.cu — paged-KV attention for the b200 worker.
 //
 // KV cache layout (per layer):  [num_blocks][2 (K,V)][n_kv][BS tokens][D] bf16, i.e. one
 // contiguous "page" of BS*D*2 bytes per (block, K|V, kv-head).  Inside a token row the 16-byte
@@ -18,7 +18,7 @@
 //   warps (one per query head of the group) share a 4-stage page ring filled by a producer
 //   warp; causal masking by absolute position; K/V are read back from the paged cache, so
 //   chunked prefill over an existing context needs no special case.
-// Gemma-2 extras (SURVEY.md §8 f1), compiled as separate instantiations so the Llama kernels keep
+// Gemma-2 extras, compiled as separate instantiations so the Llama kernels keep
 // their code: kCap = attention-logit soft-capping (score <- cap * tanh(score * scale / cap)), and a
 // runtime sliding window (query at position p sees keys p - window < j <= p; pages that lie entirely
 // before the window are never fetched).  D = 256 (Gemma-2 head size) uses 2-stage rings.

@@ -1,7 +1,6 @@
 // elementwise.cu — the HBM-bound, coalesced, 16-byte-vectorised kernels of the hot path:
 // embedding gather (K1), RMSNorm / fused add+RMSNorm (K2), RoPE + paged KV write (K4+K5),
-// SwiGLU (K10), row gather and greedy argmax (K13).  See SURVEY.md §2.1 for the vLLM ops
-// these replace.  All rounding points follow the oracle (oracle/ops.py), which follows
+// SwiGLU (K10), row gather and greedy argmax (K13), in place of vLLM's ops.  All rounding points follow the oracle (oracle/ops.py), which follows
 // vLLM's native op definitions / HF transformers' Llama.
 #include <stdarg.h>
 
@@ -166,7 +165,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 }
 
 // ------------------------------------------------------------------------------------------
-// Gemma-2 norms (SURVEY.md §8 f1).  GemmaRMSNorm multiplies by (1 + w) and rounds ONCE:
+// Gemma-2 norms.  GemmaRMSNorm multiplies by (1 + w) and rounds ONCE:
 //   y = bf16( (x * rsqrt(mean(x^2) + eps)) * (1 + w) )      all in fp32 until the final cast.
 // gemma_norm_add_norm fuses the sandwich around a residual add (two row reductions, the row
 // stays in registers):  a = norm(x, w_post);  residual = bf16(residual + a);  x = norm(residual, w_next)

@@ -2,7 +2,7 @@
 // token batch, composed from the op-level kernels.  Replaces GPUModelRunner.execute_model for
 // LlamaForCausalLM behind the reference worker (vllm/model_executor/models/llama.py:316-333,
 // 395-431): same layer wiring and rounding points, B200-native kernels.
-// B200Q_ARCH_GEMMA2 (SURVEY.md §8 f1; vllm/model_executor/models/gemma2.py): same skeleton with
+// B200Q_ARCH_GEMMA2 (vllm/model_executor/models/gemma2.py): same skeleton with
 // scaled embeddings, (1+w) sandwich norms around both residual adds, soft-capped attention with
 // alternating sliding-window layers, GeGLU, tied LM head and final-logit soft-capping.
 #include <stdlib.h>

@@ -1,4 +1,4 @@
-"""Synthetic model directories, tokenizers and JSONL job files (SURVEY.md §7.1 step 1, §8d).
+"""Synthetic model directories, tokenizers and JSONL job files.
 
 No tokenizer, config or checkpoint exists on disk in the build/bench environment and there is no
 network, so both the native worker and the oracle harness run on locally synthesised assets:
@@ -8,7 +8,7 @@ network, so both the native worker and the oracle harness run on locally synthes
     usual ids when the vocabulary is large enough), whitespace pre-tokenisation, a BOS-prepending
     post-processor and a Llama-3-style chat template.  "w17 w4 w99" tokenises to exactly
     [BOS, 17, 4, 99] and decodes back to the same text, so prompt length is exact.
-  * config.json / generation_config.json with the real Llama dimensions (SURVEY.md App. E),
+  * config.json / generation_config.json with the real Llama dimensions,
   * optional seeded safetensors weights (Normal(0, 0.02), unit norms) for small models,
   * JSONL job files: {"id": "job-0000001", "prompt": "<127 random words>"}  => 128 prompt ids.
 """

@@ -51,7 +51,7 @@ class ModelSpec:
     # the first of them.  vLLM stops on tokenizer.eos_token_id plus all generation_config ids.
     eos_token_ids: Tuple[int, ...] = ()
     name: str = "llama"
-    # architecture: "llama" (Llama / Mistral-style decoders) or "gemma2" 
+    # architecture: "llama" (Llama / Mistral-style decoders) or "gemma2"
     arch: str = "llama"
     query_pre_attn_scalar: Optional[float] = None  # gemma2: attention scale = this ** -0.5
     attn_softcap: float = 0.0                      # gemma2: 50
@@ -155,7 +155,7 @@ class ModelSpec:
         return (self.n_q_heads + 2 * self.n_kv_heads) * self.head_dim
 
     def weight_bytes_per_step(self) -> int:
-        """bf16 bytes streamed per decode step: all layer matrices + LM head (SURVEY §8d)."""
+        """bf16 bytes streamed per decode step: all layer matrices + LM head."""
         per_layer = (self.qkv_dim * self.hidden + self.hidden * self.n_q_heads * self.head_dim
                      + 3 * self.intermediate * self.hidden)
         return 2 * (self.n_layers * per_layer + self.vocab * self.hidden)
@@ -164,7 +164,7 @@ class ModelSpec:
         return 2 * self.n_layers * self.n_kv_heads * self.head_dim * 2
 
 
-# Appendix E of SURVEY.md
+# published configurations
 LLAMA_3_8B = ModelSpec(hidden=4096, n_layers=32, n_q_heads=32, n_kv_heads=8, head_dim=128,
                        intermediate=14336, vocab=128256, rms_eps=1e-5, rope_theta=500000.0,
                        tie_embeddings=False, max_position_embeddings=8192, eos_token_id=128001,
@@ -176,7 +176,7 @@ LLAMA_32_1B = ModelSpec(hidden=2048, n_layers=16, n_q_heads=32, n_kv_heads=8, he
                                       "original_max_position_embeddings": 8192},
                         tie_embeddings=True, max_position_embeddings=131072, eos_token_id=128009,
                         bos_token_id=128000, name="llama-3.2-1b")
-# google/gemma-2-9b(-it) and Unbabel/Tower-Plus-9B (BASELINE configs #4, #5) share this shape
+# google/gemma-2-9b(-it) and Unbabel/Tower-Plus-9B share this shape
 GEMMA_2_9B = ModelSpec(hidden=3584, n_layers=42, n_q_heads=16, n_kv_heads=8, head_dim=256,
                        intermediate=14336, vocab=256000, rms_eps=1e-6, rope_theta=10000.0,
                        tie_embeddings=True, max_position_embeddings=8192, eos_token_id=1,

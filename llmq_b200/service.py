@@ -3,7 +3,7 @@
 Pure host logic with no llmq import, so it can be driven directly (bench.py, tests) exactly the
 way ``B200Worker._process_job`` drives it: ``future = service.submit(ids, ...); await future``.
 
-Threading model (SURVEY.md §8b): the asyncio event-loop thread owns AMQP, tokenisation and
+Threading model: the asyncio event-loop thread owns AMQP, tokenisation and
 futures; ONE engine thread owns the CUDA context and runs the continuous-batching step loop
 (`b200q_engine_step`, GIL released inside the C call).
 """
@@ -35,7 +35,7 @@ class _TokenTable:
     """Generated tokens of the live requests as one int32 matrix (row = request slot = the engine's
     request id), so that a step's (ids, tokens) arrays are stored with two vectorised numpy
     operations instead of a Python loop over the batch: with thousands of sequences per step that
-    loop sits between two GPU steps and idles the device (host fast path)."""
+    loop sits between two GPU steps and idles the device."""
 
     def __init__(self):
         import numpy as np

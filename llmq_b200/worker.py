@@ -5,7 +5,7 @@ four abstract methods (:57-75) with the same constructor signature, prompt const
 handling and error convention as the reference ``VLLMWorker`` (ref:llmq/workers/vllm_worker.py)
 — the job envelope, Result construction, publishing and acking stay in the untouched base class.
 
-Threading model (SURVEY.md §8b): the asyncio event-loop thread owns AMQP, tokenisation and
+Threading model: the asyncio event-loop thread owns AMQP, tokenisation and
 futures; ONE engine thread owns the CUDA context and runs the continuous-batching step loop
 (`b200q_engine_step`, GIL released inside the C call); ``_process_job`` is
 ``submit(request); await future``.
@@ -52,7 +52,7 @@ class B200Worker(BaseWorker):
     async def _initialize_processor(self) -> None:
         tp, dp = self.tensor_parallel_size or 1, self.data_parallel_size or 1
         if tp != 1 or dp != 1:
-            # the path shards by running one worker per GPU against the same queue (SURVEY §8e)
+            # the path shards by running one worker per GPU against the same queue
             raise ValueError(
                 f"b200 worker runs one replica per GPU (got -tp {tp} -dp {dp}); start one worker "
                 "per GPU with CUDA_VISIBLE_DEVICES=<i> instead")

@@ -1,5 +1,4 @@
-"""oracle/gemma2.py — CPU restatement of the Gemma-2 architecture (the next model
-family; BASELINE configs #4 Tower-Plus-9B and #5 Gemma-2-9B-it are Gemma-2-shaped).
+"""oracle/gemma2.py — CPU restatement of the Gemma-2 architecture.
 TEST INFRASTRUCTURE ONLY (see oracle/ops.py).  Parity target of the B200Q_ARCH_GEMMA2 path of
 libb200q (tests/test_gemma2_gpu.py); pinned against transformers' Gemma2ForCausalLM goldens
 (tests/test_oracle_golden.py).

@@ -133,7 +133,7 @@ class LlamaOracle:
 def random_llama_weights(dims: LlamaDims, seed: int = 1234, std: float = 0.02,
                          dtype=torch.bfloat16) -> Dict[str, torch.Tensor]:
     """Seeded synthetic checkpoint in HF naming: Normal(0, std) matrices, unit norm weights
-    (not vLLM's near-zero dummy init, which makes argmax tie-fragile)."""
+   ."""
     g = torch.Generator().manual_seed(seed)
 
     def mat(r, c):

@@ -16,7 +16,7 @@ needs_reference = pytest.mark.skipif(REFERENCE is None, reason="the reference ll
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a B200 (run with -m gpu under gpurun)")
+    config.addinivalue_line("markers", "gpu: needs a B200 (run with -m gpu)")
 
 
 @pytest.fixture(scope="session")

@@ -1,4 +1,4 @@
-"""Minimal in-process stand-in for the `aio_pika` surface llmq uses (SURVEY.md Appendix C).
+"""Minimal in-process stand-in for the `aio_pika` surface llmq uses.
 
 TEST / BENCH INFRASTRUCTURE ONLY.  This image has neither `aio_pika` nor a RabbitMQ server, so the
 reference's host code (ref:llmq/core/broker.py, ref:llmq/workers/base.py) is run unmodified on

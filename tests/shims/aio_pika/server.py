@@ -5,7 +5,7 @@ TEST / BENCH INFRASTRUCTURE ONLY — this image has no RabbitMQ; a deployment us
     python -m aio_pika.server --port 5673          (with tests/shims on PYTHONPATH)
     B200Q_SHIM_BROKER=127.0.0.1:5673  ...any llmq process using the stand-in...
 
-Semantics are those the reference relies on (SURVEY.md Appendix C): named queues on the default
+Semantics are those the reference relies on: named queues on the default
 exchange, per-channel prefetch window, round-robin between consumers, ack / reject(requeue),
 un-acked deliveries return to the queue when a connection drops, passive declare of a missing
 queue fails, purge.

@@ -1,5 +1,5 @@
 """placeholder for the optional `semhash` dependency, which ref:llmq/workers/__init__.py:5 imports
-unconditionally (semantic dedup worker — out of scope). TEST SHIM ONLY."""
+unconditionally (semantic dedup worker). TEST SHIM ONLY."""
 
 
 class SemHash:  # pragma: no cover

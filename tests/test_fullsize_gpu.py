@@ -1,4 +1,4 @@
-"""Size-independent properties at BASELINE.json's full model sizes (random-init Llama-3.2-1B and
+"""Size-independent properties at full model sizes (random-init Llama-3.2-1B and
 Llama-3-8B, 128-token prompts): the oracle cannot run these in seconds, so parity is carried by
 (a) the op/model tests on small shapes and (b) these invariants of the same code at full size:
 determinism, batch invariance (a request's tokens do not depend on its batch-mates), chunked
@@ -72,7 +72,7 @@ def test_fullsize_invariants(cuda, key):
 
 @pytest.mark.parametrize("key", ["llama-3-8b", "llama-3.2-1b"])
 def test_fullwidth_two_layer_logits_and_ids_match_the_oracle(cuda, key):
-    """the oracle comparison at BASELINE widths.  Two decoder layers with the
+    """The oracle comparison at full widths.  Two decoder layers with the
     REAL hidden / intermediate / head / vocab sizes (K = 4096 and 14336 accumulations, V = 128256
     argmax, llama3 rope scaling and tied head for the 1B) on a seeded checkpoint; the batch is the
     bench's shape — 36 prompts x 128 tokens = 4608 prefill rows in ONE step, which dispatches the

@@ -1,5 +1,4 @@
-"""GPU parity of the Gemma-2 path (BASELINE configs #4 Tower-Plus-9B and #5
-Gemma-2-9B-it are Gemma-2-shaped) through the C ABI: the new op-level entry points against
+"""GPU parity of the Gemma-2 path through the C ABI: the new op-level entry points against
 oracle/gemma2.py, the whole forward against the oracle AND against the committed transformers
 Gemma2ForCausalLM goldens (tests/golden/hf_gemma2_tiny.npz), and the engine's greedy decoding
 (sliding window crossed during decode, head_dim 256) against the oracle."""

@@ -1,4 +1,4 @@
-"""CPU-side checks of the Gemma-2 support (SURVEY.md §8 f1): config parsing, weight naming and
+"""CPU-side checks of the Gemma-2 support: config parsing, weight naming and
 fusion, the ctypes view of the extended model config."""
 import torch
 
@@ -10,7 +10,7 @@ def test_gemma2_builtin_spec_roundtrip():
     assert (r.arch, r.head_dim, r.sliding_window, r.attn_softcap, r.final_softcap, r.tie_embeddings) == \
         ("gemma2", 256, 4096, 50.0, 30.0, True)
     assert abs(r.attn_scale - 1 / 16) < 1e-9 and r.embed_scale == 59.75  # bf16(sqrt(3584))
-    # SURVEY §8(d)-style bookkeeping: bytes streamed per decode step, KV bytes per token
+    # bookkeeping: bytes streamed per decode step, KV bytes per token
     assert s.weight_bytes_per_step() == 2 * (42 * (8192 * 3584 + 3584 * 4096 + 3 * 14336 * 3584) + 256000 * 3584)
     assert s.kv_bytes_per_token() == 2 * 42 * 8 * 256 * 2
     assert BUILTIN_SPECS["llama-3-8b"].arch == "llama" and BUILTIN_SPECS["llama-3-8b"].embed_scale == 0.0

@@ -120,7 +120,7 @@ def test_chat_prompt_carries_double_bos_like_the_reference(patched):
     w.service = S.GenerationService(FakeEngine(), tok, 1)
     text = w.build_prompt(Job(id="c", messages=[{"role": "user", "content": "w5"}]))
     ids = tok(text, add_special_tokens=True).input_ids
-    assert ids[0] == ids[1] == tok.bos_token_id  # SURVEY.md Appendix D1
+    assert ids[0] == ids[1] == tok.bos_token_id
     assert w.stop_strings(Job(id="a", prompt="x")) is None
     assert w.stop_strings(Job(id="a", prompt="x", stop=[tok.eos_token])) is None  # inert special
     assert w.stop_strings(Job(id="a", prompt="x", stop=["END", tok.eos_token])) == ["END"]
@@ -152,7 +152,7 @@ def test_job_stream_is_sharding_invariant():
 
 
 def test_config1_dummy_worker_1k_jobs_through_broker(monkeypatch):
-    """BASELINE config #1: the reference's own DummyWorker (unmodified), 1k synthetic JSONL jobs
+    """The reference's own DummyWorker (unmodified), 1k synthetic JSONL jobs
     through the broker — plumbing only.  Its 1 s sleep per job is patched to 1 ms."""
     import llmq.workers.dummy_worker as DW
     aio_pika.reset_brokers()
@@ -353,7 +353,7 @@ def test_token_table_matches_a_dict_of_lists_model():
 
 
 def test_engine_failure_rejects_and_requeues_instead_of_dropping(patched, monkeypatch):
-    """SURVEY §8b error convention: only ValueError drops a job (ack).  A device / engine failure
+    """Error convention: only ValueError drops a job (ack).  A device / engine failure
     must surface as a non-ValueError from _process_job so that the reference's BaseWorker rejects
     the message with requeue=True (base.py:237-245) and another worker can pick it up; once the
     engine thread has died every later submit fails the same way (no silent hang)."""
@@ -402,7 +402,7 @@ def test_engine_failure_rejects_and_requeues_instead_of_dropping(patched, monkey
 
 
 def test_reference_quirks_are_replicated_not_fixed(patched):
-    """behaviours of the reference worker that a drop-in must keep.
+    """Behaviours of the reference worker that a drop-in must keep.
     D4 — a prompt is always passed through str.format (ref:llmq/core/models.py:46), so braces in a
     later pipeline stage's input (= the previous model's output) raise KeyError / IndexError
     (=> reject + requeue by the base class) or ValueError (=> dropped); D6 — chat jobs report the
@@ -425,7 +425,7 @@ def test_reference_quirks_are_replicated_not_fixed(patched):
 
 
 def test_absurd_max_tokens_fails_one_job_not_the_engine_thread(monkeypatch):
-    """a job carrying max_tokens=3e9 used to raise MemoryError while sizing its token-table
+    """A job carrying max_tokens=3e9 used to raise MemoryError while sizing its token-table
     row, inside the engine thread, which killed generation for every request.  It is clamped to
     the engine's max_model_len now, and any per-request admission failure surfaces as ValueError
     for that request only (=> ack/drop by the base class), the others complete."""
@@ -454,7 +454,7 @@ def test_absurd_max_tokens_fails_one_job_not_the_engine_thread(monkeypatch):
 
 
 def test_fatal_engine_error_resolves_queued_and_in_hand_requests(monkeypatch):
-    """when the engine thread dies, requests still in the inbox and the one being
+    """When the engine thread dies, requests still in the inbox and the one being
     admitted must get their futures resolved too (their AMQP messages would otherwise stay un-acked
     for ever), and the worker is told to stop consuming."""
     tok = build_tokenizer(VOCAB)
@@ -500,7 +500,7 @@ def test_worker_stops_consuming_when_the_engine_dies(patched):
 
 
 def test_stop_scanner_is_incremental_and_matches_whole_text_search():
-    """stop strings were found by re-decoding the whole output after every
+    """Stop strings were found by re-decoding the whole output after every
     token (O(n^2)).  _StopScanner decodes a bounded tail per token; on an 8192-token output (the
     reference's default VLLM_MAX_TOKENS) it must (a) find the same cut as a search of the full
     text, (b) call decode on short windows only."""
@@ -578,7 +578,7 @@ def test_detokenize_equals_vllms_prompt_primed_decode_stream():
 
 
 def test_every_eos_id_of_the_model_ends_generation(tmp_path):
-    """ADVICE r1: instruct models list several EOS ids (Llama-3.x-Instruct: 128001/128008/128009;
+    """Instruct models list several EOS ids (Llama-3.x-Instruct: 128001/128008/128009;
     gemma-2-it adds <end_of_turn> in generation_config.json); vLLM stops on all of them, so must
     the native engine — otherwise chat jobs run on to VLLM_MAX_TOKENS."""
     from llmq_b200.fixtures import DryRunEngine
@@ -611,7 +611,7 @@ def test_every_eos_id_of_the_model_ends_generation(tmp_path):
 
 
 def test_default_max_model_len_is_the_models_own(monkeypatch):
-    """with VLLM_MAX_MODEL_LEN unset the reference leaves the context length to vLLM
+    """With VLLM_MAX_MODEL_LEN unset the reference leaves the context length to vLLM
     (= max_position_embeddings), not 4096; prompts of 4096+ tokens on an 8k model must be served"""
     import llmq_b200.model as M
     seen = {}

@@ -1,7 +1,7 @@
 """The reference's CLI surface end to end across PROCESSES, CPU only: a TCP broker (the aio_pika
 stand-in's server), two `llmq worker dummy` processes (the reference's unmodified worker + CLI),
 `llmq submit` of a JSONL file and `llmq receive` of the results — queue-sharded data parallelism
-exactly as llmq deploys it (competing consumers on one queue, SURVEY.md §8e)."""
+exactly as llmq deploys it (competing consumers on one queue)."""
 import json
 import os
 import subprocess
@@ -69,7 +69,7 @@ def test_two_worker_processes_share_one_queue(tmp_path):
 
 @pytest.mark.skipif(REF is None, reason="reference llmq package not available")
 def test_queue_bench_tool_pipeline_mode_with_the_reference_dummy_worker(tmp_path):
-    """tools/queue_bench.py (the process-level harness of BASELINE configs #3-#5) in its two-stage pipeline
+    """tools/queue_bench.py (the process-level harness) in its two-stage pipeline
     mode, with the reference's own DummyWorker processes standing in for the GPU workers: broker process,
     `llmq worker pipeline CFG STAGE` processes, stage-1 results routed to stage 2 by the reference's
     publish_pipeline_result, final results counted from `pipeline.<name>.results`."""

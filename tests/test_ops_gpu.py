@@ -1,5 +1,5 @@
 """GPU parity of every op-level C-ABI entry point against the CPU oracle (oracle/ops.py).
-Run under gpurun:  python -m pytest tests -m gpu -x -q"""
+Run on a B200:  python -m pytest tests -m gpu -x -q"""
 import math
 
 import numpy as np

@@ -76,7 +76,7 @@ def test_rope_llama3_scaling_matches_vllm_formula():
 
 
 def test_gemma2_oracle_matches_hf_golden():
-    """SURVEY.md §8 f1 groundwork: the Gemma-2 restatement (soft-capping, sliding window, GeGLU,
+    """The Gemma-2 restatement (soft-capping, sliding window, GeGLU,
     (1+w) norms, post-norms, scaled tied embeddings) against transformers' Gemma2ForCausalLM"""
     from oracle.gemma2 import Gemma2Dims, Gemma2Oracle, random_gemma2_weights
     meta = json.load(open(os.path.join(G, "hf_gemma2_meta.json")))

@@ -1,5 +1,5 @@
 """Parity against the REAL reference engine: greedy token ids produced by vLLM 0.22.0 on a B200
-(tools/vllm_incumbent.py golden, temperature forced to 0 — SURVEY.md §8c) for seeded
+(tools/vllm_incumbent.py golden, temperature forced to 0) for seeded
 checkpoints that `llmq_b200.fixtures.seeded_state_dict` reproduces bit for bit.
 
 vLLM does not agree with itself bit for bit (its compiled and eager modes differ on 4 of the 12

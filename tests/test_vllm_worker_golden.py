@@ -1,10 +1,10 @@
-"""Parity against the reference's OWN worker at BASELINE widths.
+"""Parity against the reference's OWN worker at full widths.
 
 `tests/golden/vllm_worker_golden_<case>.json.gz` were produced on a B200 by
 `tools/oracle_vllm_worker.py golden`: the reference's `VLLMWorker` (ref:llmq/workers/vllm_worker.py:11,
 unmodified, vLLM 0.22.0) behind the unmodified `BaseWorker` / `BrokerManager`, instrumented only to
 decode greedily and to record token ids and the top-2 logprob margin of every decision.  Seeded
-random-init checkpoints with the REAL widths of the BASELINE models:
+random-init checkpoints with the REAL widths of the models:
   llama32_1b    Llama-3.2-1B, all 16 layers          llama3_8b_w4   Llama-3-8B widths, 4 layers
 76 jobs each (64 of the canonical 128-token benchmark stream + 12 ragged lengths), 128 new tokens,
 twice: as the reference configures vLLM (compiled, CUDA graphs) and with enforce_eager.
@@ -86,7 +86,7 @@ def check_divergences(ours, run, what):
 
 @pytest.mark.parametrize("case", CASES)
 def test_fixture_is_the_canonical_job_stream_and_our_tokenisation(case):
-    """the prompt ids vLLM's renderer produced for the reference worker's text prompt
+    """The prompt ids vLLM's renderer produced for the reference worker's text prompt
     (add_special_tokens=True: one BOS) are exactly what GenerationService.encode produces, and the
     text the reference worker returned is what GenerationService.detokenize makes of the same ids
     (vLLM's DecodeStream is primed with the prompt: the text is the CONTINUATION of the prompt, which

@@ -181,7 +181,7 @@ def test_b200_worker_end_to_end_from_gemma2_model_dir(cuda, tmp_path, monkeypatc
 
 
 def test_two_engines_back_to_back_in_one_process_get_the_same_kv_pool(cuda):
-    """VERDICT r1 weak #1 / ADVICE: `gpu_memory_utilization` sizes the KV pool from what the device
+    """`gpu_memory_utilization` sizes the KV pool from what the device
     has left; memory this process had freed to torch's caching allocator (the previous engine's
     pool) used to be counted as in use, so a second engine in the same process got 0 blocks.
     Building, closing and rebuilding at the same utilisation must give the same pool (± a few MB of
@@ -214,12 +214,11 @@ def test_two_engines_back_to_back_in_one_process_get_the_same_kv_pool(cuda):
 
 @needs_reference
 def test_two_stage_pipeline_on_the_gpu_with_braces_in_stage1_output(cuda, tmp_path, monkeypatch):
-    """config #4 (SURVEY §8 f2) with real model output: two B200Worker stages on the GPU, stage 1's
+    """config #4 with real model output: two B200Worker stages on the GPU, stage 1's
     text routed into stage 2's queue by the reference's unmodified `publish_pipeline_result`
     (ref:llmq/core/broker.py:145-193).  The reference formats every prompt with str.format
     (ref:llmq/core/models.py:46), so a stage-1 OUTPUT that contains a stray brace makes the stage-2
-    job un-formattable: ValueError => logged + acked/dropped (ref:llmq/workers/base.py:228-235,
-    SURVEY App. D4).  The quirk is replicated, not fixed: such jobs produce no final result, all
+    job un-formattable: ValueError => logged + acked/dropped (ref:llmq/workers/base.py:228-235).  The quirk is replicated, not fixed: such jobs produce no final result, all
     others produce exactly the greedy continuation of their stage-1 text."""
     import json
 

@@ -1,4 +1,4 @@
-"""Host-path ceiling of the b200 worker, measured WITHOUT a GPU (SURVEY.md §8 f4).
+"""Host-path ceiling of the b200 worker, measured WITHOUT a GPU.
 
 The C++ engine runs in its dry-run mode (real scheduler, real paged-KV bookkeeping and per-step
 metadata packing, fabricated tokens, no CUDA), so what is timed is everything the host does per

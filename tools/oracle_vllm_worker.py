@@ -1,11 +1,11 @@
-"""OracleVLLMWorker — the reference's own worker as the GPU oracle (SURVEY.md §8c, §7.1-2(ii)).
+"""OracleVLLMWorker — the reference's own worker as the GPU oracle.
 
 The reference worker (ref:llmq/workers/vllm_worker.py:11) is run UNMODIFIED on a B200 behind the
 unmodified `BaseWorker` / `BrokerManager` (on the aio_pika stand-in: the image has no RabbitMQ);
 this subclass only makes it usable as a parity oracle, without touching /root/reference:
 
   * :146 `await self.engine.get_tokenizer()` — vLLM >= 0.22 returns the tokenizer synchronously, so
-    the engine's `get_tokenizer` is wrapped into an awaitable (SURVEY fact #5);
+    the engine's `get_tokenizer` is wrapped into an awaitable;
   * :161-165 `SamplingParams(temperature=0.7, ...)` — the module-level name `SamplingParams` is
     replaced by a factory that forces `temperature=0.0` (greedy, the oracle mode) and asks for the
     top-2 logprobs of every generated token (their difference is the logit margin of that step,
@@ -18,7 +18,7 @@ this subclass only makes it usable as a parity oracle, without touching /root/re
   python tools/oracle_vllm_worker.py pack                   (here)
       -> tests/golden/vllm_worker_golden_<case>.json.gz     (committed fixtures)
 
-Cases are seeded random-init checkpoints with the REAL widths of the BASELINE models
+Cases are seeded random-init checkpoints with the REAL widths of the models
 (`llmq_b200.fixtures.seeded_state_dict` reproduces them bit for bit anywhere):
   llama3_8b_w4  : Llama-3-8B hidden/intermediate/heads/vocab, 4 of the 32 layers
   llama32_1b    : Llama-3.2-1B, all 16 layers (tied embeddings, llama3 rope scaling)

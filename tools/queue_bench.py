@@ -1,5 +1,4 @@
-"""Process-level benchmark with the reference's measurement shape (ref:performance_benchmark.py:193-394,
-BASELINE.md §2): a broker process, N worker PROCESSES started through the CLI (one per GPU), the
+"""Process-level benchmark with the reference's measurement shape (ref:performance_benchmark.py:193-394): a broker process, N worker PROCESSES started through the CLI (one per GPU), the
 queue pre-loaded with synthetic JSONL jobs, clock from first delivery to last result.
 
   config #3 (queue-sharded data parallel, ref:utils/run_llmq_benchmark.slurm:52-72):

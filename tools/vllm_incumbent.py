@@ -5,7 +5,7 @@ ref:llmq/workers/vllm_worker.py:105-123,161-186) — on the same B200, developme
                                             #   -> gpurun_out/vllm_golden_<name>.json (copied to tests/golden/)
   python tools/vllm_incumbent.py throughput # Llama-3-8B dims, dummy weights, 128-in/128-out
 
-Differences from the reference worker, all deliberate (SURVEY.md §8c): temperature is forced to 0
+Differences from the reference worker, all deliberate: temperature is forced to 0
 (the reference hard-codes 0.7 unseeded), prompts are passed as token ids (same ids the reference
 would get from tokenising the text), and the engine is the synchronous `LLM` front-end over the
 same EngineCore instead of `AsyncLLMEngine` behind an AMQP consumer.
