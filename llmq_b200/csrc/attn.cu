@@ -207,19 +207,19 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S_::RING_BYTES + S_::MERGE_FLOATS * 4) +
                    warp * DEC_STAGES;
 
-  const int ctx = __ldg(ctx_lens + seq);
-  // the query sits at position ctx-1 and sees keys [lo, ctx); pages before lo's page are skipped
-  const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
-  const int page0 = lo / BS;
-  const int n_pages = (ctx + BS - 1) / BS - page0;
-  const int my_n = n_pages > wg ? (n_pages - wg + n_warps - 1) / n_warps : 0;
-
   if (lane == 0) {
 #pragma unroll
     for (int s = 0; s < DEC_STAGES; ++s) mbar_init(bars + s, 1);
     mbar_fence_init();
   }
   __syncwarp();
+  follow_previous(q, out, kv_layer, block_table, ctx_lens);
+  const int ctx = __ldg(ctx_lens + seq);
+  // the query sits at position ctx-1 and sees keys [lo, ctx); pages before lo's page are skipped
+  const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
+  const int page0 = lo / BS;
+  const int n_pages = (ctx + BS - 1) / BS - page0;
+  const int my_n = n_pages > wg ? (n_pages - wg + n_warps - 1) / n_warps : 0;
 
   const int32_t* bt = block_table + (long long)seq * bt_stride + page0;
   const long long page_stride = (long long)G_::PAGE_BYTES;  // bytes per (block,kv,head) page
@@ -456,6 +456,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
     mbar_fence_init();
   }
   __syncwarp();
+  follow_previous(q, out, kv_layer, block_table, ctx_lens);
   if (first >= total) return;
 
   const long long page_stride = (long long)G_::PAGE_BYTES;
@@ -661,6 +662,7 @@ __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
   uint64_t* empty = full + PF_STAGES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y;
+  follow_previous(q, out, kv_layer, block_table, tiles);
   if (long_keys > 0 && portion_keys(tiles, n_tiles, blockIdx.x, lane) >= long_keys) return;
   const int4 tile = __ldg(tiles + blockIdx.x);
   const int bt_row = tile.x, row0 = tile.y, n_rows = tile.z, pos0 = tile.w;
@@ -925,9 +927,9 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
   const ScoreConsts sc = score_consts(scale, softcap);
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = decode_config<D, BS, kShared>(splits, n_seqs, n_kv, &attr, st);
-  B200Q_CUDA(cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv,
-                                n_q / n_kv, sc.c0, sc.c1, window));
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, cfg.gridDim, DEC_WARPS * 32, cfg.dynamicSmemBytes, st, splits, (const bf16*)q, q_stride, (bf16*)out,
+                          (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -961,10 +963,9 @@ static int launch_decode_stream(const void* q, int q_stride, void* out, const vo
   const int want = (total + DEC_WARPS - 1) / DEC_WARPS;
   const int grid = want < max_ctas ? want : max_ctas;
   const ScoreConsts sc = score_consts(scale, softcap);
-  kern<<<grid, DEC_WARPS * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out,
-                                                (const uint8_t*)kv, bt, bt_stride, ctx, n_seqs, n_q,
-                                                n_kv, n_q / n_kv, sc.c0, sc.c1, window);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, DEC_WARPS * 32, S_::TOTAL, st, 1, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt,
+                          bt_stride, ctx, n_seqs, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -985,11 +986,9 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
                   PfCfg<D>::MAX_G);
   const ScoreConsts sc = score_consts(scale, softcap);
   dim3 grid(n_tiles, n_kv);
-  kern<<<grid, (G + 1) * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out,
-                                              (const uint8_t*)kv, bt, bt_stride,
-                                              (const int4*)tiles, n_tiles, n_q, n_kv, G, sc.c0, sc.c1, window,
-                                              long_keys);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, (G + 1) * 32, S_::TOTAL, st, 1, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt,
+                          bt_stride, (const int4*)tiles, n_tiles, n_q, n_kv, G, sc.c0, sc.c1, window, long_keys));
+  count_launch();
   return B200Q_OK;
 }
 

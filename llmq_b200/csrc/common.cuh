@@ -22,6 +22,13 @@ int prefill_attn(int route, const void* q, int q_stride, void* out, const void* 
 void bump_tuning_epoch();
 int tuning_epoch();
 
+// The projections (gemm_tcgen05.cu) as a forward pass calls them.  fixed_w: no kernel that may still run when this one begins writes the
+// weights, so they are fetched before follow_previous; that holds where the first kernel of the same pass was not launched early.
+int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st);
+int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w, cudaStream_t st, const float** partials_out,
+                 int* splits_out);
+int linear_gated(bool gelu, const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st);
+
 #define B200Q_CHECK_ARG(cond, ...)          \
   do {                                      \
     if (!(cond)) {                          \
@@ -142,6 +149,10 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, in
       ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
+// the same box into L2 only.  Nothing is read by it as far as the memory model goes, so that it may run ahead of follow_previous.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tmap), "r"(c0), "r"(c1) : "memory");
+}
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, int c0, int c1, int c2, int c3, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
@@ -175,6 +186,47 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
       "{%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// ---- kernels that begin while the one before them on the stream still runs -------------------
+// launch_early starts a kernel as soon as every block of the one before it has called follow_previous (or has ended), wherever an SM has
+// room: the launch, barriers, tensor memory and what may be asked into L2 ahead no longer lie between the two.  follow_previous waits
+// until that kernel has ended and what it wrote can be seen; nothing that another kernel may write is read, and nothing is written,
+// before it.  Every thread calls it, so the kernel two places back has ended as well; and it is called once the block has its tensor
+// memory (a block barrier between), which a block of the next kernel could otherwise take from it and hold until this one ends.  The
+// pointers that the kernel reads through go through it: a load marked read-only (__ldg, const __restrict__) is not held back by the wait
+// alone.  B200, in a graph of dependent kernels: 2.0 us instead of 3.4 from one small kernel to the next; the routed feed-forward of 128
+// rows (8 kernels) 73.2 -> 58.9 us, a decode step of four layers of the 1B model at 48 sequences (37 kernels) 371 -> 349 us.
+template <typename T>
+__device__ __forceinline__ void pin_behind(T*& p) {
+  asm volatile("" : "+l"(p)::"memory");
+}
+template <typename T>
+__device__ __forceinline__ void pin_behind(T* __restrict__& p) {
+  asm volatile("" : "+l"(p)::"memory");
+}
+template <typename... P>
+__device__ __forceinline__ void follow_previous(P&... p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (pin_behind(p), ...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
 }
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(256) embed_kernel(const int32_t* __restrict__ 
                                                     const int32_t* __restrict__ prev_out,
                                                     const uint4* __restrict__ table,
                                                     uint4* __restrict__ out, int T, int chunks) {
+  follow_previous(ids, prev_out, table, out);
   long long total = (long long)T * chunks;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256) embed_scaled_kernel(const int32_t* __rest
                                                            const uint4* __restrict__ table,
                                                            uint4* __restrict__ out, int T, int chunks,
                                                            float scale) {
+  follow_previous(ids, prev_out, table, out);
   long long total = (long long)T * chunks;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -101,8 +103,8 @@ template <bool kAdd, bool kPartials = false>
 __global__ void __launch_bounds__(NORM_THREADS)
     rmsnorm_kernel(const uint4* __restrict__ x_in, uint4* __restrict__ residual,
                    const uint4* __restrict__ w, uint4* __restrict__ y, int chunks, float inv_h,
-                   float eps, const float* __restrict__ ws = nullptr, int splits = 0,
-                   long long mn = 0) {
+                   float eps, const float* __restrict__ ws, int splits, long long mn) {
+  follow_previous(x_in, residual, w, y, ws);
   const long long row = blockIdx.x;
   const uint4* xr = x_in + row * chunks;
   uint4 v[NORM_MAX_CHUNKS];
@@ -210,6 +212,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
                       const uint4* __restrict__ w_post, const uint4* __restrict__ w_next,
                       uint4* __restrict__ y, int chunks, float inv_h, float eps) {
   __shared__ float red[NORM_THREADS / 32];
+  follow_previous(x_in, residual, w_post, w_next, y);
   const long long row = blockIdx.x;
   const uint4* xr = x_in + row * chunks;
   uint4 v[NORM_MAX_CHUNKS];
@@ -260,6 +263,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 // final-logit soft-capping with every eager bf16 rounding: l <- bf16(bf16(tanh(bf16(l / cap))) * cap)
 __global__ void __launch_bounds__(256)
     softcap_kernel(uint4* __restrict__ logits, long long n_chunks, float cap) {
+  follow_previous(logits);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_chunks;
        i += (long long)gridDim.x * blockDim.x) {
     uint4 a = ld_v4(logits + i);
@@ -313,6 +317,7 @@ __global__ void __launch_bounds__(256)
                         const int32_t* __restrict__ slot_mapping, uint4* __restrict__ kv_layer,
                         int n_q, int n_kv, int D, int block_size, const float* __restrict__ ws,
                         int splits, long long mn) {
+  follow_previous(qkv, cos_sin, positions, slot_mapping, kv_layer, ws);
   const int t = blockIdx.x;
   const int cpr = D / 8;        // 16 B chunks per head row
   const int half = cpr / 2;     // chunk pairs per head
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     swiglu_kernel(const uint4* __restrict__ gate_up, uint4* __restrict__ out, int T, int ichunks) {
+  follow_previous(gate_up, out);
   long long total = (long long)T * ichunks;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -394,6 +400,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     gather_rows_kernel(const uint4* __restrict__ x, const int32_t* __restrict__ rows,
                        uint4* __restrict__ out, int n, int chunks) {
+  follow_previous(x, rows, out);
   long long total = (long long)n * chunks;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -415,6 +422,7 @@ __device__ __forceinline__ void amax_update(float v, int i, float& best, int& bi
 
 __global__ void __launch_bounds__(1024)
     argmax_kernel(const bf16* __restrict__ logits, int32_t* __restrict__ ids, int V) {
+  follow_previous(logits, ids);
   const bf16* row = logits + (long long)blockIdx.x * V;
   float best = -INFINITY;
   int bi = 0x7fffffff;
@@ -504,6 +512,7 @@ constexpr int SAMPLE_THREADS = 512;
 __global__ void __launch_bounds__(SAMPLE_THREADS, 3)
     sample_kernel(const bf16* __restrict__ logits, const int32_t* __restrict__ params,
                   int32_t* __restrict__ ids, int V) {
+  follow_previous(logits, params, ids);
   const int split = blockIdx.x, splits = gridDim.x, r_ = blockIdx.y;
   const bf16* row = logits + (long long)r_ * V;
   const float temp = __int_as_float(params[4 * r_ + 0]);
@@ -643,9 +652,9 @@ int b200q_gemma_rmsnorm(const void* x, const void* w, void* y, int T, int H, flo
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "gemma_rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  gemma_norm_kernel<false><<<T, NORM_THREADS, 0, as_stream(stream)>>>(
-      (const uint4*)x, nullptr, (const uint4*)w, nullptr, (uint4*)y, H / 8, 1.f / (float)H, eps);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(gemma_norm_kernel<false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
+                          (const uint4*)w, nullptr, (uint4*)y, H / 8, 1.f / (float)H, eps));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -655,10 +664,9 @@ int b200q_gemma_norm_add_norm(void* x, void* residual, const void* w_post, const
                   "gemma_norm_add_norm: bad shape T=%d H=%d", T, H);
   B200Q_CHECK_ARG(x && residual && w_post && w_next, "gemma_norm_add_norm: null argument");
   if (T == 0) return B200Q_OK;
-  gemma_norm_kernel<true><<<T, NORM_THREADS, 0, as_stream(stream)>>>(
-      (const uint4*)x, (uint4*)residual, (const uint4*)w_post, (const uint4*)w_next, (uint4*)x, H / 8,
-      1.f / (float)H, eps);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(gemma_norm_kernel<true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
+                          (const uint4*)w_post, (const uint4*)w_next, (uint4*)x, H / 8, 1.f / (float)H, eps));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -667,8 +675,8 @@ int b200q_softcap_bf16(void* logits, int64_t n, float cap, void* stream) {
                   (long long)n, (double)cap);
   B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(logits) & 15) == 0, "softcap: logits not 16-byte aligned");
   if (n == 0) return B200Q_OK;
-  softcap_kernel<<<grid_for(n / 8, 256), 256, 0, as_stream(stream)>>>((uint4*)logits, n / 8, cap);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(softcap_kernel, grid_for(n / 8, 256), 256, 0, as_stream(stream), 1, (uint4*)logits, n / 8, cap));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -676,9 +684,9 @@ int b200q_rmsnorm(const void* x, const void* w, void* y, int T, int H, float eps
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  rmsnorm_kernel<false><<<T, NORM_THREADS, 0, as_stream(stream)>>>(
-      (const uint4*)x, nullptr, (const uint4*)w, (uint4*)y, H / 8, 1.f / (float)H, eps);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(rmsnorm_kernel<false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
+                          (const uint4*)w, (uint4*)y, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -687,9 +695,9 @@ int b200q_add_rmsnorm(void* x, void* residual, const void* w, int T, int H, floa
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "add_rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  rmsnorm_kernel<true><<<T, NORM_THREADS, 0, as_stream(stream)>>>(
-      (const uint4*)x, (uint4*)residual, (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(rmsnorm_kernel<true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
+                          (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -699,10 +707,9 @@ int b200q_add_rmsnorm_splitk(void* x, void* residual, const void* w, const float
                   "add_rmsnorm_splitk: bad shape T=%d H=%d", T, H);
   B200Q_CHECK_ARG(partials && splits >= 1 && splits <= 16, "add_rmsnorm_splitk: bad partials (splits=%d)", splits);
   if (T == 0) return B200Q_OK;
-  rmsnorm_kernel<true, true><<<T, NORM_THREADS, 0, as_stream(stream)>>>(
-      nullptr, (uint4*)residual, (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, partials, splits,
-      (long long)T * H);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(rmsnorm_kernel<true, true>, T, NORM_THREADS, 0, as_stream(stream), 1, nullptr, (uint4*)residual,
+                          (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, partials, splits, (long long)T * H));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -713,10 +720,9 @@ int b200q_rope_kvwrite(void* qkv, const void* cos_sin, const int32_t* positions,
                   "rope_kvwrite: bad shape T=%d n_q=%d n_kv=%d D=%d bs=%d", T, n_q, n_kv, D,
                   block_size);
   if (T == 0) return B200Q_OK;
-  rope_kvwrite_kernel<false><<<T, 256, 0, as_stream(stream)>>>(
-      (uint4*)qkv, (const uint4*)cos_sin, positions, slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size,
-      nullptr, 0, 0);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(rope_kvwrite_kernel<false>, T, 256, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
+                          slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size, nullptr, 0, 0));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -728,10 +734,9 @@ int b200q_rope_kvwrite_splitk(void* qkv, const float* partials, int splits, cons
                   block_size);
   B200Q_CHECK_ARG(partials && splits >= 1 && splits <= 16, "rope_kvwrite_splitk: bad partials (splits=%d)", splits);
   if (T == 0) return B200Q_OK;
-  rope_kvwrite_kernel<true><<<T, 256, 0, as_stream(stream)>>>(
-      (uint4*)qkv, (const uint4*)cos_sin, positions, slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size,
-      partials, splits, (long long)T * (n_q + 2 * n_kv) * D);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(rope_kvwrite_kernel<true>, T, 256, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
+                          slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size, partials, splits, (long long)T * (n_q + 2 * n_kv) * D));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -739,9 +744,9 @@ int b200q_swiglu(const void* gate_up, void* out, int T, int I, void* stream) {
   B200Q_CHECK_ARG(T >= 0 && I > 0 && I % 8 == 0, "swiglu: bad shape T=%d I=%d", T, I);
   if (T == 0) return B200Q_OK;
   int ic = I / 8;
-  swiglu_kernel<<<grid_for((long long)T * ic, 256), 256, 0, as_stream(stream)>>>(
-      (const uint4*)gate_up, (uint4*)out, T, ic);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(swiglu_kernel, grid_for((long long)T * ic, 256), 256, 0, as_stream(stream), 1, (const uint4*)gate_up, (uint4*)out,
+                          T, ic));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -749,17 +754,17 @@ int b200q_gather_rows(const void* x, const int32_t* rows, void* out, int n, int 
   B200Q_CHECK_ARG(n >= 0 && H > 0 && H % 8 == 0, "gather_rows: bad shape n=%d H=%d", n, H);
   if (n == 0) return B200Q_OK;
   int chunks = H / 8;
-  gather_rows_kernel<<<grid_for((long long)n * chunks, 256), 256, 0, as_stream(stream)>>>(
-      (const uint4*)x, rows, (uint4*)out, n, chunks);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(gather_rows_kernel, grid_for((long long)n * chunks, 256), 256, 0, as_stream(stream), 1, (const uint4*)x, rows,
+                          (uint4*)out, n, chunks));
+  count_launch();
   return B200Q_OK;
 }
 
 int b200q_argmax_bf16(const void* logits, int32_t* ids, int B, int V, void* stream) {
   B200Q_CHECK_ARG(B >= 0 && V > 0, "argmax: bad shape B=%d V=%d", B, V);
   if (B == 0) return B200Q_OK;
-  argmax_kernel<<<B, 1024, 0, as_stream(stream)>>>((const bf16*)logits, ids, V);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(argmax_kernel, B, 1024, 0, as_stream(stream), 1, (const bf16*)logits, ids, V));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -771,18 +776,10 @@ int b200q_sample_bf16(const void* logits, const int32_t* params, int32_t* ids, i
   // (a grid's second dimension ends at 65535 rows)
   for (int at = 0; at < B; at += 65535) {
     const int rows = B - at < 65535 ? B - at : 65535;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = rows >= 444 ? 1 : (444 + rows - 1) / rows < 8 ? (444 + rows - 1) / rows : 8;  // three CTAs per SM
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(attr.val.clusterDim.x, rows);
-    cfg.blockDim = dim3(SAMPLE_THREADS);
-    cfg.stream = as_stream(stream);
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    B200Q_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, (const bf16*)logits + (long long)at * V, params + 4 * (long long)at, ids + at, V));
-    B200Q_LAUNCH_CHECK();
+    const int splits = rows >= 444 ? 1 : (444 + rows - 1) / rows < 8 ? (444 + rows - 1) / rows : 8;  // three CTAs per SM
+    B200Q_CUDA(launch_early(sample_kernel, dim3(splits, rows), SAMPLE_THREADS, 0, as_stream(stream), splits,
+                            (const bf16*)logits + (long long)at * V, params + 4 * (long long)at, ids + at, V));
+    count_launch();
   }
   return B200Q_OK;
 }

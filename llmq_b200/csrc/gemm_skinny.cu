@@ -7,7 +7,9 @@
 //     partial tiles meet in distributed shared memory, are added in the order of the splits (deterministic) and stored once:
 //     no scratch round trip and no second launch;
 //   * no tile loop: a CTA works one tile, and where the ring takes half of an SM's memory the second CTA of the SM covers its
-//     start and its end.
+//     start and its end;
+//   * the first weights are asked for before the kernel before this one has ended (follow_previous): into the ring where nobody can
+//     still be writing them (fixed_w), into L2 otherwise.
 // A gated unit (SwiGLU, GeGLU, clamped) works on gate rows in the first 128 rows of a 256-row tile and up rows in the other.
 #include "tcgen05.cuh"
 
@@ -18,6 +20,7 @@ constexpr int SK_BK = 64;
 constexpr int SK_TILE_BYTES = 128 * SK_BK * 2;  // 128 weight rows of one k-block
 constexpr int SK_MAX_STAGES = 8;
 constexpr int SK_MAX_SPLITS = 8;
+constexpr long long SK_AHEAD_BYTES = 24000000;  // weights of a product that are asked for before the kernel before it has ended
 
 struct SkinnyArgs {
   bf16* C;
@@ -27,6 +30,8 @@ struct SkinnyArgs {
   long long ldc, patience;  // patience: cycles that the product warp waits for a stage
   float limit;
   int M, N, K, mp, stages, a_bytes, cols, chunk;  // mp: M padded to 16; chunk: columns (rows of A) per exchange
+  int fixed_w;  // see linear() in common.cuh
+  int ahead;    // k-blocks of weights that are asked for before the kernel before this one has ended
 };
 
 // After a wait ran out, before the block's memory is given back: what the first thread asked for has come, and what was issued has been
@@ -71,19 +76,36 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
   int asked = 0;  // (of the fetching thread) stages asked for
+  // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
+  // (short reductions keep the order that the kernels for larger steps add in)
+  const int kb_first = kb0 + (kb1 - kb0 >= 16 ? tile * 5 % (kb1 - kb0) : 0), early = min(a.stages, kb1 - kb0);
+  if (warp == 0 && lane == 0) {  // the first weights while the kernels before this one end
+    int kb = kb_first;
+    for (int i = 0; i < min(a.ahead, kb1 - kb0); ++i, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
+      if (a.fixed_w && i < early) {
+        mbar_expect_tx(full + i, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
+        tma_load_2d(smem + i * stage_bytes, &tmap_w, kb * SK_BK, tile * NT, full + i);
+      } else {
+        tma_prefetch_2d(&tmap_w, kb * SK_BK, tile * NT);
+      }
+    }
+  }
+  __syncwarp();
+  const float* bias = a.bias;
+  follow_previous(bias);
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
-      // (short reductions keep the order that the kernels for larger steps add in)
-      int kb = kb0 + (kb1 - kb0 >= 16 ? tile * 5 % (kb1 - kb0) : 0);
+      int kb = kb_first;
       for (; asked < kb1 - kb0; ++asked, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
-        if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, &dead, a.failed)) break;
         uint8_t* sw = smem + stage * stage_bytes;
-        mbar_expect_tx(full + stage, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
-        tma_load_2d(sw, &tmap_w, kb * SK_BK, tile * NT, full + stage);
+        if (!a.fixed_w || asked >= early) {
+          if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, &dead, a.failed)) break;
+          mbar_expect_tx(full + stage, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
+          tma_load_2d(sw, &tmap_w, kb * SK_BK, tile * NT, full + stage);
+        }
         tma_load_2d(sw + WT * SK_TILE_BYTES, &tmap_a, kb * SK_BK, 0, full + stage);
         if (++stage == a.stages) {
           stage = 0;
@@ -199,8 +221,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if constexpr (kAct == ACT_CLAMPED) {
-              const float* b = a.bias + (long long)tile * NT + n + j;
-              o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), a.bias ? __ldg(b) : 0.f, a.bias ? __ldg(b + 128) : 0.f,
+              const float* b = bias + (long long)tile * NT + n + j;
+              o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), bias ? __ldg(b) : 0.f, bias ? __ldg(b + 128) : 0.f,
                                   a.limit);
             } else {
               o[j] = gated_unit<kAct>(__float_as_uint(o[j]), __float_as_uint(u[j]));
@@ -305,6 +327,8 @@ static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_
   if (a.stages > SK_MAX_STAGES) a.stages = SK_MAX_STAGES;
   a.chunk = a.stages * stage / (WT * 512) & ~15;
   if (a.chunk > a.mp) a.chunk = a.mp;
+  a.ahead = (int)(SK_AHEAD_BYTES / ((long long)(a.N / (WT * 128)) * p.splits * WT * SK_TILE_BYTES));
+  if (a.ahead < a.stages) a.ahead = a.stages;
   CUtensorMap tw, ta;
   rc = get_tmap(W, a.N, a.K, WT * 128, &tw);
   if (rc) return rc;
@@ -314,19 +338,9 @@ static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_
     set_error("gemm: no host-visible flag for bounded waits");
     return B200Q_ECUDA;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.splits, a.N / (WT * 128));
-  cfg.blockDim = dim3(SK_THREADS);
-  cfg.dynamicSmemBytes = a.stages * stage + 1024;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = a.parts ? 1 : p.splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  B200Q_CUDA(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<WT, kAct>, tw, ta, a));
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(gemm_skinny_kernel<WT, kAct>, dim3(p.splits, a.N / (WT * 128)), SK_THREADS, a.stages * stage + 1024, st,
+                          a.parts ? 1 : p.splits, tw, ta, a));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -365,8 +379,9 @@ int gemm_skinny_splits(int M, int N, int K) {
 
 // C (or, `parts`: the fp32 partial tiles [splits][M][N]) of up to 128 rows; `act`: ACT_*
 int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int act, long long ldc, const float* bias, float limit,
-                float* parts, cudaStream_t st) {
+                float* parts, bool fixed_w, cudaStream_t st) {
   SkinnyArgs a{};
+  a.fixed_w = fixed_w;
   a.C = (bf16*)C;
   a.parts = parts;
   a.bias = bias;

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                      const __grid_constant__ CUtensorMap tmap_b, bf16* __restrict__ C, int M,
                      int N, int K, int splits, float* __restrict__ ws, int a_bytes,
-                     long long ldc, GateArgs gate) {
+                     long long ldc, GateArgs gate, int fixed_w) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;
   // a_bytes: bytes one A k-block really carries.  For M < 128 the tensor map's box holds only the
   // rows that exist (rounded up to the 8-row swizzle atom), not 128: the other rows of the UMMA's A
@@ -193,6 +193,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  int early = 0;  // k-blocks whose weights are asked for while the kernel before this one ends
+  if (warp == 0 && lane == 0) {
+    const int rest = blockIdx.x / m_tiles, n_blk = rest / splits, kb0 = (rest % splits) * k_blocks;
+    for (int kb = 0; kb < STAGES && kb < k_blocks; ++kb) {
+      if (fixed_w) {
+        mbar_expect_tx(full + kb, (uint32_t)(a_bytes + Cfg::B_BYTES));
+        tma_load_2d(smem + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmap_b, (kb0 + kb) * GEMM_BK, n_blk * BN, full + kb);
+        ++early;
+      } else {
+        tma_prefetch_2d(&tmap_b, (kb0 + kb) * GEMM_BK, n_blk * BN);
+      }
+    }
+  }
+  __syncwarp();
+  follow_previous(gate.bias);
 
   if (warp == 0) {
     // ===== TMA producer =====
@@ -203,12 +218,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const int m_blk = tile % m_tiles, rest = tile / m_tiles;
         const int n_blk = rest / splits, kb0 = (rest % splits) * k_blocks;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          mbar_wait(empty + stage, phase ^ 1u);
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
-          mbar_expect_tx(full + stage, (uint32_t)(a_bytes + Cfg::B_BYTES));
+          if (early > 0) {
+            --early;
+          } else {
+            mbar_wait(empty + stage, phase ^ 1u);
+            mbar_expect_tx(full + stage, (uint32_t)(a_bytes + Cfg::B_BYTES));
+            tma_load_2d(sb, &tmap_b, (kb0 + kb) * GEMM_BK, n_blk * BN, full + stage);
+          }
           tma_load_2d(sa, &tmap_a, (kb0 + kb) * GEMM_BK, m_blk * GEMM_BM, full + stage);
-          tma_load_2d(sb, &tmap_b, (kb0 + kb) * GEMM_BK, n_blk * BN, full + stage);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -304,6 +323,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const float4* __restrict__ ws, uint4* __restrict__ out, long long mn8,
                          int splits) {
+  follow_previous(ws, out);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < mn8;
        i += (long long)gridDim.x * blockDim.x) {
     float4 a = ws[2 * i], b = ws[2 * i + 1];
@@ -396,7 +416,7 @@ template <int BN, int kAct = ACT_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                       const __grid_constant__ CUtensorMap tmap_b, bf16* __restrict__ C, int M,
-                      int N, int K, long long ldc, GateArgs gate) {
+                      int N, int K, long long ldc, GateArgs gate, int fixed_w) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;
   using Cfg = Gemm2Cfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
@@ -439,6 +459,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   cluster_sync_all();  // peer barriers are initialised before anybody signals them
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  int early = 0;  // (as above)
+  if (warp == 0 && lane == 0) {
+    const int row = cluster_id / m_tiles * BN + (int)rank * (BN / 2);
+    for (int kb = 0; kb < STAGES && kb < k_blocks; ++kb) {
+      if (fixed_w) {
+        const uint32_t lfull = mapa_shared(full + kb, 0);
+        mbar_expect_tx_cluster(lfull, Cfg::STAGE_BYTES);
+        tma_load_2d_2sm(smem + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmap_b, kb * GEMM_BK, row, lfull);
+        ++early;
+      } else {
+        tma_prefetch_2d(&tmap_b, kb * GEMM_BK, row);
+      }
+    }
+  }
+  __syncwarp();
+  follow_previous(gate.bias);
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs): own A rows + own half of B, completion on the LEADER =====
@@ -448,13 +484,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
         const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          mbar_wait(empty + stage, phase ^ 1u);
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
           const uint32_t lfull = mapa_shared(full + stage, 0);
-          mbar_expect_tx_cluster(lfull, Cfg::STAGE_BYTES);
+          if (early > 0) {
+            --early;
+          } else {
+            mbar_wait(empty + stage, phase ^ 1u);
+            mbar_expect_tx_cluster(lfull, Cfg::STAGE_BYTES);
+            tma_load_2d_2sm(sb, &tmap_b, kb * GEMM_BK, n_blk * BN + (int)rank * (BN / 2), lfull);
+          }
           tma_load_2d_2sm(sa, &tmap_a, kb * GEMM_BK, m_blk * 256 + (int)rank * 128, lfull);
-          tma_load_2d_2sm(sb, &tmap_b, kb * GEMM_BK, n_blk * BN + (int)rank * (BN / 2), lfull);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -670,7 +710,7 @@ static int splitk_scratch(int splits, int M, int N, float** out) {
 template <int BN, int kAct = ACT_NONE>
 static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int K,
                        cudaStream_t st, int splits = 1, const float** partials_out = nullptr, long long ldc = 0,
-                       GateArgs gate = {nullptr, 0.f}) {
+                       GateArgs gate = {nullptr, 0.f}, bool fixed_w = false) {
   using Cfg = GemmCfg<BN>;
   CUtensorMap ta, tb;
   const int a_rows = M < GEMM_BM ? (M + 7) & ~7 : GEMM_BM;  // one m-tile: load only the rows that exist
@@ -692,16 +732,15 @@ static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int 
     rc = splitk_scratch(splits, M, N, &ws);
     if (rc) return rc;
   }
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st>>>(ta, tb, (bf16*)C, M, N, K, splits, ws,
-                                                    a_rows * GEMM_BK * 2,
-                                                    ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K, splits, ws, a_rows * GEMM_BK * 2,
+                          ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate, (int)fixed_w));
+  count_launch();
   if (partials_out) *partials_out = ws;  // the caller fuses the reduction into the consumer of C
   if (splits > 1 && !partials_out) {
     const long long mn8 = (long long)M * N / 8;
     const int rgrid = (int)((mn8 + 255) / 256 < 148 * 8 ? (mn8 + 255) / 256 : 148 * 8);
-    splitk_reduce_kernel<<<rgrid, 256, 0, st>>>((const float4*)ws, (uint4*)C, mn8, splits);
-    B200Q_LAUNCH_CHECK();
+    B200Q_CUDA(launch_early(splitk_reduce_kernel, rgrid, 256, 0, st, 1, (const float4*)ws, (uint4*)C, mn8, splits));
+    count_launch();
   }
   return B200Q_OK;
 }
@@ -710,7 +749,7 @@ static int g_gemm2_pairs = 0;  // co-resident CTA pairs reported by the occupanc
 
 template <int BN, int kAct = ACT_NONE>
 static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int K,
-                        cudaStream_t st, long long ldc = 0, GateArgs gate = {nullptr, 0.f}) {
+                        cudaStream_t st, long long ldc = 0, GateArgs gate = {nullptr, 0.f}, bool fixed_w = false) {
   using Cfg = Gemm2Cfg<BN>;
   CUtensorMap ta, tb;
   int rc = get_tmap(A, M, K, GEMM_BM, &ta);
@@ -749,9 +788,9 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
     g_gemm2_pairs = pairs;
   }
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st>>>(ta, tb, (bf16*)C, M, N, K,
-                                                  ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K,
+                          ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate, (int)fixed_w));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -860,26 +899,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int mt_per_group = (ga.M + GEMM_BM - 1) / GEMM_BM;
-  const int m_tiles = ga.tab ? *ga.n_mt : mt_per_group * ga.groups;
-  const int n_tiles = N / BN;
-  const int num_tiles = m_tiles * n_tiles;
-  const int k_blocks = K / GEMM_BK;
-  auto tile_of = [&](int tile, int& g, int& row0, int& row_end, int& n_blk) {
-    const int mt = tile % m_tiles;
-    n_blk = tile / m_tiles;
-    if (ga.tab) {
-      const int4 e = ga.tab[mt];
-      g = e.x;
-      row0 = e.y;
-      row_end = e.z;
-    } else {
-      g = mt / mt_per_group;
-      row0 = (mt % mt_per_group) * GEMM_BM;
-      row_end = ga.M;
-    }
-  };
-
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -899,6 +918,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  follow_previous();
+  const int mt_per_group = (ga.M + GEMM_BM - 1) / GEMM_BM;
+  const int m_tiles = ga.tab ? *ga.n_mt : mt_per_group * ga.groups;
+  const int n_tiles = N / BN;
+  const int num_tiles = m_tiles * n_tiles;
+  const int k_blocks = K / GEMM_BK;
+  auto tile_of = [&](int tile, int& g, int& row0, int& row_end, int& n_blk) {
+    const int mt = tile % m_tiles;
+    n_blk = tile / m_tiles;
+    if (ga.tab) {
+      const int4 e = ga.tab[mt];
+      g = e.x;
+      row0 = e.y;
+      row_end = e.z;
+    } else {
+      g = mt / mt_per_group;
+      row0 = (mt % mt_per_group) * GEMM_BM;
+      row_end = ga.M;
+    }
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1010,8 +1049,8 @@ static int launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, void* C,
     attr_set = true;
   }
   const int grid = max_tiles < num_sms() ? max_tiles : num_sms();
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st>>>(ta, tb, C, N, K, ga);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, C, N, K, ga));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -1022,7 +1061,7 @@ using namespace b200q;
 // shared body of the fused gate_up GEMMs (SwiGLU / GeGLU)
 template <int kAct>
 static int gemm_gated(const char* what, const void* A, const void* W, void* C, int M, int N, int K,
-                      void* stream, long long ldc = 0, GateArgs gate = {nullptr, 0.f}) {
+                      void* stream, long long ldc = 0, GateArgs gate = {nullptr, 0.f}, bool fixed_w = false) {
   B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 256 == 0,
                   "%s: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%256==0)", what, M, N, K);
   B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
@@ -1032,11 +1071,84 @@ static int gemm_gated(const char* what, const void* A, const void* W, void* C, i
   if (M == 0) return B200Q_OK;
   cudaStream_t st = as_stream(stream);
   if (use_skinny(M, N, K, true))
-    return gemm_skinny(A, W, C, M, N, K, kAct, ldc > 0 ? ldc : N / 2, gate.bias, gate.limit, nullptr, st);
+    return gemm_skinny(A, W, C, M, N, K, kAct, ldc > 0 ? ldc : N / 2, gate.bias, gate.limit, nullptr, fixed_w, st);
   if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && choose_tile(M, N, true).pair))
-    return launch_gemm2<256, kAct>(A, W, C, M, N, K, st, ldc, gate);
-  return launch_gemm<256, kAct>(A, W, C, M, N, K, st, 1, nullptr, ldc, gate);
+    return launch_gemm2<256, kAct>(A, W, C, M, N, K, st, ldc, gate, fixed_w);
+  return launch_gemm<256, kAct>(A, W, C, M, N, K, st, 1, nullptr, ldc, gate, fixed_w);
 }
+
+namespace b200q {
+
+int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st) {
+  B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 64 == 0,
+                  "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
+  B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
+                      (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+                      (reinterpret_cast<uintptr_t>(C) & 15) == 0,
+                  "gemm: operands must be 16-byte aligned");
+  if (M == 0) return B200Q_OK;
+  if (use_skinny(M, N, K, false)) return gemm_skinny(A, W, C, M, N, K, ACT_NONE, N, nullptr, 0.f, nullptr, fixed_w, st);
+  int bn = g_gemm_force_bn;
+  if (g_gemm_mode == 2 && M > GEMM_BM) {
+    if ((bn == 0 || bn == 256) && N % 256 == 0) return launch_gemm2<256>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+    if ((bn == 0 || bn == 128) && N % 128 == 0) return launch_gemm2<128>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+  }
+  {
+    // split-K for decode-sized batches: when a projection has too few 128-wide output tiles to
+    // put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
+    // B200Q_BATCH_INVARIANT=1 (read once): never split K, so every output element is reduced in
+    // one sequential pass (the attention kernels do likewise) and a request's tokens cannot depend on its batch-mates (like
+    // VLLM_BATCH_INVARIANT); costs decode-sized GEMMs up to 2x
+    const int splits = choose_splits(M, N, K, batch_invariant(), bn);
+    if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
+  }
+  if (bn == 0) {
+    const TileChoice t = choose_tile(M, N, false);
+    if (t.pair && g_gemm_mode == 0)
+      return t.bn == 256 ? launch_gemm2<256>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w) : launch_gemm2<128>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+    bn = t.bn;
+  }
+  if (N % bn != 0) bn = (N % 128 == 0) ? 128 : 64;
+  if (bn == 256) return launch_gemm<256>(A, W, C, M, N, K, st, 1, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
+  if (bn == 128) return launch_gemm<128>(A, W, C, M, N, K, st, 1, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
+  return launch_gemm<64>(A, W, C, M, N, K, st, 1, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
+}
+
+int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w, cudaStream_t st, const float** partials_out,
+                 int* splits_out) {
+  B200Q_CHECK_ARG(partials_out && splits_out, "gemm_splitk: null output argument");
+  *partials_out = nullptr;
+  *splits_out = 1;
+  B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 64 == 0,
+                  "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
+  B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0,
+                  "gemm: operands must be 16-byte aligned");
+  if (M == 0 || g_gemm_mode == 2 || g_gemm_force_bn != 0) return B200Q_OK;
+  if (use_skinny(M, N, K, false)) {
+    const int n = gemm_skinny_splits(M, N, K);
+    if (n <= 1 || N > 8192) return B200Q_OK;
+    float* ws = nullptr;
+    int rc = splitk_scratch(n, M, N, &ws);
+    if (!rc) rc = gemm_skinny(A, W, nullptr, M, N, K, ACT_NONE, N, nullptr, 0.f, ws, fixed_w, st);
+    if (rc) return rc;
+    *partials_out = ws;
+    *splits_out = n;
+    return B200Q_OK;
+  }
+  const int splits = choose_splits(M, N, K, batch_invariant(), 0);
+  if (splits <= 1) return B200Q_OK;
+  int rc = launch_gemm<128>(A, W, nullptr, M, N, K, st, splits, partials_out, 0, GateArgs{nullptr, 0.f}, fixed_w);
+  if (rc) return rc;
+  *splits_out = splits;
+  return B200Q_OK;
+}
+
+int linear_gated(bool gelu, const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st) {
+  return gelu ? gemm_gated<ACT_GEGLU>("gemm_geglu", A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w)
+              : gemm_gated<ACT_SWIGLU>("gemm_swiglu", A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+}
+
+}  // namespace b200q
 
 extern "C" {
 
@@ -1106,39 +1218,7 @@ int b200q_gemm_set_mode(int mode) {
 }
 
 int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, void* stream) {
-  B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 64 == 0,
-                  "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
-  B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
-                      (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
-                      (reinterpret_cast<uintptr_t>(C) & 15) == 0,
-                  "gemm: operands must be 16-byte aligned");
-  if (M == 0) return B200Q_OK;
-  cudaStream_t st = as_stream(stream);
-  if (use_skinny(M, N, K, false)) return gemm_skinny(A, W, C, M, N, K, ACT_NONE, N, nullptr, 0.f, nullptr, st);
-  int bn = g_gemm_force_bn;
-  if (g_gemm_mode == 2 && M > GEMM_BM) {
-    if ((bn == 0 || bn == 256) && N % 256 == 0) return launch_gemm2<256>(A, W, C, M, N, K, st);
-    if ((bn == 0 || bn == 128) && N % 128 == 0) return launch_gemm2<128>(A, W, C, M, N, K, st);
-  }
-  {
-    // split-K for decode-sized batches: when a projection has too few 128-wide output tiles to
-    // put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
-    // B200Q_BATCH_INVARIANT=1 (read once): never split K, so every output element is reduced in
-    // one sequential pass (the attention kernels do likewise) and a request's tokens cannot depend on its batch-mates (like
-    // VLLM_BATCH_INVARIANT); costs decode-sized GEMMs up to 2x
-    const int splits = choose_splits(M, N, K, batch_invariant(), bn);
-    if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits);
-  }
-  if (bn == 0) {
-    const TileChoice t = choose_tile(M, N, false);
-    if (t.pair && g_gemm_mode == 0)
-      return t.bn == 256 ? launch_gemm2<256>(A, W, C, M, N, K, st) : launch_gemm2<128>(A, W, C, M, N, K, st);
-    bn = t.bn;
-  }
-  if (N % bn != 0) bn = (N % 128 == 0) ? 128 : 64;
-  if (bn == 256) return launch_gemm<256>(A, W, C, M, N, K, st);
-  if (bn == 128) return launch_gemm<128>(A, W, C, M, N, K, st);
-  return launch_gemm<64>(A, W, C, M, N, K, st);
+  return linear(A, W, C, M, N, K, false, as_stream(stream));
 }
 
 // The split-K half of b200q_gemm_bf16 on its own: when the dispatcher would split the reduction
@@ -1148,33 +1228,8 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
 // b200q_rope_kvwrite_splitk), saving a launch and a round trip per projection.  *splits_out = 1
 // means nothing was launched: call b200q_gemm_bf16 instead.  The scratch is overwritten by the next
 // split-K GEMM on the stream.
-int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, void* stream,
-                           const float** partials_out, int* splits_out) {
-  B200Q_CHECK_ARG(partials_out && splits_out, "gemm_splitk: null output argument");
-  *partials_out = nullptr;
-  *splits_out = 1;
-  B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 64 == 0,
-                  "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
-  B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0,
-                  "gemm: operands must be 16-byte aligned");
-  if (M == 0 || g_gemm_mode == 2 || g_gemm_force_bn != 0) return B200Q_OK;
-  if (use_skinny(M, N, K, false)) {
-    const int n = gemm_skinny_splits(M, N, K);
-    if (n <= 1 || N > 8192) return B200Q_OK;
-    float* ws = nullptr;
-    int rc = splitk_scratch(n, M, N, &ws);
-    if (!rc) rc = gemm_skinny(A, W, nullptr, M, N, K, ACT_NONE, N, nullptr, 0.f, ws, as_stream(stream));
-    if (rc) return rc;
-    *partials_out = ws;
-    *splits_out = n;
-    return B200Q_OK;
-  }
-  const int splits = choose_splits(M, N, K, batch_invariant(), 0);
-  if (splits <= 1) return B200Q_OK;
-  int rc = launch_gemm<128>(A, W, nullptr, M, N, K, as_stream(stream), splits, partials_out);
-  if (rc) return rc;
-  *splits_out = splits;
-  return B200Q_OK;
+int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, void* stream, const float** partials_out, int* splits_out) {
+  return linear_parts(A, W, M, N, K, false, as_stream(stream), partials_out, splits_out);
 }
 
 // K9+K10 fused: out[M, N/2] = swiglu(A . W^T) where W [N, K] holds gate/up rows interleaved in
@@ -1182,12 +1237,12 @@ int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, vo
 // rows).  Same rounding points as b200q_gemm_bf16 followed by b200q_swiglu.
 int b200q_gemm_swiglu_bf16(const void* A, const void* W, void* C, int M, int N, int K,
                            void* stream) {
-  return gemm_gated<ACT_SWIGLU>("gemm_swiglu", A, W, C, M, N, K, stream);
+  return linear_gated(false, A, W, C, M, N, K, false, as_stream(stream));
 }
 
 // Gemma-2's GeGLU (gelu_tanh(gate) * up) in the same fused epilogue, same weight interleaving
 int b200q_gemm_geglu_bf16(const void* A, const void* W, void* C, int M, int N, int K, void* stream) {
-  return gemm_gated<ACT_GEGLU>("gemm_geglu", A, W, C, M, N, K, stream);
+  return linear_gated(true, A, W, C, M, N, K, false, as_stream(stream));
 }
 
 // the clamped gated unit (with biases unless NULL) in the same epilogue; C has rows of ldc elements

@@ -1319,6 +1319,7 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restric
 }
 __global__ void __launch_bounds__(256) copy_f32_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                        long long n) {
+  follow_previous(in, out);
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
     out[e] = in[e];
 }
@@ -1744,8 +1745,8 @@ int b200q_f32_to_bf16(const float* in, void* out, int64_t n, void* stream) {
 int b200q_copy_f32(const float* in, float* out, int64_t n, void* stream) {
   B200Q_CHECK_ARG(in && out && n >= 0, "copy_f32: bad argument");
   if (n == 0) return B200Q_OK;
-  copy_f32_kernel<<<grid_for(n), 256, 0, as_stream(stream)>>>(in, out, n);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(copy_f32_kernel, grid_for(n), 256, 0, as_stream(stream), 1, in, out, (long long)n));
+  count_launch();
   return B200Q_OK;
 }
 

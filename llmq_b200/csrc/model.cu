@@ -275,7 +275,8 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
   const double kv_tok_bytes = 2.0 * NKV * D * 2;  // K+V bytes per cached token per layer
 
   const bool gemma = c.arch == B200Q_ARCH_GEMMA2;
-  // token ids < 0 are indirections into the previous step's sampled ids (async stepping)
+  // token ids < 0 are indirections into the previous step's sampled ids (async stepping).  (The one kernel of a pass that is not launched
+  // early: all that came before it on the stream has ended when it begins, which is what fixed_w asks for.)
   B200Q_TRY(B200Q_PROF_ELEMENTWISE, 2.0 * T * H * 2,
             b200q_embed_ex(b->token_ids, b->prev_out_ids, m->embed, m->residual, T, H,
                            gemma ? c.embed_scale : 0.f, stream));
@@ -297,10 +298,10 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
     *part = nullptr;
     *splits = 1;
     if (fuse) {
-      int rc2 = b200q_gemm_bf16_splitk(A, W, T, N, K, stream, part, splits);
+      int rc2 = linear_parts(A, W, T, N, K, true, cst, part, splits);
       if (rc2 || *splits > 1) return rc2;
     }
-    return b200q_gemm_bf16(A, W, C, T, N, K, stream);
+    return linear(A, W, C, T, N, K, true, cst);
   };
   // (a caller without a host copy of the portions: every sequence that ends a portion samples)
   const int32_t* portions = b->h_seq_desc && b->n_rows >= b->n_dec ? b->h_seq_desc + 4 * (long long)b->n_dec : nullptr;
@@ -342,11 +343,11 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
     B200Q_TRY(B200Q_PROF_GEMM, 2.0 * T * H * QD, gemm_maybe_split(m->attn, L.o, m->x, H, QD, &part, &splits));
     if (gemma) {
       B200Q_TRY(B200Q_PROF_ELEMENTWISE, 4.0 * T * H * 2, b200q_gemma_norm_add_norm(m->x, m->residual, L.post_attn_norm, L.pre_ffn_norm, T, H, c.rms_eps, stream));
-      B200Q_TRY(B200Q_PROF_GEMM, 4.0 * T * I * H, b200q_gemm_geglu_bf16(m->x, L.gate_up, m->act, T, 2 * I, H, stream));
+      B200Q_TRY(B200Q_PROF_GEMM, 4.0 * T * I * H, linear_gated(true, m->x, L.gate_up, m->act, T, 2 * I, H, true, cst));
     } else {
       B200Q_TRY(B200Q_PROF_ELEMENTWISE, 4.0 * T * H * 2, add_norm(L.post_norm, part, splits));
       // gate_up GEMM with the SwiGLU fused into its epilogue (weights interleaved at bind time)
-      B200Q_TRY(B200Q_PROF_GEMM, 4.0 * T * I * H, b200q_gemm_swiglu_bf16(m->x, L.gate_up, m->act, T, 2 * I, H, stream));
+      B200Q_TRY(B200Q_PROF_GEMM, 4.0 * T * I * H, linear_gated(false, m->x, L.gate_up, m->act, T, 2 * I, H, true, cst));
     }
     B200Q_TRY(B200Q_PROF_GEMM, 2.0 * T * H * I, gemm_maybe_split(m->act, L.down, m->x, H, I, &pend, &pend_splits));
     if (gemma && li + 1 < c.n_layers)
@@ -364,7 +365,7 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
   }
   if (b->n_sample > 0) {
     B200Q_TRY(B200Q_PROF_ELEMENTWISE, 2.0 * b->n_sample * H * 2, b200q_gather_rows(m->x, b->sample_rows, m->sel, b->n_sample, H, stream));
-    B200Q_TRY(B200Q_PROF_GEMM, 2.0 * b->n_sample * (double)c.vocab * H, b200q_gemm_bf16(m->sel, m->lm_head, m->logits, b->n_sample, c.vocab, H, stream));
+    B200Q_TRY(B200Q_PROF_GEMM, 2.0 * b->n_sample * (double)c.vocab * H, linear(m->sel, m->lm_head, m->logits, b->n_sample, c.vocab, H, true, cst));
     if (c.final_softcap > 0.f)
       B200Q_TRY(B200Q_PROF_ELEMENTWISE, 2.0 * b->n_sample * c.vocab * 2,
                 b200q_softcap_bf16(m->logits, (int64_t)b->n_sample * c.vocab, c.final_softcap, stream));

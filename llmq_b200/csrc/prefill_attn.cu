@@ -79,7 +79,7 @@ __device__ __forceinline__ int block_portion_keys(const FaArgs& a, int first, in
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int i = first + 32 * h + lane;
-    const int4 t = __ldg(a.tiles + min(i, a.n_tiles - 1));
+    const int4 t = a.tiles[min(i, a.n_tiles - 1)];
     const int n = min(max(t.z, 0), 16);
     keys[h] = t.w + n;
     // (lane 0 compares with lane 31 of the half before)
@@ -107,7 +107,7 @@ struct FaBlock {
   __device__ __forceinline__ void fetch(const FaArgs& a, const FaOrder& o, int u, int lane) {
     ahead_first = u < o.units ? o.block(u / a.n_kv) * a.per_block : a.n_tiles;
     ahead_count = min(a.per_block, a.n_tiles - ahead_first);
-    ahead = lane < ahead_count ? __ldg(a.tiles + ahead_first + lane) : make_int4(0, 0, 0, 0);
+    ahead = lane < ahead_count ? a.tiles[ahead_first + lane] : make_int4(0, 0, 0, 0);
   }
   template <bool kSplit>
   __device__ __forceinline__ void begin(const FaArgs& a, const FaOrder& o, FaUnit at, int lane) {
@@ -175,7 +175,7 @@ __device__ __forceinline__ void fa_row_again(const FaArgs& a, const int32_t* bt,
   for (int j0 = lo & ~31; j0 <= pos; j0 += 32) {
     const int j = j0 + lane, t = j & 15;
     const bool seen = j >= lo && j <= pos;
-    const int blk = seen ? __ldg(bt + (j >> 4)) : 0;
+    const int blk = seen ? bt[j >> 4] : 0;
     float s = -INFINITY;
     if (seen) {
       const uint8_t* row = a.kv + ((long long)blk * 2 * a.n_kv + kvh) * page_bytes + t * (D * 2);
@@ -241,7 +241,7 @@ __device__ __noinline__ void fa_rows_again(const FaArgs& a, const FaOrder order)
     int keys = 0;
     if constexpr (kSplit) keys = block_portion_keys(a, first, lane);
     for (int i = 0; i < count; ++i) {
-      const int4 t = __ldg(a.tiles + first + i);
+      const int4 t = a.tiles[first + i];
       if (kSplit && __shfl_sync(0xffffffffu, keys, i) < a.long_keys) continue;
       const int rows = min(max(t.z, 0), 16) * a.G;
       for (int f = warp; f < rows; f += 8) {
@@ -285,14 +285,6 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
   const bool sort = n_blocks <= FA_SORTED && n_blocks * a.n_kv > (int)gridDim.x;  // (one unit each: nothing to deal out)
   const FaOrder order{sort ? sorted : nullptr, n_blocks, n_blocks * a.n_kv};
 
-  if constexpr (kSplit) {  // no tile sees so many keys: nothing to do here
-    bool any = false;
-    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {
-      const int4 t = __ldg(a.tiles + i);
-      any |= t.w + min(max(t.z, 0), 16) >= a.long_keys;
-    }
-    if (!__syncthreads_or(any)) return;
-  }
   if (threadIdx.x == 0) {
     dead = redo = 0;
     for (int s = 0; s < STG; ++s) {
@@ -312,11 +304,24 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     mbar_fence_init();
   }
   if (warp == 9) tmem_alloc(&tmem_slot, 512);
+  __syncthreads();
+  follow_previous();
+  if constexpr (kSplit) {  // no tile sees so many keys: nothing to do here
+    bool any = false;
+    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {
+      const int4 t = a.tiles[i];
+      any |= t.w + min(max(t.z, 0), 16) >= a.long_keys;
+    }
+    if (!__syncthreads_or(any)) {
+      if (warp == 9) tmem_dealloc(tmem_slot, 512);
+      return;
+    }
+  }
   if (sort) {
     for (int i = threadIdx.x; i < n_blocks; i += FA_THREADS) steps_in[i] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {  // the last token of a run sees most keys
-      const int4 t = __ldg(a.tiles + i), n = __ldg(a.tiles + min(i + 1, a.n_tiles - 1));
+      const int4 t = a.tiles[i], n = a.tiles[min(i + 1, a.n_tiles - 1)];
       const bool ends = i + 1 == a.n_tiles || (i + 1) % a.per_block == 0 || n.x != t.x || n.y != t.y + t.z || n.w != t.w + t.z;
       const int all = t.w + t.z, keys = a.window > 0 ? min(all, a.window) : all;
       if (ends && (!kSplit || all >= a.long_keys)) atomicAdd(steps_in + i / a.per_block, max(keys, 0) / KT + 2);  // (start and end: about one step)
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
         const int n_pages = (total + 15) / 16 - k0 / 16;
         auto page_of = [&](int j) {
           const int at_page = j * PAGES + lane;
-          return lane < PAGES && at_page < n_pages && j < steps ? __ldg(bt + at_page) : 0;
+          return lane < PAGES && at_page < n_pages && j < steps ? bt[at_page] : 0;
         };
         // one step's keys or values; keys are asked for a step ahead of values, whose slot is free that much later
         auto load = [&](int which, int j, int blk) {
@@ -894,8 +899,8 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
   }
   const long long units = (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv;
   const int grid = units < FA_SMS ? (int)units : FA_SMS;
-  kern<<<grid, FA_THREADS, C::SMEM, st>>>(map, a);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(kern, grid, FA_THREADS, C::SMEM, st, 1, map, a));
+  count_launch();
   return B200Q_OK;
 }
 

@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* __r
                                                                 int n_groups, int keep, int shared,
                                                                 int32_t* __restrict__ idx, float* __restrict__ wts) {
   __shared__ float gscore[4][ROUTE_MAX_GROUPS];
+  follow_previous(logits, corr, idx, wts);
   const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + wi;
   if (t >= Tn) return;
@@ -308,6 +309,7 @@ __global__ void __launch_bounds__(1024) moe_plan_part_kernel(const int32_t* __re
                                                              int32_t* __restrict__ perm_tok, int32_t* __restrict__ pair_pos,
                                                              int32_t* __restrict__ tile_tab, int32_t* __restrict__ n_tiles) {
   extern __shared__ int32_t si[];  // counts[E] | offs[E+1] | cursor[E]
+  follow_previous(idx, group_off, perm_tok, pair_pos, tile_tab, n_tiles);
   int32_t* counts = si;
   int32_t* offs = si + E;
   int32_t* cursor = offs + E + 1;
@@ -394,6 +396,7 @@ __global__ void __launch_bounds__(256) residual_add_routed_v8_kernel(float* __re
                                                                      const int32_t* __restrict__ idx,
                                                                      const float* __restrict__ wts, int top, int n_real,
                                                                      const bf16* __restrict__ h, int Tn, int W8) {
+  follow_previous(x, eout, pair_pos, idx, wts, h);
   const long long total = (long long)Tn * W8;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
     const int t = (int)(e / W8), c = (int)(e - (long long)t * W8) * 8;
@@ -536,12 +539,12 @@ int b200q_moe_route_grouped(const float* logits, const float* correction, int T_
                   "moe_route_grouped: bad argument (E=%d top=%d groups=%d keep=%d; groups divide E, at most %d groups, "
                   "top fits the kept groups)", E, top, n_groups, keep, ROUTE_MAX_GROUPS);
   if (T_ == 0) return B200Q_OK;
-  moe_route_grouped_kernel<false><<<(T_ + 3) / 4, 128, 0, as_stream(stream)>>>(logits, E, correction, T_, E, top, n_groups,
-                                                                              keep, 0, idx, wts);
-  B200Q_LAUNCH_CHECK();
-  moe_plan_part_kernel<<<1, 1024, (size_t)(3 * E + 1) * sizeof(int32_t), as_stream(stream)>>>(
-      idx, T_ * top, top, E, e_gemm, group_off, perm_tok, pair_pos, tile_tab, n_tiles);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(moe_route_grouped_kernel<false>, (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, E, correction, T_, E, top,
+                          n_groups, keep, 0, idx, wts));
+  count_launch();
+  B200Q_CUDA(launch_early(moe_plan_part_kernel, 1, 1024, (size_t)(3 * E + 1) * sizeof(int32_t), as_stream(stream), 1, idx, T_ * top, top, E,
+                          e_gemm, group_off, perm_tok, pair_pos, tile_tab, n_tiles));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -556,12 +559,12 @@ int b200q_moe_route_gated(const float* logits, int ld, const float* correction, 
                   "the kept groups)", E, top, n_groups, keep, ROUTE_MAX_GROUPS);
   if (T_ == 0) return B200Q_OK;
   const int per = top + shared, n = E + shared;
-  moe_route_grouped_kernel<true><<<(T_ + 3) / 4, 128, 0, as_stream(stream)>>>(logits, ld, correction, T_, E, top, n_groups,
-                                                                             keep, shared, idx, wts);
-  B200Q_LAUNCH_CHECK();
-  moe_plan_part_kernel<<<1, 1024, (size_t)(3 * n + 1) * sizeof(int32_t), as_stream(stream)>>>(
-      idx, T_ * per, per, n, n, group_off, perm_tok, pair_pos, tile_tab, n_tiles);
-  B200Q_LAUNCH_CHECK();
+  B200Q_CUDA(launch_early(moe_route_grouped_kernel<true>, (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, ld, correction, T_, E, top,
+                          n_groups, keep, shared, idx, wts));
+  count_launch();
+  B200Q_CUDA(launch_early(moe_plan_part_kernel, 1, 1024, (size_t)(3 * n + 1) * sizeof(int32_t), as_stream(stream), 1, idx, T_ * per, per, n,
+                          n, group_off, perm_tok, pair_pos, tile_tab, n_tiles));
+  count_launch();
   return B200Q_OK;
 }
 
@@ -595,8 +598,8 @@ int b200q_residual_add_routed(float* x, const void* expert_out, const int32_t* p
   if (T_ == 0) return B200Q_OK;
   if (dtype == B200Q_DTYPE_BF16 && W % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(expert_out) | reinterpret_cast<uintptr_t>(h)) & 15) == 0)
-    residual_add_routed_v8_kernel<<<grid_for((long long)T_ * W / 8), 256, 0, as_stream(stream)>>>(
-        x, (const bf16*)expert_out, pair_pos, idx, wts, top, n_real, (const bf16*)h, T_, W / 8);
+    B200Q_CUDA(launch_early(residual_add_routed_v8_kernel, grid_for((long long)T_ * W / 8), 256, 0, as_stream(stream), 1, x,
+                            (const bf16*)expert_out, pair_pos, idx, wts, top, n_real, (const bf16*)h, T_, W / 8));
   else
     DISPATCH_T(dtype, (residual_add_routed_kernel<T><<<grid_for((long long)T_ * W), 256, 0, as_stream(stream)>>>(
                           x, (const T*)expert_out, pair_pos, idx, wts, top, n_real, (const T*)h, T_, W)));

@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(256) silu_glu_kernel(const T* __restrict__ gu,
 }
 __global__ void __launch_bounds__(256) silu_glu_v8_kernel(const bf16* __restrict__ gu, bf16* __restrict__ y,
                                                           long long rows, int F) {
+  follow_previous(gu, y);
   const int per = F / 8;
   const long long total = rows * per;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -648,8 +649,9 @@ int b200q_silu_glu(const void* gate_up, void* y, int64_t rows, int F, int dtype,
   if (rows == 0) return B200Q_OK;
   if (dtype == B200Q_DTYPE_BF16 && F % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
-    silu_glu_v8_kernel<<<grid_for(rows * (F / 8)), 256, 0, as_stream(stream)>>>((const bf16*)gate_up, (bf16*)y, rows, F);
-    B200Q_LAUNCH_CHECK();
+    B200Q_CUDA(launch_early(silu_glu_v8_kernel, grid_for(rows * (F / 8)), 256, 0, as_stream(stream), 1, (const bf16*)gate_up, (bf16*)y,
+                            (long long)rows, F));
+    count_launch();
     return B200Q_OK;
   }
   DISPATCH_T(dtype, (silu_glu_kernel<T><<<grid_for(rows * F), 256, 0, as_stream(stream)>>>((const T*)gate_up, (T*)y,

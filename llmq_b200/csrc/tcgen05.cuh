@@ -235,6 +235,6 @@ int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const 
 bool gemm_skinny_ok(int M, int N, int K, bool gated);
 int gemm_skinny_splits(int M, int N, int K);
 int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int act, long long ldc, const float* bias, float limit,
-                float* parts, cudaStream_t st);
+                float* parts, bool fixed_w, cudaStream_t st);
 
 }  // namespace b200q
