@@ -10,7 +10,8 @@
 //     start and its end;
 //   * the first weights are asked for before the kernel before this one has ended (follow_previous): into the ring where nobody can
 //     still be writing them (fixed_w), into L2 otherwise.
-// A gated unit (SwiGLU, GeGLU, clamped) works on gate rows in the first 128 rows of a 256-row tile and up rows in the other.
+// A gated unit (SwiGLU, GeGLU, clamped) works on a 128-row tile of 64 gate rows and the 64 rows that they gate: few or no splits whose
+// parts would have to meet (28672 x 4096, 100 rows: 44.7 us, 48.0 with tiles of 128 + 128 rows; 16384 x 2048, 48 rows: 14.2, 16.3).
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -48,7 +49,9 @@ template <int WT, int kAct>
 __global__ void __launch_bounds__(SK_THREADS, 2)
     gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const SkinnyArgs a) {
   constexpr int NT = WT * 128;
-  static_assert(kAct == ACT_NONE || WT == 2, "a gated unit needs both halves");
+  // (a gated unit's tile is 64 gate rows and the 64 rows that they gate, out of a block of 256 weight rows)
+  constexpr bool kGated = kAct != ACT_NONE;
+  static_assert(!kGated || WT == 1, "a gated unit's tile is 128 rows");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], done;
@@ -56,6 +59,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   __shared__ int dead;  // a wait ran out: the other roles stop as well
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int split = blockIdx.x, splits = gridDim.x, tile = blockIdx.y;
+  const int gate_row = tile / 2 * 256 + tile % 2 * 64;
   const int kb_all = a.K / SK_BK, kb0 = split * kb_all / splits, kb1 = (split + 1) * kb_all / splits;
   const int stage_bytes = WT * SK_TILE_BYTES + a.mp * (SK_BK * 2);
 
@@ -79,12 +83,23 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   // every tile begins at another k-block: all of them asking for the same rows of A at once cost 2-4 % at 64 rows and more
   // (short reductions keep the order that the kernels for larger steps add in)
   const int kb_first = kb0 + (kb1 - kb0 >= 16 ? tile * 5 % (kb1 - kb0) : 0), early = min(a.stages, kb1 - kb0);
+  auto load_w = [&](uint8_t* to, int kb, uint64_t* bar) {
+    if constexpr (kGated) {
+      tma_load_2d(to, &tmap_w, kb * SK_BK, gate_row, bar);
+      tma_load_2d(to + SK_TILE_BYTES / 2, &tmap_w, kb * SK_BK, gate_row + 128, bar);
+    } else {
+      tma_load_2d(to, &tmap_w, kb * SK_BK, tile * NT, bar);
+    }
+  };
   if (warp == 0 && lane == 0) {  // the first weights while the kernels before this one end
     int kb = kb_first;
     for (int i = 0; i < min(a.ahead, kb1 - kb0); ++i, kb = kb + 1 < kb1 ? kb + 1 : kb0) {
       if (a.fixed_w && i < early) {
         mbar_expect_tx(full + i, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
-        tma_load_2d(smem + i * stage_bytes, &tmap_w, kb * SK_BK, tile * NT, full + i);
+        load_w(smem + i * stage_bytes, kb, full + i);
+      } else if constexpr (kGated) {
+        tma_prefetch_2d(&tmap_w, kb * SK_BK, gate_row);
+        tma_prefetch_2d(&tmap_w, kb * SK_BK, gate_row + 128);
       } else {
         tma_prefetch_2d(&tmap_w, kb * SK_BK, tile * NT);
       }
@@ -104,7 +119,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
         if (!a.fixed_w || asked >= early) {
           if (!mbar_wait_or_fail(empty + stage, phase ^ 1u, &dead, a.failed)) break;
           mbar_expect_tx(full + stage, (uint32_t)(WT * SK_TILE_BYTES + a.a_bytes));
-          tma_load_2d(sw, &tmap_w, kb * SK_BK, tile * NT, full + stage);
+          load_w(sw, kb, full + stage);
         }
         tma_load_2d(sw + WT * SK_TILE_BYTES, &tmap_a, kb * SK_BK, 0, full + stage);
         if (++stage == a.stages) {
@@ -119,7 +134,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
     int stage = 0;
     uint32_t phase = 0;
     for (int i = kb0; i < kb1; ++i) {
-      if (!__all_sync(0xffffffffu, mbar_wait_or_fail(full + stage, phase, &dead, a.failed, a.patience))) break;
+      if (!mbar_wait_warp(full + stage, phase, &dead, a.failed, a.patience)) break;
       tc_fence_after();
       if (elect_one()) {
         const uint32_t sw = smem_u32(smem + stage * stage_bytes), sa = sw + WT * SK_TILE_BYTES;
@@ -143,44 +158,59 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
   }
 
   // ---- the accumulators: lane = weight row, column = row of A ----
-  float* red = reinterpret_cast<float*>(smem);  // [chunk][NT]; the ring is free once every product has been made
   const bool epi = warp >= 2;
   const int quarter = warp & 3, row = quarter * 32 + lane;
   if (epi) {
-    mbar_wait_or_fail(&done, 0, &dead, a.failed);
+    mbar_wait_or_fail<16>(&done, 0, &dead, a.failed);
     __syncwarp();
     tc_fence_after();
   }
   // (products that stop early say so before `done`: copies may then still arrive in the ring, which is left alone)
   const bool give = epi && *(volatile int*)&dead == 0;
+  // 32 columns of the accumulator: a load takes some 0.2 us, so that both are asked for before the first is used (2048 x 2048 in five
+  // parts, 48 rows: 1.6 -> 0.6 us from the last product to the end of the CTA; 64 columns at a time are no faster and take the registers
+  // that the next kernel's CTAs need beside this one's)
+  auto columns = [&](int h, int c, int n, uint32_t(&v)[2][16]) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+      if (16 * x < n) tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * a.mp + c + 16 * x), v[x]);
+    tmem_ld_wait();
+  };
   if (a.parts) {
     if (epi) {
       float* dst = a.parts + (long long)split * a.M * a.N + (long long)tile * NT + row;
 #pragma unroll 1
       for (int h = 0; h < WT; ++h)
 #pragma unroll 1
-        for (int c = 0; c < a.mp; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * a.mp + c), v);
-          tmem_ld_wait();
+        for (int c = 0; c < a.M; c += 32) {
+          uint32_t v[2][16];
+          columns(h, c, a.M - c, v);
+          float* d = dst + h * 128 + (long long)c * a.N;
+          const int n = a.M - c;
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c + j < a.M) dst[(long long)(c + j) * a.N + h * 128] = __uint_as_float(v[j]);
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int j = 0; j < 16; ++j, d += a.N)
+              if (16 * x + j < n) *d = __uint_as_float(v[x][j]);
         }
     }
   } else {
+    float* red = reinterpret_cast<float*>(smem);
     for (int c0 = 0; c0 < a.M; c0 += a.chunk) {
       if (give) {
         const int cn = min(a.chunk, a.mp - c0);
 #pragma unroll 1
         for (int h = 0; h < WT; ++h)
 #pragma unroll 1
-          for (int c = 0; c < cn; c += 16) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * a.mp + c0 + c), v);
-            tmem_ld_wait();
+          for (int c = 0; c < cn; c += 32) {
+            uint32_t v[2][16];
+            columns(h, c0 + c, cn - c, v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) red[(c + j) * NT + h * 128 + row] = __uint_as_float(v[j]);
+            for (int x = 0; x < 2; ++x)
+              if (c + 16 * x < cn) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) red[(c + 16 * x + j) * NT + h * 128 + row] = __uint_as_float(v[x][j]);
+              }
           }
       }
       if (splits > 1)
@@ -188,40 +218,40 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
       else
         __syncthreads();
       // rows split, split + splits, ... of the chunk are this CTA's to add and store, four columns of C per thread
-      constexpr int OUT = kAct != ACT_NONE ? 128 : NT, GR = OUT / 4;
+      constexpr int OUT = kGated ? NT / 2 : NT, GR = OUT / 4;
       const int rows = min(a.chunk, a.M - c0), mine = rows > split ? (rows - split + splits - 1) / splits : 0;
       for (int i = threadIdx.x; i < mine * GR; i += SK_THREADS) {
         const int r = (i / GR) * splits + split, n = (i % GR) * 4;
         const float* src = red + r * NT + n;
         // (all partial sums are asked for before the first is added: a remote read takes about 200 cycles)
-        float4 p[SK_MAX_SPLITS], q[kAct != ACT_NONE ? SK_MAX_SPLITS : 1];
+        float4 p[SK_MAX_SPLITS], q[kGated ? SK_MAX_SPLITS : 1];
         if (splits > 1) {
 #pragma unroll
           for (int s = 0; s < SK_MAX_SPLITS; ++s)
             if (s < splits) {
               const uint32_t at = mapa_shared(src, s);
               p[s] = ld_cluster_v4(at);
-              if constexpr (kAct != ACT_NONE) q[s] = ld_cluster_v4(at + 512);
+              if constexpr (kGated) q[s] = ld_cluster_v4(at + OUT * 4);
             }
         } else {
           p[0] = *reinterpret_cast<const float4*>(src);
-          if constexpr (kAct != ACT_NONE) q[0] = *reinterpret_cast<const float4*>(src + 128);
+          if constexpr (kGated) q[0] = *reinterpret_cast<const float4*>(src + OUT);
         }
         float4 x = p[0], y = x;
-        if constexpr (kAct != ACT_NONE) y = q[0];
+        if constexpr (kGated) y = q[0];
 #pragma unroll
         for (int s = 1; s < SK_MAX_SPLITS; ++s)
           if (s < splits) {
             x.x += p[s].x; x.y += p[s].y; x.z += p[s].z; x.w += p[s].w;
-            if constexpr (kAct != ACT_NONE) { y.x += q[s].x; y.y += q[s].y; y.z += q[s].z; y.w += q[s].w; }
+            if constexpr (kGated) { y.x += q[s].x; y.y += q[s].y; y.z += q[s].z; y.w += q[s].w; }
           }
         float o[4] = {x.x, x.y, x.z, x.w};
-        if constexpr (kAct != ACT_NONE) {
+        if constexpr (kGated) {
           const float u[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if constexpr (kAct == ACT_CLAMPED) {
-              const float* b = bias + (long long)tile * NT + n + j;
+              const float* b = bias + gate_row + n + j;
               o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), bias ? __ldg(b) : 0.f, bias ? __ldg(b + 128) : 0.f,
                                   a.limit);
             } else {
@@ -282,13 +312,14 @@ struct SkinnyPlan {
   bool alone;
   int splits;
 };
-// Measured on B200, weights from HBM, back to back in a graph, us (new kernel / the kernels of gemm_tcgen05.cu before it):
-//   rows                        1            64           100
-//   4096 x 4096            10.6 / 12.5  12.3 / 13.7  13.3 / 14.5
-//   4096 x 14336           24.1 / 26.5  26.1 / 29.4  28.1 / 29.9
-//   16384 x 2048 gated     15.6 / 45.8  19.6 / 46.1  22.1 / 45.9
-//   28672 x 4096 gated     41.5 / 70.5  48.4 / 72.9  53.1 / 72.5
-//   3072 x 2048             6.8 /  8.3   8.7 / 10.9   9.4 / 12.1   (the launch itself is most of it)
+// Measured on B200, weights from HBM, back to back in a graph, us (here / the kernels of gemm_tcgen05.cu; both begin while the product
+// before them ends):
+//   rows                        1            48           100          128
+//   3072 x 2048             5.2 /  6.3   6.8 /  8.0   8.0 /  9.6   8.5 / 10.5
+//   4096 x 4096             8.6 /  9.2  10.4 / 10.6  11.2 / 11.7  11.8 / 13.1
+//   4096 x 14336           21.3 / 22.4  23.8 / 24.7  24.3 / 26.7  25.2 / 28.9
+//   16384 x 2048 gated     12.9 / 43.2  14.4 / 43.7  17.3 / 44.1  18.1 / 25.1
+//   28672 x 4096 gated     38.7 / 66.4  41.1 / 68.3  45.7 / 68.8  47.7 / 50.2
 // Splits: up to 64 rows two CTAs per SM with three or more stages each are best; with more rows a stage grows and one CTA per SM
 // with the whole memory as its ring is (28.7 against 29.7 us at 4096 x 14336, 100 rows), unless the tiles alone would leave half
 // of the SMs idle.  All clusters have to be resident at once: a cluster lies within a processing cluster of the chip, and one
@@ -330,7 +361,7 @@ static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_
   a.ahead = (int)(SK_AHEAD_BYTES / ((long long)(a.N / (WT * 128)) * p.splits * WT * SK_TILE_BYTES));
   if (a.ahead < a.stages) a.ahead = a.stages;
   CUtensorMap tw, ta;
-  rc = get_tmap(W, a.N, a.K, WT * 128, &tw);
+  rc = get_tmap(W, a.N, a.K, kAct != ACT_NONE ? 64 : WT * 128, &tw);
   if (rc) return rc;
   rc = get_tmap(A, a.M, a.K, a_rows, &ta);
   if (rc) return rc;
@@ -345,7 +376,7 @@ static int launch_skinny(const void* A, const void* W, SkinnyArgs a, cudaStream_
 }
 
 // Tiles of 256 rows halve what a CTA re-reads of A, tiles of 128 give twice the CTAs: 256 only where 128 would give more than
-// two for every SM (and for gated units, which need both halves).
+// two for every SM.
 static bool wide_tiles(int N) { return N % 256 == 0 && N / 256 >= 148; }
 
 // Which products the kernel above takes; us, here / kernels of gemm_tcgen05.cu:
@@ -358,11 +389,11 @@ static bool wide_tiles(int N) { return N % 256 == 0 && N / 256 >= 148; }
 //     at 128; K = 8192 1.02 at 100; two CTAs per SM hide some of it: 24576 x 2048 0.97 at 64 rows, 1.08 at 128.
 //   * plain, tiles of 256 (vocabulary sizes): up to 32 rows (128256 x 2048 86 / 88); up to 112 where K >= 4096 and the tiles fill rounds
 //     of two CTAs per SM (128256 x 4096 177 / 179 at 100 rows, 1.7 rounds; but 50176 x 5120 98 / 89, 0.66).
-//   * gated: below 128 rows always: the kernels there spend 15 to 20 us on the division of rows that do not exist (28672 x 4096 54 / 73 at
-//     113, 2048 x 512 6 / 40 at one row).  At 128: 16384 x 2048 24 / 28, but 28672 x 3584 51 / 49, 2048 x 512 16 / 15.
+//   * gated: always (16384 x 2048 13 / 43 at one row, 18 / 25 at 128; 28672 x 4096 46 / 69 at 112, 47.7 / 50.2 at 128; 2048 x 512 5 / 32,
+//     9.8 / 13.7); the kernels there spend 15 to 20 us on the division of rows that do not exist.
 bool gemm_skinny_ok(int M, int N, int K, bool gated) {
   if (M < 1 || M > 128 || K % SK_BK != 0 || N % (gated ? 256 : 128) != 0 || N / 128 > 65535) return false;
-  if (gated) return M < 128 || (K >= 1024 && N / 256 <= 74);
+  if (gated) return true;
   if (wide_tiles(N)) {
     const int tiles = N / 256, rounds = (tiles + 295) / 296;
     return M <= 32 || (M <= 112 && K >= 4096 && 5 * tiles >= 4 * 296 * rounds);
@@ -391,9 +422,9 @@ int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int 
   a.M = M;
   a.N = N;
   a.K = K;
-  if (act == ACT_SWIGLU) return launch_skinny<2, ACT_SWIGLU>(A, W, a, st);
-  if (act == ACT_GEGLU) return launch_skinny<2, ACT_GEGLU>(A, W, a, st);
-  if (act == ACT_CLAMPED) return launch_skinny<2, ACT_CLAMPED>(A, W, a, st);
+  if (act == ACT_SWIGLU) return launch_skinny<1, ACT_SWIGLU>(A, W, a, st);
+  if (act == ACT_GEGLU) return launch_skinny<1, ACT_GEGLU>(A, W, a, st);
+  if (act == ACT_CLAMPED) return launch_skinny<1, ACT_CLAMPED>(A, W, a, st);
   return wide_tiles(N) ? launch_skinny<2, ACT_NONE>(A, W, a, st) : launch_skinny<1, ACT_NONE>(A, W, a, st);
 }
 

@@ -137,6 +137,24 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// the same for a whole warp, whose lanes agree on the outcome; flag and clock are looked at every 64 tries (a look in between costs 140
+// cycles where the data is about to come)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* dead, int* failed, long long limit) {
+  if (limit >= 0) {
+    long long t0 = 0;
+    for (int n = 0;; ++n) {
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+      if (n % 64 != 63) continue;
+      if (n == 63) t0 = clock64();
+      if (__any_sync(0xffffffffu, *dead || clock64() - t0 > limit)) break;
+    }
+  }
+  *dead = 1;
+  __threadfence_block();
+  *(volatile int*)failed = 1;
+  return false;
+}
+
 // ---- q-tiles of prompt attention: {block table row, first row, rows, first position} -----------
 // keys that the last token of tile i's portion sees (a whole warp asks; neighbouring tiles of one sequence that continue each other are a
 // portion), as far as 31 tiles on: exact for a comparison with up to 512

@@ -124,3 +124,32 @@ def test_waits_that_run_out(cuda):
     r = subprocess.run([sys.executable, "-c", "from tests.test_gemm_skinny_gpu import give_up; give_up()"], cwd=root, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "right again" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("M", [31, 32, 33, 48, 96, 97])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (512, 4096), (33024, 128), (38144, 128)])
+def test_rows_at_the_edges_of_accumulator_loads(cuda, M, N, K):
+    """32 rows of A leave tensor memory at a time, 16 to a load: one load, a half, none of the second; tiles of 128 and 256 weight rows"""
+    test_plain(cuda, M, N, K)
+    test_gated(cuda, M, N, K, "swiglu")
+    test_gated(cuda, M, N, K, "clamped_bias")
+
+
+@pytest.mark.parametrize("M", [1, 16, 33, 64, 128])
+def test_parts_are_the_sum(cuda, M):
+    """the parts of a split reduction that the next kernel adds up are those that the product itself adds"""
+    import ctypes as C
+    from llmq_b200 import lib
+    N, K = 2048, 2048
+    a, w = rnd(cuda, M, K, seed=M), rnd(cuda, N, K, seed=N + K, scale=K ** -0.5)
+    ptr, splits = lib.gemm_bf16_splitk(a, w)
+    assert splits > 1
+    torch.cuda.synchronize()
+    parts = torch.empty(splits, M, N, device=cuda)
+    lib.check(lib.load().b200q_copy_f32(C.c_void_p(ptr), C.c_void_p(parts.data_ptr()), parts.numel(), torch.cuda.current_stream().cuda_stream))
+    c = torch.empty(M, N, dtype=BF, device=cuda)
+    lib.gemm_bf16(a, w, c)
+    total = parts[0].clone()
+    for s in range(1, splits):
+        total += parts[s]
+    assert torch.equal(total.to(BF), c)
