@@ -28,6 +28,10 @@ namespace b200q {
 
 constexpr int DEC_WARPS = 4;
 constexpr int PF_STAGES = 4;
+// cached rows that a forward pass asks into L2 while the kernels before the attention run (their tables are older than the pass; the rows
+// are read behind follow_previous, so what a kernel of the pass writes into a page is seen).  48 sequences of 100 to 900 tokens, D = 64,
+// 8 kv heads: 13.3 -> 11.8 us from the end of the kernel before to the end of the attention.
+constexpr long long DEC_AHEAD_BYTES = 48000000;
 // decode ring depth per warp: 3 pages of K+V in flight (2 at D = 256, where a page is 8 KB)
 template <int D>
 struct DecCfg {
@@ -193,7 +197,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
                        const uint8_t* __restrict__ kv_layer,
                        const int32_t* __restrict__ block_table, int bt_stride,
                        const int32_t* __restrict__ ctx_lens, int n_q, int n_kv, int G,
-                       float c0, float c1, int window) {
+                       float c0, float c1, int window, int ahead) {
+  // ahead: pages per warp that are asked into L2 before the kernel before this one has ended; 0: that one may write the tables
   using G_ = Geo<D, BS>;
   using S_ = DecSmem<D, BS>;
   constexpr int DEC_STAGES = S_::STAGES;
@@ -213,7 +218,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
     mbar_fence_init();
   }
   __syncwarp();
-  follow_previous(q, out, kv_layer, block_table, ctx_lens);
+  if (ahead == 0) follow_previous(q, out, kv_layer, block_table, ctx_lens);
+  // (without a window the first page's place in the table does not wait for the length; what lies behind the sequence is not used)
+  const int32_t* bt_row = block_table + (long long)seq * bt_stride;
+  const int guess = window <= 0 && wg + n_warps * lane < bt_stride ? __ldg(bt_row + wg + n_warps * lane) : 0;
   const int ctx = __ldg(ctx_lens + seq);
   // the query sits at position ctx-1 and sees keys [lo, ctx); pages before lo's page are skipped
   const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
@@ -221,11 +229,21 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   const int n_pages = (ctx + BS - 1) / BS - page0;
   const int my_n = n_pages > wg ? (n_pages - wg + n_warps - 1) / n_warps : 0;
 
-  const int32_t* bt = block_table + (long long)seq * bt_stride + page0;
+  const int32_t* bt = bt_row + page0;
   const long long page_stride = (long long)G_::PAGE_BYTES;  // bytes per (block,kv,head) page
   // page address: ((blk*2 + kv) * n_kv + kvh) * PAGE_BYTES
   int ids_base = 0;
-  int ids = (lane < my_n) ? __ldg(bt + wg + n_warps * lane) : 0;
+  int ids = window <= 0 ? guess : (lane < my_n) ? __ldg(bt + wg + n_warps * lane) : 0;
+  if (ahead > 0) {
+    if (lane < min(my_n, ahead)) {
+      const uint32_t bytes = (uint32_t)min(BS, ctx - (page0 + wg + n_warps * lane) * BS) * G_::ROW_BYTES;
+      const uint8_t* kp = kv_layer + ((long long)ids * 2 * n_kv + kvh) * page_stride;
+      bulk_prefetch_l2(kp, bytes);
+      bulk_prefetch_l2(kp + n_kv * page_stride, bytes);
+    }
+    __syncwarp();
+    follow_previous(q, out, kv_layer);
+  }
 
   auto issue = [&](int k) {  // whole warp calls; k = warp-local page index
     if (k - ids_base >= 32) {
@@ -366,51 +384,63 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
       mo[D + 1] = l;
     }
   }
-  if constexpr (!kShared) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < G * D; idx += DEC_WARPS * 32) {
-      const int r = idx / D, d = idx % D;
-      float M = -INFINITY;
+  __syncthreads();
+  // one state per CTA; where CTAs share the sequence it goes, not yet divided, to [G][D] | maxima [G] | sums [G] in the ring, which is free
+  float* state = reinterpret_cast<float*>(smem);
+  for (int idx = threadIdx.x; idx < G * D; idx += DEC_WARPS * 32) {
+    const int r = idx / D, d = idx % D;
+    float M = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, merge[(w * 8 + r) * (D + 2) + D]);
-      float num = 0.f, den = 0.f;
+    for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, merge[(w * 8 + r) * (D + 2) + D]);
+    float num = 0.f, den = 0.f;
 #pragma unroll
-      for (int w = 0; w < DEC_WARPS; ++w) {
-        const float* mo = merge + (w * 8 + r) * (D + 2);
-        const float wgt = (mo[D] == -INFINITY) ? 0.f : exp2f(mo[D] - M);
-        num += wgt * mo[d];
-        den += wgt * mo[D + 1];
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float* mo = merge + (w * 8 + r) * (D + 2);
+      const float wgt = (mo[D] == -INFINITY) ? 0.f : exp2f(mo[D] - M);
+      num += wgt * mo[d];
+      den += wgt * mo[D + 1];
+    }
+    if constexpr (kShared) {
+      state[idx] = num;
+      if (d == 0) {
+        state[G * D + r] = M;
+        state[G * D + G + r] = den;
       }
+    } else {
       const float v = den > 0.f ? num / den : 0.f;
       out[(long long)seq * n_q * D + (long long)(kvh * G + r) * D + d] = __float2bfloat16_rn(v);
     }
-    return;
   }
-  cluster_sync_all();
-  for (int idx = split * DEC_WARPS * 32 + threadIdx.x; idx < G * D; idx += splits * DEC_WARPS * 32) {
-    const int r = idx / D, d = idx % D;
-    float M = -INFINITY, num = 0.f, den = 0.f;
-    // (warps of the cluster in order; two passes, so that the largest maximum is known before anything is added)
-    for (int s = 0; s < splits; ++s) {
-      const uint32_t base = mapa_shared(merge, s);
+  if constexpr (kShared) {
+    cluster_sync_all();
+    // this CTA's share of the outputs; the states of all CTAs are asked for before the first is used (a remote read takes some 200 cycles)
+    const int per = (G * D + splits - 1) / splits;
+    for (int idx = split * per + threadIdx.x; idx < min((split + 1) * per, G * D); idx += DEC_WARPS * 32) {
+      const int r = idx / D, d = idx % D;
+      float v[8], m_s[8], l_s[8];
 #pragma unroll
-      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, ld_cluster_f32(base + ((w * 8 + r) * (D + 2) + D) * 4));
-    }
-    for (int s = 0; s < splits; ++s) {
-      const uint32_t base = mapa_shared(merge, s);
-#pragma unroll
-      for (int w = 0; w < DEC_WARPS; ++w) {
-        const uint32_t mo = base + (w * 8 + r) * (D + 2) * 4;
-        const float m_w = ld_cluster_f32(mo + D * 4), v_w = ld_cluster_f32(mo + d * 4), l_w = ld_cluster_f32(mo + (D + 1) * 4);
-        const float wgt = m_w == -INFINITY ? 0.f : exp2f(m_w - M);
-        num += wgt * v_w;
-        den += wgt * l_w;
+      for (int x = 0; x < 8; ++x) {
+        const uint32_t base = mapa_shared(state, min(x, splits - 1));
+        v[x] = ld_cluster_f32(base + idx * 4);
+        m_s[x] = ld_cluster_f32(base + (G * D + r) * 4);
+        l_s[x] = ld_cluster_f32(base + (G * D + G + r) * 4);
       }
+      float M = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+      for (int x = 0; x < 8; ++x)
+        if (x < splits) M = fmaxf(M, m_s[x]);
+#pragma unroll
+      for (int x = 0; x < 8; ++x)
+        if (x < splits) {
+          const float wgt = m_s[x] == -INFINITY ? 0.f : exp2f(m_s[x] - M);
+          num += wgt * v[x];
+          den += wgt * l_s[x];
+        }
+      const float o_v = den > 0.f ? num / den : 0.f;
+      out[(long long)seq * n_q * D + (long long)(kvh * G + r) * D + d] = __float2bfloat16_rn(o_v);
     }
-    const float v = den > 0.f ? num / den : 0.f;
-    out[(long long)seq * n_q * D + (long long)(kvh * G + r) * D + d] = __float2bfloat16_rn(v);
+    cluster_sync_all();  // nobody leaves while a peer still reads
   }
-  cluster_sync_all();  // nobody leaves while a peer still reads
 }
 
 // ------------------------------------------------------------------------------------------
@@ -920,7 +950,7 @@ static int decode_splits(int n_seqs, int n_kv, int bt_stride, int window) {
 template <int D, int BS, bool kCap, bool kShared>
 static int launch_decode_form(int splits, const void* q, int q_stride, void* out, const void* kv,
                          const int32_t* bt, int bt_stride, const int32_t* ctx, int n_seqs, int n_q,
-                         int n_kv, float scale, float softcap, int window, cudaStream_t st) {
+                         int n_kv, float scale, float softcap, int window, int ahead, cudaStream_t st) {
   auto kern = decode_attn_kernel<D, BS, kCap, kShared>;
   const int rc = prepare_decode<D, BS, kCap, kShared>();
   if (rc) return rc;
@@ -928,20 +958,26 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = decode_config<D, BS, kShared>(splits, n_seqs, n_kv, &attr, st);
   B200Q_CUDA(launch_early(kern, cfg.gridDim, DEC_WARPS * 32, cfg.dynamicSmemBytes, st, splits, (const bf16*)q, q_stride, (bf16*)out,
-                          (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window));
+                          (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window, ahead));
   count_launch();
   return B200Q_OK;
 }
 
 template <int D, int BS, bool kCap>
 static int launch_decode(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* ctx,
-                         int n_seqs, int n_q, int n_kv, float scale, float softcap, int window, cudaStream_t st) {
+                         int n_seqs, int n_q, int n_kv, float scale, float softcap, int window, bool tables_known, cudaStream_t st) {
   const int splits = decode_splits<D, BS, kCap>(n_seqs, n_kv, bt_stride, window);
+  int ahead = 0;
+  if (tables_known) {
+    const long long each = (long long)n_seqs * n_kv * splits * DEC_WARPS * 2 * Geo<D, BS>::PAGE_BYTES;
+    ahead = DEC_AHEAD_BYTES / each < 32 ? (int)(DEC_AHEAD_BYTES / each) : 32;
+    if (ahead < 1) ahead = 1;
+  }
   if (splits > 1)
     return launch_decode_form<D, BS, kCap, true>(splits, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap,
-                                                 window, st);
+                                                 window, ahead, st);
   return launch_decode_form<D, BS, kCap, false>(1, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap, window,
-                                                st);
+                                                ahead, st);
 }
 
 template <int D, int BS, bool kCap>
@@ -1008,6 +1044,28 @@ int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const 
                       st);
 }
 
+int decode_attn(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                const int32_t* ctx_lens, int n_seqs, int n_q, int n_kv, int D, int block_size, float scale, float softcap, int window,
+                bool tables_known, cudaStream_t st) {
+  B200Q_CHECK_ARG(n_seqs >= 0 && n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 8,
+                  "decode_attn: unsupported heads n_q=%d n_kv=%d (GQA group must be <= 8)", n_q,
+                  n_kv);
+  B200Q_CHECK_ARG(block_size == 16 && (D == 64 || D == 128 || D == 256),
+                  "decode_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D,
+                  block_size);
+  if (n_seqs == 0) return B200Q_OK;
+  // streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
+  // another order of sums)
+  const bool stream_variant =
+      g_decode_variant >= 2 ||
+      (g_decode_variant == 0 && !batch_invariant() && (long long)n_seqs * n_kv >= 16LL * attn_num_sms());
+  if (stream_variant)
+    B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
+                        ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);
+  B200Q_ATTN_DISPATCH(launch_decode, q, q_stride, out, kv_layer, block_table, bt_stride, ctx_lens,
+                      n_seqs, n_q, n_kv, scale, softcap, window, tables_known, st);
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -1026,24 +1084,8 @@ int b200q_decode_attn_ex(const void* q, int q_stride, void* out, const void* kv_
                          const int32_t* block_table, int bt_stride, const int32_t* ctx_lens,
                          int n_seqs, int n_q, int n_kv, int D, int block_size, float scale,
                          float softcap, int window, void* stream) {
-  B200Q_CHECK_ARG(n_seqs >= 0 && n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 8,
-                  "decode_attn: unsupported heads n_q=%d n_kv=%d (GQA group must be <= 8)", n_q,
-                  n_kv);
-  B200Q_CHECK_ARG(block_size == 16 && (D == 64 || D == 128 || D == 256),
-                  "decode_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D,
-                  block_size);
-  if (n_seqs == 0) return B200Q_OK;
-  cudaStream_t st = as_stream(stream);
-  // streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
-  // another order of sums)
-  const bool stream_variant =
-      g_decode_variant >= 2 ||
-      (g_decode_variant == 0 && !batch_invariant() && (long long)n_seqs * n_kv >= 16LL * attn_num_sms());
-  if (stream_variant)
-    B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
-                        ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);
-  B200Q_ATTN_DISPATCH(launch_decode, q, q_stride, out, kv_layer, block_table, bt_stride, ctx_lens,
-                      n_seqs, n_q, n_kv, scale, softcap, window, st);
+  return decode_attn(q, q_stride, out, kv_layer, block_table, bt_stride, ctx_lens, n_seqs, n_q, n_kv, D, block_size, scale, softcap, window,
+                     false, as_stream(stream));
 }
 
 int b200q_decode_attn(const void* q, int q_stride, void* out, const void* kv_layer,

@@ -22,6 +22,11 @@ int prefill_attn(int route, const void* q, int q_stride, void* out, const void* 
 void bump_tuning_epoch();
 int tuning_epoch();
 
+// single-token attention (attn.cu) as a forward pass calls it.  tables_known: block table and context lengths were there before the pass, so
+// that the pages can be asked into L2 while the kernels before this one still run (see linear).
+int decode_attn(const void* q, int q_stride, void* out, const void* kv_layer, const int32_t* block_table, int bt_stride,
+                const int32_t* ctx_lens, int n_seqs, int n_q, int n_kv, int D, int block_size, float scale, float softcap, int window,
+                bool tables_known, cudaStream_t st);
 // The projections (gemm_tcgen05.cu) as a forward pass calls them.  fixed_w: no kernel that may still run when this one begins writes the
 // weights, so they are fetched before follow_previous; that holds where the first kernel of the same pass was not launched early.
 int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st);
@@ -139,6 +144,10 @@ __device__ __forceinline__ void tma_bulk_g2s(void* smem_dst, const void* gsrc, u
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
       ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+// so many bytes (a multiple of 16) into L2 only; as with tma_prefetch_2d, nothing is read by it
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 // 2-D tiled tensor-map load
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int c0, int c1,

@@ -334,9 +334,9 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
                                  NKV, D, c.block_size, stream));
     // gemma2: even layers are the sliding-window ones (HF layer_types: sliding, full, sliding, ...)
     const int window = (gemma && li % 2 == 0) ? c.sliding_window : 0;
-    B200Q_TRY(B200Q_PROF_DECODE_ATTN, (double)b->sum_ctx_dec * kv_tok_bytes, b200q_decode_attn_ex(m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
+    B200Q_TRY(B200Q_PROF_DECODE_ATTN, (double)b->sum_ctx_dec * kv_tok_bytes, decode_attn(m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
                                 b->ctx_lens, b->n_dec, NQ, NKV, D, c.block_size, c.attn_scale,
-                                c.attn_softcap, window, stream));
+                                c.attn_softcap, window, true, cst));
     B200Q_TRY(B200Q_PROF_PREFILL_ATTN, (double)b->prefill_flops_per_layer, prefill_attn(prefill_route[window > 0], m->qkv, QKV, m->attn, kv_layer, b->block_table, b->bt_stride,
                                  b->tiles, b->n_tiles, NQ, NKV, D, c.block_size, c.attn_scale,
                                  c.attn_softcap, window, as_stream(stream)));

@@ -121,3 +121,39 @@ def test_forward_reads_weights_that_were_just_written(cuda):
         forward()
         assert torch.equal(logits, want[name]), i
     model.close()
+
+
+def test_rows_of_a_pass_see_each_other(cuda):
+    """two tokens of one sequence in one pass: the second reads from an earlier page what the first writes in the same pass, although
+    the pages are asked into L2 before that is written"""
+    import ctypes as C
+
+    from llmq_b200 import lib as L
+    from tests.test_model_gpu import TINY, build
+    model, _, _ = build(TINY["d64"])
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)
+    ids = torch.empty(2, dtype=torch.int32, device=cuda)
+
+    def forward(rows):   # (token, position) each, one sequence on pages 5 and 9
+        n = len(rows)
+        meta = {"tok": ints([t for t, _ in rows]), "pos": ints([p for _, p in rows]), "slot": ints([(5, 9)[p // 16] * 16 + p % 16 for _, p in rows]),
+                "bt": ints([[5, 9] + [0] * 6] * n), "ctx": ints([p + 1 for _, p in rows]), "tiles": ints([[0, 0, 0, 0]]), "rows": ints(list(range(n)))}
+        p = {k: t.data_ptr() for k, t in meta.items()}
+        batch = L.Batch(T=n, n_dec=n, n_tiles=0, n_sample=n, bt_stride=8, token_ids=p["tok"], positions=p["pos"], slot_mapping=p["slot"],
+                        block_table=p["bt"], ctx_lens=p["ctx"], tiles=p["tiles"], sample_rows=p["rows"], out_ids=ids.data_ptr())
+        L.check(model.lib.b200q_model_forward(model.handle, C.byref(batch), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        return model.logits_view(n).float().clone()
+
+    g = torch.Generator(device=cuda).manual_seed(3)
+    model.kv.copy_(torch.randn(model.kv.shape, generator=g, device=cuda).to(BF))
+    keep = model.kv.clone()
+    forward([(17, 15)])
+    want = forward([(40, 16)])[0]
+    for _ in range(5):
+        model.kv.copy_(keep)
+        model.kv[:, 5, :, :, 15] = 30.0     # (what is read if the first token's row is not waited for)
+        got = forward([(17, 15), (40, 16)])[1]
+        # one row or two: the same kernels and orders of sums
+        assert torch.equal(got, want)
+    model.close()
