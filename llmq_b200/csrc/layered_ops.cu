@@ -1320,8 +1320,13 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restric
 __global__ void __launch_bounds__(256) copy_f32_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                        long long n) {
   follow_previous(in, out);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-    out[e] = in[e];
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    for (long long e = first; e < n / 4; e += step) reinterpret_cast<float4*>(out)[e] = reinterpret_cast<const float4*>(in)[e];
+    for (long long e = n / 4 * 4 + first; e < n; e += step) out[e] = in[e];
+  } else {
+    for (long long e = first; e < n; e += step) out[e] = in[e];
+  }
 }
 
 }  // namespace b200q
@@ -1745,7 +1750,7 @@ int b200q_f32_to_bf16(const float* in, void* out, int64_t n, void* stream) {
 int b200q_copy_f32(const float* in, float* out, int64_t n, void* stream) {
   B200Q_CHECK_ARG(in && out && n >= 0, "copy_f32: bad argument");
   if (n == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(copy_f32_kernel, grid_for(n), 256, 0, as_stream(stream), 1, in, out, (long long)n));
+  B200Q_CUDA(launch_early(copy_f32_kernel, grid_for((n + 3) / 4), 256, 0, as_stream(stream), 1, in, out, (long long)n));
   count_launch();
   return B200Q_OK;
 }

@@ -2,6 +2,7 @@
 // previous row travels in the sequence's state slot, blends of a row with its predecessor, the squared-ReLU
 // unit, routing of a grouped mixture with identity experts, residual sums, re-injection input, logit soft cap.
 // Norms, blends, router arithmetic and the residual are fp32 whatever the model's element type is.
+#include <limits.h>
 #include <stdlib.h>
 
 #include "layered_common.cuh"
@@ -208,7 +209,13 @@ __global__ void __launch_bounds__(256) decay_from_logits_kernel(float* __restric
 // GATED: scores are the sigmoids of the logits, a group counts with the sum of its two largest choices, the weights are the
 // chosen scores as they are, and `shared` appends one pair per token for expert E with weight 1.
 constexpr int ROUTE_MAX_GROUPS = 256;
-template <bool GATED>
+// Q > 0: E <= 32 Q; a lane keeps its experts' scores and choices instead of making them again for every pick, and the largest of a warp
+// comes from one reduction of ordered integers (16 experts, 4 picks: 4.9 -> 3.7 us).
+__device__ __forceinline__ int ordered_bits(float v) {
+  const int b = __float_as_int(v);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+template <bool GATED, int Q>
 __global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* __restrict__ logits, int ld,
                                                                 const float* __restrict__ corr, int Tn, int E, int top,
                                                                 int n_groups, int keep, int shared,
@@ -258,9 +265,43 @@ __global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* __r
   }
   float chosen_s = 0.f;
   int chosen_i = -1;
+  if constexpr (Q > 0) {
+    float s_e[Q], v_e[Q];
+    uint32_t left = 0;  // bit j: expert lane + 32 j is in a kept group and has not been picked
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+      const int e = lane + 32 * j;
+      s_e[j] = v_e[j] = 0.f;
+      if (e < E && gsc[e / gs] != 0.f) {
+        s_e[j] = score(e);
+        v_e[j] = s_e[j] + corr[e];
+        if (v_e[j] == v_e[j]) left |= 1u << j;  // (what is not a number is never picked, as in the loop below)
+      }
+    }
+    for (int k = 0; k < top; ++k) {
+      float bv = -INFINITY, bs = 0.f;
+      int bj = -1;
+#pragma unroll
+      for (int j = 0; j < Q; ++j)
+        if ((left >> j & 1u) && (bj < 0 || v_e[j] > bv)) {  // (the lowest index first)
+          bv = v_e[j];
+          bs = s_e[j];
+          bj = j;
+        }
+      const int key = bj < 0 ? INT_MIN : ordered_bits(bv == 0.f ? 0.f : bv), top_key = __reduce_max_sync(0xffffffffu, key);
+      const int mine = bj >= 0 && key == top_key ? lane + 32 * bj : 0x7fffffff;
+      const int bi = __reduce_min_sync(0xffffffffu, mine);
+      bs = __shfl_sync(0xffffffffu, bs, bi & 31);
+      if (bi == mine && bj >= 0) left &= ~(1u << bj);
+      if (lane == k) {
+        chosen_s = bi == 0x7fffffff ? 0.f : bs;
+        chosen_i = bi;
+      }
+    }
+  }
   float prev_v = INFINITY;
   int prev_i = -1;
-  for (int k = 0; k < top; ++k) {
+  for (int k = 0; Q == 0 && k < top; ++k) {
     float bv = -INFINITY, bs = 0.f;
     int bi = 0x7fffffff;
     for (int e = lane; e < E; e += 32) {
@@ -300,6 +341,15 @@ __global__ void __launch_bounds__(128) moe_route_grouped_kernel(const float* __r
     idx[(long long)t * per + top] = E;
     wts[(long long)t * per + top] = 1.f;
   }
+}
+
+template <bool GATED>
+static auto route_kernel(int E) {
+  return E <= 32    ? moe_route_grouped_kernel<GATED, 1>
+         : E <= 64  ? moe_route_grouped_kernel<GATED, 2>
+         : E <= 128 ? moe_route_grouped_kernel<GATED, 4>
+         : E <= 256 ? moe_route_grouped_kernel<GATED, 8>
+                    : moe_route_grouped_kernel<GATED, 0>;
 }
 
 // grouping of the pairs by expert (one CTA), as for the other mixtures, with the tile table limited to the
@@ -402,19 +452,35 @@ __global__ void __launch_bounds__(256) residual_add_routed_v8_kernel(float* __re
     const int t = (int)(e / W8), c = (int)(e - (long long)t * W8) * 8;
     const long long at = (long long)t * W8 * 8 + c;
     float ff[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < top; ++k) {
-      const long long p = (long long)t * top + k;
-      const uint4 v = idx[p] < n_real ? ld_v4(eout + (long long)pair_pos[p] * W8 * 8 + c) : ld_v4(h + at);
-      const uint32_t q[4] = {v.x, v.y, v.z, v.w};
-      const float wk = wts[p];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        ff[2 * i] = fmaf(wk, bf16_lo(q[i]), ff[2 * i]);
-        ff[2 * i + 1] = fmaf(wk, bf16_hi(q[i]), ff[2 * i + 1]);
-      }
-    }
     float4* xo = reinterpret_cast<float4*>(x + at);
     float4 a = xo[0], b = xo[1];
+    // four choices at a time: their places are asked for together, then their rows (one by one 4.4 us for 128 tokens, 4 choices each)
+    for (int k0 = 0; k0 < top; k0 += 4) {
+      const long long p0 = (long long)t * top + k0;
+      int id[4], pos[4];
+      float wk[4];
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool on = k0 + k < top;
+        id[k] = on ? idx[p0 + k] : n_real;
+        pos[k] = on ? pair_pos[p0 + k] : 0;
+        wk[k] = on ? wts[p0 + k] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k0 + k < top) v[k] = id[k] < n_real ? ld_v4(eout + (long long)pos[k] * W8 * 8 + c) : ld_v4(h + at);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k0 + k < top) {
+          const uint32_t q[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            ff[2 * i] = fmaf(wk[k], bf16_lo(q[i]), ff[2 * i]);
+            ff[2 * i + 1] = fmaf(wk[k], bf16_hi(q[i]), ff[2 * i + 1]);
+          }
+        }
+    }
     a.x += ff[0]; a.y += ff[1]; a.z += ff[2]; a.w += ff[3];
     b.x += ff[4]; b.y += ff[5]; b.z += ff[6]; b.w += ff[7];
     xo[0] = a;
@@ -539,8 +605,8 @@ int b200q_moe_route_grouped(const float* logits, const float* correction, int T_
                   "moe_route_grouped: bad argument (E=%d top=%d groups=%d keep=%d; groups divide E, at most %d groups, "
                   "top fits the kept groups)", E, top, n_groups, keep, ROUTE_MAX_GROUPS);
   if (T_ == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(moe_route_grouped_kernel<false>, (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, E, correction, T_, E, top,
-                          n_groups, keep, 0, idx, wts));
+  B200Q_CUDA(launch_early(route_kernel<false>(E), (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, E, correction, T_, E, top, n_groups, keep, 0,
+                          idx, wts));
   count_launch();
   B200Q_CUDA(launch_early(moe_plan_part_kernel, 1, 1024, (size_t)(3 * E + 1) * sizeof(int32_t), as_stream(stream), 1, idx, T_ * top, top, E,
                           e_gemm, group_off, perm_tok, pair_pos, tile_tab, n_tiles));
@@ -559,8 +625,8 @@ int b200q_moe_route_gated(const float* logits, int ld, const float* correction, 
                   "the kept groups)", E, top, n_groups, keep, ROUTE_MAX_GROUPS);
   if (T_ == 0) return B200Q_OK;
   const int per = top + shared, n = E + shared;
-  B200Q_CUDA(launch_early(moe_route_grouped_kernel<true>, (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, ld, correction, T_, E, top,
-                          n_groups, keep, shared, idx, wts));
+  B200Q_CUDA(launch_early(route_kernel<true>(E), (T_ + 3) / 4, 128, 0, as_stream(stream), 1, logits, ld, correction, T_, E, top, n_groups, keep,
+                          shared, idx, wts));
   count_launch();
   B200Q_CUDA(launch_early(moe_plan_part_kernel, 1, 1024, (size_t)(3 * n + 1) * sizeof(int32_t), as_stream(stream), 1, idx, T_ * per, per, n,
                           n, group_off, perm_tok, pair_pos, tile_tab, n_tiles));
