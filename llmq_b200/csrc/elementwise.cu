@@ -2,6 +2,7 @@
 // embedding gather (K1), RMSNorm / fused add+RMSNorm (K2), RoPE + paged KV write (K4+K5),
 // SwiGLU (K10), row gather and greedy argmax (K13), in place of vLLM's ops.  All rounding points follow the oracle (oracle/ops.py), which follows
 // vLLM's native op definitions / HF transformers' Llama.
+#include <limits.h>
 #include <stdarg.h>
 
 #include "tcgen05.cuh"
@@ -411,7 +412,8 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------------------------------------------
 // K13 greedy argmax over bf16 logits; lowest index wins ties (torch.argmax behaviour).
-// One 1024-thread CTA per row.  V need not be a multiple of 8 (tail handled scalar).
+// A cluster of gridDim.x CTAs shares a row, four 16-byte loads in flight per thread (48 rows of 128256 logits: 15.3 us with the end of the
+// step, 9.7 so).  V need not be a multiple of 8 (tail handled scalar).
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void amax_update(float v, int i, float& best, int& bi) {
   if (v > best || (v == best && i < bi)) {
@@ -420,160 +422,26 @@ __device__ __forceinline__ void amax_update(float v, int i, float& best, int& bi
   }
 }
 
-__global__ void __launch_bounds__(1024)
-    argmax_kernel(const bf16* __restrict__ logits, int32_t* __restrict__ ids, int V) {
-  follow_previous(logits, ids);
-  const bf16* row = logits + (long long)blockIdx.x * V;
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  const int nvec = ((reinterpret_cast<uintptr_t>(row) & 15) == 0) ? V / 8 : 0;
-  const uint4* rv = reinterpret_cast<const uint4*>(row);
-  for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
-    uint4 a = ld_nc_v4(rv + c);
-    const uint32_t* ap = reinterpret_cast<const uint32_t*>(&a);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      amax_update(bf16_lo(ap[k]), c * 8 + 2 * k, best, bi);
-      amax_update(bf16_hi(ap[k]), c * 8 + 2 * k + 1, best, bi);
-    }
-  }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x)
-    amax_update(__bfloat162float(row[i]), i, best, bi);
+// the largest of the block's threads and then of the cluster's CTAs; thread 0 of CTA 0 returns with it
+template <int THREADS>
+__device__ __forceinline__ void amax_cluster(float& best, int& bi) {
+  const int split = blockIdx.x, splits = gridDim.x;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     float ov = __shfl_xor_sync(0xffffffffu, best, o);
     int oi = __shfl_xor_sync(0xffffffffu, bi, o);
     amax_update(ov, oi, best, bi);
   }
-  __shared__ float sv[32];
-  __shared__ int si[32];
+  __shared__ float sv[THREADS / 32];
+  __shared__ int si[THREADS / 32];
   if ((threadIdx.x & 31) == 0) {
     sv[threadIdx.x >> 5] = best;
     si[threadIdx.x >> 5] = bi;
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    best = threadIdx.x < (blockDim.x >> 5) ? sv[threadIdx.x] : -INFINITY;
-    bi = threadIdx.x < (blockDim.x >> 5) ? si[threadIdx.x] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      amax_update(ov, oi, best, bi);
-    }
-    if (threadIdx.x == 0) ids[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
-  }
-}
-
-// ------------------------------------------------------------------------------------------
-// K13 sampler at temperature > 0: the reference's default path (SamplingParams(temperature=0.7),
-// ref:llmq/workers/vllm_worker.py:161-165; vLLM: probs = softmax(logits/T); probs.div_(q).argmax
-// with q ~ Exp(1), vllm/v1/sample/ops/topk_topp_sampler.py:395-416).  argmax_i p_i/q_i ==
-// argmax_i (logit_i/T - log q_i), so no softmax pass is needed: one read of the bf16 logits row.
-// q_i = -log(u_i), u_i from Philox4x32-10 keyed by the request's seed with counter
-// (element index / 4, token position) — counter-based, so a request's samples do not depend on
-// its batch-mates.  temperature == 0 rows fall back to the greedy argmax (lowest index on ties).
-// params: int32[B][4] = {float bits of temperature, seed lo, seed hi, position}.
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                              uint32_t k0, uint32_t k1, uint32_t (&out)[4]) {
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-    c0 = hi1 ^ c1 ^ k0;
-    c1 = lo1;
-    c2 = hi0 ^ c3 ^ k1;
-    c3 = lo0;
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
-  }
-  out[0] = c0;
-  out[1] = c1;
-  out[2] = c2;
-  out[3] = c3;
-}
-
-// -log(-log u), u = (n + 1/2) / 2^24 with n = the upper 24 bits.  n + 1/2 takes 25 bits from 2^23 on and rounds half a step up or down (to
-// u = 1 for the largest n, whose noise is 17.3 and not infinite): what was rounded off, d = +-2^-25, comes back as log u = log u' + d / u',
-// 1 / u' = 2 - u' being near enough (off by 1.5e-8 of 0.69 at u' = 1/2).  Below 2^23, d = 0.
-__device__ __forceinline__ float gumbel_from_bits(uint32_t x) {
-  const float n = (float)(x >> 8), n5 = n + 0.5f, u = n5 * (1.0f / 16777216.0f);
-  const float d = ((n - n5) + 0.5f) * (1.0f / 16777216.0f);
-  return -logf(-fmaf(d, 2.f - u, logf(u)));
-}
-
-// A cluster of gridDim.x CTAs shares a row (a row per CTA left most SMs idle or one deep: 60 us for 128 rows of 128256 logits, 33 so).
-// Bound: integer work of the random numbers, 20 instructions per logit.  The two logarithms of a logit's noise are taken only where
-// the logit could still win: its value t + noise exceeds the best so far only if -log u < e^(t - best), and -log u >= 1 - u, which the
-// bits give directly.  The margin covers the roundings of t, best and the exponential (|best| * 1e-6 + 1.5e-3 in base 2, some ten times
-// what they are), so what is left out is smaller than the best, and the result is the one that all logarithms give.
-constexpr int SAMPLE_THREADS = 512;
-__global__ void __launch_bounds__(SAMPLE_THREADS, 3)
-    sample_kernel(const bf16* __restrict__ logits, const int32_t* __restrict__ params,
-                  int32_t* __restrict__ ids, int V) {
-  follow_previous(logits, params, ids);
-  const int split = blockIdx.x, splits = gridDim.x, r_ = blockIdx.y;
-  const bf16* row = logits + (long long)r_ * V;
-  const float temp = __int_as_float(params[4 * r_ + 0]);
-  const uint32_t k0 = (uint32_t)params[4 * r_ + 1], k1 = (uint32_t)params[4 * r_ + 2];
-  const uint32_t pos = (uint32_t)params[4 * r_ + 3];
-  const bool greedy = !(temp > 0.f);
-  const float inv_t = greedy ? 1.f : 1.f / temp;
-  const float log2e = 1.4426950408889634f;
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  float bound = -INFINITY;  // (best of the warp) * log2 e - margin
-  // groups of 4 consecutive elements share one Philox block: counter = (group, position, 0, 0)
-  const int n4 = V / 4, step = splits * SAMPLE_THREADS;
-  for (int g0 = split * SAMPLE_THREADS; g0 < n4; g0 += step) {  // (whole warps go round together)
-    const int g = g0 + threadIdx.x;
-    if (g < n4) {
-      const uint2 a = *reinterpret_cast<const uint2*>(row + 4 * g);  // 4 bf16 (V*2 B rows are 8 B aligned)
-      float v[4] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y)};
-      if (greedy) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) amax_update(v[k], 4 * g + k, best, bi);
-      } else {
-        uint32_t r[4];
-        philox4x32_10((uint32_t)g, pos, 0u, 0u, k0, k1, r);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float t = v[k] * inv_t;
-          float least;  // e^(t - best), a little more
-          asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(least) : "f"(fmaf(t, log2e, -bound)));
-          // 1 - u >= 2 - f - 2^-23 with f = 1 + the upper 23 bits
-          const float one_less_u = (2.f - __uint_as_float(0x3f800000u | (r[k] >> 9))) - 1.1920929e-7f;
-          if (!(one_less_u > least)) amax_update(v[k] * inv_t + gumbel_from_bits(r[k]), 4 * g + k, best, bi);
-        }
-      }
-    }
-    if (!greedy) {
-      // the warp's best, through integers of the same order
-      int o = __float_as_int(best);
-      o ^= (o >> 31) & 0x7fffffff;
-      o = __reduce_max_sync(0xffffffffu, o);
-      o ^= (o >> 31) & 0x7fffffff;
-      const float top = __int_as_float(o);
-      bound = fmaf(top, log2e, -(1.5e-3f + fabsf(top) * 1e-6f));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    amax_update(ov, oi, best, bi);
-  }
-  __shared__ float sv[32];
-  __shared__ int si[32];
-  if ((threadIdx.x & 31) == 0) {
-    sv[threadIdx.x >> 5] = best;
-    si[threadIdx.x >> 5] = bi;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    best = threadIdx.x < (blockDim.x >> 5) ? sv[threadIdx.x] : -INFINITY;
-    bi = threadIdx.x < (blockDim.x >> 5) ? si[threadIdx.x] : 0x7fffffff;
+    best = threadIdx.x < THREADS / 32 ? sv[threadIdx.x] : -INFINITY;
+    bi = threadIdx.x < THREADS / 32 ? si[threadIdx.x] : 0x7fffffff;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -592,7 +460,188 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 3)
         amax_update(ld_cluster_f32(mapa_shared(sv, s)), __float_as_int(ld_cluster_f32(mapa_shared(si, s))), best, bi);
     cluster_sync_all();
   }
+}
+
+constexpr int ARGMAX_THREADS = 512;
+__global__ void __launch_bounds__(ARGMAX_THREADS)
+    argmax_kernel(const bf16* __restrict__ logits, int32_t* __restrict__ ids, int V) {
+  follow_previous(logits, ids);
+  const int split = blockIdx.x, r_ = blockIdx.y;
+  const bf16* row = logits + (long long)r_ * V;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  const int nvec = ((reinterpret_cast<uintptr_t>(row) & 15) == 0) ? V / 8 : 0;
+  const uint4* rv = reinterpret_cast<const uint4*>(row);
+  const int step = gridDim.x * ARGMAX_THREADS, first = split * ARGMAX_THREADS + threadIdx.x;
+  for (int c0 = first; c0 < nvec; c0 += 4 * step) {
+    uint4 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c0 + u * step < nvec) a[u] = ld_nc_v4(rv + c0 + u * step);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c0 + u * step < nvec) {
+        const uint32_t* ap = reinterpret_cast<const uint32_t*>(&a[u]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          amax_update(bf16_lo(ap[k]), (c0 + u * step) * 8 + 2 * k, best, bi);
+          amax_update(bf16_hi(ap[k]), (c0 + u * step) * 8 + 2 * k + 1, best, bi);
+        }
+      }
+  }
+  for (int i = nvec * 8 + first; i < V; i += step) amax_update(__bfloat162float(row[i]), i, best, bi);
+  amax_cluster<ARGMAX_THREADS>(best, bi);
   if (split == 0 && threadIdx.x == 0) ids[r_] = bi == 0x7fffffff ? 0 : bi;
+}
+
+// ------------------------------------------------------------------------------------------
+// K13 sampler at temperature > 0: the reference's default path (SamplingParams(temperature=0.7),
+// ref:llmq/workers/vllm_worker.py:161-165; vLLM: probs = softmax(logits/T); probs.div_(q).argmax
+// with q ~ Exp(1), vllm/v1/sample/ops/topk_topp_sampler.py:395-416).  argmax_i p_i/q_i ==
+// argmax_i (logit_i/T - log q_i), so no softmax pass is needed: one read of the bf16 logits row.
+// q_i = -log(u_i), u_i from Philox4x32-10 keyed by the request's seed with counter
+// (element index / 4, token position) — counter-based, so a request's samples do not depend on
+// its batch-mates.  temperature == 0 rows fall back to the greedy argmax (lowest index on ties).
+// params: int32[B][4] = {float bits of temperature, seed lo, seed hi, position}.
+// ------------------------------------------------------------------------------------------
+// counter (c0, c1, 0, 0); k0, k1: the key of every round
+__device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, const uint32_t (&k0)[10], const uint32_t (&k1)[10], uint32_t (&out)[4]) {
+  uint32_t c2 = 0, c3 = 0;
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c0, p1 = (uint64_t)0xCD9E8D57u * c2;
+    c0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0[r];
+    c1 = (uint32_t)p1;
+    c2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1[r];
+    c3 = (uint32_t)p0;
+  }
+  out[0] = c0;
+  out[1] = c1;
+  out[2] = c2;
+  out[3] = c3;
+}
+
+// -log(-log u), u = (n + 1/2) / 2^24 with n = the upper 24 bits.  n + 1/2 takes 25 bits from 2^23 on and rounds half a step up or down (to
+// u = 1 for the largest n, whose noise is 17.3 and not infinite): what was rounded off, d = +-2^-25, comes back as log u = log u' + d / u',
+// 1 / u' = 2 - u' being near enough (off by 1.5e-8 of 0.69 at u' = 1/2).  Below 2^23, d = 0.
+__device__ __forceinline__ float gumbel_from_bits(uint32_t x) {
+  const float n = (float)(x >> 8), n5 = n + 0.5f, u = n5 * (1.0f / 16777216.0f);
+  const float d = ((n - n5) + 0.5f) * (1.0f / 16777216.0f);
+  return -logf(-fmaf(d, 2.f - u, logf(u)));
+}
+
+// A cluster of gridDim.x CTAs shares a row.  Bound: integer work of the random numbers.  The two logarithms of a logit's noise are taken
+// only where the logit could still win: its value t + noise exceeds the best so far only if -log u < e^(t - best), and -log u >= 1 - u,
+// which the bits give directly; four logits (one block of random numbers) are looked at together, by the largest t and the largest u among
+// them.  The margin covers the roundings of t, best and the exponential (|best| * 1e-6 + 1.5e-3 in base 2, some ten times what they are),
+// so what is left out is smaller than the best, and the result is the one that all logarithms give.  The best so far is the CTA's, in
+// shared memory: a warp sees a few thousand logits only, and would take logarithms for a third of them on its own.  128 rows of 128256
+// logits 35 -> 25 us, 1024 rows 181 -> 132 (issue slots 58 % busy, half of them the random numbers).
+constexpr int SAMPLE_THREADS = 512;
+__device__ __forceinline__ int order_float(float v) {  // integers of the same order
+  const int o = __float_as_int(v);
+  return o ^ ((o >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float unorder_float(int o) { return __int_as_float(o ^ ((o >> 31) & 0x7fffffff)); }
+
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
+    sample_kernel(const bf16* __restrict__ logits, const int32_t* __restrict__ params,
+                  int32_t* __restrict__ ids, int V) {
+  __shared__ int top_s;  // the CTA's best so far, through order_float
+  if (threadIdx.x == 0) top_s = INT_MIN;
+  __syncthreads();
+  follow_previous(logits, params, ids);
+  const int split = blockIdx.x, splits = gridDim.x, r_ = blockIdx.y;
+  const bf16* row = logits + (long long)r_ * V;
+  const float temp = __int_as_float(params[4 * r_ + 0]);
+  // (the round keys are kept: made again for every block they are a fifth of its instructions)
+  uint32_t k0[10], k1[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+    k0[i] = (uint32_t)params[4 * r_ + 1] + (uint32_t)i * 0x9E3779B9u;
+    k1[i] = (uint32_t)params[4 * r_ + 2] + (uint32_t)i * 0xBB67AE85u;
+    asm volatile("" : "+r"(k0[i]), "+r"(k1[i]));
+  }
+  const uint32_t pos = (uint32_t)params[4 * r_ + 3];
+  const bool greedy = !(temp > 0.f);
+  const float inv_t = greedy ? 1.f : 1.f / temp;
+  const float log2e = 1.4426950408889634f;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  // groups of 4 consecutive elements share one Philox block: counter = (group, position, 0, 0)
+  constexpr int AT_ONCE = 2;
+  const int n4 = V / 4, step = splits * SAMPLE_THREADS, first = split * SAMPLE_THREADS + threadIdx.x;
+  const uint2 none = make_uint2(0xff80ff80u, 0xff80ff80u);
+  auto fetch = [&](int g) { return g < n4 ? *reinterpret_cast<const uint2*>(row + 4 * (long long)g) : none; };  // (8 B aligned: V*2 B rows)
+  if (greedy) {
+    for (int g = first; g < n4; g += step) {
+      const uint2 a = fetch(g);
+      const float v[4] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y)};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) amax_update(v[k], 4 * g + k, best, bi);
+    }
+  } else {
+    uint2 a[AT_ONCE];
+#pragma unroll
+    for (int x = 0; x < AT_ONCE; ++x) a[x] = fetch(first + x * step);
+    for (int g0 = first; g0 - (int)threadIdx.x < n4; g0 += AT_ONCE * step) {  // (whole CTAs go round together)
+      uint2 next[AT_ONCE];
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x) next[x] = fetch(g0 + (AT_ONCE + x) * step);
+      const float top = unorder_float(*(volatile int*)&top_s);  // (nothing yet: not a number, and every logit is looked at)
+      const float bound = fmaf(top, log2e, -(1.5e-3f + fabsf(top) * 1e-6f));
+      bool look[AT_ONCE], any = false;
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x) {
+        uint32_t r[4];
+        philox4x32_10((uint32_t)(g0 + x * step), pos, k0, k1, r);
+        const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[x].x), *reinterpret_cast<const __nv_bfloat162*>(&a[x].y));
+        const float t = fmaxf(__low2float(m), __high2float(m)) * inv_t;
+        float least;  // e^(t - best), a little more
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(least) : "f"(fmaf(t, log2e, -bound)));
+        // 1 - u >= 2 - f - 2^-23 with f = 1 + the upper 23 bits
+        const uint32_t most = max(max(r[0], r[1]), max(r[2], r[3]));
+        const float one_less_u = (2.f - __uint_as_float(0x3f800000u | (most >> 9))) - 1.1920929e-7f;
+        look[x] = !(one_less_u > least) && g0 + x * step < n4;
+        any |= look[x];
+      }
+      if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+        for (int x = 0; x < AT_ONCE; ++x)
+          if (look[x]) {  // (seldom: its random numbers once more)
+            uint32_t r[4];
+            philox4x32_10((uint32_t)(g0 + x * step), pos, k0, k1, r);
+            const float v[4] = {bf16_lo(a[x].x), bf16_hi(a[x].x), bf16_lo(a[x].y), bf16_hi(a[x].y)};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) amax_update(v[k] * inv_t + gumbel_from_bits(r[k]), 4 * (g0 + x * step) + k, best, bi);
+          }
+        const int o = __reduce_max_sync(0xffffffffu, order_float(best));
+        if ((threadIdx.x & 31) == 0) atomicMax(&top_s, o);
+      }
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x) a[x] = next[x];
+    }
+  }
+  amax_cluster<SAMPLE_THREADS>(best, bi);
+  if (split == 0 && threadIdx.x == 0) ids[r_] = bi == 0x7fffffff ? 0 : bi;
+}
+
+// CTAs per row: the least (rounds of resident clusters) x (a CTA's share of a row and its start and end).  A cluster lies within one of the
+// chip's eight processing clusters, which has room for `room` CTAs (17 SMs counted, so that 48 clusters of 6 do not count as resident:
+// 48 rows of 128256 logits 14.9 us with 5 CTAs each, 18.7 with 6).  128 rows: 24.9 us with 2, 30.8 with 3, 37.8 with 1; 300 rows 55 / 60 /
+// 58; 1024 rows 149 / 182 / 132; one row 8 CTAs 8, 2 CTAs 13.
+static int row_splits(int rows, int room, int most) {
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= 8 && s <= most; ++s) {
+    const long long resident = 8LL * (room / s);
+    const double t = (double)((rows + resident - 1) / resident) * (1.0 / s + 0.1);
+    if (t < 0.95 * least) {
+      least = t;
+      best = s;
+    }
+  }
+  return best;
 }
 
 }  // namespace b200q
@@ -763,8 +812,12 @@ int b200q_gather_rows(const void* x, const int32_t* rows, void* out, int n, int 
 int b200q_argmax_bf16(const void* logits, int32_t* ids, int B, int V, void* stream) {
   B200Q_CHECK_ARG(B >= 0 && V > 0, "argmax: bad shape B=%d V=%d", B, V);
   if (B == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(argmax_kernel, B, 1024, 0, as_stream(stream), 1, (const bf16*)logits, ids, V));
-  count_launch();
+  for (int at = 0; at < B; at += 65535) {  // (a grid's second dimension ends at 65535 rows)
+    const int rows = B - at < 65535 ? B - at : 65535, splits = row_splits(rows, 4 * 17, V / (16 * ARGMAX_THREADS) + 1);
+    B200Q_CUDA(launch_early(argmax_kernel, dim3(splits, rows), ARGMAX_THREADS, 0, as_stream(stream), splits,
+                            (const bf16*)logits + (long long)at * V, ids + at, V));
+    count_launch();
+  }
   return B200Q_OK;
 }
 
@@ -776,7 +829,7 @@ int b200q_sample_bf16(const void* logits, const int32_t* params, int32_t* ids, i
   // (a grid's second dimension ends at 65535 rows)
   for (int at = 0; at < B; at += 65535) {
     const int rows = B - at < 65535 ? B - at : 65535;
-    const int splits = rows >= 444 ? 1 : (444 + rows - 1) / rows < 8 ? (444 + rows - 1) / rows : 8;  // three CTAs per SM
+    const int splits = row_splits(rows, 2 * 17, V / (8 * SAMPLE_THREADS) + 1);
     B200Q_CUDA(launch_early(sample_kernel, dim3(splits, rows), SAMPLE_THREADS, 0, as_stream(stream), splits,
                             (const bf16*)logits + (long long)at * V, params + 4 * (long long)at, ids + at, V));
     count_launch();

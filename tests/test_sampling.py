@@ -149,3 +149,25 @@ def test_masked_rows_and_ties(cuda, B):
     expect(got, ref, temps, seeds, positions)
     for i, k in enumerate(kind):
         assert k != 2 or got[i] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 9, 40, 48, 68, 130, 300, 600])   # rows of 8 CTAs down to one
+@pytest.mark.parametrize("V", [4, 2048, 16 * 512 * 8 + 4, 16 * 512 * 8 + 5])
+def test_argmax_over_shared_rows(cuda, B, V):
+    """the lowest of the largest, in whatever CTA's share it lies; rows that are not 16-byte aligned, rows without a largest"""
+    from llmq_b200 import lib
+    g = torch.Generator().manual_seed(B * V)
+    rows = torch.randn(B, V, generator=g).to(torch.bfloat16)
+    kind = [i % 4 for i in range(B)]
+    for i, k in enumerate(kind):
+        if k == 1:
+            rows[i, torch.randint(0, V, (3,), generator=g)] = 9.0
+        elif k == 2:
+            rows[i] = -float("inf")
+        elif k == 3:
+            rows[i, V - 1] = float("inf")
+    ids = torch.full((B,), -1, dtype=torch.int32, device=cuda)
+    lib.argmax_bf16(rows.to(cuda), ids)
+    want = [int((r == r.max()).nonzero()[0, 0]) for r in rows.float()]
+    assert ids.cpu().tolist() == want
