@@ -60,19 +60,22 @@ constexpr int EPI_SMEM_PER_WARP = 32 * 128;  // 32 rows x 64 bf16
 template <int BN, int kAct>
 __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long long ldc,
                                               int row0, int M, uint8_t* patch, int lane,
-                                              const float* gate_bias = nullptr, float limit = 0.f) {
+                                              const float* gate_bias = nullptr, float limit = 0.f, int cols = BN) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;  // gated epilogue: tile = [gate (BN/2) | up (BN/2)]
   constexpr int OUT_BN = kSwiGLU ? BN / 2 : BN;
   // (no row of this warp exists: its accumulators are sums of zeros, which the gated units' division treats as a special case: 384 rows
   // x 2048 x 512 gated 29 us, 15 without)
   if (row0 >= M) return;
+  // (kRagged: columns of C in this tile, a multiple of 32; the last tile of a row may have fewer than BN)
+  constexpr bool kRagged = BN % 128 != 0 && BN > 64;
   const uint32_t patch_s = smem_u32(patch);
 #pragma unroll 1
-  for (int c0 = 0; c0 < OUT_BN; c0 += 64) {
+  for (int c0 = 0; c0 < (kRagged ? cols : OUT_BN); c0 += 64) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {  // two 32-column TMEM loads -> 64 output columns of this row
       uint32_t v[32];
       uint4 o[4];
+      if (kRagged && c0 + 32 * h >= cols) break;
       if constexpr (!kSwiGLU) {
         tmem_ld32(taddr + (uint32_t)(c0 + 32 * h), v);
         tmem_ld_wait();
@@ -133,7 +136,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
       asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
                    : "r"(a));
-      if (row0 + rr < M) st_v4(ctile + (long long)rr * ldc + c0 + c * 8, o);
+      if (row0 + rr < M && (!kRagged || c0 + c * 8 < cols)) st_v4(ctile + (long long)rr * ldc + c0 + c * 8, o);
     }
     __syncwarp();
   }
@@ -355,7 +358,7 @@ struct Gemm2Cfg {
   static constexpr int B_BYTES = (BN / 2) * GEMM_BK * 2;       // this CTA's half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = GEMM_SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : GEMM_SMEM_BUDGET / STAGE_BYTES;
-  static constexpr int TMEM_COLS = 2 * BN;
+  static constexpr int TMEM_COLS = BN > 128 ? 512 : 256;       // two accumulators, a power of two
   static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + 4 * 4096;
 };
 
@@ -434,7 +437,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int m_tiles = (M + 255) / 256;
-  const int n_tiles = N / BN;
+  const int n_tiles = (N + BN - 1) / BN;  // (BN = 160, 192: the last one may be ragged, its rows of W behind the end are zeros)
   const int num_tiles = m_tiles * n_tiles;
   const int k_blocks = K / GEMM_BK;
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
@@ -552,7 +555,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       bf16* ctile = C + (long long)row0 * ldc + (long long)n_blk * OUT_BN;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
       epilogue_rows<BN, kAct>(taddr, ctile, ldc, row0, M, epi_smem + (warp - 2) * EPI_SMEM_PER_WARP, lane,
-                                kAct == ACT_CLAMPED && gate.bias ? gate.bias + (long long)n_blk * BN : nullptr, gate.limit);
+                                kAct == ACT_CLAMPED && gate.bias ? gate.bias + (long long)n_blk * BN : nullptr, gate.limit,
+                                min(BN, N - n_blk * BN));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(tmem_empty + acc, 0));
@@ -763,7 +767,7 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_TOTAL));
     attr_set = true;
   }
-  const int tiles = ((M + 255) / 256) * (N / BN);
+  const int tiles = ((M + 255) / 256) * ((N + BN - 1) / BN);
   // the tile loop is static round-robin over CO-RESIDENT CTA pairs: size the grid by what the
   // hardware can really keep resident at once (GPC/TPC pairing can make this < SMs/2)
   static int pairs = 0;
@@ -796,9 +800,11 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
 
 // Which kernel and tile: the least (rounds of the persistent loop) x (time of a round).  Rounds: tiles over 148 SMs, or tiles of 256 rows
 // over 74 CTA pairs.  A round's time beside the 128 x 256 tile's (K 14336, one round, us: 85.5; pair 256 x 256 70-74, pair 256 x 128
-// 50.7, 128 x 128 55, 128 x 64 50; K 8192 the same shares, 49.5 / 41.5 / 29.8 / 32 / 29): the pair kernels fetch half the weight rows
-// per SM, narrow tiles are bound by what they fetch.  Before, the pair kernel was taken for whole rounds of 74 tiles only:
-// 768 x 3584 x 14336 86 -> 71 us, 512 x 4096 x 14336 58 -> 53, 1536 x 2048 x 8192 50 -> 43.
+// 50.7, 128 x 128 55, 128 x 64 50; pairs of 256 x 192 59, 256 x 160 55, whose last tile of a row may be ragged; K 8192 the same shares,
+// 49.5 / 41.5 / 29.8 / 32 / 29): the pair kernels fetch half the weight rows per SM, narrow tiles are bound by what they fetch.  Before, the pair kernel was taken for whole rounds of 74 tiles only:
+// 768 x 3584 x 14336 86 -> 71 us, 512 x 4096 x 14336 58 -> 53, 1536 x 2048 x 8192 50 -> 43.  The widths of 160 and 192 fill rounds that 256
+// leaves half empty: 750 x 3584 x 14336 69 -> 59 us, 1500 x 4096 x 14336 140 -> 125, 1024 x 6144 x 4096 42 -> 37, 3000 x 2048 x 8192 81 -> 73
+// (108 sizes looked at: the rule is within 1 % of the best tile for 94 of them, at worst 16 % off at 300 x 2048).
 struct TileChoice {
   bool pair;
   int bn;
@@ -808,13 +814,15 @@ static TileChoice choose_tile(int M, int N, bool gated) {
     bool pair;
     int bn;
     double cost;
-  } all[5] = {{true, 256, 0.84}, {false, 256, 1.0}, {true, 128, 0.595}, {false, 128, 0.645}, {false, 64, 0.585}};
+  } all[7] = {{true, 256, 0.84},  {false, 256, 1.0},   {true, 192, 0.70},  {true, 160, 0.65},
+              {true, 128, 0.595}, {false, 128, 0.645}, {false, 64, 0.585}};
   TileChoice best{false, N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64};
   double least = 1e30;
   for (const auto& c : all) {
-    if (N % c.bn || (gated && c.bn != 256) || (c.pair && M <= GEMM_BM)) continue;
+    const bool ragged = c.bn == 160 || c.bn == 192;
+    if ((ragged ? N < c.bn : N % c.bn != 0) || (gated && c.bn != 256) || (c.pair && M <= GEMM_BM)) continue;
     const long long rows = c.pair ? 256 : GEMM_BM, slots = c.pair ? num_sms() / 2 : num_sms();
-    const long long tiles = (M + rows - 1) / rows * (N / c.bn);
+    const long long tiles = (M + rows - 1) / rows * ((N + c.bn - 1) / c.bn);
     const double t = (double)((tiles + slots - 1) / slots) * c.cost;
     if (t < least - 1e-9) {
       least = t;
@@ -1121,9 +1129,11 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
   }
   if (bn == 0) {
     const TileChoice t = choose_tile(M, N, false);
+    if (t.bn == 192 && g_gemm_mode == 0) return launch_gemm2<192>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+    if (t.bn == 160 && g_gemm_mode == 0) return launch_gemm2<160>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
     if (t.pair && g_gemm_mode == 0)
       return t.bn == 256 ? launch_gemm2<256>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w) : launch_gemm2<128>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
-    bn = t.bn;
+    bn = t.bn == 192 || t.bn == 160 ? 256 : t.bn;
   }
   if (N % bn != 0) bn = (N % 128 == 0) ? 128 : 64;
   if (bn == 256) return launch_gemm<256>(A, W, C, M, N, K, st, 1, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
