@@ -435,11 +435,23 @@ def _p(t) -> int:
     return t.data_ptr()
 
 
-def _stream(stream=None) -> int:
-    import torch
+_raw_stream = _device = None
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+
+def _stream(stream=None) -> int:
+    """handle of `stream`, or of the calling thread's current one on its current device.  torch.cuda.current_stream() makes a stream object
+    for it, 3.2 us of the 8.2 us that a small product's call took; the functions behind it take 0.2."""
+    if stream is not None:
+        return stream.cuda_stream
+    global _raw_stream, _device
+    if _raw_stream is None:
+        import torch
+
+        s = torch.cuda.current_stream().cuda_stream   # (brings CUDA up where nothing has yet)
+        _device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda d: torch.cuda.current_stream(d).cuda_stream)
+        return s
+    return _raw_stream(_device())
 
 
 # ---- thin op wrappers (used by tests/bench; the worker goes through Engine) ------------------

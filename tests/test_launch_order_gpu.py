@@ -157,3 +157,25 @@ def test_rows_of_a_pass_see_each_other(cuda):
         # one row or two: the same kernels and orders of sums
         assert torch.equal(got, want)
     model.close()
+
+
+def test_calls_go_to_the_current_stream(cuda):
+    """of the thread that calls, inside and outside of a stream context"""
+    import threading
+
+    from llmq_b200 import lib
+    assert lib._stream() == torch.cuda.current_stream().cuda_stream
+    s, other, seen = torch.cuda.Stream(), torch.cuda.Stream(), {}
+
+    def look():
+        with torch.cuda.stream(other):
+            seen["there"] = lib._stream()
+        seen["outside"] = lib._stream()
+
+    with torch.cuda.stream(s):
+        assert lib._stream() == s.cuda_stream != 0
+        t = threading.Thread(target=look)
+        t.start()
+        t.join()
+    assert seen == {"there": other.cuda_stream, "outside": torch.cuda.default_stream().cuda_stream}
+    assert lib._stream() == torch.cuda.current_stream().cuda_stream and lib._stream(s) == s.cuda_stream
