@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   if (ahead == 0) follow_previous(q, out, kv_layer, block_table, ctx_lens);
   // (without a window the first page's place in the table does not wait for the length; what lies behind the sequence is not used)
   const int32_t* bt_row = block_table + (long long)seq * bt_stride;
-  const int guess = window <= 0 && wg + n_warps * lane < bt_stride ? __ldg(bt_row + wg + n_warps * lane) : 0;
-  const int ctx = __ldg(ctx_lens + seq);
+  const int guess = window <= 0 && wg + n_warps * lane < bt_stride ? bt_row[wg + n_warps * lane] : 0;
+  const int ctx = ctx_lens[seq];
   // the query sits at position ctx-1 and sees keys [lo, ctx); pages before lo's page are skipped
   const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
   const int page0 = lo / BS;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   const long long page_stride = (long long)G_::PAGE_BYTES;  // bytes per (block,kv,head) page
   // page address: ((blk*2 + kv) * n_kv + kvh) * PAGE_BYTES
   int ids_base = 0;
-  int ids = window <= 0 ? guess : (lane < my_n) ? __ldg(bt + wg + n_warps * lane) : 0;
+  int ids = window <= 0 ? guess : (lane < my_n) ? bt[wg + n_warps * lane] : 0;
   if (ahead > 0) {
     if (lane < min(my_n, ahead)) {
       const uint32_t bytes = (uint32_t)min(BS, ctx - (page0 + wg + n_warps * lane) * BS) * G_::ROW_BYTES;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   auto issue = [&](int k) {  // whole warp calls; k = warp-local page index
     if (k - ids_base >= 32) {
       ids_base += 32;
-      ids = (ids_base + lane < my_n) ? __ldg(bt + wg + n_warps * (ids_base + lane)) : 0;
+      ids = (ids_base + lane < my_n) ? bt[wg + n_warps * (ids_base + lane)] : 0;
     }
     const int blk = __shfl_sync(0xffffffffu, ids, k - ids_base);
     const int p = page0 + wg + n_warps * k;
@@ -495,12 +495,12 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
   // ---- issue cursor: runs up to DEC_STAGES pages ahead of the consumer, across item borders ----
   // with a sliding window an item's pages run from first_page(ctx) to the last one
   auto first_page = [&](int ctx) { return (window > 0 && ctx > window) ? (ctx - window) / BS : 0; };
-  int i_item = first, i_ctx = max(__ldg(ctx_lens + first / n_kv), 1);
+  int i_item = first, i_ctx = max(ctx_lens[first / n_kv], 1);
   int i_page = first_page(i_ctx);
   int i_npages = (i_ctx + BS - 1) / BS;
   int i_ids_base = i_page;
   int i_ids = (i_ids_base + lane < i_npages)
-                  ? __ldg(block_table + (long long)(first / n_kv) * bt_stride + i_ids_base + lane)
+                  ? block_table[(long long)(first / n_kv) * bt_stride + i_ids_base + lane]
                   : 0;
   int issued = 0;
   bool i_done = false;
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
     if (i_page - i_ids_base >= 32) {
       i_ids_base += 32;
       i_ids = (i_ids_base + lane < i_npages)
-                  ? __ldg(block_table + (long long)(i_item / n_kv) * bt_stride + i_ids_base + lane)
+                  ? block_table[(long long)(i_item / n_kv) * bt_stride + i_ids_base + lane]
                   : 0;
     }
     const int blk = __shfl_sync(0xffffffffu, i_ids, i_page - i_ids_base);
@@ -538,12 +538,12 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
         return;
       }
       const int seq = i_item / n_kv;
-      i_ctx = max(__ldg(ctx_lens + seq), 1);
+      i_ctx = max(ctx_lens[seq], 1);
       i_npages = (i_ctx + BS - 1) / BS;
       i_page = first_page(i_ctx);
       i_ids_base = i_page;
       i_ids = (i_ids_base + lane < i_npages)
-                  ? __ldg(block_table + (long long)seq * bt_stride + i_ids_base + lane)
+                  ? block_table[(long long)seq * bt_stride + i_ids_base + lane]
                   : 0;
     }
   };
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
     }
   };
   uint32_t qn[D / 16][2];  // prefetched Q of the NEXT item
-  int n_ctx = max(__ldg(ctx_lens + first / n_kv), 1);
+  int n_ctx = max(ctx_lens[first / n_kv], 1);
   load_q(first, qn);
   int consumed = 0;
   for (int item = first; item < total; item += n_warps) {
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 2)
     const int n_pages = (ctx + BS - 1) / BS;
     const int lo = (window > 0 && ctx > window) ? ctx - window : 0;
     if (item + n_warps < total) {  // prefetch the next item's Q and context length
-      n_ctx = max(__ldg(ctx_lens + (item + n_warps) / n_kv), 1);
+      n_ctx = max(ctx_lens[(item + n_warps) / n_kv], 1);
       load_q(item + n_warps, qn);
     }
     // TPV (D = 256): O^T tiles [dim = 16 i + lane/4 (+8)][head = 2(lane&3), +1], D/16 x 4 registers;
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
   const int kvh = blockIdx.y;
   follow_previous(q, out, kv_layer, block_table, tiles);
   if (long_keys > 0 && portion_keys(tiles, n_tiles, blockIdx.x, lane) >= long_keys) return;
-  const int4 tile = __ldg(tiles + blockIdx.x);
+  const int4 tile = tiles[blockIdx.x];
   const int bt_row = tile.x, row0 = tile.y, n_rows = tile.z, pos0 = tile.w;
   const int total_kv = pos0 + n_rows;  // keys 0 .. pos0+n_rows-1 are visible to this tile
   const int n_pages = (total_kv + BS - 1) / BS;
@@ -727,7 +727,7 @@ __global__ void __launch_bounds__((PfCfg<D>::MAX_G + 1) * 32)
         __syncwarp();
       }
       if (lane == 0) {
-        const int blk = __ldg(bt + p);
+        const int blk = bt[p];
         const uint32_t bytes = (uint32_t)n_valid * G_::ROW_BYTES;
         const uint8_t* kp =
             kv_layer + (((long long)blk * 2 + 0) * n_kv + kvh) * (long long)G_::PAGE_BYTES;

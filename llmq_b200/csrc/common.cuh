@@ -90,6 +90,15 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
                : "l"(p));
   return r;
 }
+// read once, not to be kept in L1; unlike ld_nc_v4 also right for what another kernel writes while this one is already on the chip
+__device__ __forceinline__ uint4 ld_once_v4(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p)
+               : "memory");
+  return r;
+}
 __device__ __forceinline__ uint4 ld_v4(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st_v4(void* p, uint4 v) { *reinterpret_cast<uint4*>(p) = v; }
 
@@ -202,10 +211,11 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
 // room: the launch, barriers, tensor memory and what may be asked into L2 ahead no longer lie between the two.  follow_previous waits
 // until that kernel has ended and what it wrote can be seen; nothing that another kernel may write is read, and nothing is written,
 // before it.  Every thread calls it, so the kernel two places back has ended as well; and it is called once the block has its tensor
-// memory (a block barrier between), which a block of the next kernel could otherwise take from it and hold until this one ends.  The
-// pointers that the kernel reads through go through it: a load marked read-only (__ldg, const __restrict__) is not held back by the wait
-// alone.  B200, in a graph of dependent kernels: 2.0 us instead of 3.4 from one small kernel to the next; the routed feed-forward of 128
-// rows (8 kernels) 73.2 -> 58.9 us, a decode step of four layers of the 1B model at 48 sequences (37 kernels) 371 -> 349 us.
+// memory (a block barrier between), which a block of the next kernel could otherwise take from it and hold until this one ends.  What
+// another kernel may write while this one waits is not read-only for this one's lifetime: no __ldg or ld.global.nc in such a kernel, and
+// the pointers that it reads through go through follow_previous, so that the compiler makes no such loads of const __restrict__ ones.
+// B200, in a graph of dependent kernels: 2.0 us instead of 3.4 from one small kernel to the next; the routed feed-forward of 128 rows
+// (8 kernels) 73.2 -> 58.9 us, a decode step of four layers of the 1B model at 48 sequences (37 kernels) 371 -> 349 us.
 template <typename T>
 __device__ __forceinline__ void pin_behind(T*& p) {
   asm volatile("" : "+l"(p)::"memory");

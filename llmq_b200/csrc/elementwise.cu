@@ -31,7 +31,7 @@ int tuning_epoch() { return __atomic_load_n(&g_epoch, __ATOMIC_RELAXED); }
 // back, so a decode row's input token is still on the device (engine.cu, async stepping).
 __device__ __forceinline__ int resolve_token(const int32_t* __restrict__ ids,
                                              const int32_t* __restrict__ prev_out, int t) {
-  int id = __ldg(ids + t);
+  int id = ids[t];
   if (id < 0) id = prev_out[-1 - id];  // plain load: written by the previous step's sampler
   return id;
 }
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) embed_kernel(const int32_t* __restrict__ 
        i += (long long)gridDim.x * blockDim.x) {
     int t = (int)(i / chunks), c = (int)(i % chunks);
     int id = resolve_token(ids, prev_out, t);
-    out[i] = ld_nc_v4(table + (long long)id * chunks + c);
+    out[i] = ld_once_v4(table + (long long)id * chunks + c);
   }
 }
 
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) embed_scaled_kernel(const int32_t* __rest
        i += (long long)gridDim.x * blockDim.x) {
     int t = (int)(i / chunks), c = (int)(i % chunks);
     int id = resolve_token(ids, prev_out, t);
-    uint4 a = ld_nc_v4(table + (long long)id * chunks + c);
+    uint4 a = ld_once_v4(table + (long long)id * chunks + c);
     uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
 #pragma unroll
     for (int k = 0; k < 4; ++k) ap[k] = pack_bf16x2(bf16_lo(ap[k]) * scale, bf16_hi(ap[k]) * scale);
@@ -79,13 +79,13 @@ constexpr int NORM_MAX_CHUNKS = 4;  // H <= 256*4*8 = 8192
 
 // 8 consecutive outputs of a split-K GEMM: the fp32 partials ws[s][row][col] added in split order
 // (the same order and rounding as the stand-alone reduction) and rounded to bf16
-__device__ __forceinline__ uint4 sum_partials_bf16(const float* __restrict__ ws, long long off,
+__device__ __forceinline__ uint4 sum_partials_bf16(const float* ws, long long off,
                                                    long long mn, int splits) {
-  float4 a = __ldg(reinterpret_cast<const float4*>(ws + off));
-  float4 b = __ldg(reinterpret_cast<const float4*>(ws + off + 4));
+  float4 a = *reinterpret_cast<const float4*>(ws + off);
+  float4 b = *reinterpret_cast<const float4*>(ws + off + 4);
   for (int sp = 1; sp < splits; ++sp) {
-    const float4 c = __ldg(reinterpret_cast<const float4*>(ws + sp * mn + off));
-    const float4 d = __ldg(reinterpret_cast<const float4*>(ws + sp * mn + off + 4));
+    const float4 c = *reinterpret_cast<const float4*>(ws + sp * mn + off);
+    const float4 d = *reinterpret_cast<const float4*>(ws + sp * mn + off + 4);
     a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
     b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
   }
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
     int c = threadIdx.x + j * NORM_THREADS;
     if (c < chunks) {
       uint4 a = v[j];
-      uint4 ww = __ldg(w + c);
+      uint4 ww = ld_v4(w + c);
       uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
       const uint32_t* wp = reinterpret_cast<const uint32_t*>(&ww);
 #pragma unroll
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
       int c = threadIdx.x + j * NORM_THREADS;
       if (c < chunks) {
         uint4 a = v[j];
-        gemma_scale_chunk(a, __ldg(w_post + c), inv);
+        gemma_scale_chunk(a, ld_v4(w_post + c), inv);
         uint4 r = ld_v4(residual + row * chunks + c);
         uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
         const uint32_t* rp = reinterpret_cast<const uint32_t*>(&r);
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
     int c = threadIdx.x + j * NORM_THREADS;
     if (c < chunks) {
       uint4 a = v[j];
-      gemma_scale_chunk(a, __ldg(w_out + c), inv);
+      gemma_scale_chunk(a, ld_v4(w_out + c), inv);
       st_v4(y + row * chunks + c, a);
     }
   }
@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(256)
   const int half = cpr / 2;     // chunk pairs per head
   const int row_chunks = (n_q + 2 * n_kv) * cpr;
   uint4* row = qkv + (long long)t * row_chunks;
-  const int pos = __ldg(positions + t);
-  const int slot = __ldg(slot_mapping + t);
+  const int pos = positions[t];
+  const int slot = slot_mapping[t];
   const uint4* cs_row = cos_sin + (long long)pos * cpr;  // [cos (D/2) | sin (D/2)]
   const int blk = slot >= 0 ? slot / block_size : 0;
   const int off = slot >= 0 ? slot % block_size : 0;
@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(256)
         x1 = ld_v4(row + head * cpr + c);
         x2 = ld_v4(row + head * cpr + c + half);
       }
-      uint4 cs = __ldg(cs_row + c);
-      uint4 sn = __ldg(cs_row + half + c);
+      uint4 cs = ld_v4(cs_row + c);
+      uint4 sn = ld_v4(cs_row + half + c);
       rope_chunk_pair(x1, x2, cs, sn);
       if (head < n_q) {
         st_v4(row + head * cpr + c, x1);
@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(256)
        i += (long long)gridDim.x * blockDim.x) {
     long long t = i / ichunks;
     int c = (int)(i % ichunks);
-    uint4 g = ld_nc_v4(gate_up + t * 2 * ichunks + c);
-    uint4 u = ld_nc_v4(gate_up + t * 2 * ichunks + ichunks + c);
+    uint4 g = ld_once_v4(gate_up + t * 2 * ichunks + c);
+    uint4 u = ld_once_v4(gate_up + t * 2 * ichunks + ichunks + c);
     uint32_t* gp = reinterpret_cast<uint32_t*>(&g);
     const uint32_t* up = reinterpret_cast<const uint32_t*>(&u);
 #pragma unroll
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(256)
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     int r = (int)(i / chunks), c = (int)(i % chunks);
-    out[i] = ld_v4(x + (long long)__ldg(rows + r) * chunks + c);
+    out[i] = ld_v4(x + (long long)rows[r] * chunks + c);
   }
 }
 
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(ARGMAX_THREADS)
     uint4 a[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c0 + u * step < nvec) a[u] = ld_nc_v4(rv + c0 + u * step);
+      if (c0 + u * step < nvec) a[u] = ld_once_v4(rv + c0 + u * step);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (c0 + u * step < nvec) {

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
           for (int j = 0; j < 4; ++j) {
             if constexpr (kAct == ACT_CLAMPED) {
               const float* b = bias + gate_row + n + j;
-              o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), bias ? __ldg(b) : 0.f, bias ? __ldg(b + 128) : 0.f,
+              o[j] = clamped_unit(__float_as_uint(o[j]), __float_as_uint(u[j]), bias ? b[0] : 0.f, bias ? b[128] : 0.f,
                                   a.limit);
             } else {
               o[j] = gated_unit<kAct>(__float_as_uint(o[j]), __float_as_uint(u[j]));

@@ -97,7 +97,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 x = gate_bias ? __ldg(bg + j) : zero, y = gate_bias ? __ldg(bu + j) : zero;
+            const float4 x = gate_bias ? bg[j] : zero, y = gate_bias ? bu[j] : zero;
             v[4 * j + 0] = __float_as_uint(clamped_unit(v[4 * j + 0], u[4 * j + 0], x.x, y.x, limit));
             v[4 * j + 1] = __float_as_uint(clamped_unit(v[4 * j + 1], u[4 * j + 1], x.y, y.y, limit));
             v[4 * j + 2] = __float_as_uint(clamped_unit(v[4 * j + 2], u[4 * j + 2], x.z, y.z, limit));

@@ -159,7 +159,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 // keys that the last token of tile i's portion sees (a whole warp asks; neighbouring tiles of one sequence that continue each other are a
 // portion), as far as 31 tiles on: exact for a comparison with up to 512
 __device__ __forceinline__ int portion_keys(const int4* tiles, int n_tiles, int i, int lane) {
-  const int4 t = __ldg(tiles + min(i + lane, n_tiles - 1));
+  const int4 t = tiles[min(i + lane, n_tiles - 1)];
   const int n = min(max(t.z, 0), 16);
   const int x = __shfl_up_sync(0xffffffffu, t.x, 1), y = __shfl_up_sync(0xffffffffu, t.y + n, 1), w = __shfl_up_sync(0xffffffffu, t.w + n, 1);
   const uint32_t ends = __ballot_sync(0xffffffffu, lane > 0 && (i + lane >= n_tiles || x != t.x || y != t.y || w != t.w));
