@@ -216,13 +216,20 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
 // the pointers that it reads through go through follow_previous, so that the compiler makes no such loads of const __restrict__ ones.
 // B200, in a graph of dependent kernels: 2.0 us instead of 3.4 from one small kernel to the next; the routed feed-forward of 128 rows
 // (8 kernels) 73.2 -> 58.9 us, a decode step of four layers of the 1B model at 48 sequences (37 kernels) 371 -> 349 us.
+// (pinned as an address of global memory, which the compiler would otherwise forget that it is)
+template <typename T>
+__device__ __forceinline__ T* pinned_global(T* p) {
+  size_t at = __cvta_generic_to_global(p);
+  asm volatile("" : "+l"(at)::"memory");
+  return reinterpret_cast<T*>(__cvta_global_to_generic(at));
+}
 template <typename T>
 __device__ __forceinline__ void pin_behind(T*& p) {
-  asm volatile("" : "+l"(p)::"memory");
+  p = pinned_global(p);
 }
 template <typename T>
 __device__ __forceinline__ void pin_behind(T* __restrict__& p) {
-  asm volatile("" : "+l"(p)::"memory");
+  p = pinned_global<T>(p);
 }
 template <typename... P>
 __device__ __forceinline__ void follow_previous(P&... p) {

@@ -5,6 +5,8 @@
 #include <limits.h>
 #include <stdarg.h>
 
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -76,6 +78,18 @@ __global__ void __launch_bounds__(256) embed_scaled_kernel(const int32_t* __rest
 // ------------------------------------------------------------------------------------------
 constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAX_CHUNKS = 4;  // H <= 256*4*8 = 8192
+// The kernels are made for 1, 2 and 4 chunks of a row per thread, and a thread asks for two or more of them, and of their weights, before it
+// stores the first: pointers that went through follow_previous are not known to lie apart, so that the compiler leaves every load behind
+// the store ahead of it.  us, add + norm before kernels began early / with the loads as the compiler left them / now: 48 rows of 8192
+// 4.0 / 4.3 / 3.1, 750 of 8192 6.8 / 8.7 / 6.6, 750 of 4096 4.5 / 5.0 / 4.1, 4608 of 2048 10.0 / 9.7 / 9.4.  Registers decide the rest: a
+// kernel for four chunks whatever the width takes 11.0 for the last of these, norms alone with all four weights of a thread at once 32.9
+// instead of 28.2 for 4608 rows of 8192.
+template <typename F>
+static int norm_chunks(int H, F&& launch) {
+  const int n = (H / 8 + NORM_THREADS - 1) / NORM_THREADS;
+  return n <= 1 ? launch(std::integral_constant<int, 1>{}) : n == 2 ? launch(std::integral_constant<int, 2>{})
+                                                                    : launch(std::integral_constant<int, NORM_MAX_CHUNKS>{});
+}
 
 // 8 consecutive outputs of a split-K GEMM: the fp32 partials ws[s][row][col] added in split order
 // (the same order and rounding as the stand-alone reduction) and rounded to bf16
@@ -100,7 +114,7 @@ __device__ __forceinline__ uint4 sum_partials_bf16(const float* ws, long long of
 // kPartials: x is not read from x_in but reduced on the fly from the fp32 partials of a split-K GEMM
 // (decode-sized batches): the projection's reduce pass, the residual add and the norm become ONE
 // launch instead of two, and the bf16 GEMM output never makes a round trip through memory.
-template <bool kAdd, bool kPartials = false>
+template <int CH, bool kAdd, bool kPartials = false>
 __global__ void __launch_bounds__(NORM_THREADS)
     rmsnorm_kernel(const uint4* __restrict__ x_in, uint4* __restrict__ residual,
                    const uint4* __restrict__ w, uint4* __restrict__ y, int chunks, float inv_h,
@@ -108,17 +122,31 @@ __global__ void __launch_bounds__(NORM_THREADS)
   follow_previous(x_in, residual, w, y, ws);
   const long long row = blockIdx.x;
   const uint4* xr = x_in + row * chunks;
-  uint4 v[NORM_MAX_CHUNKS];
+  constexpr bool kAhead = !kPartials;  // (beside the sums of parts, weights that come with the row cost more registers than they give)
+  constexpr int WN = kAhead ? CH : 2;
+  uint4 v[CH], res[2], weight[WN];
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_CHUNKS; ++j) {
+  for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
     if (c < chunks) {
-      uint4 a;
-      if constexpr (kPartials) a = sum_partials_bf16(ws, (row * chunks + c) * 8, mn, splits);
-      else a = ld_v4(xr + c);
+      if constexpr (kPartials) v[j] = sum_partials_bf16(ws, (row * chunks + c) * 8, mn, splits);
+      else v[j] = ld_v4(xr + c);
+      if constexpr (kAhead) weight[j] = ld_v4(w + c);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < CH; ++j) {
+    int c = threadIdx.x + j * NORM_THREADS;
+    if (kAdd && j % 2 == 0) {
+#pragma unroll
+      for (int i = 0; i < 2 && j + i < CH; ++i)
+        if (c + i * NORM_THREADS < chunks) res[i] = ld_v4(residual + row * chunks + c + i * NORM_THREADS);
+    }
+    if (c < chunks) {
+      uint4 a = v[j];
       if (kAdd) {
-        uint4 r = ld_v4(residual + row * chunks + c);
+        uint4 r = res[j % 2];
         uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
         const uint32_t* rp = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
@@ -147,11 +175,16 @@ __global__ void __launch_bounds__(NORM_THREADS)
   for (int i = 0; i < NORM_THREADS / 32; ++i) tot += red[i];
   const float inv = __frsqrt_rn(tot * inv_h + eps);
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_CHUNKS; ++j) {
+  for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
+    if (!kAhead && j % 2 == 0) {
+#pragma unroll
+      for (int i = 0; i < 2 && j + i < CH; ++i)
+        if (c + i * NORM_THREADS < chunks) weight[i] = ld_v4(w + c + i * NORM_THREADS);
+    }
     if (c < chunks) {
       uint4 a = v[j];
-      uint4 ww = ld_v4(w + c);
+      uint4 ww = weight[j % WN];
       uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
       const uint32_t* wp = reinterpret_cast<const uint32_t*>(&ww);
 #pragma unroll
@@ -207,7 +240,7 @@ __device__ __forceinline__ void gemma_scale_chunk(uint4& a, const uint4& ww, flo
   }
 }
 
-template <bool kSandwich>
+template <int CH, bool kSandwich>
 __global__ void __launch_bounds__(NORM_THREADS)
     gemma_norm_kernel(const uint4* __restrict__ x_in, uint4* __restrict__ residual,
                       const uint4* __restrict__ w_post, const uint4* __restrict__ w_next,
@@ -216,10 +249,10 @@ __global__ void __launch_bounds__(NORM_THREADS)
   follow_previous(x_in, residual, w_post, w_next, y);
   const long long row = blockIdx.x;
   const uint4* xr = x_in + row * chunks;
-  uint4 v[NORM_MAX_CHUNKS];
+  uint4 v[CH], res[2], weight[2];
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_CHUNKS; ++j) {
+  for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
     if (c < chunks) {
       v[j] = ld_v4(xr + c);
@@ -231,12 +264,20 @@ __global__ void __launch_bounds__(NORM_THREADS)
     // a = norm(x, w_post); residual <- bf16(residual + a); then the second norm over the new residual
     ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < NORM_MAX_CHUNKS; ++j) {
+    for (int j = 0; j < CH; ++j) {
       int c = threadIdx.x + j * NORM_THREADS;
+      if (j % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < 2 && j + i < CH; ++i)
+          if (c + i * NORM_THREADS < chunks) {
+            weight[i] = ld_v4(w_post + c + i * NORM_THREADS);
+            res[i] = ld_v4(residual + row * chunks + c + i * NORM_THREADS);
+          }
+      }
       if (c < chunks) {
         uint4 a = v[j];
-        gemma_scale_chunk(a, ld_v4(w_post + c), inv);
-        uint4 r = ld_v4(residual + row * chunks + c);
+        gemma_scale_chunk(a, weight[j % 2], inv);
+        uint4 r = res[j % 2];
         uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
         const uint32_t* rp = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
@@ -251,11 +292,16 @@ __global__ void __launch_bounds__(NORM_THREADS)
   }
   const uint4* w_out = kSandwich ? w_next : w_post;
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_CHUNKS; ++j) {
+  for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
+    if (j % 2 == 0) {
+#pragma unroll
+      for (int i = 0; i < 2 && j + i < CH; ++i)
+        if (c + i * NORM_THREADS < chunks) weight[i] = ld_v4(w_out + c + i * NORM_THREADS);
+    }
     if (c < chunks) {
       uint4 a = v[j];
-      gemma_scale_chunk(a, ld_v4(w_out + c), inv);
+      gemma_scale_chunk(a, weight[j % 2], inv);
       st_v4(y + row * chunks + c, a);
     }
   }
@@ -701,10 +747,12 @@ int b200q_gemma_rmsnorm(const void* x, const void* w, void* y, int T, int H, flo
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "gemma_rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(gemma_norm_kernel<false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
-                          (const uint4*)w, nullptr, (uint4*)y, H / 8, 1.f / (float)H, eps));
-  count_launch();
-  return B200Q_OK;
+  return norm_chunks(H, [&](auto ch) -> int {
+    B200Q_CUDA(launch_early(gemma_norm_kernel<decltype(ch)::value, false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
+                            (const uint4*)w, nullptr, (uint4*)y, H / 8, 1.f / (float)H, eps));
+    count_launch();
+    return B200Q_OK;
+  });
 }
 
 int b200q_gemma_norm_add_norm(void* x, void* residual, const void* w_post, const void* w_next, int T,
@@ -713,10 +761,12 @@ int b200q_gemma_norm_add_norm(void* x, void* residual, const void* w_post, const
                   "gemma_norm_add_norm: bad shape T=%d H=%d", T, H);
   B200Q_CHECK_ARG(x && residual && w_post && w_next, "gemma_norm_add_norm: null argument");
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(gemma_norm_kernel<true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
-                          (const uint4*)w_post, (const uint4*)w_next, (uint4*)x, H / 8, 1.f / (float)H, eps));
-  count_launch();
-  return B200Q_OK;
+  return norm_chunks(H, [&](auto ch) -> int {
+    B200Q_CUDA(launch_early(gemma_norm_kernel<decltype(ch)::value, true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
+                            (const uint4*)w_post, (const uint4*)w_next, (uint4*)x, H / 8, 1.f / (float)H, eps));
+    count_launch();
+    return B200Q_OK;
+  });
 }
 
 int b200q_softcap_bf16(void* logits, int64_t n, float cap, void* stream) {
@@ -733,10 +783,12 @@ int b200q_rmsnorm(const void* x, const void* w, void* y, int T, int H, float eps
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(rmsnorm_kernel<false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
-                          (const uint4*)w, (uint4*)y, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
-  count_launch();
-  return B200Q_OK;
+  return norm_chunks(H, [&](auto ch) -> int {
+    B200Q_CUDA(launch_early(rmsnorm_kernel<decltype(ch)::value, false>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, nullptr,
+                            (const uint4*)w, (uint4*)y, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
+    count_launch();
+    return B200Q_OK;
+  });
 }
 
 int b200q_add_rmsnorm(void* x, void* residual, const void* w, int T, int H, float eps,
@@ -744,10 +796,12 @@ int b200q_add_rmsnorm(void* x, void* residual, const void* w, int T, int H, floa
   B200Q_CHECK_ARG(T >= 0 && H > 0 && H % 8 == 0 && H <= NORM_THREADS * NORM_MAX_CHUNKS * 8,
                   "add_rmsnorm: bad shape T=%d H=%d", T, H);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(rmsnorm_kernel<true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
-                          (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
-  count_launch();
-  return B200Q_OK;
+  return norm_chunks(H, [&](auto ch) -> int {
+    B200Q_CUDA(launch_early(rmsnorm_kernel<decltype(ch)::value, true>, T, NORM_THREADS, 0, as_stream(stream), 1, (const uint4*)x, (uint4*)residual,
+                            (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, nullptr, 0, 0));
+    count_launch();
+    return B200Q_OK;
+  });
 }
 
 int b200q_add_rmsnorm_splitk(void* x, void* residual, const void* w, const float* partials,
@@ -756,10 +810,12 @@ int b200q_add_rmsnorm_splitk(void* x, void* residual, const void* w, const float
                   "add_rmsnorm_splitk: bad shape T=%d H=%d", T, H);
   B200Q_CHECK_ARG(partials && splits >= 1 && splits <= 16, "add_rmsnorm_splitk: bad partials (splits=%d)", splits);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(rmsnorm_kernel<true, true>, T, NORM_THREADS, 0, as_stream(stream), 1, nullptr, (uint4*)residual,
-                          (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, partials, splits, (long long)T * H));
-  count_launch();
-  return B200Q_OK;
+  return norm_chunks(H, [&](auto ch) -> int {
+    B200Q_CUDA(launch_early(rmsnorm_kernel<decltype(ch)::value, true, true>, T, NORM_THREADS, 0, as_stream(stream), 1, nullptr, (uint4*)residual,
+                            (const uint4*)w, (uint4*)x, H / 8, 1.f / (float)H, eps, partials, splits, (long long)T * H));
+    count_launch();
+    return B200Q_OK;
+  });
 }
 
 int b200q_rope_kvwrite(void* qkv, const void* cos_sin, const int32_t* positions,

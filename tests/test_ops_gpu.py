@@ -38,6 +38,36 @@ def test_add_rmsnorm(cuda, T, H):
     bf16_close(xg, y_ref, what="add_rmsnorm")
 
 
+@pytest.mark.parametrize("H", [8, 2040, 2048, 2056, 4096, 4104, 6152, 8192])
+def test_norms_at_chunk_edges(cuda, H):
+    """widths of one, two and four chunks per thread, the first of the next, the last thread's own"""
+    from llmq_b200 import lib
+    from oracle.gemma2 import gemma_rms_norm
+    T = 3
+    x, r, w, w2 = rnd(T, H, seed=1, scale=3.0), rnd(T, H, seed=2), rnd(H, seed=3), rnd(H, seed=4, scale=0.3)
+    y = torch.empty(T, H, dtype=BF, device=cuda)
+    lib.rmsnorm(x.to(cuda), w.to(cuda), y, 1e-5)
+    bf16_close(y, O.rms_norm(x.float(), w.float(), 1e-5), what="rmsnorm")
+    lib.gemma_rmsnorm(x.to(cuda), w2.to(cuda), y, 1e-6)
+    bf16_close(y, gemma_rms_norm(x.float(), w2.float(), 1e-6, "bf16"), what="gemma_rmsnorm")
+    y_ref, r_ref = O.add_rms_norm(x.float(), r.float(), w.float(), 1e-5)
+    xg, rg = x.to(cuda), r.to(cuda)
+    lib.add_rmsnorm(xg, rg, w.to(cuda), 1e-5)
+    assert torch.equal(rg.float().cpu(), r_ref)
+    bf16_close(xg, y_ref, what="add_rmsnorm")
+    # parts whose sum in their order is x
+    parts = torch.stack([x.float() * 0.5, x.float() * 0.25, x.float() * 0.25]).to(cuda)
+    xs, rs = torch.empty(T, H, dtype=BF, device=cuda), r.to(cuda)
+    lib.add_rmsnorm_splitk(xs, rs, w.to(cuda), parts.data_ptr(), 3, 1e-5)
+    assert torch.equal(rs, rg) and torch.equal(xs, xg)
+    a = gemma_rms_norm(x.float(), w2.float(), 1e-6, "bf16")
+    res = (r.float() + a.float()).to(BF)
+    xg, rg = x.to(cuda), r.to(cuda)
+    lib.gemma_norm_add_norm(xg, rg, w2.to(cuda), w.to(cuda), 1e-6)
+    bf16_close(rg, res.float(), what="gemma residual")
+    bf16_close(xg, gemma_rms_norm(rg.float().cpu(), w.float(), 1e-6, "bf16"), what="gemma_norm_add_norm")
+
+
 def test_embed_gather_argmax(cuda):
     from llmq_b200 import lib
     V, H, T = 1000, 512, 77
