@@ -582,7 +582,9 @@ __device__ __forceinline__ float gumbel_from_bits(uint32_t x) {
 // them.  The margin covers the roundings of t, best and the exponential (|best| * 1e-6 + 1.5e-3 in base 2, some ten times what they are),
 // so what is left out is smaller than the best, and the result is the one that all logarithms give.  The best so far is the CTA's, in
 // shared memory: a warp sees a few thousand logits only, and would take logarithms for a third of them on its own.  128 rows of 128256
-// logits 35 -> 25 us, 1024 rows 181 -> 132 (issue slots 58 % busy, half of them the random numbers).
+// logits 35 -> 25 us, 1024 rows 181 -> 133 (issue slots 58 % busy, half of them the random numbers).  Two CTAs per SM:
+// with three, which leave 40 registers to a thread, 28 and 142.  Rows of temperature 0:
+// 48 / 128 / 300 / 1024 of them 6.4 / 10.0 / 22 / 69 us (8.6 / 14.7 / 30 / 92 before).
 constexpr int SAMPLE_THREADS = 512;
 __device__ __forceinline__ int order_float(float v) {  // integers of the same order
   const int o = __float_as_int(v);
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
   const int split = blockIdx.x, splits = gridDim.x, r_ = blockIdx.y;
   const bf16* row = logits + (long long)r_ * V;
   const float temp = __int_as_float(params[4 * r_ + 0]);
-  // (the round keys are kept: made again for every block they are a fifth of its instructions)
+  // (the round keys are kept: 1024 rows 132.6 us, 133.4 with keys made again for every block; 128 rows 24.6 either way)
   uint32_t k0[10], k1[10];
 #pragma unroll
   for (int i = 0; i < 10; ++i) {
@@ -620,17 +622,44 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
   const uint2 none = make_uint2(0xff80ff80u, 0xff80ff80u);
   auto fetch = [&](int g) { return g < n4 ? *reinterpret_cast<const uint2*>(row + 4 * (long long)g) : none; };  // (8 B aligned: V*2 B rows)
   if (greedy) {
-    for (int g = first; g < n4; g += step) {
-      const uint2 a = fetch(g);
-      const float v[4] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y)};
+    auto take = [&](int g, uint2 q) {
+      const float v[4] = {bf16_lo(q.x), bf16_hi(q.x), bf16_lo(q.y), bf16_hi(q.y)};
 #pragma unroll
       for (int k = 0; k < 4; ++k) amax_update(v[k], 4 * g + k, best, bi);
-    }
+    };
+    int g = first;
+    auto round = [&](auto at_once) {  // so many loads in flight
+      constexpr int N = decltype(at_once)::value;
+      for (; g < n4 - (N - 1) * step; g += N * step) {
+        uint2 a[N];
+#pragma unroll
+        for (int x = 0; x < N; ++x) a[x] = fetch(g + x * step);
+#pragma unroll
+        for (int x = 0; x < N; ++x) take(g + x * step, a[x]);
+      }
+    };
+    round(std::integral_constant<int, 4>{});
+    round(std::integral_constant<int, 2>{});
+    round(std::integral_constant<int, 1>{});
   } else {
+    auto take = [&](int g, uint2 q) {  // the four logits of group g with their noise
+      uint32_t r[4];
+      philox4x32_10((uint32_t)g, pos, k0, k1, r);
+      const float v[4] = {bf16_lo(q.x), bf16_hi(q.x), bf16_lo(q.y), bf16_hi(q.y)};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) amax_update(v[k] * inv_t + gumbel_from_bits(r[k]), 4 * g + k, best, bi);
+    };
     uint2 a[AT_ONCE];
 #pragma unroll
     for (int x = 0; x < AT_ONCE; ++x) a[x] = fetch(first + x * step);
-    for (int g0 = first; g0 - (int)threadIdx.x < n4; g0 += AT_ONCE * step) {  // (whole CTAs go round together)
+    // (a row of one round: nothing to compare with before it has been looked at)
+    const bool one_round = n4 <= AT_ONCE * step;
+    if (one_round) {
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x)
+        if (first + x * step < n4) take(first + x * step, a[x]);
+    }
+    for (int g0 = first; !one_round && g0 - (int)threadIdx.x < n4; g0 += AT_ONCE * step) {  // (whole CTAs go round together)
       uint2 next[AT_ONCE];
 #pragma unroll
       for (int x = 0; x < AT_ONCE; ++x) next[x] = fetch(g0 + (AT_ONCE + x) * step);
@@ -654,13 +683,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
       if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
         for (int x = 0; x < AT_ONCE; ++x)
-          if (look[x]) {  // (seldom: its random numbers once more)
-            uint32_t r[4];
-            philox4x32_10((uint32_t)(g0 + x * step), pos, k0, k1, r);
-            const float v[4] = {bf16_lo(a[x].x), bf16_hi(a[x].x), bf16_lo(a[x].y), bf16_hi(a[x].y)};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) amax_update(v[k] * inv_t + gumbel_from_bits(r[k]), 4 * (g0 + x * step) + k, best, bi);
-          }
+          if (look[x]) take(g0 + x * step, a[x]);  // (seldom: its random numbers once more)
         const int o = __reduce_max_sync(0xffffffffu, order_float(best));
         if ((threadIdx.x & 31) == 0) atomicMax(&top_s, o);
       }
@@ -672,17 +695,27 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
   if (split == 0 && threadIdx.x == 0) ids[r_] = bi == 0x7fffffff ? 0 : bi;
 }
 
-// CTAs per row: the least (rounds of resident clusters) x (a CTA's share of a row and its start and end).  A cluster lies within one of the
-// chip's eight processing clusters, which has room for `room` CTAs (17 SMs counted, so that 48 clusters of 6 do not count as resident:
-// 48 rows of 128256 logits 14.9 us with 5 CTAs each, 18.7 with 6).  128 rows: 24.9 us with 2, 30.8 with 3, 37.8 with 1; 300 rows 55 / 60 /
-// 58; 1024 rows 149 / 182 / 132; one row 8 CTAs 8, 2 CTAs 13.
-static int row_splits(int rows, int room, int most) {
+// CTAs per row: the least rounds x (a CTA's share of a row and its start) + what a cluster and every CTA cost, in the time of one logit of a
+// CTA that works alone (of the argmax 0.05 ns, of the sampler 0.13).  Rounds: rows over the clusters that are resident at once, a last one
+// that is not full counted in part (`last`), because rows do not end together.  A cluster lies within one of the chip's eight processing clusters,
+// which has room for `room` CTAs (17 SMs counted, so that 48 clusters of 6 do not count as resident: 48 rows of 128256 logits 14.9 us with 5
+// CTAs each, 18.7 with 6).  Fitted to 1 to 1024 rows of 4096 to 256000 logits with 1 to 8 CTAs each: 1 (sampler) and 2 % (argmax) behind
+// the best number on average.  Sampler, us: 128 rows of 128256 24.8 with 2 CTAs each, 30 with 3, 35 with 1; 1024 rows 133 / 149 with 1 / 2;
+// one row 7.4 with 8, 12.9 with 2.  Argmax: 128 rows of 32000 4.1 / 4.8 / 5.3 with 1 / 2 / 4, of 128256 12.1 / 10.0 / 8.9; 300 rows of
+// 128256 20.8 / 16.8 / 17.4 with 1 / 2 / 3.
+struct RowCosts {
+  int room, per_cta;  // CTAs that a processing cluster has room for; logits below which a row is not shared any further
+  double cluster, last;
+};
+constexpr RowCosts ARGMAX_COSTS{4 * 17, 16 * ARGMAX_THREADS, 20000, 0.4}, SAMPLE_COSTS{2 * 17, 8 * SAMPLE_THREADS, 5000, 0.3};
+static int row_splits(int rows, int V, const RowCosts& c) {
   int best = 1;
   double least = 1e30;
-  for (int s = 1; s <= 8 && s <= most; ++s) {
-    const long long resident = 8LL * (room / s);
-    const double t = (double)((rows + resident - 1) / resident) * (1.0 / s + 0.1);
-    if (t < 0.95 * least) {
+  for (int s = 1; s <= 8 && s <= V / c.per_cta + 1; ++s) {
+    const int resident = 8 * (c.room / s);
+    const double full = (double)rows / resident, rounds = c.last * ((rows + resident - 1) / resident) + (1.0 - c.last) * (full > 1.0 ? full : 1.0);
+    const double t = rounds * ((double)V / s + 4000.0) + (s > 1 ? c.cluster : 0.0) + 20.0 * rows * s;
+    if (t < least) {
       least = t;
       best = s;
     }
@@ -869,7 +902,7 @@ int b200q_argmax_bf16(const void* logits, int32_t* ids, int B, int V, void* stre
   B200Q_CHECK_ARG(B >= 0 && V > 0, "argmax: bad shape B=%d V=%d", B, V);
   if (B == 0) return B200Q_OK;
   for (int at = 0; at < B; at += 65535) {  // (a grid's second dimension ends at 65535 rows)
-    const int rows = B - at < 65535 ? B - at : 65535, splits = row_splits(rows, 4 * 17, V / (16 * ARGMAX_THREADS) + 1);
+    const int rows = B - at < 65535 ? B - at : 65535, splits = row_splits(rows, V, ARGMAX_COSTS);
     B200Q_CUDA(launch_early(argmax_kernel, dim3(splits, rows), ARGMAX_THREADS, 0, as_stream(stream), splits,
                             (const bf16*)logits + (long long)at * V, ids + at, V));
     count_launch();
@@ -885,7 +918,7 @@ int b200q_sample_bf16(const void* logits, const int32_t* params, int32_t* ids, i
   // (a grid's second dimension ends at 65535 rows)
   for (int at = 0; at < B; at += 65535) {
     const int rows = B - at < 65535 ? B - at : 65535;
-    const int splits = row_splits(rows, 2 * 17, V / (8 * SAMPLE_THREADS) + 1);
+    const int splits = row_splits(rows, V, SAMPLE_COSTS);
     B200Q_CUDA(launch_early(sample_kernel, dim3(splits, rows), SAMPLE_THREADS, 0, as_stream(stream), splits,
                             (const bf16*)logits + (long long)at * V, params + 4 * (long long)at, ids + at, V));
     count_launch();

@@ -124,7 +124,7 @@ def test_largest_bits_do_not_win_by_themselves(cuda, low):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B", [1, 56, 64, 74, 89, 111, 148, 222, 444])   # rows of 8, 8, 7, 6, 5, 4, 3, 2 and 1 CTAs
+@pytest.mark.parametrize("B", [1, 56, 64, 74, 89, 111, 148, 222, 444])   # rows of 5 CTAs down to one
 def test_masked_rows_and_ties(cuda, B):
     V = 4 * 512 * 8 + 12   # (some CTAs of a row of eight take a second, short turn)
     rows = torch.randn(B, V, generator=torch.Generator().manual_seed(B)) * 3
@@ -171,3 +171,15 @@ def test_argmax_over_shared_rows(cuda, B, V):
     lib.argmax_bf16(rows.to(cuda), ids)
     want = [int((r == r.max()).nonzero()[0, 0]) for r in rows.float()]
     assert ids.cpu().tolist() == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 130, 600])
+@pytest.mark.parametrize("V", [4, 508, 2052, 4096, 4100, 6148, 8196])
+def test_rows_of_a_few_rounds(cuda, B, V):
+    """a row that its CTAs see in one round (every logit with its noise), one logit group more, and rows of temperature 0 with four, two and
+    one loads in flight"""
+    rows = torch.randn(B, V, generator=torch.Generator().manual_seed(B + V)) * 2
+    rows[B // 2, V - 1] = 40.0
+    temps, seeds, positions = [(0.7, 0.0, 1.3)[i % 3] for i in range(B)], [7 + i for i in range(B)], [5 * i for i in range(B)]
+    expect(draw_on_gpu(cuda, rows, temps, seeds, positions), rows, temps, seeds, positions)
