@@ -1022,6 +1022,19 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
                   PfCfg<D>::MAX_G);
   const ScoreConsts sc = score_consts(scale, softcap);
   dim3 grid(n_tiles, n_kv);
+  // Launched early, but for numbers of CTAs that an empty chip takes evenly and that come to lie two or three on one SM and none on another
+  // where those of the kernel before still hold their places (us, plainly / early: D = 128, 4 portions of 30 to 60 tokens, 104 CTAs 4.9 / 5.6,
+  // 3 of 60 to 120, 144 CTAs 6.4 / 7.3, but 32 of 16, 256 CTAs 5.1 / 4.9 and one of 128, 64 CTAs 7.1 / 6.6; D = 64, of which an SM holds
+  // more: 32 of 16, 256 CTAs 3.95 / 4.32, one of 512, 256 CTAs 18.6 / 21.6, 12 of 40 to 80, 432 CTAs 6.3 / 6.7, but 104 CTAs 4.4 / 4.3 and
+  // 20 of 10 to 100, 620 CTAs 8.9 / 8.3).
+  const long long ctas = (long long)n_tiles * n_kv, sms = attn_num_sms();
+  const bool uneven = D == 64 ? ctas > sms - 20 && ctas <= 13 * sms / 4 : 2 * ctas > sms && ctas <= sms;
+  if (uneven) {
+    kern<<<grid, (G + 1) * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, (const int4*)tiles,
+                                                n_tiles, n_q, n_kv, G, sc.c0, sc.c1, window, long_keys);
+    B200Q_LAUNCH_CHECK();
+    return B200Q_OK;
+  }
   B200Q_CUDA(launch_early(kern, grid, (G + 1) * 32, S_::TOTAL, st, 1, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt,
                           bt_stride, (const int4*)tiles, n_tiles, n_q, n_kv, G, sc.c0, sc.c1, window, long_keys));
   count_launch();

@@ -231,10 +231,12 @@ template <typename T>
 __device__ __forceinline__ void pin_behind(T* __restrict__& p) {
   p = pinned_global<T>(p);
 }
+// (the wait alone, where a block may find that it has nothing to do; follow_previous comes behind it once the block has its tensor memory)
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P>
 __device__ __forceinline__ void follow_previous(P&... p) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_previous();
   (pin_behind(p), ...);
 }
 template <typename... P, typename... A>

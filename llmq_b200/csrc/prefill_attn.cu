@@ -72,14 +72,25 @@ struct FaUnit {  // a CTA's place: unit u, at x of its round
   }
 };
 
+// An entry of a table (tiles, pages).  D = 64: a load instruction of its own; as the compiler places plain ones, one prompt of 6000 tokens
+// takes 287 us instead of 270 and 4 of 300 to 1200 43.9 instead of 41.2.  D = 128 and 256 lose 1 to 2 % by it.
+template <int D, typename T>
+__device__ __forceinline__ T table_entry(const T* p) {
+  if constexpr (D == 64)
+    return __ldca(p);
+  else
+    return *p;
+}
+
 // portion_keys of the tiles first .. first + 15, one per lane
+template <int D>
 __device__ __forceinline__ int block_portion_keys(const FaArgs& a, int first, int lane) {
   uint64_t ends = 0;  // bit p: tile first + p does not continue the one before it
   int keys[2], x = 0, y = 0, w = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int i = first + 32 * h + lane;
-    const int4 t = a.tiles[min(i, a.n_tiles - 1)];
+    const int4 t = table_entry<D>(a.tiles + min(i, a.n_tiles - 1));
     const int n = min(max(t.z, 0), 16);
     keys[h] = t.w + n;
     // (lane 0 compares with lane 31 of the half before)
@@ -99,6 +110,7 @@ __device__ __forceinline__ int block_portion_keys(const FaArgs& a, int first, in
 }
 
 // the runs of a block, seen by a whole warp: lane l holds tile l of the block
+template <int D>
 struct FaBlock {
   int4 t, ahead;
   uint32_t starts;  // bit l: tile l begins a run
@@ -107,7 +119,7 @@ struct FaBlock {
   __device__ __forceinline__ void fetch(const FaArgs& a, const FaOrder& o, int u, int lane) {
     ahead_first = u < o.units ? o.block(u / a.n_kv) * a.per_block : a.n_tiles;
     ahead_count = min(a.per_block, a.n_tiles - ahead_first);
-    ahead = lane < ahead_count ? a.tiles[ahead_first + lane] : make_int4(0, 0, 0, 0);
+    ahead = lane < ahead_count ? table_entry<D>(a.tiles + ahead_first + lane) : make_int4(0, 0, 0, 0);
   }
   template <bool kSplit>
   __device__ __forceinline__ void begin(const FaArgs& a, const FaOrder& o, FaUnit at, int lane) {
@@ -118,7 +130,7 @@ struct FaBlock {
     fetch(a, o, at.u, lane);
     t.z = min(max(t.z, 0), 16);
     if constexpr (kSplit)
-      if (block_portion_keys(a, first, lane) < a.long_keys) t.z = 0;  // (no rows: no run)
+      if (block_portion_keys<D>(a, first, lane) < a.long_keys) t.z = 0;  // (no rows: no run)
     const int br = __shfl_up_sync(0xffffffffu, t.x, 1), r0 = __shfl_up_sync(0xffffffffu, t.y, 1), nn = __shfl_up_sync(0xffffffffu, t.z, 1),
               p0 = __shfl_up_sync(0xffffffffu, t.w, 1);
     const bool next = lane > 0 && lane < count && br == t.x && r0 + nn == t.y && p0 + nn == t.w;
@@ -175,7 +187,7 @@ __device__ __forceinline__ void fa_row_again(const FaArgs& a, const int32_t* bt,
   for (int j0 = lo & ~31; j0 <= pos; j0 += 32) {
     const int j = j0 + lane, t = j & 15;
     const bool seen = j >= lo && j <= pos;
-    const int blk = seen ? bt[j >> 4] : 0;
+    const int blk = seen ? table_entry<D>(bt + (j >> 4)) : 0;
     float s = -INFINITY;
     if (seen) {
       const uint8_t* row = a.kv + ((long long)blk * 2 * a.n_kv + kvh) * page_bytes + t * (D * 2);
@@ -239,9 +251,9 @@ __device__ __noinline__ void fa_rows_again(const FaArgs& a, const FaOrder order)
   for (FaUnit w; w.u < order.units; w.step()) {
     const int kvh = w.u % a.n_kv, first = order.block(w.u / a.n_kv) * a.per_block, count = min(a.per_block, a.n_tiles - first);
     int keys = 0;
-    if constexpr (kSplit) keys = block_portion_keys(a, first, lane);
+    if constexpr (kSplit) keys = block_portion_keys<D>(a, first, lane);
     for (int i = 0; i < count; ++i) {
-      const int4 t = a.tiles[first + i];
+      const int4 t = table_entry<D>(a.tiles + first + i);
       if (kSplit && __shfl_sync(0xffffffffu, keys, i) < a.long_keys) continue;
       const int rows = min(max(t.z, 0), 16) * a.G;
       for (int f = warp; f < rows; f += 8) {
@@ -303,25 +315,23 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     mbar_init(&pv_done, 1);
     mbar_fence_init();
   }
+  if constexpr (kSplit) {  // no tile sees so many keys: nothing to do here
+    wait_for_previous();
+    bool any = false;
+    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {
+      const int4 t = table_entry<D>(a.tiles + i);
+      any |= t.w + min(max(t.z, 0), 16) >= a.long_keys;
+    }
+    if (!__syncthreads_or(any)) return;
+  }
   if (warp == 9) tmem_alloc(&tmem_slot, 512);
   __syncthreads();
   follow_previous();
-  if constexpr (kSplit) {  // no tile sees so many keys: nothing to do here
-    bool any = false;
-    for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {
-      const int4 t = a.tiles[i];
-      any |= t.w + min(max(t.z, 0), 16) >= a.long_keys;
-    }
-    if (!__syncthreads_or(any)) {
-      if (warp == 9) tmem_dealloc(tmem_slot, 512);
-      return;
-    }
-  }
   if (sort) {
     for (int i = threadIdx.x; i < n_blocks; i += FA_THREADS) steps_in[i] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < a.n_tiles; i += FA_THREADS) {  // the last token of a run sees most keys
-      const int4 t = a.tiles[i], n = a.tiles[min(i + 1, a.n_tiles - 1)];
+      const int4 t = table_entry<D>(a.tiles + i), n = table_entry<D>(a.tiles + min(i + 1, a.n_tiles - 1));
       const bool ends = i + 1 == a.n_tiles || (i + 1) % a.per_block == 0 || n.x != t.x || n.y != t.y + t.z || n.w != t.w + t.z;
       const int all = t.w + t.z, keys = a.window > 0 ? min(all, a.window) : all;
       if (ends && (!kSplit || all >= a.long_keys)) atomicAdd(steps_in + i / a.per_block, max(keys, 0) / KT + 2);  // (start and end: about one step)
@@ -360,7 +370,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     // ===== pages =====
     if (lane == 0) tma_prefetch_desc(&kv_map);
     int n_loaded[2] = {0, 0};
-    FaBlock b;
+    FaBlock<D> b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
       b.template begin<kSplit>(a, order, w, lane);
@@ -375,7 +385,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
         const int n_pages = (total + 15) / 16 - k0 / 16;
         auto page_of = [&](int j) {
           const int at_page = j * PAGES + lane;
-          return lane < PAGES && at_page < n_pages && j < steps ? bt[at_page] : 0;
+          return lane < PAGES && at_page < n_pages && j < steps ? table_entry<D>(bt + at_page) : 0;
         };
         // one step's keys or values; keys are asked for a step ahead of values, whose slot is free that much later
         auto load = [&](int which, int j, int blk) {
@@ -450,7 +460,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
       __syncwarp();
       tc_fence_after();
     };
-    FaBlock b;
+    FaBlock<D> b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
       b.template begin<kSplit>(a, order, w, lane);
@@ -560,7 +570,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
     constexpr int LPR = D / 8, RPP = 64 / LPR;  // lanes per row, rows per pass of the two warps
     const int tid = threadIdx.x - 320, c = tid % LPR;
     uint32_t par[2] = {1, 1};
-    FaBlock b;
+    FaBlock<D> b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
       b.template begin<kSplit>(a, order, w, lane);
@@ -643,7 +653,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) prefill_attn_kernel(const __gri
       return fmaf(v, a.c0, -base);
     };
     auto both = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
-    FaBlock b;
+    FaBlock<D> b;
     b.fetch(a, order, blockIdx.x, lane);
     for (FaUnit w; w.u < order.units; w.step()) {
       b.template begin<kSplit>(a, order, w, lane);
@@ -899,8 +909,18 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
   }
   const long long units = (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv;
   const int grid = units < FA_SMS ? (int)units : FA_SMS;
-  B200Q_CUDA(launch_early(kern, grid, FA_THREADS, C::SMEM, st, 1, map, a));
-  count_launch();
+  // Launched early where a CTA has no more than two units, or units of one step of keys.  CTAs that find their SMs as those of the kernel
+  // before leave them come to lie elsewhere than the launch of an empty chip puts them, and where long units are dealt out over several
+  // rounds that costs more than the start that is saved (D = 128, us, plainly / early: 12 portions of 100 to 700 tokens 56.8 / 61.3, 8 of 512
+  // 47.0 / 50.5, 16 of 256 37.4 / 39.5, 4 of 300 to 1200 51.0 / 53.0; but one of 512 22.2 / 21.5, 36 of 128 32.8 / 32.5; D = 64 60 of 128
+  // 44.5 / 42.7, 8 of 512 37.6 / 40.2; D = 256, 4 heads, 8 of 512 30.8 / 29.9, 40 of 50 to 200 41.0 / 43.0).
+  if (units <= 2 * FA_SMS || a.bt_stride * 16 <= C::KT) {
+    B200Q_CUDA(launch_early(kern, grid, FA_THREADS, C::SMEM, st, 1, map, a));
+    count_launch();
+  } else {
+    kern<<<grid, FA_THREADS, C::SMEM, st>>>(map, a);
+    B200Q_LAUNCH_CHECK();
+  }
   return B200Q_OK;
 }
 

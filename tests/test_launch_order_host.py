@@ -73,6 +73,7 @@ def test_no_thread_leaves_ahead_of_the_wait():
     for kernel in early(found):
         for f, is_kernel, body in found[kernel]:
             if is_kernel and "follow_previous(" in body:
+                wait = min(body.index(w) for w in ("follow_previous(", "wait_for_previous(") if w in body)
                 # (a `return` of a lambda ahead of it does not end the kernel)
-                ahead = re.sub(r"\[&?\]\s*\([^)]*\)\s*\{[^{}]*(?:\{[^{}]*\}[^{}]*)*\}", "", body[:body.index("follow_previous(")])
+                ahead = re.sub(r"\[&?\]\s*\([^)]*\)\s*\{[^{}]*(?:\{[^{}]*\}[^{}]*)*\}", "", body[:wait])
                 assert not re.search(r"\breturn\b", ahead), (f, kernel)
