@@ -440,7 +440,11 @@ __global__ void __launch_bounds__(256) residual_add_routed_kernel(float* __restr
   }
 }
 
-// bf16 rows, 8 channels per thread: the token's chosen rows are read with 16-byte loads
+// bf16 rows, 8 channels per thread: the token's chosen rows are read with 16-byte loads.  AT choices at a time: their places are asked for
+// together, then their rows.  Four where every thread has one piece of a row, so that nothing else hides the reads (128 tokens of 4 choices,
+// 2048 wide 4.3 -> 3.3 us), one where threads have more: the registers of four cost as much in threads (2000 tokens of 6, 3072 wide 33 us,
+// 46 with four; 2000 of 4, 2048 wide 11.2 / 12.4).
+template <int AT>
 __global__ void __launch_bounds__(256) residual_add_routed_v8_kernel(float* __restrict__ x, const bf16* __restrict__ eout,
                                                                      const int32_t* __restrict__ pair_pos,
                                                                      const int32_t* __restrict__ idx,
@@ -453,25 +457,25 @@ __global__ void __launch_bounds__(256) residual_add_routed_v8_kernel(float* __re
     const long long at = (long long)t * W8 * 8 + c;
     float ff[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float4* xo = reinterpret_cast<float4*>(x + at);
-    float4 a = xo[0], b = xo[1];
-    // four choices at a time: their places are asked for together, then their rows (one by one 4.4 us for 128 tokens, 4 choices each)
-    for (int k0 = 0; k0 < top; k0 += 4) {
+    float4 a, b;
+    if constexpr (AT > 1) a = xo[0], b = xo[1];
+    for (int k0 = 0; k0 < top; k0 += AT) {
       const long long p0 = (long long)t * top + k0;
-      int id[4], pos[4];
-      float wk[4];
-      uint4 v[4];
+      int id[AT], pos[AT];
+      float wk[AT];
+      uint4 v[AT];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < AT; ++k) {
         const bool on = k0 + k < top;
         id[k] = on ? idx[p0 + k] : n_real;
         pos[k] = on ? pair_pos[p0 + k] : 0;
         wk[k] = on ? wts[p0 + k] : 0.f;
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < AT; ++k)
         if (k0 + k < top) v[k] = id[k] < n_real ? ld_v4(eout + (long long)pos[k] * W8 * 8 + c) : ld_v4(h + at);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < AT; ++k)
         if (k0 + k < top) {
           const uint32_t q[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
 #pragma unroll
@@ -481,6 +485,7 @@ __global__ void __launch_bounds__(256) residual_add_routed_v8_kernel(float* __re
           }
         }
     }
+    if constexpr (AT == 1) a = xo[0], b = xo[1];
     a.x += ff[0]; a.y += ff[1]; a.z += ff[2]; a.w += ff[3];
     b.x += ff[4]; b.y += ff[5]; b.z += ff[6]; b.w += ff[7];
     xo[0] = a;
@@ -664,8 +669,9 @@ int b200q_residual_add_routed(float* x, const void* expert_out, const int32_t* p
   if (T_ == 0) return B200Q_OK;
   if (dtype == B200Q_DTYPE_BF16 && W % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(expert_out) | reinterpret_cast<uintptr_t>(h)) & 15) == 0)
-    B200Q_CUDA(launch_early(residual_add_routed_v8_kernel, grid_for((long long)T_ * W / 8), 256, 0, as_stream(stream), 1, x,
-                            (const bf16*)expert_out, pair_pos, idx, wts, top, n_real, (const bf16*)h, T_, W / 8));
+    B200Q_CUDA(launch_early((long long)T_ * W / 8 <= 148 * 2048 ? residual_add_routed_v8_kernel<4> : residual_add_routed_v8_kernel<1>,
+                            grid_for((long long)T_ * W / 8), 256, 0, as_stream(stream), 1, x, (const bf16*)expert_out, pair_pos, idx, wts, top,
+                            n_real, (const bf16*)h, T_, W / 8));
   else
     DISPATCH_T(dtype, (residual_add_routed_kernel<T><<<grid_for((long long)T_ * W), 256, 0, as_stream(stream)>>>(
                           x, (const T*)expert_out, pair_pos, idx, wts, top, n_real, (const T*)h, T_, W)));

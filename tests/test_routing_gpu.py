@@ -48,22 +48,19 @@ def test_picks(cuda, E, groups, keep):
 
 
 @pytest.mark.parametrize("top", [1, 3, 4, 5, 8, 9])
-@pytest.mark.parametrize("W", [8, 2056])
-def test_sums_of_routed_rows(cuda, top, W):
+@pytest.mark.parametrize("T,W", [(13, 8), (13, 2056), (1179, 2056), (1180, 2056)])   # four choices at a time, at last one
+def test_sums_of_routed_rows(cuda, top, T, W):
     from llmq_b200 import lib as L
     lib = L.load()
     g = torch.Generator().manual_seed(top * W)
-    T, real = 13, 6
+    real = 6
     x, eo = torch.randn(T, W, generator=g), torch.randn(T * top, W, generator=g).to(torch.bfloat16)
     h, wts = torch.randn(T, W, generator=g).to(torch.bfloat16), torch.rand(T * top, generator=g)
     idx, pair = torch.randint(0, real + 2, (T * top,), generator=g).to(torch.int32), torch.randperm(T * top, generator=g).to(torch.int32)
     d = [v.to(cuda) for v in (x, eo, pair, idx, wts, h)]
     L.check(lib.b200q_residual_add_routed(*[v.data_ptr() for v in d[:5]], top, real, d[5].data_ptr(), T, W, L.DTYPE_BF16, None))
     torch.cuda.synchronize()
-    want = x.double()
-    for t in range(T):
-        for k in range(top):
-            p = t * top + k
-            want[t] += wts[p].double() * (eo[pair[p]] if idx[p] < real else h[t]).double()
+    rows = torch.where((idx < real)[:, None], eo[pair.long()], h.repeat_interleave(top, 0)).double()
+    want = x.double() + (wts.double()[:, None] * rows).view(T, top, W).sum(1)
     # top + 1 fp32 additions of terms of order 1
     assert float((d[0].cpu().double() - want).abs().max()) < 2e-6 * (top + 2)
