@@ -104,7 +104,7 @@ int b200q_gemm_bf16(const void* A_dev, const void* W_dev, void* C_dev,
 
 /* Decode-sized batches: the split-K form of b200q_gemm_bf16 WITHOUT its reduce pass.  If the library
  *     would split the reduction for this shape, the fp32 partial tiles are left in its scratch
- *     (*partials = [splits][M][N], valid until the next split-K GEMM on the stream) and *splits > 1;
+ *     (*partials = [splits][M][N], the stream's or, during capture, the graph's; valid until the next split product there) and *splits > 1;
  *     the caller folds sum-in-split-order + bf16 rounding into the consumer (the two *_splitk ops
  *     below).  *splits == 1: nothing was launched, call b200q_gemm_bf16.  Results are bit-identical
  *     to the unfused sequence. */

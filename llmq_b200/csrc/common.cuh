@@ -33,6 +33,17 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
 int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w, cudaStream_t st, const float** partials_out,
                  int* splits_out);
 int linear_gated(bool gelu, const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st);
+// While one of these lives, split products that the calling thread asks for leave their parts in `*slot` (allocated at the first): a pass
+// runs under one of its model's
+class SplitScratchOf {
+ public:
+  explicit SplitScratchOf(void** slot);
+  ~SplitScratchOf();
+  SplitScratchOf(const SplitScratchOf&) = delete;
+
+ private:
+  void** before_;
+};
 
 #define B200Q_CHECK_ARG(cond, ...)          \
   do {                                      \

@@ -17,8 +17,10 @@
 // tensor-bound (2*M*N*K flops against the measured bf16 peak).
 #include <stdlib.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "tcgen05.cuh"
 
@@ -709,15 +711,135 @@ static int num_sms() {
   return n;
 }
 
-// fixed-size scratch of partial tiles (8 splits x 256 rows x 8192 cols fp32 = 64 MiB), allocated once and never moved: CUDA
-// graphs captured by the engine bake this pointer into their kernel nodes
-static int splitk_scratch(int splits, int M, int N, float** out) {
-  static float* ws = nullptr;
+// ---- scratch of partial tiles -----------------------------------------------------------------------
+// Whoever orders its products by itself has its own, so that nobody's parts are overwritten before they are added: a model (its passes run
+// one behind the other; SplitScratchOf), a stream, and a graph in the making, whose replays may run beside the stream that it was captured
+// on.  A buffer never moves while it has an owner: graphs bake its address in.
+static constexpr size_t SPLIT_BYTES = (size_t)8 * 256 * 8192 * sizeof(float);  // 8 splits x 256 rows x 8192 columns: 64 MiB
+thread_local void** t_model_scratch = nullptr;
+SplitScratchOf::SplitScratchOf(void** slot) : before_(t_model_scratch) { t_model_scratch = slot; }
+SplitScratchOf::~SplitScratchOf() { t_model_scratch = before_; }
+
+namespace {
+// (cudaMalloc and its like are refused to every thread while any stream is being captured in the default mode, unless the thread says that it
+// knows)
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+struct SplitBuffer {
+  void* p = nullptr;
+  size_t bytes = 0;
+  int device = 0;
+  unsigned long long stream = 0, capture = 0, used = 0;  // capture: of the graph that owns it; 0: the stream does
+  std::atomic<bool> free{false};                         // the graph is gone
+};
+std::mutex g_split_mu;
+std::vector<SplitBuffer*> g_split;  // (never shrinks in entries that a callback may still name)
+constexpr int SPLIT_STREAMS = 16;     // buffers of streams; further streams take over the one that was not used for longest
+constexpr size_t SPLIT_SPARE = 2 * SPLIT_BYTES;  // kept of what graphs have given back
+
+int split_alloc(size_t bytes, void** p) {
+  RelaxedCapture relaxed;
+  B200Q_CUDA(cudaMalloc(p, bytes));
+  return B200Q_OK;
+}
+}  // namespace
+
+static int splitk_scratch(int splits, int M, int N, cudaStream_t st, float** out) {
   const size_t need = (size_t)splits * M * N * sizeof(float);
-  const size_t cap = (size_t)8 * 256 * 8192 * sizeof(float);
-  B200Q_CHECK_ARG(need <= cap, "split-K scratch too small for M=%d N=%d splits=%d", M, N, splits);
-  if (!ws) B200Q_CUDA(cudaMalloc(&ws, cap));
-  *out = ws;
+  B200Q_CHECK_ARG(need <= SPLIT_BYTES, "split-K scratch too small for M=%d N=%d splits=%d", M, N, splits);
+  if (t_model_scratch) {
+    if (!*t_model_scratch)
+      if (int rc = split_alloc(SPLIT_BYTES, t_model_scratch)) return rc;
+    *out = (float*)*t_model_scratch;
+    return B200Q_OK;
+  }
+  int device = 0;
+  unsigned long long id = 0, capture = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  const cudaGraphNode_t* nodes = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t n_nodes = 0;
+  cudaGetDevice(&device);
+  if (cudaStreamGetCaptureInfo_v3(st, &status, &capture, &graph, &nodes, &edges, &n_nodes) != cudaSuccess ||
+      status != cudaStreamCaptureStatusActive) {
+    cudaGetLastError();  // (a product that cannot run here fails at its launch)
+    capture = 0;
+    B200Q_CUDA(cudaStreamGetId(st, &id));  // (a handle may come back as that of another stream)
+  } else {
+    id = (unsigned long long)reinterpret_cast<uintptr_t>(st);
+  }
+  static unsigned long long clock = 0;
+  std::lock_guard<std::mutex> lock(g_split_mu);
+  SplitBuffer *own = nullptr, *oldest = nullptr;
+  int streams = 0;
+  for (SplitBuffer* b : g_split) {
+    if (!b->p || b->device != device || b->free.load()) continue;
+    if (b->stream == id && b->capture == capture && b->bytes >= need) own = b;
+    if (b->capture == 0) {
+      ++streams;
+      if (!oldest || b->used < oldest->used) oldest = b;
+    }
+  }
+  if (!own && capture == 0) {
+    if (streams >= SPLIT_STREAMS) {
+      RelaxedCapture relaxed;
+      if (cudaDeviceSynchronize() == cudaSuccess)
+        own = oldest;
+      else
+        cudaGetLastError();  // (something is being captured: one more buffer)
+    }
+    if (!own) {
+      own = new SplitBuffer;
+      if (int rc = split_alloc(own->bytes = SPLIT_BYTES, &own->p)) {
+        delete own;
+        return rc;
+      }
+      g_split.push_back(own);
+    }
+    // what graphs have given back, down to a spare or two
+    size_t spare = 0;
+    for (SplitBuffer* b : g_split)
+      if (b->p && b->free.load() && (spare += b->bytes) > SPLIT_SPARE) {
+        RelaxedCapture relaxed;
+        spare -= b->bytes;
+        if (cudaFree(b->p) == cudaSuccess)
+          b->p = nullptr;
+        else
+          cudaGetLastError();
+      }
+  } else if (!own) {
+    size_t bytes = (size_t)1 << 20;
+    while (bytes < need) bytes *= 2;
+    for (SplitBuffer* b : g_split)  // the smallest that fits of those given back
+      if (b->p && b->free.load() && b->device == device && b->bytes >= need && (!own || b->bytes < own->bytes)) own = b;
+    if (!own) {
+      for (SplitBuffer* b : g_split)
+        if (!b->p) own = b;
+      const bool fresh = !own;
+      if (fresh) own = new SplitBuffer;
+      if (int rc = split_alloc(own->bytes = bytes, &own->p)) {
+        own->p = nullptr;
+        if (fresh) delete own;
+        return rc;
+      }
+      if (fresh) g_split.push_back(own);
+    }
+    own->free.store(true);  // (until the graph holds it)
+    cudaUserObject_t held;
+    B200Q_CUDA(cudaUserObjectCreate(&held, own, [](void* b) { static_cast<SplitBuffer*>(b)->free.store(true); }, 1,
+                                    cudaUserObjectNoDestructorSync));
+    B200Q_CUDA(cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove));
+    own->free.store(false);
+  }
+  own->device = device;
+  own->stream = id;
+  own->capture = capture;
+  own->used = ++clock;
+  *out = (float*)own->p;
   return B200Q_OK;
 }
 
@@ -742,8 +864,11 @@ static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int 
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (N / BN) * splits;
   const int grid = tiles < num_sms() ? tiles : num_sms();
   float* ws = nullptr;
+  static std::mutex pair;  // (no other thread's product on the same stream between a product and the sum of its parts)
+  std::unique_lock<std::mutex> together(pair, std::defer_lock);
   if (splits > 1) {
-    rc = splitk_scratch(splits, M, N, &ws);
+    if (!partials_out) together.lock();
+    rc = splitk_scratch(splits, M, N, st, &ws);
     if (rc) return rc;
   }
   B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K, splits, ws, a_rows * GEMM_BK * 2,
@@ -1165,7 +1290,7 @@ int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w
     const int n = gemm_skinny_splits(M, N, K);
     if (n <= 1 || N > 8192) return B200Q_OK;
     float* ws = nullptr;
-    int rc = splitk_scratch(n, M, N, &ws);
+    int rc = splitk_scratch(n, M, N, st, &ws);
     if (!rc) rc = gemm_skinny(A, W, nullptr, M, N, K, ACT_NONE, N, nullptr, 0.f, ws, fixed_w, st);
     if (rc) return rc;
     *partials_out = ws;
@@ -1270,8 +1395,8 @@ int b200q_gemm_bf16(const void* A, const void* W, void* C, int M, int N, int K, 
 // ([splits][M][N], *partials_out) and NO reduce pass runs — the caller folds the fixed-order sum and
 // the bf16 rounding into the kernel that consumes the projection (b200q_add_rmsnorm_splitk,
 // b200q_rope_kvwrite_splitk), saving a launch and a round trip per projection.  *splits_out = 1
-// means nothing was launched: call b200q_gemm_bf16 instead.  The scratch is overwritten by the next
-// split-K GEMM on the stream.
+// means nothing was launched: call b200q_gemm_bf16 instead.  The scratch is the stream's, or the graph's that is being captured, and
+// is overwritten by the next split product there (a call of b200q_gemm_bf16 may be one); passes of a model leave it alone.
 int b200q_gemm_bf16_splitk(const void* A, const void* W, int M, int N, int K, void* stream, const float** partials_out, int* splits_out) {
   return linear_parts(A, W, M, N, K, false, as_stream(stream), partials_out, splits_out);
 }

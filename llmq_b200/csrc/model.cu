@@ -104,6 +104,7 @@ int b200q_model_destroy(b200q_model_t m) {
   if (m) {
     for (cudaEvent_t e : m->ev_pool) cudaEventDestroy(e);
     layered_destroy(m);
+    if (m->split_ws) cudaFree(m->split_ws);
   }
   delete m;
   return B200Q_OK;
@@ -229,6 +230,7 @@ int b200q_model_profile_collect(b200q_model_t m, b200q_profile* out, int reset) 
 
 int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
   B200Q_CHECK_ARG(m && b, "forward: null argument");
+  const SplitScratchOf own(&m->split_ws);
   if (m->lay) return layered_forward(m, b, stream);
   const b200q_model_config& c = m->cfg;
   if (!m->embed || !m->final_norm || !m->lm_head || !m->kv || !m->rope || !m->ws) {

@@ -126,6 +126,7 @@ struct b200q_model {
        *sel = nullptr, *logits = nullptr;
   // fold the split-K reduce of decode-sized projections into the consuming kernel (B200Q_FUSE_SPLITK=0: off)
   bool fuse_splitk = true;
+  void* split_ws = nullptr;  // parts of split reductions (SplitScratchOf)
   b200q_layered* lay = nullptr;  // B200Q_ARCH_RAMOPEL: everything layer-specific lives here
   // optional per-category device timing (CUDA events on the forward's stream)
   bool profiling = false;
