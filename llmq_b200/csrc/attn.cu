@@ -872,10 +872,14 @@ static int prepare_decode() {
   return B200Q_OK;
 }
 
+template <bool kShared>
+static dim3 decode_grid(int splits, int n_seqs, int n_kv) {
+  return kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
+}
 template <int D, int BS, bool kShared>
 static cudaLaunchConfig_t decode_config(int splits, int n_seqs, int n_kv, cudaLaunchAttribute* attr, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
+  cfg.gridDim = decode_grid<kShared>(splits, n_seqs, n_kv);
   cfg.blockDim = dim3(DEC_WARPS * 32);
   cfg.dynamicSmemBytes = DecSmem<D, BS>::TOTAL;
   cfg.stream = st;
@@ -955,10 +959,8 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
   const int rc = prepare_decode<D, BS, kCap, kShared>();
   if (rc) return rc;
   const ScoreConsts sc = score_consts(scale, softcap);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = decode_config<D, BS, kShared>(splits, n_seqs, n_kv, &attr, st);
-  B200Q_CUDA(launch_early(kern, cfg.gridDim, DEC_WARPS * 32, cfg.dynamicSmemBytes, st, splits, (const bf16*)q, q_stride, (bf16*)out,
-                          (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window, ahead));
+  B200Q_CUDA(launch_early(kern, decode_grid<kShared>(splits, n_seqs, n_kv), DEC_WARPS * 32, DecSmem<D, BS>::TOTAL, st, splits, (const bf16*)q,
+                          q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window, ahead));
   count_launch();
   return B200Q_OK;
 }

@@ -11,7 +11,8 @@
 //   * the first weights are asked for before the kernel before this one has ended (follow_previous): into the ring where nobody can
 //     still be writing them (fixed_w), into L2 otherwise.
 // A gated unit (SwiGLU, GeGLU, clamped) works on a 128-row tile of 64 gate rows and the 64 rows that they gate: few or no splits whose
-// parts would have to meet (28672 x 4096, 100 rows: 44.7 us, 48.0 with tiles of 128 + 128 rows; 16384 x 2048, 48 rows: 14.2, 16.3).
+// parts would have to meet (28672 x 4096, 100 rows: 45.7 us, 48.0 with tiles of 128 + 128 rows; 16384 x 2048, 48 rows: 14.4, 16.3;
+// but 6144 x 4096, 100 rows 17.9, 17.0: few tiles, each of which fetches all rows of A).
 #include "tcgen05.cuh"
 
 namespace b200q {

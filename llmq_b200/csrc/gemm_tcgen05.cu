@@ -19,6 +19,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -944,7 +945,7 @@ struct TileChoice {
   bool pair;
   int bn;
 };
-static TileChoice choose_tile(int M, int N, bool gated) {
+static TileChoice choose_tile(int M, int N, bool gated, bool pairs) {
   const struct {
     bool pair;
     int bn;
@@ -955,7 +956,7 @@ static TileChoice choose_tile(int M, int N, bool gated) {
   double least = 1e30;
   for (const auto& c : all) {
     const bool ragged = c.bn == 160 || c.bn == 192;
-    if ((ragged ? N < c.bn : N % c.bn != 0) || (gated && c.bn != 256) || (c.pair && M <= GEMM_BM)) continue;
+    if ((ragged ? N < c.bn : N % c.bn != 0) || (gated && c.bn != 256) || (c.pair && (!pairs || M <= GEMM_BM))) continue;
     const long long rows = c.pair ? 256 : GEMM_BM, slots = c.pair ? num_sms() / 2 : num_sms();
     const long long tiles = (M + rows - 1) / rows * ((N + c.bn - 1) / c.bn);
     const double t = (double)((tiles + slots - 1) / slots) * c.cost;
@@ -1232,7 +1233,7 @@ static int gemm_gated(const char* what, const void* A, const void* W, void* C, i
   cudaStream_t st = as_stream(stream);
   if (use_skinny(M, N, K, true))
     return gemm_skinny(A, W, C, M, N, K, kAct, ldc > 0 ? ldc : N / 2, gate.bias, gate.limit, nullptr, fixed_w, st);
-  if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && choose_tile(M, N, true).pair))
+  if ((g_gemm_mode == 2 && M > GEMM_BM) || (g_gemm_mode == 0 && choose_tile(M, N, true, true).pair))
     return launch_gemm2<256, kAct>(A, W, C, M, N, K, st, ldc, gate, fixed_w);
   return launch_gemm<256, kAct>(A, W, C, M, N, K, st, 1, nullptr, ldc, gate, fixed_w);
 }
@@ -1263,12 +1264,16 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
     if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
   }
   if (bn == 0) {
-    const TileChoice t = choose_tile(M, N, false);
-    if (t.bn == 192 && g_gemm_mode == 0) return launch_gemm2<192>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
-    if (t.bn == 160 && g_gemm_mode == 0) return launch_gemm2<160>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
-    if (t.pair && g_gemm_mode == 0)
-      return t.bn == 256 ? launch_gemm2<256>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w) : launch_gemm2<128>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
-    bn = t.bn == 192 || t.bn == 160 ? 256 : t.bn;
+    const TileChoice t = choose_tile(M, N, false, g_gemm_mode == 0);
+    auto pair = [&](auto width) {
+      return launch_gemm2<decltype(width)::value>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
+    };
+    if (t.pair)
+      return t.bn == 256   ? pair(std::integral_constant<int, 256>{})
+             : t.bn == 192 ? pair(std::integral_constant<int, 192>{})
+             : t.bn == 160 ? pair(std::integral_constant<int, 160>{})
+                           : pair(std::integral_constant<int, 128>{});
+    bn = t.bn;
   }
   if (N % bn != 0) bn = (N % 128 == 0) ? 128 : 64;
   if (bn == 256) return launch_gemm<256>(A, W, C, M, N, K, st, 1, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
@@ -1370,6 +1375,9 @@ int b200q_gemm_set_tile_n(int bn) {
 // test/tuning hook: 0 = auto, 1 = 1-CTA kernels only, 2 = 2-CTA (cta_group::2) kernel whenever legal
 // diagnostics: co-resident CTA pairs the 2-CTA kernel's grid is sized to (0 until first use)
 int b200q_gemm_resident_pairs(void) { return g_gemm2_pairs; }
+
+// test hook: columns of the tiles of a product of more than 128 rows whose reduction is not split
+int b200q_gemm_tile_n(int M, int N) { return g_gemm_force_bn ? g_gemm_force_bn : choose_tile(M, N, false, g_gemm_mode == 0).bn; }
 
 // test/tuning hook: 0 = auto split-K, 1 = off, n > 1 = force n splits (decode-sized M only)
 int b200q_gemm_set_splitk(int n) {

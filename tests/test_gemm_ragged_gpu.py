@@ -1,5 +1,5 @@
-"""Products of more than 128 rows whose rounds are filled by tiles of 160 and 192 columns (csrc/gemm_tcgen05.cu: choose_tile): columns
-that those widths do not divide, a last tile of 32, 64 and 128 columns or without a half, rows at the edges of the pair's 256."""
+"""Products of more than 128 rows whose rounds are filled by tiles of 160 and 192 columns (csrc/gemm_tcgen05.cu: choose_tile): every width
+that a last tile of a row can have, rows at the edges of the pair's 256, one row of pair tiles and several."""
 import pytest
 import torch
 
@@ -9,13 +9,9 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 
-# 160 columns: 3584 = 22 x 160 + 64, 3392 = 21 x 160 + 32; 192: 4096 = 21 x 192 + 64, 2304 = 12 x 192, 6144 = 32 x 192, 3712 = 19 x 192 + 64,
-# 8192 = 42 x 192 + 128
-@pytest.mark.parametrize("M,N", [(513, 3584), (750, 3584), (768, 3392), (640, 4096), (768, 3712), (1281, 2304), (1500, 2304), (512, 6144), (1024, 6144),
-                                 (513, 8192), (3000, 2048), (1537, 4096)])
-@pytest.mark.parametrize("K", [64, 1088])
-def test_ragged_tiles(cuda, M, N, K):
+def check(cuda, M, N, K, width):
     from llmq_b200 import lib
+    assert lib.load().b200q_gemm_tile_n(M, N) == width, (M, N)
     g = torch.Generator(device=cuda).manual_seed(M + N + K)
     a = torch.randn(M, K, generator=g, device=cuda).to(BF)
     w = (torch.randn(N, K, generator=g, device=cuda) * K ** -0.5).to(BF)
@@ -31,7 +27,26 @@ def test_ragged_tiles(cuda, M, N, K):
         try:
             c = torch.empty(M, N, dtype=BF, device=cuda)
             if N % bn == 0:
+                assert lib.load().b200q_gemm_tile_n(M, N) == bn
                 lib.gemm_bf16(a, w, c)
                 assert torch.equal(c, whole[:M])
         finally:
             lib.gemm_set_tile_n(0)
+
+
+# 129 to 256 rows, one row of pair tiles: 160 columns from 9472 + 64 to 74 x 160 = 11840, 192 up to 74 x 192 = 14208
+@pytest.mark.parametrize("M", [129, 255, 256])
+@pytest.mark.parametrize("N,width", [(9536, 160), (9600, 160), (9664, 160), (9728, 160), (9792, 160), (11840, 160),      # last tile of 96, 160, 64, 128, 32, 160
+                                     (11904, 192), (11968, 192), (12032, 192), (14208, 192)])                              # 192, 64, 128, 192
+@pytest.mark.parametrize("K", [64, 1088])
+def test_one_row_of_tiles(cuda, M, N, width, K):
+    check(cuda, M, N, K, width)
+
+
+# three rows of pair tiles and more
+@pytest.mark.parametrize("M,N,width", [(513, 3392, 160), (750, 3584, 160), (768, 3712, 160), (768, 3840, 160), (640, 4096, 192), (513, 4608, 192),
+                                       (1281, 2304, 192), (1500, 2304, 192), (512, 6144, 192), (1024, 6144, 192), (257, 6912, 192),
+                                       (3000, 2048, 192)])
+@pytest.mark.parametrize("K", [64, 1088])
+def test_rows_of_tiles(cuda, M, N, width, K):
+    check(cuda, M, N, K, width)
