@@ -54,7 +54,7 @@ GEMMA2_CASE = dict(hidden=256, n_layers=4, n_q_heads=4, n_kv_heads=2, head_dim=6
 
 
 def gemma2_golden(out_dir):
-    """Gemma-2 (the next architecture): HF Gemma2ForCausalLM on CPU -> goldens for
+    """Gemma-2 (the second architecture served): HF Gemma2ForCausalLM on CPU -> goldens for
     oracle/gemma2.py; 48 tokens > the 16-token sliding window, so both layer types are exercised"""
     from transformers import Gemma2Config, Gemma2ForCausalLM
 

@@ -1,5 +1,5 @@
 """Host-side logic of the worker slot, CPU only: the reference's BaseWorker / BrokerManager /
-Job / Result code runs UNMODIFIED (from baseline/_ref or /root/reference) on the aio_pika
+Job / Result code runs UNMODIFIED (from baseline/_ref or the mounted reference) on the aio_pika
 stand-in, with B200Worker plugged in and a fake engine in place of the GPU."""
 import asyncio
 import json

@@ -1,5 +1,5 @@
 """The drop-in itself on a B200: the reference's BaseWorker / BrokerManager (unmodified, from
-baseline/_ref or /root/reference) + B200Worker loading a model DIRECTORY (config.json, safetensors,
+baseline/_ref or the mounted reference) + B200Worker loading a model DIRECTORY (config.json, safetensors,
 tokenizer files — what `llmq worker run <model> <queue>` gets), jobs in through the broker,
 results out of `<queue>.results`, texts compared with the CPU oracle's greedy decode."""
 import asyncio

@@ -2,7 +2,7 @@
 
 The reference worker (ref:llmq/workers/vllm_worker.py:11) is run UNMODIFIED on a B200 behind the
 unmodified `BaseWorker` / `BrokerManager` (on the aio_pika stand-in: the image has no RabbitMQ);
-this subclass only makes it usable as a parity oracle, without touching /root/reference:
+this subclass only makes it usable as a parity oracle, without touching the reference:
 
   * :146 `await self.engine.get_tokenizer()` — vLLM >= 0.22 returns the tokenizer synchronously, so
     the engine's `get_tokenizer` is wrapped into an awaitable;
@@ -14,7 +14,7 @@ this subclass only makes it usable as a parity oracle, without touching /root/re
     vLLM tokenised) beside the text the worker returns.
 
   python tools/oracle_vllm_worker.py golden [case ...]      (on the B200 box)
-      -> gpurun_out/vllm_worker_golden_<case>.json
+      -> build/vllm_worker_golden_<case>.json
   python tools/oracle_vllm_worker.py pack                   (here)
       -> tests/golden/vllm_worker_golden_<case>.json.gz     (committed fixtures)
 
@@ -47,7 +47,7 @@ for _p in (os.path.join(ROOT, "baseline", "_ref"), "/root/reference"):
 os.environ.setdefault("HF_HUB_OFFLINE", "1")
 os.environ.setdefault("VLLM_NO_USAGE_STATS", "1")
 os.environ.setdefault("LLMQ_LOG_LEVEL", "WARNING")
-OUT = os.path.join(ROOT, "gpurun_out")
+OUT = os.path.join(ROOT, "build")
 
 from llmq_b200.model import LLAMA_32_1B, LLAMA_3_8B, ModelSpec  # noqa: E402
 
@@ -236,7 +236,7 @@ def golden(cases):
 
 
 def pack():
-    """gpurun_out/vllm_worker_golden_<case>.json -> tests/golden/vllm_worker_golden_<case>.json.gz"""
+    """build/vllm_worker_golden_<case>.json -> tests/golden/vllm_worker_golden_<case>.json.gz"""
     import glob
     import gzip
 

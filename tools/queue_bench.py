@@ -169,7 +169,7 @@ def main():
     ap.add_argument("--prefetch", type=int, default=5000)
     ap.add_argument("--budget", type=int, default=4608)
     ap.add_argument("--timeout", type=float, default=600)
-    ap.add_argument("--out-dir", default=os.path.join(ROOT, "gpurun_out"))
+    ap.add_argument("--out-dir", default=os.path.join(ROOT, "build"))
     args = ap.parse_args()
     if not args.vocab:
         from llmq_b200.model import BUILTIN_SPECS

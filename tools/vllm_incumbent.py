@@ -2,7 +2,7 @@
 ref:llmq/workers/vllm_worker.py:105-123,161-186) — on the same B200, development/measurement tool.
 
   python tools/vllm_incumbent.py golden     # greedy token ids on a small seeded checkpoint
-                                            #   -> gpurun_out/vllm_golden_<name>.json (copied to tests/golden/)
+                                            #   -> build/vllm_golden_<name>.json (copied to tests/golden/)
   python tools/vllm_incumbent.py throughput # Llama-3-8B dims, dummy weights, 128-in/128-out
 
 Differences from the reference worker, all deliberate: temperature is forced to 0
@@ -20,7 +20,7 @@ sys.path.insert(0, ROOT)
 os.environ.setdefault("VLLM_ENABLE_V1_MULTIPROCESSING", "0")
 os.environ.setdefault("HF_HUB_OFFLINE", "1")
 os.environ.setdefault("VLLM_NO_USAGE_STATS", "1")
-OUT = os.path.join(ROOT, "gpurun_out")
+OUT = os.path.join(ROOT, "build")
 os.makedirs(OUT, exist_ok=True)
 
 import numpy as np  # noqa: E402
@@ -188,7 +188,7 @@ def same_lease():
     clock from submission to the last token (ramp and tail included), for every max_num_seqs in
     MAX_NUM_SEQS (default 128,750,4608: the engine default the reference runs with, its production
     scripts' 750 (ref:utils/run_llmq_benchmark.slurm:32-33) and the headline configuration).
-    Every run is its own process.  -> gpurun_out/same_lease_vllm_vs_native.json"""
+    Every run is its own process.  -> build/same_lease_vllm_vs_native.json"""
     import subprocess
 
     seqs_list = [int(x) for x in os.environ.get("MAX_NUM_SEQS", "128,750,4608").split(",")]
