@@ -714,51 +714,41 @@ static int num_sms() {
 
 // ---- scratch of partial tiles -----------------------------------------------------------------------
 // Whoever orders its products by itself has its own, so that nobody's parts are overwritten before they are added: a model (its passes run
-// one behind the other; SplitScratchOf), a stream, and a graph in the making, whose replays may run beside the stream that it was captured
-// on.  A buffer never moves while it has an owner: graphs bake its address in.
-static constexpr size_t SPLIT_BYTES = (size_t)8 * 256 * 8192 * sizeof(float);  // 8 splits x 256 rows x 8192 columns: 64 MiB
-thread_local void** t_model_scratch = nullptr;
-SplitScratchOf::SplitScratchOf(void** slot) : before_(t_model_scratch) { t_model_scratch = slot; }
-SplitScratchOf::~SplitScratchOf() { t_model_scratch = before_; }
+// one behind the other; a piece of its workspace), a stream, and a graph in the making, whose replays may run beside the stream that it was
+// captured on.  Nothing here waits for the device or frees: either would end other threads' captures.  A stream's buffer stays with its
+// handle (which comes back for another stream only once the work of the one before is done), a graph's comes back with the last of the
+// graph and its executables and serves whoever asks next.  Sizes go by powers of two from 1 MiB, so that streams hold twice what their
+// largest product needs at most.
+struct ModelScratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+static thread_local ModelScratch t_model_scratch;
+SplitScratchOf::SplitScratchOf(void* p, size_t bytes) : p_(t_model_scratch.p), bytes_(t_model_scratch.bytes) { t_model_scratch = {p, bytes}; }
+SplitScratchOf::~SplitScratchOf() { t_model_scratch = {p_, bytes_}; }
 
 namespace {
-// (cudaMalloc and its like are refused to every thread while any stream is being captured in the default mode, unless the thread says that it
-// knows)
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 struct SplitBuffer {
   void* p = nullptr;
   size_t bytes = 0;
   int device = 0;
-  unsigned long long stream = 0, capture = 0, used = 0;  // capture: of the graph that owns it; 0: the stream does
-  std::atomic<bool> free{false};                         // the graph is gone
+  cudaStream_t stream = nullptr;
+  unsigned long long capture = 0;  // of the graph that owns it; 0: the stream does
+  std::atomic<bool> free{false};   // the graph is gone
 };
 std::mutex g_split_mu;
-std::vector<SplitBuffer*> g_split;  // (never shrinks in entries that a callback may still name)
-constexpr int SPLIT_STREAMS = 16;     // buffers of streams; further streams take over the one that was not used for longest
-constexpr size_t SPLIT_SPARE = 2 * SPLIT_BYTES;  // kept of what graphs have given back
-
-int split_alloc(size_t bytes, void** p) {
-  RelaxedCapture relaxed;
-  B200Q_CUDA(cudaMalloc(p, bytes));
-  return B200Q_OK;
-}
+std::vector<SplitBuffer*> g_split;  // (entries stay: a graph's callback names its own)
 }  // namespace
 
 static int splitk_scratch(int splits, int M, int N, cudaStream_t st, float** out) {
   const size_t need = (size_t)splits * M * N * sizeof(float);
   B200Q_CHECK_ARG(need <= SPLIT_BYTES, "split-K scratch too small for M=%d N=%d splits=%d", M, N, splits);
-  if (t_model_scratch) {
-    if (!*t_model_scratch)
-      if (int rc = split_alloc(SPLIT_BYTES, t_model_scratch)) return rc;
-    *out = (float*)*t_model_scratch;
+  if (need <= t_model_scratch.bytes) {
+    *out = (float*)t_model_scratch.p;
     return B200Q_OK;
   }
   int device = 0;
-  unsigned long long id = 0, capture = 0;
+  unsigned long long capture = 0;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   cudaGraph_t graph = nullptr;
   const cudaGraphNode_t* nodes = nullptr;
@@ -769,77 +759,46 @@ static int splitk_scratch(int splits, int M, int N, cudaStream_t st, float** out
       status != cudaStreamCaptureStatusActive) {
     cudaGetLastError();  // (a product that cannot run here fails at its launch)
     capture = 0;
-    B200Q_CUDA(cudaStreamGetId(st, &id));  // (a handle may come back as that of another stream)
-  } else {
-    id = (unsigned long long)reinterpret_cast<uintptr_t>(st);
   }
-  static unsigned long long clock = 0;
   std::lock_guard<std::mutex> lock(g_split_mu);
-  SplitBuffer *own = nullptr, *oldest = nullptr;
-  int streams = 0;
+  SplitBuffer *own = nullptr, *spare = nullptr;
   for (SplitBuffer* b : g_split) {
-    if (!b->p || b->device != device || b->free.load()) continue;
-    if (b->stream == id && b->capture == capture && b->bytes >= need) own = b;
-    if (b->capture == 0) {
-      ++streams;
-      if (!oldest || b->used < oldest->used) oldest = b;
+    if (b->device != device || b->bytes < need) continue;
+    if (b->free.load()) {
+      if (!spare || b->bytes < spare->bytes) spare = b;
+    } else if (b->stream == st && b->capture == capture && (!own || b->bytes > own->bytes)) {
+      own = b;
     }
   }
-  if (!own && capture == 0) {
-    if (streams >= SPLIT_STREAMS) {
-      RelaxedCapture relaxed;
-      if (cudaDeviceSynchronize() == cudaSuccess)
-        own = oldest;
-      else
-        cudaGetLastError();  // (something is being captured: one more buffer)
-    }
+  if (!own) {
+    own = spare;
     if (!own) {
+      size_t bytes = (size_t)1 << 20;
+      while (bytes < need) bytes *= 2;
+      // (refused to every thread while any stream is captured in the default mode, unless the thread says that it knows)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      void* p = nullptr;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t e = cudaMalloc(&p, bytes);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      B200Q_CUDA(e);
       own = new SplitBuffer;
-      if (int rc = split_alloc(own->bytes = SPLIT_BYTES, &own->p)) {
-        delete own;
-        return rc;
-      }
+      own->p = p;
+      own->bytes = bytes;
+      own->device = device;
+      own->free.store(true);
       g_split.push_back(own);
     }
-    // what graphs have given back, down to a spare or two
-    size_t spare = 0;
-    for (SplitBuffer* b : g_split)
-      if (b->p && b->free.load() && (spare += b->bytes) > SPLIT_SPARE) {
-        RelaxedCapture relaxed;
-        spare -= b->bytes;
-        if (cudaFree(b->p) == cudaSuccess)
-          b->p = nullptr;
-        else
-          cudaGetLastError();
-      }
-  } else if (!own) {
-    size_t bytes = (size_t)1 << 20;
-    while (bytes < need) bytes *= 2;
-    for (SplitBuffer* b : g_split)  // the smallest that fits of those given back
-      if (b->p && b->free.load() && b->device == device && b->bytes >= need && (!own || b->bytes < own->bytes)) own = b;
-    if (!own) {
-      for (SplitBuffer* b : g_split)
-        if (!b->p) own = b;
-      const bool fresh = !own;
-      if (fresh) own = new SplitBuffer;
-      if (int rc = split_alloc(own->bytes = bytes, &own->p)) {
-        own->p = nullptr;
-        if (fresh) delete own;
-        return rc;
-      }
-      if (fresh) g_split.push_back(own);
+    if (capture) {
+      cudaUserObject_t held;
+      B200Q_CUDA(cudaUserObjectCreate(&held, own, [](void* b) { static_cast<SplitBuffer*>(b)->free.store(true); }, 1,
+                                      cudaUserObjectNoDestructorSync));
+      B200Q_CUDA(cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove));
     }
-    own->free.store(true);  // (until the graph holds it)
-    cudaUserObject_t held;
-    B200Q_CUDA(cudaUserObjectCreate(&held, own, [](void* b) { static_cast<SplitBuffer*>(b)->free.store(true); }, 1,
-                                    cudaUserObjectNoDestructorSync));
-    B200Q_CUDA(cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove));
+    own->stream = st;
+    own->capture = capture;
     own->free.store(false);
   }
-  own->device = device;
-  own->stream = id;
-  own->capture = capture;
-  own->used = ++clock;
   *out = (float*)own->p;
   return B200Q_OK;
 }

@@ -600,15 +600,17 @@ void layered_destroy(b200q_model* m) {
   m->lay = nullptr;
 }
 
-int64_t layered_workspace_bytes(b200q_model* m) { return layout(m, nullptr); }
+// (behind the layout: parts of split reductions)
+int64_t layered_workspace_bytes(b200q_model* m) { return layout(m, nullptr) + (int64_t)SPLIT_BYTES; }
 
 int layered_bind_workspace(b200q_model* m, void* p, int64_t bytes) {
-  const int64_t need = layout(m, nullptr);
+  const int64_t need = layered_workspace_bytes(m);
   B200Q_CHECK_ARG(bytes >= need, "workspace too small: %lld < %lld", (long long)bytes, (long long)need);
   B200Q_CHECK_ARG((reinterpret_cast<uintptr_t>(p) & 255) == 0, "workspace must be 256-byte aligned");
   m->ws = (uint8_t*)p;
   m->ws_bytes = bytes;
-  layout(m, (uint8_t*)p);
+  m->split_ws = (uint8_t*)p + layout(m, (uint8_t*)p);
+  m->split_bytes = SPLIT_BYTES;
   return B200Q_OK;
 }
 

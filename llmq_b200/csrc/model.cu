@@ -31,6 +31,15 @@ static int64_t qkv_dim(const b200q_model_config& c) {
   return (int64_t)(c.n_q_heads + 2 * c.n_kv_heads) * c.head_dim;
 }
 
+// parts of the largest split product of a pass (projections and heads of more than 8192 columns are not split)
+static int64_t split_bytes(const b200q_model_config& c) {
+  int64_t n = qkv_dim(c) > c.hidden ? qkv_dim(c) : c.hidden;
+  if (c.vocab <= 8192 && c.vocab > n) n = c.vocab;
+  const int64_t rows = c.max_tokens > c.max_seqs ? c.max_tokens : c.max_seqs;
+  const int64_t b = 8 * (rows < 256 ? rows : 256) * n * (int64_t)sizeof(float);
+  return b < (int64_t)SPLIT_BYTES ? b : (int64_t)SPLIT_BYTES;
+}
+
 static int check_cfg(const b200q_model_config* c) {
   B200Q_CHECK_ARG(c != nullptr, "model config is null");
   B200Q_CHECK_ARG(c->hidden > 0 && c->hidden % 64 == 0 && c->hidden <= 8192,
@@ -75,6 +84,7 @@ int64_t b200q_model_workspace_bytes(const b200q_model_config* c) {
   b += align256(T * (int64_t)c->intermediate * 2);                       // act
   b += align256(S * (int64_t)c->hidden * 2);                             // sel
   b += align256(S * (int64_t)c->vocab * 2);                              // logits
+  b += align256(split_bytes(*c));
   return b;
 }
 
@@ -104,7 +114,6 @@ int b200q_model_destroy(b200q_model_t m) {
   if (m) {
     for (cudaEvent_t e : m->ev_pool) cudaEventDestroy(e);
     layered_destroy(m);
-    if (m->split_ws) cudaFree(m->split_ws);
   }
   delete m;
   return B200Q_OK;
@@ -196,6 +205,8 @@ int b200q_model_bind_workspace(b200q_model_t m, void* p, int64_t bytes) {
   m->act = take(T * (int64_t)c.intermediate * 2);
   m->sel = take(S * (int64_t)c.hidden * 2);
   m->logits = take(S * (int64_t)c.vocab * 2);
+  m->split_bytes = (size_t)split_bytes(c);
+  m->split_ws = take(split_bytes(c));
   return B200Q_OK;
 }
 
@@ -230,7 +241,7 @@ int b200q_model_profile_collect(b200q_model_t m, b200q_profile* out, int reset) 
 
 int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
   B200Q_CHECK_ARG(m && b, "forward: null argument");
-  const SplitScratchOf own(&m->split_ws);
+  const SplitScratchOf own(m->split_ws, m->split_bytes);
   if (m->lay) return layered_forward(m, b, stream);
   const b200q_model_config& c = m->cfg;
   if (!m->embed || !m->final_norm || !m->lm_head || !m->kv || !m->rope || !m->ws) {

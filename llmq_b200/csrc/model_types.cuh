@@ -126,7 +126,8 @@ struct b200q_model {
        *sel = nullptr, *logits = nullptr;
   // fold the split-K reduce of decode-sized projections into the consuming kernel (B200Q_FUSE_SPLITK=0: off)
   bool fuse_splitk = true;
-  void* split_ws = nullptr;  // parts of split reductions (SplitScratchOf)
+  void* split_ws = nullptr;  // parts of split reductions (SplitScratchOf), a piece of the workspace
+  size_t split_bytes = 0;
   b200q_layered* lay = nullptr;  // B200Q_ARCH_RAMOPEL: everything layer-specific lives here
   // optional per-category device timing (CUDA events on the forward's stream)
   bool profiling = false;
