@@ -229,6 +229,8 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
 // the pointers that it reads through go through follow_previous, so that the compiler makes no such loads of const __restrict__ ones.
 // B200, in a graph of dependent kernels: 2.0 us instead of 3.4 from one small kernel to the next; the routed feed-forward of 128 rows
 // (8 kernels) 73.2 -> 58.9 us, a decode step of four layers of the 1B model at 48 sequences (37 kernels) 371 -> 349 us.
+// (Blocks that take the places which the kernel before leaves may come to lie two on one SM and none on another: kernels that lose more by
+// that than a start costs, 1 to 1.5 us, are launched plainly for those sizes, see launch_prefill in attn.cu and prefill_attn.cu.)
 // (pinned as an address of global memory, which the compiler would otherwise forget that it is)
 template <typename T>
 __device__ __forceinline__ T* pinned_global(T* p) {
