@@ -907,14 +907,16 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     attr_set = true;
   }
-  const long long units = (long long)((a.n_tiles + a.per_block - 1) / a.per_block) * a.n_kv;
+  const int blocks = (a.n_tiles + a.per_block - 1) / a.per_block;
+  const long long units = (long long)blocks * a.n_kv;
   const int grid = units < FA_SMS ? (int)units : FA_SMS;
   // Launched early where a CTA has no more than two units, or units of one step of keys.  CTAs that find their SMs as those of the kernel
   // before leave them come to lie elsewhere than the launch of an empty chip puts them, and where long units are dealt out over several
   // rounds that costs more than the start that is saved (D = 128, us, plainly / early: 12 portions of 100 to 700 tokens 56.8 / 61.3, 8 of 512
   // 47.0 / 50.5, 16 of 256 37.4 / 39.5, 4 of 300 to 1200 51.0 / 53.0; but one of 512 22.2 / 21.5, 36 of 128 32.8 / 32.5; D = 64 60 of 128
-  // 44.5 / 42.7, 8 of 512 37.6 / 40.2; D = 256, 4 heads, 8 of 512 30.8 / 29.9, 40 of 50 to 200 41.0 / 43.0).
-  if (units <= 2 * FA_SMS || a.bt_stride * 16 <= C::KT) {
+  // 44.5 / 42.7, 8 of 512 37.6 / 40.2; D = 256, 4 heads, 8 of 512 30.8 / 29.9, 40 of 50 to 200 41.0 / 43.0).  At D = 256 up to 64 blocks gain or
+  // are even with any number of heads (8 heads: 16 of 256 45.9 / 45.1, 3 of 333 to 2048 88.4 / 87.2, 8 of 512 even; 6 of 300 to 600 46.8 / 48.4).
+  if (units <= 2 * FA_SMS || a.bt_stride * 16 <= C::KT || (D == 256 && blocks <= 64)) {
     B200Q_CUDA(launch_early(kern, grid, FA_THREADS, C::SMEM, st, 1, map, a));
     count_launch();
   } else {
