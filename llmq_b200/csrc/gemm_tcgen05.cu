@@ -94,6 +94,12 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
         tmem_ld32(taddr + (uint32_t)(c0 + 32 * h), v);
         tmem_ld32(taddr + (uint32_t)(BN / 2 + c0 + 32 * h), u);
         tmem_ld_wait();
+        // (a row that does not exist, beside rows that do: as above; 300 rows of 16384 x 2048 64.4 -> 35.2 us, 200 of 28672 x 4096
+        // 88.3 -> 64.0, 2001 403 -> 354)
+        if (row0 + lane >= M) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0x3f800000u;
+        }
         if constexpr (kAct == ACT_CLAMPED) {
           const float4* bg = reinterpret_cast<const float4*>(gate_bias + c0 + 32 * h);
           const float4* bu = reinterpret_cast<const float4*>(gate_bias + BN / 2 + c0 + 32 * h);
