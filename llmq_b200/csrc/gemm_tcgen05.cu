@@ -707,6 +707,39 @@ int get_page_tmap(const void* kv, int D, CUtensorMap* out) {
   return B200Q_OK;
 }
 
+int get_head_rows_tmap(const void* p, int n_q, int D, long long stride, int heads, int rows, int cols, CUtensorMap* out) {
+  static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
+  static std::mutex mu;
+  const TmapKey key{p, stride << 16 | n_q, D, (heads * 128 + rows) * 64 + cols - 1};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return B200Q_OK;
+  }
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled entry point unavailable (driver too old / no driver)");
+    return B200Q_ECUDA;
+  }
+  cuuint64_t gdim[3] = {(cuuint64_t)D, (cuuint64_t)n_q, 0x0ffffffeull};
+  cuuint64_t gstride[2] = {(cuuint64_t)D * 2, (cuuint64_t)stride * 2};
+  cuuint32_t box[3] = {(cuuint32_t)cols, (cuuint32_t)heads, (cuuint32_t)rows};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUtensorMap m;
+  CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d) for rows of %d heads of %d at %p", (int)r, n_q, D, p);
+    return B200Q_ECUDA;
+  }
+  if (cache.size() > 4096) cache.clear();
+  cache[key] = m;
+  *out = m;
+  return B200Q_OK;
+}
+
 static int num_sms() {
   static int n = 0;
   if (n == 0) {

@@ -245,6 +245,10 @@ int get_tmap(const void* ptr, long long rows, long long cols, int box_rows, CUte
 // [two groups of 8 rows][64-column slices][8 rows][128 bytes]; coordinates {0, 0, 0, page * 2}.
 int get_page_tmap(const void* kv, int D, CUtensorMap* out);
 
+// rows of n_q heads of D bf16 values, `stride` elements apart, from p on (as many as there are; the caller knows).  One box is `cols` (32 or
+// 64) columns of `heads` heads of `rows` rows, with a swizzle as wide as its columns; coordinates {column, head, row}.
+int get_head_rows_tmap(const void* p, int n_q, int D, long long stride, int heads, int rows, int cols, CUtensorMap* out);
+
 // prompt portions over short contexts (attn.cu); long_keys > 0: portions of so many keys and more are left out
 int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
                   int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, int long_keys, cudaStream_t st);

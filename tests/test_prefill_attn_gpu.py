@@ -123,6 +123,13 @@ def test_lengths(cuda, n):
         check(cuda, D, 4, 2, [(n, 33)], seed=n + 1)
 
 
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 8, 8), (128, 16, 8), (256, 16, 8)])
+@pytest.mark.parametrize("cap", [0.0, 50.0, 12.0, 2.0])     # none; arguments of tanh up to 0.1, to 0.3 and beyond: 3 terms, 5 terms, all of it
+def test_many_runs_to_a_cta(cuda, D, n_q, n_kv, cap):
+    """more runs than the ring between the roles holds, of 1 to 6 steps, whole query tiles and parts of them"""
+    check(cuda, D, n_q, n_kv, [(17 * i % 90 if i % 3 else 0, 9 + 31 * i % 290) for i in range(220)], cap=cap, seed=5, routes=(1,))
+
+
 def step(cuda, D, n_q, n_kv, portions, seed, scale, cap=0.0, window=0, wide=True, rows_of=None, k_scale=1.0):
     """one call's inputs on the GPU and the call"""
     from llmq_b200 import lib
