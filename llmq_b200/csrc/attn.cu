@@ -22,6 +22,8 @@
 // their code: kCap = attention-logit soft-capping (score <- cap * tanh(score * scale / cap)), and a
 // runtime sliding window (query at position p sees keys p - window < j <= p; pages that lie entirely
 // before the window are never fetched).  D = 256 (Gemma-2 head size) uses 2-stage rings.
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -37,6 +39,11 @@ template <int D>
 struct DecCfg {
   static constexpr int STAGES = D > 128 ? 2 : 3;
 };
+__device__ __forceinline__ float dec_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 // score -> log2-domain logit.  plain: s * (scale * log2 e).  capped: tanh(s * scale / cap) * (cap * log2 e)
 template <bool kCap>
@@ -179,19 +186,20 @@ __device__ __forceinline__ void zero_tail_rows(uint8_t* v_page, int n_valid, int
 // ------------------------------------------------------------------------------------------
 // K7 decode
 // ------------------------------------------------------------------------------------------
-template <int D, int BS>
+// PAGES: pages that a warp takes at once; two of them twice in its ring
+template <int D, int BS, int PAGES>
 struct DecSmem {
-  static constexpr int STAGES = DecCfg<D>::STAGES;
-  static constexpr int STAGE_BYTES = 2 * Geo<D, BS>::PAGE_BYTES;
+  static constexpr int STAGES = PAGES > 1 ? 2 : DecCfg<D>::STAGES;
+  static constexpr int STAGE_BYTES = PAGES * 2 * Geo<D, BS>::PAGE_BYTES;
   static constexpr int RING_BYTES = DEC_WARPS * STAGES * STAGE_BYTES;
   static constexpr int MERGE_FLOATS = DEC_WARPS * 8 * (D + 2);
   static constexpr int TOTAL = RING_BYTES + MERGE_FLOATS * 4 + DEC_WARPS * STAGES * 8;
 };
 
 // A cluster of gridDim.x CTAs shares a sequence's pages where there are few sequences: warp w of CTA r takes pages r * DEC_WARPS + w,
-// + warps of the cluster, ...; the CTAs read each other's partial states through distributed shared memory and each adds up and stores
+// + warps of the cluster, ..., PAGES of them at once; the CTAs read each other's partial states through distributed shared memory and each adds up and stores
 // its share of the outputs.
-template <int D, int BS, bool kCap, bool kShared>
+template <int D, int BS, bool kCap, bool kShared, int PAGES>
 __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
     decode_attn_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out,
                        const uint8_t* __restrict__ kv_layer,
@@ -200,7 +208,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
                        float c0, float c1, int window, int ahead) {
   // ahead: pages per warp that are asked into L2 before the kernel before this one has ended; 0: that one may write the tables
   using G_ = Geo<D, BS>;
-  using S_ = DecSmem<D, BS>;
+  using S_ = DecSmem<D, BS, PAGES>;
   constexpr int DEC_STAGES = S_::STAGES;
   extern __shared__ __align__(128) uint8_t smem[];
   const int seq = kShared ? blockIdx.y : blockIdx.x, kvh = kShared ? blockIdx.z : blockIdx.y;
@@ -245,33 +253,43 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
     follow_previous(q, out, kv_layer);
   }
 
-  auto issue = [&](int k) {  // whole warp calls; k = warp-local page index
-    if (k - ids_base >= 32) {
+  const int turns = (my_n + PAGES - 1) / PAGES;
+  auto issue = [&](int t) {  // whole warp calls; pages t * PAGES, ... of this warp
+    if (t * PAGES - ids_base >= 32) {
       ids_base += 32;
       ids = (ids_base + lane < my_n) ? bt[wg + n_warps * (ids_base + lane)] : 0;
     }
-    const int blk = __shfl_sync(0xffffffffu, ids, k - ids_base);
-    const int p = page0 + wg + n_warps * k;
-    const int n_valid = min(BS, ctx - p * BS);
-    const int st = k % DEC_STAGES;
-    uint8_t* ks = ring + st * S_::STAGE_BYTES;
-    uint8_t* vs = ks + G_::PAGE_BYTES;
-    if (n_valid < BS) {
-      zero_tail_rows<D, BS>(vs, n_valid, lane);
+    const int st = t % DEC_STAGES;
+    uint8_t* to = ring + st * S_::STAGE_BYTES;
+    int blk[PAGES], n_valid[PAGES], all = 0;
+#pragma unroll
+    for (int x = 0; x < PAGES; ++x) {
+      const int k = t * PAGES + x;
+      blk[x] = __shfl_sync(0xffffffffu, ids, (k - ids_base) & 31);
+      n_valid[x] = x == 0 || k < my_n ? min(BS, ctx - (page0 + wg + n_warps * k) * BS) : 0;
+      all += n_valid[x];
+    }
+    if (all < PAGES * BS) {
+#pragma unroll
+      for (int x = 0; x < PAGES; ++x)
+        zero_tail_rows<D, BS>(to + (2 * x + 1) * G_::PAGE_BYTES, n_valid[x], lane);
       __syncwarp();
     }
     if (lane == 0) {
-      const uint32_t bytes = (uint32_t)n_valid * G_::ROW_BYTES;
-      const uint8_t* kp = kv_layer + (((long long)blk * 2 + 0) * n_kv + kvh) * page_stride;
-      const uint8_t* vp = kv_layer + (((long long)blk * 2 + 1) * n_kv + kvh) * page_stride;
-      mbar_expect_tx(bars + st, 2 * bytes);
-      tma_bulk_g2s(ks, kp, bytes, bars + st);
-      tma_bulk_g2s(vs, vp, bytes, bars + st);
+      mbar_expect_tx(bars + st, (uint32_t)all * (2 * G_::ROW_BYTES));
+#pragma unroll
+      for (int x = 0; x < PAGES; ++x) {
+        const uint32_t bytes = (uint32_t)n_valid[x] * G_::ROW_BYTES;
+        const uint8_t* kp = kv_layer + ((long long)blk[x] * 2 * n_kv + kvh) * page_stride;
+        if (x == 0 || bytes > 0) {
+          tma_bulk_g2s(to + 2 * x * G_::PAGE_BYTES, kp, bytes, bars + st);
+          tma_bulk_g2s(to + (2 * x + 1) * G_::PAGE_BYTES, kp + n_kv * page_stride, bytes, bars + st);
+        }
+      }
     }
   };
 
-  const int n_pro = my_n < DEC_STAGES ? my_n : DEC_STAGES;
-  for (int k = 0; k < n_pro; ++k) issue(k);
+  for (int t = 0; t < min(turns, DEC_STAGES); ++t) issue(t);
 
   // Q fragments: rows 0..G-1 of the 16-row tile are the G query heads of this kv head
   uint32_t qa[D / 16][4];
@@ -296,57 +314,65 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
   for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m = -INFINITY, l = 0.f;
 
-  for (int k = 0; k < my_n; ++k) {
-    const int st = k % DEC_STAGES;
-    const uint32_t phase = (uint32_t)(k / DEC_STAGES) & 1u;
-    mbar_wait(bars + st, phase);
-    const int p = page0 + wg + n_warps * k;
-    const int n_valid = min(BS, ctx - p * BS);
-    const int t_lo = lo - p * BS;  // first visible token of this page (<= 0 except on the window's first page)
-    const uint32_t k_s = smem_u32(ring + st * S_::STAGE_BYTES);
-    const uint32_t v_s = k_s + G_::PAGE_BYTES;
+  for (int t = 0; t < turns; ++t) {
+    const int st = t % DEC_STAGES;
+    mbar_wait(bars + st, (uint32_t)(t / DEC_STAGES) & 1u);
+    const uint32_t at = smem_u32(ring + st * S_::STAGE_BYTES);
 
-    float s[BS / 8][4];
-    qk_page<D, BS, false>(k_s, qa, s, lane);
-
+    float s[PAGES][BS / 8][4];
     float mx = -INFINITY;
 #pragma unroll
-    for (int nt = 0; nt < G_::NT; ++nt) {
-      const int t0 = nt * 8 + (lane & 3) * 2;
-      s[nt][0] = (t0 < n_valid && t0 >= t_lo) ? score_xform<kCap>(s[nt][0], c0, c1) : -INFINITY;
-      s[nt][1] = (t0 + 1 < n_valid && t0 + 1 >= t_lo) ? score_xform<kCap>(s[nt][1], c0, c1) : -INFINITY;
-      mx = fmaxf(mx, fmaxf(s[nt][0], s[nt][1]));
+    for (int x = 0; x < PAGES; ++x)
+      qk_page<D, BS, false>(at + 2 * x * G_::PAGE_BYTES, qa, s[x], lane);
+#pragma unroll
+    for (int x = 0; x < PAGES; ++x) {
+      const int first = (page0 + wg + n_warps * (t * PAGES + x)) * BS;
+      // visible tokens of this page: up to n_valid (a page that is not there: none), from t_lo (<= 0 except on the window's first page)
+      const int n_valid = ctx - first, t_lo = lo - first;
+#pragma unroll
+      for (int nt = 0; nt < G_::NT; ++nt) {
+        const int t0 = nt * 8 + (lane & 3) * 2;
+        s[x][nt][0] = (t0 < n_valid && t0 >= t_lo) ? score_xform<kCap>(s[x][nt][0], c0, c1) : -INFINITY;
+        s[x][nt][1] = (t0 + 1 < n_valid && t0 + 1 >= t_lo) ? score_xform<kCap>(s[x][nt][1], c0, c1) : -INFINITY;
+        mx = fmaxf(mx, fmaxf(s[x][nt][0], s[x][nt][1]));
+      }
     }
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float m_new = fmaxf(m, mx);  // finite: every page has >= 1 valid token
-    const float alpha = exp2f(m - m_new);
+    const float m_new = fmaxf(m, mx);  // finite: the first page has >= 1 visible token
+    const float alpha = dec_ex2(m - m_new);
     float psum = 0.f;
 #pragma unroll
-    for (int nt = 0; nt < G_::NT; ++nt) {
-      s[nt][0] = exp2f(s[nt][0] - m_new);
-      s[nt][1] = exp2f(s[nt][1] - m_new);
-      s[nt][2] = 0.f;
-      s[nt][3] = 0.f;
-      psum += s[nt][0] + s[nt][1];
-    }
+    for (int x = 0; x < PAGES; ++x)
+#pragma unroll
+      for (int nt = 0; nt < G_::NT; ++nt) {
+        s[x][nt][0] = dec_ex2(s[x][nt][0] - m_new);
+        s[x][nt][1] = dec_ex2(s[x][nt][1] - m_new);
+        s[x][nt][2] = 0.f;
+        s[x][nt][3] = 0.f;
+        psum += s[x][nt][0] + s[x][nt][1];
+      }
     l = l * alpha + psum;
     m = m_new;
     if constexpr (TPV) {
       float a0, a1;
       per_head_pair(alpha, lane, a0, a1);
       scale_ot<D>(o, a0, a1);
-      pv_page_t<D, BS>(v_s, s, o, lane);
+#pragma unroll
+      for (int x = 0; x < PAGES; ++x)
+        pv_page_t<D, BS>(at + (2 * x + 1) * G_::PAGE_BYTES, s[x], o, lane);
     } else {
 #pragma unroll
       for (int i = 0; i < NO; ++i) {
         o[i][0] *= alpha;
         o[i][1] *= alpha;
       }
-      pv_page<D, BS, false>(v_s, s, o, lane);
+#pragma unroll
+      for (int x = 0; x < PAGES; ++x)
+        pv_page<D, BS, false>(at + (2 * x + 1) * G_::PAGE_BYTES, s[x], o, lane);
     }
     __syncwarp();
-    if (k + DEC_STAGES < my_n) issue(k + DEC_STAGES);
+    if (t + DEC_STAGES < turns) issue(t + DEC_STAGES);
   }
 
   // ---- merge the 4 per-warp partial states ----
@@ -861,12 +887,12 @@ static int attn_num_sms() {
   return n;
 }
 
-template <int D, int BS, bool kCap, bool kShared>
+template <int D, int BS, bool kCap, bool kShared, int PAGES>
 static int prepare_decode() {
   static bool attr_set = false;
   if (!attr_set) {
-    B200Q_CUDA(cudaFuncSetAttribute(decode_attn_kernel<D, BS, kCap, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    DecSmem<D, BS>::TOTAL));
+    B200Q_CUDA(cudaFuncSetAttribute(decode_attn_kernel<D, BS, kCap, kShared, PAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    DecSmem<D, BS, PAGES>::TOTAL));
     attr_set = true;
   }
   return B200Q_OK;
@@ -876,12 +902,12 @@ template <bool kShared>
 static dim3 decode_grid(int splits, int n_seqs, int n_kv) {
   return kShared ? dim3(splits, n_seqs, n_kv) : dim3(n_seqs, n_kv);  // (only x goes beyond 65535)
 }
-template <int D, int BS, bool kShared>
+template <int D, int BS, bool kShared, int PAGES>
 static cudaLaunchConfig_t decode_config(int splits, int n_seqs, int n_kv, cudaLaunchAttribute* attr, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = decode_grid<kShared>(splits, n_seqs, n_kv);
   cfg.blockDim = dim3(DEC_WARPS * 32);
-  cfg.dynamicSmemBytes = DecSmem<D, BS>::TOTAL;
+  cfg.dynamicSmemBytes = DecSmem<D, BS, PAGES>::TOTAL;
   cfg.stream = st;
   attr->id = cudaLaunchAttributeClusterDimension;
   attr->val.clusterDim.x = splits;
@@ -892,7 +918,7 @@ static cudaLaunchConfig_t decode_config(int splits, int n_seqs, int n_kv, cudaLa
 }
 
 // how many clusters of `splits` CTAs are resident at once (asked for once per size)
-template <int D, int BS, bool kCap>
+template <int D, int BS, bool kCap, int PAGES>
 static int decode_resident(int splits) {
   static int known[9];
   int& n = known[splits];
@@ -900,16 +926,16 @@ static int decode_resident(int splits) {
     int v = 0;
     cudaError_t e;
     if (splits == 1) {
-      e = prepare_decode<D, BS, kCap, false>()
+      e = prepare_decode<D, BS, kCap, false, PAGES>()
               ? cudaErrorUnknown
-              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, decode_attn_kernel<D, BS, kCap, false>, DEC_WARPS * 32,
-                                                              DecSmem<D, BS>::TOTAL);
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, decode_attn_kernel<D, BS, kCap, false, PAGES>,
+                                                              DEC_WARPS * 32, DecSmem<D, BS, PAGES>::TOTAL);
       v *= attn_num_sms();
     } else {
       cudaLaunchAttribute attr;
-      const cudaLaunchConfig_t cfg = decode_config<D, BS, true>(splits, attn_num_sms(), 1, &attr, nullptr);
-      e = prepare_decode<D, BS, kCap, true>() ? cudaErrorUnknown
-                                              : cudaOccupancyMaxActiveClusters(&v, decode_attn_kernel<D, BS, kCap, true>, &cfg);
+      const cudaLaunchConfig_t cfg = decode_config<D, BS, true, PAGES>(splits, attn_num_sms(), 1, &attr, nullptr);
+      e = prepare_decode<D, BS, kCap, true, PAGES>() ? cudaErrorUnknown
+                                              : cudaOccupancyMaxActiveClusters(&v, decode_attn_kernel<D, BS, kCap, true, PAGES>, &cfg);
     }
     if (e != cudaSuccess || v <= 0) {
       cudaGetLastError();
@@ -928,38 +954,60 @@ static int decode_resident(int splits) {
 // pages per warp.  The contexts are taken to fill the block table.  Fitted to 1800 sizes (1 to 90 sequences of 256 to 8000 tokens), 1 to
 // 2.5 % slower than the best number of CTAs on average; against one CTA each 0.78 of the time, nowhere more than 1.09.  6 sequences of
 // 3000 to 8100 tokens, D = 64, 8 kv heads: 22 us, 65 with one CTA each.  B200Q_BATCH_INVARIANT=1: always one, whatever the batch.
-template <int D, int BS, bool kCap>
-static int decode_splits(int n_seqs, int n_kv, int bt_stride, int window) {
-  if (batch_invariant() || g_decode_variant == 1) return 1;
-  constexpr double ROUND = D > 128 ? 4 : 8, PAGE = D > 128 ? 0.83 : D > 64 ? 0.58 : 0.5, SHARE = D > 128 ? 2 : D > 64 ? 3 : 1.5;
+// Pages at once: two where that is not paid for with CTAs.  The chain of a page (scores, maximum, exponentials, values: a warp works on
+// one at a time, a few warps to a scheduler) is what bounds all but the largest steps, and two pages share it: D = 64, whose CTAs still come
+// three to an SM, 32 sequences of 100 to 900 tokens 12.9 -> 10.9 us, one of 8000 11.8 -> 9.8, 100 of 33 to 2560 52.2 -> 47.8; D = 128, where
+// it leaves one CTA per SM, one of 8000 14.8 -> 12.5, 8 of 20 to 500 7.8 -> 6.3, but 128 of 129 to 256 23.7 -> 31.3: with costs of its own
+// beside the other (1087 times fitted, of both forms, 0.6 % slower than the best; 4.4 % without).  D = 256: the ring would hold one turn.
+struct DecodePlan {
+  int splits, pages;  // CTAs per sequence, pages that a warp takes at once
+};
+struct DecodeCosts {
+  double round, page, share;
+};
+template <int D, int BS, bool kCap, int PAGES>
+static void decode_plan_of(int n_seqs, int n_kv, int bt_stride, int window, DecodeCosts c, DecodePlan* best, double* least) {
   const long long n = (long long)n_seqs * n_kv;
-  const int sms = attn_num_sms(), per_sm = decode_resident<D, BS, kCap>(1) / sms;
+  const int sms = attn_num_sms(), per_sm = decode_resident<D, BS, kCap, PAGES>(1) / sms;
   const int pages = window > 0 && (window + 15) / 16 + 1 < bt_stride ? (window + 15) / 16 + 1 : bt_stride;
-  int best = 1;
-  double least = 0;
   for (int s = 1; s <= 8 && (s == 1 || pages >= 4 * DEC_WARPS * s); ++s) {
-    const long long resident = decode_resident<D, BS, kCap>(s), rounds = (n + resident - 1) / resident, deep = (n * s + sms - 1) / sms;
-    const double chain = (pages + DEC_WARPS * s - 1) / (DEC_WARPS * s) * PAGE * (1 + 0.15 * ((deep < per_sm ? deep : per_sm) - 1));
+    const long long resident = decode_resident<D, BS, kCap, PAGES>(s), rounds = (n + resident - 1) / resident, deep = (n * s + sms - 1) / sms;
+    const double chain = (pages + DEC_WARPS * s - 1) / (DEC_WARPS * s) * c.page * (1 + 0.15 * ((deep < per_sm ? deep : per_sm) - 1));
     const double bytes_us = (double)n * pages * (2 * BS * D * 2) / 9e6;
-    const double work = rounds * (ROUND + chain);
-    const double t = 2 + (work > bytes_us ? work : bytes_us) + (s > 1 ? SHARE + (s & (s - 1) ? 0.5 : 0) : 0);
-    if (s == 1 || t < 0.97 * least) {
-      least = t;
-      best = s;
+    const double work = rounds * (c.round + chain);
+    const double t = 2 + (work > bytes_us ? work : bytes_us) + (s > 1 ? c.share + (s & (s - 1) ? 0.5 : 0) : 0);
+    if (best->splits == 0 || t < 0.97 * *least) {
+      *least = t;
+      *best = {s, PAGES};
     }
   }
+}
+template <int D, int BS, bool kCap>
+static DecodePlan decode_plan(int n_seqs, int n_kv, int bt_stride, int window) {
+  if (batch_invariant() || g_decode_variant == 1) return {1, D == 64 ? 2 : 1};
+  DecodePlan best{0, 1};
+  double least = 0;
+  // (a warp has no more than two of 8 pages: 50 tokens, D = 64, 2.75 us one at a time, 3.05 with room for another)
+  const bool few = bt_stride <= 2 * DEC_WARPS;
+  if (D != 64 || few)
+    decode_plan_of<D, BS, kCap, 1>(n_seqs, n_kv, bt_stride, window,
+                                   D > 128 ? DecodeCosts{4, 0.83, 2} : D > 64 ? DecodeCosts{8, 0.58, 3} : DecodeCosts{8, 0.5, 1.5}, &best, &least);
+  if constexpr (D <= 128)
+    if (!few)
+      decode_plan_of<D, BS, kCap, 2>(n_seqs, n_kv, bt_stride, window, D > 64 ? DecodeCosts{7.3, 0.59, 1.9} : DecodeCosts{8, 0.5, 1.5}, &best,
+                                     &least);
   return best;
 }
 
-template <int D, int BS, bool kCap, bool kShared>
+template <int D, int BS, bool kCap, bool kShared, int PAGES>
 static int launch_decode_form(int splits, const void* q, int q_stride, void* out, const void* kv,
                          const int32_t* bt, int bt_stride, const int32_t* ctx, int n_seqs, int n_q,
                          int n_kv, float scale, float softcap, int window, int ahead, cudaStream_t st) {
-  auto kern = decode_attn_kernel<D, BS, kCap, kShared>;
-  const int rc = prepare_decode<D, BS, kCap, kShared>();
+  auto kern = decode_attn_kernel<D, BS, kCap, kShared, PAGES>;
+  const int rc = prepare_decode<D, BS, kCap, kShared, PAGES>();
   if (rc) return rc;
   const ScoreConsts sc = score_consts(scale, softcap);
-  B200Q_CUDA(launch_early(kern, decode_grid<kShared>(splits, n_seqs, n_kv), DEC_WARPS * 32, DecSmem<D, BS>::TOTAL, st, splits, (const bf16*)q,
+  B200Q_CUDA(launch_early(kern, decode_grid<kShared>(splits, n_seqs, n_kv), DEC_WARPS * 32, DecSmem<D, BS, PAGES>::TOTAL, st, splits, (const bf16*)q,
                           q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, ctx, n_q, n_kv, n_q / n_kv, sc.c0, sc.c1, window, ahead));
   count_launch();
   return B200Q_OK;
@@ -968,18 +1016,24 @@ static int launch_decode_form(int splits, const void* q, int q_stride, void* out
 template <int D, int BS, bool kCap>
 static int launch_decode(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* ctx,
                          int n_seqs, int n_q, int n_kv, float scale, float softcap, int window, bool tables_known, cudaStream_t st) {
-  const int splits = decode_splits<D, BS, kCap>(n_seqs, n_kv, bt_stride, window);
+  const DecodePlan plan = decode_plan<D, BS, kCap>(n_seqs, n_kv, bt_stride, window);
   int ahead = 0;
   if (tables_known) {
-    const long long each = (long long)n_seqs * n_kv * splits * DEC_WARPS * 2 * Geo<D, BS>::PAGE_BYTES;
+    const long long each = (long long)n_seqs * n_kv * plan.splits * DEC_WARPS * 2 * Geo<D, BS>::PAGE_BYTES;
     ahead = DEC_AHEAD_BYTES / each < 32 ? (int)(DEC_AHEAD_BYTES / each) : 32;
     if (ahead < 1) ahead = 1;
   }
-  if (splits > 1)
-    return launch_decode_form<D, BS, kCap, true>(splits, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap,
-                                                 window, ahead, st);
-  return launch_decode_form<D, BS, kCap, false>(1, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap, window,
-                                                ahead, st);
+  auto launch = [&](auto pages) {
+    constexpr int P = decltype(pages)::value;
+    if (plan.splits > 1)
+      return launch_decode_form<D, BS, kCap, true, P>(plan.splits, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap,
+                                                      window, ahead, st);
+    return launch_decode_form<D, BS, kCap, false, P>(1, q, q_stride, out, kv, bt, bt_stride, ctx, n_seqs, n_q, n_kv, scale, softcap, window,
+                                                     ahead, st);
+  };
+  if constexpr (D <= 128)
+    if (plan.pages == 2) return launch(std::integral_constant<int, 2>{});
+  return launch(std::integral_constant<int, 1>{});
 }
 
 template <int D, int BS, bool kCap>
