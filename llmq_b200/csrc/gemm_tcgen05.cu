@@ -63,7 +63,8 @@ constexpr int EPI_SMEM_PER_WARP = 32 * 128;  // 32 rows x 64 bf16
 template <int BN, int kAct>
 __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long long ldc,
                                               int row0, int M, uint8_t* patch, int lane,
-                                              const float* gate_bias = nullptr, float limit = 0.f, int cols = BN) {
+                                              const float* gate_bias = nullptr, float limit = 0.f, int cols = BN, int c_begin = 0,
+                                              int c_step = 64) {
   constexpr bool kSwiGLU = kAct != ACT_NONE;  // gated epilogue: tile = [gate (BN/2) | up (BN/2)]
   constexpr int OUT_BN = kSwiGLU ? BN / 2 : BN;
   // (no row of this warp exists: its accumulators are sums of zeros, which the gated units' division treats as a special case: 384 rows
@@ -73,7 +74,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, bf16* ctile, long 
   constexpr bool kRagged = BN % 128 != 0 && BN > 64;
   const uint32_t patch_s = smem_u32(patch);
 #pragma unroll 1
-  for (int c0 = 0; c0 < (kRagged ? cols : OUT_BN); c0 += 64) {
+  for (int c0 = c_begin; c0 < (kRagged ? cols : OUT_BN); c0 += c_step) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {  // two 32-column TMEM loads -> 64 output columns of this row
       uint32_t v[32];
@@ -367,6 +368,9 @@ __global__ void __launch_bounds__(256)
 // 16 KB + BN*128 B to 16 KB + BN*64 B for the same MMA work — the 1-CTA kernel is ingest-bound,
 // this one moves the bound back to the tensor pipe.
 // ==================================================================================================
+// Eight warps store: a gated tile takes four of them some 14 us, which is longer than its products up to K = 2304 and stands behind the last
+// tile of any reduction.
+constexpr int GEMM2_THREADS = 320;
 template <int BN>
 struct Gemm2Cfg {
   static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;        // 16 KB: this CTA's 128 rows
@@ -374,7 +378,7 @@ struct Gemm2Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = GEMM_SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : GEMM_SMEM_BUDGET / STAGE_BYTES;
   static constexpr int TMEM_COLS = BN > 128 ? 512 : 256;       // two accumulators, a power of two
-  static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + 4 * 4096;
+  static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + 1024 + 256 + 8 * 4096;
 };
 
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster_addr, uint32_t bytes) {
@@ -431,7 +435,7 @@ __host__ __device__ constexpr uint32_t make_idesc_2sm(int n) {
 }
 
 template <int BN, int kAct = ACT_NONE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM2_THREADS, 1)
     gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                       const __grid_constant__ CUtensorMap tmap_b, bf16* __restrict__ C, int M,
                       int N, int K, long long ldc, GateArgs gate, int fixed_w) {
@@ -446,7 +450,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   uint64_t* tmem_full = empty + STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-  uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;  // 4 warps x 4 KB transpose patches
+  uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES + 256;  // 8 warps x 4 KB transpose patches
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -467,8 +471,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
     mbar_init(tmem_full + 0, 1);
     mbar_init(tmem_full + 1, 1);
-    mbar_init(tmem_empty + 0, 8);  // 4 epilogue warps x 2 CTAs, all arriving at the leader
-    mbar_init(tmem_empty + 1, 8);
+    mbar_init(tmem_empty + 0, 16);  // 8 epilogue warps x 2 CTAs, all arriving at the leader
+    mbar_init(tmem_empty + 1, 16);
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc_2sm(tmem_slot, Cfg::TMEM_COLS);
@@ -561,7 +565,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       }
     }
   } else {
-    // ===== epilogue (both CTAs): own 128 rows of the 256-row tile =====
+    // ===== epilogue (both CTAs): own 128 rows of the 256-row tile, every other 64 columns to four of the warps =====
     const int quarter = warp & 3;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -575,7 +579,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
       epilogue_rows<BN, kAct>(taddr, ctile, ldc, row0, M, epi_smem + (warp - 2) * EPI_SMEM_PER_WARP, lane,
                                 kAct == ACT_CLAMPED && gate.bias ? gate.bias + (long long)n_blk * BN : nullptr, gate.limit,
-                                min(BN, N - n_blk * BN));
+                                min(BN, N - n_blk * BN), (warp - 2) / 4 * 64, 128);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(tmem_empty + acc, 0));
@@ -908,7 +912,7 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
   if (pairs == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms() & ~1);
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3(GEMM2_THREADS);
     cfg.dynamicSmemBytes = Cfg::SMEM_TOTAL;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -926,7 +930,7 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
     g_gemm2_pairs = pairs;
   }
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K,
+  B200Q_CUDA(launch_early(kern, grid, GEMM2_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K,
                           ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate, (int)fixed_w));
   count_launch();
   return B200Q_OK;
