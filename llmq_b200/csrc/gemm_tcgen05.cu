@@ -970,6 +970,40 @@ static TileChoice choose_tile(int M, int N, bool gated, bool pairs) {
   return best;
 }
 
+// the least (rounds x round's time) of the tiles above, in 128 x 256 tiles
+static double tile_rounds(int M, int N, const TileChoice& t) {
+  const long long rows = t.pair ? 256 : GEMM_BM, slots = t.pair ? num_sms() / 2 : num_sms();
+  const double cost = t.pair ? (t.bn == 256 ? 0.84 : t.bn == 192 ? 0.70 : t.bn == 160 ? 0.65 : 0.595) : t.bn == 256 ? 1.0 : t.bn == 128 ? 0.645 : 0.585;
+  const long long tiles = (M + rows - 1) / rows * ((N + t.bn - 1) / t.bn);
+  return (double)((tiles + slots - 1) / slots) * cost;
+}
+// Rows of A in a tile of gemm_rows.cu, 0 where the tiles above are faster.  A round there costs, in the same measure (0.38 us a k-block of
+// 64), what stands here, its start and end 2 us more.  Measured with 13 shapes of the built-in models x 25 row counts from 80 to 4608 and
+// every tile: the rule takes 0.956 of the time without these tiles on average, at worst 1.008, where always knowing the best would take
+// 0.949.  us, without / with: 300 x 128256 x 4096 317 / 248, 513 rows 497 / 416, 128 rows 181 / 171; 300 x 8192 x 3584 22.9 / 18.3; 900 x
+// 3584 x 4096 24 / 21; 1600 x 4096 x 14336 148 / 130; 4608 x 3584 x 14336 373 / 331.  Up to 128 rows only for vocabulary sizes, whose tiles
+// of 256 columns leave the last round half empty (what has fewer columns goes to gemm_skinny.cu).  Gated products gain nothing here: a
+// gate and an up tile per CTA leave fewer tiles than the rounds want.
+static int rows_tile(int M, int N, int K, const TileChoice& other) {
+  if (M <= 64 || (M <= GEMM_BM && N < 148 * 256) || N % 128 != 0) return 0;
+  const struct {
+    int rows;
+    double cost;
+  } all[8] = {{64, 0.43}, {96, 0.45}, {128, 0.49}, {160, 0.575}, {192, 0.645}, {224, 0.70}, {256, 0.83}, {320, 1.12}};
+  const double unit = 0.3817 * (K / GEMM_BK);
+  double least = 0.95 * unit * tile_rounds(M, N, other);
+  int best = 0;
+  for (const auto& c : all) {
+    const long long tiles = (long long)((N / 128 + 1) / 2) * ((M + c.rows - 1) / c.rows), pairs = num_sms() / 2;
+    const double t = (double)((tiles + pairs - 1) / pairs) * c.cost * unit + 2.0;
+    if (t < least) {
+      least = t;
+      best = c.rows;
+    }
+  }
+  return best;
+}
+
 int g_gemm_force_bn = 0;  // test hook: 0 = heuristic
 int g_gemm_splitk = 0;    // 0 = auto, 1 = never, n > 1 = force n splits where legal (tests)
 
@@ -1267,6 +1301,8 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
   }
   if (bn == 0) {
     const TileChoice t = choose_tile(M, N, false, g_gemm_mode == 0);
+    if (g_gemm_mode == 0)
+      if (const int rows = rows_tile(M, N, K, t)) return gemm_rows(A, W, C, M, N, K, rows, fixed_w, st);
     auto pair = [&](auto width) {
       return launch_gemm2<decltype(width)::value>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
     };
@@ -1377,6 +1413,12 @@ int b200q_gemm_set_tile_n(int bn) {
 // test/tuning hook: 0 = auto, 1 = 1-CTA kernels only, 2 = 2-CTA (cta_group::2) kernel whenever legal
 // diagnostics: co-resident CTA pairs the 2-CTA kernel's grid is sized to (0 until first use)
 int b200q_gemm_resident_pairs(void) { return g_gemm2_pairs; }
+
+// test hook: rows of A in the tiles of gemm_rows.cu that a product takes (0: none of them)
+int b200q_gemm_rows_tile(int M, int N, int K) {
+  if (g_gemm_mode || g_gemm_force_bn || use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 0;
+  return rows_tile(M, N, K, choose_tile(M, N, false, true));
+}
 
 // test hook: columns of the tiles of a product of more than 128 rows whose reduction is not split
 int b200q_gemm_tile_n(int M, int N) { return g_gemm_force_bn ? g_gemm_force_bn : choose_tile(M, N, false, g_gemm_mode == 0).bn; }

@@ -259,4 +259,7 @@ int gemm_skinny_splits(int M, int N, int K);
 int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int act, long long ldc, const float* bias, float limit,
                 float* parts, bool fixed_w, cudaStream_t st);
 
+// tiles of 256 weight rows and `rows` rows of A (gemm_rows.cu): a multiple of 32 up to 256, of 64 beyond; N a multiple of 128
+int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, bool fixed_w, cudaStream_t st);
+
 }  // namespace b200q
