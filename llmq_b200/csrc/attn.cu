@@ -1049,10 +1049,12 @@ static int launch_decode_stream(const void* q, int q_stride, void* out, const vo
     attr_set = true;
   }
   const int total = n_seqs * n_kv;
-  // 2 resident CTAs per SM (96 KB of page ring each); variant 3 (tests) squeezes everything
-  // through 4 CTAs so that every warp walks many items
-  const int max_ctas = g_decode_variant == 3 ? 4 : 2 * attn_num_sms();
+  // An item to a warp, so that CTAs begin as others end: dealt out evenly over two CTAs per SM, ragged items leave most of them waiting for
+  // the longest share (8 kv heads, D = 128: 4608 sequences of 129 to 256 tokens 582 -> 529 us, 1000 of 10 to 500 189 -> 164, 400 of 200
+  // 55.9 / 56.1; D = 64 323 -> 271, 115 -> 92, 34.7 / 36.5).  Items of up to 8 pages are dealt out: a CTA's start is longer than they are
+  // (1500 of 40 to 60 59 us, 66 with an item to a warp).  variant 3 (tests) squeezes everything through 4 CTAs so that every warp walks many.
   const int want = (total + DEC_WARPS - 1) / DEC_WARPS;
+  const int max_ctas = g_decode_variant == 3 ? 4 : bt_stride > 8 ? want : 2 * attn_num_sms();
   const int grid = want < max_ctas ? want : max_ctas;
   const ScoreConsts sc = score_consts(scale, softcap);
   B200Q_CUDA(launch_early(kern, grid, DEC_WARPS * 32, S_::TOTAL, st, 1, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt,
@@ -1123,11 +1125,13 @@ int decode_attn(const void* q, int q_stride, void* out, const void* kv_layer, co
                   "decode_attn: unsupported D=%d block_size=%d (D in {64,128,256}, block 16)", D,
                   block_size);
   if (n_seqs == 0) return B200Q_OK;
-  // streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
-  // another order of sums)
+  // The streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
+  // another order of sums); but up to 5000 items of which some have 40 pages and more are shared by a CTA's warps all the same, whose ends
+  // lie closer together (us, streamed / shared: 8 kv heads, D = 128, 400 sequences of 20 to 900 tokens 130 / 116, 600 of 1 to 1500
+  // 294 / 268; D = 64 76 / 61, 166 / 139; but 1000 of 10 to 500 164 / 169, D = 256 320 / 385).
+  const long long items = (long long)n_seqs * n_kv;
   const bool stream_variant =
-      g_decode_variant >= 2 ||
-      (g_decode_variant == 0 && !batch_invariant() && (long long)n_seqs * n_kv >= 16LL * attn_num_sms());
+      g_decode_variant >= 2 || (g_decode_variant == 0 && !batch_invariant() && items >= 16LL * attn_num_sms() && !(items <= 5000 && bt_stride >= 40));
   if (stream_variant)
     B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
                         ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);

@@ -30,3 +30,25 @@ def test_shared_pages(cuda, D, n_q, n_kv, ctxs, cap, window):
         ref = reference(q, *rows[i], torch.tensor([c - 1]), D ** -0.5, cap, window).to(BF)
         # probabilities are rounded to bf16 before the value product: 2^-9 each, outputs agree to ~5e-3 or 2 ulps
         bf16_close(got[i].view(1, n_q, D), ref, ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"ctx {c}")
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 16, 8), (128, 8, 8), (256, 16, 8)])
+@pytest.mark.parametrize("columns", [8, 9, 39, 40])     # dealt out over the resident warps; a warp to an item (twice); an item to a CTA
+def test_many_sequences(cuda, D, n_q, n_kv, columns):
+    """296 sequences and a few more: items enough for the streaming kernel, contexts of one token up to the whole table"""
+    from llmq_b200 import lib
+    for B, window in ((296, 0), (301, 70)):
+        ctxs = [1 + (i * i * 37) % min(16 * columns, 300) for i in range(B)]
+        ctxs[5] = 16 * columns
+        kv, bt, rows = make_cache(ctxs, n_kv, D, seed=B, wide=False)
+        assert bt.shape[1] == columns + 1
+        bt = bt[:, :columns].contiguous()
+        qkv = torch.randn(B, (n_q + 2 * n_kv) * D, generator=torch.Generator().manual_seed(7)).to(BF)
+        out = torch.full((B + 1, n_q * D), float("nan"), dtype=BF, device=cuda)
+        lib.decode_attn(qkv.to(cuda), out, kv.to(cuda), bt.to(cuda), torch.tensor(ctxs, dtype=torch.int32, device=cuda), n_q, n_kv, D, BS, D ** -0.5,
+                        softcap=20.0 if window else 0.0, window=window)
+        got = out.cpu()
+        assert torch.isnan(got[B].float()).all()
+        for i, c in enumerate(ctxs):
+            ref = reference(qkv[i: i + 1, : n_q * D].view(1, n_q, D), *rows[i], torch.tensor([c - 1]), D ** -0.5, 20.0 if window else 0.0, window).to(BF)
+            bf16_close(got[i].view(1, n_q, D), ref, ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"ctx {c}")   # (as above)
