@@ -91,24 +91,43 @@ static int norm_chunks(int H, F&& launch) {
                                                                     : launch(std::integral_constant<int, NORM_MAX_CHUNKS>{});
 }
 
-// 8 consecutive outputs of a split-K GEMM: the fp32 partials ws[s][row][col] added in split order
-// (the same order and rounding as the stand-alone reduction) and rounded to bf16
-__device__ __forceinline__ uint4 sum_partials_bf16(const float* ws, long long off,
-                                                   long long mn, int splits) {
-  float4 a = *reinterpret_cast<const float4*>(ws + off);
-  float4 b = *reinterpret_cast<const float4*>(ws + off + 4);
-  for (int sp = 1; sp < splits; ++sp) {
-    const float4 c = *reinterpret_cast<const float4*>(ws + sp * mn + off);
-    const float4 d = *reinterpret_cast<const float4*>(ws + sp * mn + off + 4);
-    a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
-    b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+// C pieces of 8 consecutive outputs of a split-K GEMM, from off[i] on: the fp32 partials ws[s][row][col] added in split order (the same order
+// and rounding as the stand-alone reduction) and rounded to bf16.  These kernels are chains of reads from L2: AT_ONCE parts of every piece
+// are asked for before the first is added.  More than the callers' 4 or 2 x 2 take registers that longer rows or fuller SMs want back.
+// 48 rows of 4 parts, us, part after part / so: a norm of 4096 3.6 / 3.2; of 2048 2.7 / 2.5; with 8 parts 4.4 / 4.2.
+template <int C, int AT_ONCE>
+__device__ __forceinline__ void sum_partials_bf16(const float* ws, const long long (&off)[C], long long mn, int splits, uint4 (&out)[C]) {
+  float4 a[C][2];
+  for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
+    float4 p[C][AT_ONCE][2];
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x)
+        if (s0 + x < splits) {
+          p[i][x][0] = *reinterpret_cast<const float4*>(ws + (s0 + x) * mn + off[i]);
+          p[i][x][1] = *reinterpret_cast<const float4*>(ws + (s0 + x) * mn + off[i] + 4);
+        }
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+#pragma unroll
+      for (int x = 0; x < AT_ONCE; ++x)
+        if (s0 + x < splits) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float4 c = p[i][x][h];
+            if (s0 + x == 0) {
+              a[i][h] = c;
+            } else {
+              a[i][h].x += c.x; a[i][h].y += c.y; a[i][h].z += c.z; a[i][h].w += c.w;
+            }
+          }
+        }
   }
-  uint4 o;
-  o.x = pack_bf16x2(a.x, a.y);
-  o.y = pack_bf16x2(a.z, a.w);
-  o.z = pack_bf16x2(b.x, b.y);
-  o.w = pack_bf16x2(b.z, b.w);
-  return o;
+#pragma unroll
+  for (int i = 0; i < C; ++i)
+    out[i] = make_uint4(pack_bf16x2(a[i][0].x, a[i][0].y), pack_bf16x2(a[i][0].z, a[i][0].w), pack_bf16x2(a[i][1].x, a[i][1].y),
+                        pack_bf16x2(a[i][1].z, a[i][1].w));
 }
 
 // kPartials: x is not read from x_in but reduced on the fly from the fp32 partials of a split-K GEMM
@@ -122,23 +141,38 @@ __global__ void __launch_bounds__(NORM_THREADS)
   follow_previous(x_in, residual, w, y, ws);
   const long long row = blockIdx.x;
   const uint4* xr = x_in + row * chunks;
-  constexpr bool kAhead = !kPartials;  // (beside the sums of parts, weights that come with the row cost more registers than they give)
-  constexpr int WN = kAhead ? CH : 2;
-  uint4 v[CH], res[2], weight[WN];
+  // (sums of parts: what does not wait for them is asked for first; otherwise the residual's chunks go two at a time behind the row's)
+  uint4 v[CH], res[kPartials ? CH : 2], weight[CH];
   float ss = 0.f;
+  if constexpr (kPartials) {
 #pragma unroll
-  for (int j = 0; j < CH; ++j) {
-    int c = threadIdx.x + j * NORM_THREADS;
-    if (c < chunks) {
-      if constexpr (kPartials) v[j] = sum_partials_bf16(ws, (row * chunks + c) * 8, mn, splits);
-      else v[j] = ld_v4(xr + c);
-      if constexpr (kAhead) weight[j] = ld_v4(w + c);
+    for (int j = 0; j < CH; ++j) {
+      const int c = threadIdx.x + j * NORM_THREADS;
+      if (c < chunks) {
+        if (kAdd) res[j] = ld_v4(residual + row * chunks + c);
+        weight[j] = ld_v4(w + c);
+      }
     }
   }
 #pragma unroll
   for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
-    if (kAdd && j % 2 == 0) {
+    if (c < chunks) {
+      if constexpr (kPartials) {
+        const long long off[1] = {(row * chunks + c) * 8};
+        uint4 sum[1];
+        sum_partials_bf16<1, 4>(ws, off, mn, splits, sum);
+        v[j] = sum[0];
+      } else {
+        v[j] = ld_v4(xr + c);
+        weight[j] = ld_v4(w + c);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < CH; ++j) {
+    int c = threadIdx.x + j * NORM_THREADS;
+    if (kAdd && !kPartials && j % 2 == 0) {
 #pragma unroll
       for (int i = 0; i < 2 && j + i < CH; ++i)
         if (c + i * NORM_THREADS < chunks) res[i] = ld_v4(residual + row * chunks + c + i * NORM_THREADS);
@@ -146,7 +180,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
     if (c < chunks) {
       uint4 a = v[j];
       if (kAdd) {
-        uint4 r = res[j % 2];
+        uint4 r = res[kPartials ? j : j % 2];
         uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
         const uint32_t* rp = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
@@ -177,14 +211,9 @@ __global__ void __launch_bounds__(NORM_THREADS)
 #pragma unroll
   for (int j = 0; j < CH; ++j) {
     int c = threadIdx.x + j * NORM_THREADS;
-    if (!kAhead && j % 2 == 0) {
-#pragma unroll
-      for (int i = 0; i < 2 && j + i < CH; ++i)
-        if (c + i * NORM_THREADS < chunks) weight[i] = ld_v4(w + c + i * NORM_THREADS);
-    }
     if (c < chunks) {
       uint4 a = v[j];
-      uint4 ww = weight[j % WN];
+      uint4 ww = weight[j];
       uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
       const uint32_t* wp = reinterpret_cast<const uint32_t*>(&ww);
 #pragma unroll
@@ -358,7 +387,7 @@ __device__ __forceinline__ void rope_chunk_pair(uint4& x1, uint4& x2, const uint
 // kPartials: the qkv row is reduced on the fly from the fp32 partials of the split-K qkv projection
 // (decode-sized batches) instead of being read back as bf16 — reduce + RoPE + KV write in one launch
 template <bool kPartials>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kPartials ? 128 : 256)
     rope_kvwrite_kernel(uint4* __restrict__ qkv, const uint4* __restrict__ cos_sin,
                         const int32_t* __restrict__ positions,
                         const int32_t* __restrict__ slot_mapping, uint4* __restrict__ kv_layer,
@@ -377,20 +406,22 @@ __global__ void __launch_bounds__(256)
   const int off = slot >= 0 ? slot % block_size : 0;
   const int n_rope_items = (n_q + n_kv) * half;
   const int n_items = n_rope_items + n_kv * cpr;
-  for (int it = threadIdx.x; it < n_items; it += blockDim.x) {
+  for (int it = blockIdx.y * blockDim.x + threadIdx.x; it < n_items; it += gridDim.y * blockDim.x) {
     if (it < n_rope_items) {
       int head = it / half, c = it % half;
       uint4 x1, x2;
+      uint4 cs = ld_v4(cs_row + c);
+      uint4 sn = ld_v4(cs_row + half + c);
       if constexpr (kPartials) {
-        const long long e = ((long long)t * row_chunks + head * cpr + c) * 8;
-        x1 = sum_partials_bf16(ws, e, mn, splits);
-        x2 = sum_partials_bf16(ws, e + (long long)half * 8, mn, splits);
+        const long long e = ((long long)t * row_chunks + head * cpr + c) * 8, off2[2] = {e, e + (long long)half * 8};
+        uint4 x[2];
+        sum_partials_bf16<2, 2>(ws, off2, mn, splits, x);
+        x1 = x[0];
+        x2 = x[1];
       } else {
         x1 = ld_v4(row + head * cpr + c);
         x2 = ld_v4(row + head * cpr + c + half);
       }
-      uint4 cs = ld_v4(cs_row + c);
-      uint4 sn = ld_v4(cs_row + half + c);
       rope_chunk_pair(x1, x2, cs, sn);
       if (head < n_q) {
         st_v4(row + head * cpr + c, x1);
@@ -407,9 +438,12 @@ __global__ void __launch_bounds__(256)
       int j = it - n_rope_items;
       int h = j / cpr, c = j % cpr;
       uint4 v;
-      if constexpr (kPartials)
-        v = sum_partials_bf16(ws, ((long long)t * row_chunks + (n_q + n_kv + h) * cpr + c) * 8, mn, splits);
-      else
+      if constexpr (kPartials) {
+        const long long off1[1] = {((long long)t * row_chunks + (n_q + n_kv + h) * cpr + c) * 8};
+        uint4 sum[1];
+        sum_partials_bf16<1, 4>(ws, off1, mn, splits, sum);
+        v = sum[0];
+      } else
         v = ld_v4(row + (n_q + n_kv + h) * cpr + c);
       uint4* dst = kv_layer + ((((long long)blk * 2 + 1) * n_kv + h) * block_size + off) * cpr;
       st_v4(dst + (c ^ (off & 7)), v);
@@ -858,7 +892,11 @@ int b200q_rope_kvwrite(void* qkv, const void* cos_sin, const int32_t* positions,
                   "rope_kvwrite: bad shape T=%d n_q=%d n_kv=%d D=%d bs=%d", T, n_q, n_kv, D,
                   block_size);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(rope_kvwrite_kernel<false>, T, 256, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
+  // A row is (n_q + n_kv) D/16 + n_kv D/8 items.  Up to 320 rows a row's rounds of 256 items go to blocks of their own, of equal size (128 rows
+  // of 32 + 8 + 8 heads, D = 128: 3.05 -> 2.61 us); above, the chip is full and one block to a row reads with more in flight (1000: 6.1, 6.7).
+  const int items = (n_q + n_kv) * D / 16 + n_kv * D / 8, blocks = T <= 320 ? (items + 255) / 256 : 1;
+  const int threads = blocks > 1 ? ((items + blocks - 1) / blocks + 31) / 32 * 32 : 256;
+  B200Q_CUDA(launch_early(rope_kvwrite_kernel<false>, dim3(T, blocks), threads, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
                           slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size, nullptr, 0, 0));
   count_launch();
   return B200Q_OK;
@@ -872,7 +910,10 @@ int b200q_rope_kvwrite_splitk(void* qkv, const float* partials, int splits, cons
                   block_size);
   B200Q_CHECK_ARG(partials && splits >= 1 && splits <= 16, "rope_kvwrite_splitk: bad partials (splits=%d)", splits);
   if (T == 0) return B200Q_OK;
-  B200Q_CUDA(launch_early(rope_kvwrite_kernel<true>, T, 256, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
+  // One item to a thread, in blocks of 128: a thread that goes on to a second item begins its reads anew.  Four parts, us, a block of 256
+  // to a row / so: 48 rows of 32 + 8 + 8 heads, D = 128 5.2 / 3.2; 16 + 8 + 8, D = 256 5.7 / 3.3; 128 rows of the first 5.5 / 3.7.
+  const int items = (n_q + n_kv) * D / 16 + n_kv * D / 8;
+  B200Q_CUDA(launch_early(rope_kvwrite_kernel<true>, dim3(T, (items + 127) / 128), 128, 0, as_stream(stream), 1, (uint4*)qkv, (const uint4*)cos_sin, positions,
                           slot_mapping, (uint4*)kv_layer, n_q, n_kv, D, block_size, partials, splits, (long long)T * (n_q + 2 * n_kv) * D));
   count_launch();
   return B200Q_OK;

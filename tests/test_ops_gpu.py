@@ -426,6 +426,32 @@ def test_splitk_partials_fused_into_norm_and_rope_are_bit_identical(cuda, M):
 
 
 
+@pytest.mark.parametrize("T,D,n_q,n_kv", [(1, 256, 1, 1), (5, 64, 32, 8), (33, 128, 32, 8), (320, 128, 5, 1), (321, 256, 3, 2)])
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 8, 16])
+def test_sums_of_parts_at_every_count(cuda, T, D, n_q, n_kv, splits):
+    """parts that come several at a time are added one after the other all the same: the bits of a plain sum in their order"""
+    from llmq_b200 import lib
+    W = (n_q + 2 * n_kv) * D
+    parts = torch.randn(splits, T, W, generator=torch.Generator().manual_seed(splits)).to(cuda)
+    total = parts[0].clone()
+    for p in parts[1:]:
+        total += p
+    want = total.to(BF)
+    res, w = rnd(T, W, seed=31).to(cuda), rnd(W, seed=32).to(cuda)
+    y_ref, r_ref, y, r = want.clone(), res.clone(), torch.empty_like(want), res.clone()
+    lib.add_rmsnorm(y_ref, r_ref, w, 1e-5)
+    lib.add_rmsnorm_splitk(y, r, w, parts.data_ptr(), splits, 1e-5)
+    assert torch.equal(r, r_ref) and torch.equal(y, y_ref)
+    table = O.rope_table(512, D, 500000.0, None).to(BF).to(cuda)
+    pos = torch.randint(0, 512, (T,), dtype=torch.int32, generator=torch.Generator().manual_seed(1)).to(cuda)
+    slots = torch.randperm(30 * 16, generator=torch.Generator().manual_seed(2))[:T].to(torch.int32).to(cuda)
+    kv_ref, kv = (torch.zeros(30, 2, n_kv, 16, D, dtype=BF, device=cuda) for _ in range(2))
+    q = torch.zeros_like(want)
+    lib.rope_kvwrite(want, table, pos, slots, kv_ref, n_q, n_kv, D, 16)
+    lib.rope_kvwrite_splitk(q, parts.data_ptr(), splits, table, pos, slots, kv, n_q, n_kv, D, 16)
+    assert torch.equal(q[:, :n_q * D], want[:, :n_q * D]) and torch.equal(kv, kv_ref)
+
+
 def test_model_forward_is_identical_with_and_without_splitk_fusion(cuda, monkeypatch):
     """whole-engine check of the same: greedy + sampled tokens with B200Q_FUSE_SPLITK on / off"""
     from llmq_b200.model import BUILTIN_SPECS, Engine
