@@ -8,8 +8,10 @@
 //     issues the products, eight warps store.  Two tiles' accumulators in tensor memory where they fit.
 //   * a lane of an accumulator is a column of C: 32 rows x 128 columns at a time are turned in shared memory and leave by TMA, which also
 //     leaves out what lies behind the last row or column.
+//   * where the tiles are too few for the chip, K is cut as well and the fp32 sums of its parts leave by plain stores, for another kernel to add.
 // The parts of a row of tiles follow each other, so that CTA pairs share weights through L2; every element of C is one sequential sum, in
-// the same order as in gemm_tcgen05.cu.  Times and the rule that takes these tiles: rows_tile in gemm_tcgen05.cu.
+// the same order as in gemm_tcgen05.cu, or one such sum to a part of K.  Times and the rule that takes these tiles: rows_tile in
+// gemm_tcgen05.cu.
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -24,6 +26,8 @@ struct GemmRowsArgs {
   int* failed;
   int M, N, K, nt, stages, parts, n_blocks;  // a tile has HALVES * nt rows of A; n_blocks: of 128 columns of C
   int fixed_w;                               // see linear() in common.cuh
+  int splits;                                // parts of K, each a tile of its own
+  float* ws;                                 // their sums, [split][M][N], for splits > 1
 };
 
 __device__ __forceinline__ void gr_arrive(uint32_t bar) {
@@ -59,8 +63,9 @@ __device__ __forceinline__ void gr_commit(uint64_t* bar) {
                : "memory");
 }
 
-// HALVES: accumulators side by side that share a tile's weights (of nt rows of A each)
-template <int HALVES>
+// HALVES: accumulators side by side that share a tile's weights (of nt rows of A each).  PARTS: a tile is a part of K (a kernel of its own, since
+// what places it costs every other tile 0.3 us)
+template <int HALVES, bool PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
     gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                      const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ GemmRowsArgs a) {
@@ -72,7 +77,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
   __shared__ int dead;  // a wait ran out: the other roles stop as well
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
-  const int n_tiles = (a.n_blocks + 1) / 2 * a.parts, k_blocks = a.K / GR_BK;
+  const int per_pair = PARTS ? a.parts * a.splits : a.parts, n_tiles = (a.n_blocks + 1) / 2 * per_pair, k_blocks = a.K / GR_BK;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int a_bytes = a.nt / 2 * (GR_BK * 2), stage_bytes = GR_W_BYTES + HALVES * a_bytes;
   const int rows_all = HALVES * a.nt, accs = 2 * rows_all <= 512 ? 2 : 1;  // accumulators of a whole tile
@@ -117,19 +122,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
     }
   };
   // the first row of W of this CTA's part of a tile
-  auto w_row = [&](int tile) { return (tile / a.parts * 2 + rank) * 128; };
+  auto w_row = [&](int tile) { return (tile / per_pair * 2 + rank) * 128; };
+  // the k-blocks of a tile: parts of K behind one another, each with all parts of M
+  auto k_begin = [&](int tile) { return PARTS ? tile % per_pair / a.parts * k_blocks / a.splits : 0; };
+  auto k_end = [&](int tile) { return PARTS ? (tile % per_pair / a.parts + 1) * k_blocks / a.splits : k_blocks; };
 
   // the first weights while the kernel before this one ends: into the ring where nobody can still be writing them, into L2 otherwise
   const uint32_t full0 = mapa_shared(full, 0);
   int early = 0;
   if (warp == 0 && lane == 0) {
-    for (int kb = 0; kb < min(a.stages, k_blocks); ++kb) {
+    const int k0 = k_begin(pair), n = min(a.stages, k_end(pair) - k0);
+    for (int s = 0; s < n; ++s) {
       if (a.fixed_w) {
-        gr_expect_tx(full0 + kb * 8, GR_W_BYTES);
-        gr_load(smem + kb * stage_bytes, &tmap_w, kb * GR_BK, w_row(pair), full0 + kb * 8);
+        gr_expect_tx(full0 + s * 8, GR_W_BYTES);
+        gr_load(smem + s * stage_bytes, &tmap_w, (k0 + s) * GR_BK, w_row(pair), full0 + s * 8);
         ++early;
       } else {
-        tma_prefetch_2d(&tmap_w, kb * GR_BK, w_row(pair));
+        tma_prefetch_2d(&tmap_w, (k0 + s) * GR_BK, w_row(pair));
       }
     }
   }
@@ -144,11 +153,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
       const void* map = weights ? &tmap_w : &tmap_a;
       const uint32_t bytes = weights ? GR_W_BYTES : HALVES * a_bytes;
       uint8_t* const to = smem + (weights ? 0 : GR_W_BYTES);
-      int stage = early % a.stages, kb = early;
+      int stage = early % a.stages, done = early;
       uint32_t phase = early / a.stages;
       for (int tile = pair; tile < n_tiles; tile += pairs) {
         const int row = weights ? w_row(tile) : tile % a.parts * rows_all + rank * (a.nt / 2);
-        for (; kb < k_blocks; ++kb) {
+        const int k1 = k_end(tile);
+        for (int kb = k_begin(tile) + done; kb < k1; ++kb) {
           const uint32_t bar = full0 + stage * 8;
           uint8_t* at = to + stage * stage_bytes;
           wait(empty + stage, phase ^ 1u);
@@ -160,7 +170,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
             phase ^= 1u;
           }
         }
-        kb = 0;
+        done = 0;
         if (*(volatile int*)&dead) break;
       }
     }
@@ -176,7 +186,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
         if (!(on = mbar_wait_warp(acc_empty + acc, acc_phase ^ 1u, &dead, a.failed, WAIT_CYCLES))) break;
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(acc * rows_all);
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        const int k0 = k_begin(tile), k1 = k_end(tile);
+        for (int kb = k0; kb < k1; ++kb) {
           if (!(on = mbar_wait_warp(full + stage, phase, &dead, a.failed, WAIT_CYCLES))) break;
           tc_fence_after();
           if (elect_one()) {
@@ -186,9 +197,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
 #pragma unroll
               for (int h = 0; h < HALVES; ++h)
                 gr_product(d + (uint32_t)(h * a.nt), make_smem_desc(sw + k * 32), make_smem_desc(sa + h * a_bytes + k * 32), idesc,
-                           (kb > 0 || k > 0) ? 1u : 0u);
+                           (kb > k0 || k > 0) ? 1u : 0u);
             gr_commit(empty + stage);
-            if (kb == k_blocks - 1) gr_commit(acc_full + acc);
+            if (kb == k1 - 1) gr_commit(acc_full + acc);
           }
           __syncwarp();
           if (++stage == a.stages) {
@@ -212,7 +223,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
     int acc = 0, n_out = 0;
     uint32_t acc_phase = 0;
     for (int tile = pair; tile < n_tiles; tile += pairs) {
-      const int block = tile / a.parts * 2 + rank, row0 = tile % a.parts * rows_all;
+      const int block = tile / per_pair * 2 + rank, row0 = tile % a.parts * rows_all;
       const int rows = min(rows_all, a.M - row0);
       wait(acc_full + acc, acc_phase);
       __syncwarp();
@@ -224,22 +235,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
           uint32_t v[32];
           tmem_ld32(at + (uint32_t)m0, v);
           tmem_ld_wait();
-          const uint32_t patch = patch0 + (uint32_t)(n_out & 1) * GR_PATCH;
-          if (copies) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          all();  // (the copy that read this patch has)
-          // row j of the patch, column quarter * 32 + lane: two boxes of 64 columns, as the copy's 128-byte swizzle
-          const uint32_t col = (uint32_t)((quarter & 1) * 64 + lane * 2), base = patch + (uint32_t)(quarter >> 1) * 4096 + (col & 15u);
+          if constexpr (PARTS) {  // a warp's row of a part is 128 bytes
+            float* to = a.ws + ((long long)(tile % per_pair / a.parts) * a.M + row0 + m0) * a.N + block * 128 + quarter * 32 + lane;
+            const int n = rows - m0;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            asm volatile("st.shared.b16 [%0], %1;" ::"r"(base + j * 128 + (((col >> 4) ^ (j & 7)) << 4)),
-                         "h"((unsigned short)f2bf_bits(__uint_as_float(v[j])))
-                         : "memory");
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          all();
-          if (copies) {
-            gr_store(&tmap_c, block * 128, row0 + m0, patch);
-            gr_store(&tmap_c, block * 128 + 64, row0 + m0, patch + 4096);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            for (int j = 0; j < 32; ++j)
+              if (j < n) to[(long long)j * a.N] = __uint_as_float(v[j]);
+          } else {
+            const uint32_t patch = patch0 + (uint32_t)(n_out & 1) * GR_PATCH;
+            if (copies) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            all();  // (the copy that read this patch has)
+            // row j of the patch, column quarter * 32 + lane: two boxes of 64 columns, as the copy's 128-byte swizzle
+            const uint32_t col = (uint32_t)((quarter & 1) * 64 + lane * 2), base = patch + (uint32_t)(quarter >> 1) * 4096 + (col & 15u);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              asm volatile("st.shared.b16 [%0], %1;" ::"r"(base + j * 128 + (((col >> 4) ^ (j & 7)) << 4)),
+                           "h"((unsigned short)f2bf_bits(__uint_as_float(v[j])))
+                           : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            all();
+            if (copies) {
+              gr_store(&tmap_c, block * 128, row0 + m0, patch);
+              gr_store(&tmap_c, block * 128 + 64, row0 + m0, patch + 4096);
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
           }
         }
       }
@@ -269,8 +288,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GR_THREADS, 1)
   }
 }
 
-template <int HALVES>
-static int launch_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, bool fixed_w, cudaStream_t st) {
+template <int HALVES, bool PARTS>
+static int launch_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, int splits, float* ws, bool fixed_w,
+                       cudaStream_t st) {
   GemmRowsArgs a{};
   a.M = M;
   a.N = N;
@@ -279,18 +299,20 @@ static int launch_rows(const void* A, const void* W, void* C, int M, int N, int 
   a.parts = (M + rows - 1) / rows;
   a.n_blocks = N / 128;
   a.fixed_w = fixed_w;
+  a.splits = splits;
+  a.ws = ws;
   a.stages = GR_RING / (GR_W_BYTES + rows / 2 * GR_BK * 2);
   if (a.stages > GR_MAX_STAGES) a.stages = GR_MAX_STAGES;
   CUtensorMap tw, ta, tc;
   int rc = get_tmap(W, N, K, 128, &tw);
   if (!rc) rc = get_tmap(A, M, K, a.nt / 2, &ta);
-  if (!rc) rc = get_tmap(C, M, N, 32, &tc);
+  if (!rc) rc = PARTS ? get_tmap(A, M, K, a.nt / 2, &tc) : get_tmap(C, M, N, 32, &tc);  // (parts leave by plain stores)
   if (rc) return rc;
   if (!wait_flag(&a.failed)) {
     set_error("gemm: no host-visible flag for bounded waits");
     return B200Q_ECUDA;
   }
-  auto kern = gemm_rows_kernel<HALVES>;
+  auto kern = gemm_rows_kernel<HALVES, PARTS>;
   static int pairs = 0;  // as many as can be resident at once
   if (pairs == 0) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
@@ -311,14 +333,20 @@ static int launch_rows(const void* A, const void* W, void* C, int M, int N, int 
     }
     pairs = n < 74 ? n : 74;
   }
-  const int tiles = (a.n_blocks + 1) / 2 * a.parts;
+  const int tiles = (a.n_blocks + 1) / 2 * a.parts * splits;
   B200Q_CUDA(launch_early(kern, 2 * (tiles < pairs ? tiles : pairs), GR_THREADS, GR_SMEM, st, 1, tw, ta, tc, a));
   count_launch();
   return B200Q_OK;
 }
 
-int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, bool fixed_w, cudaStream_t st) {
-  return rows > 256 ? launch_rows<2>(A, W, C, M, N, K, rows, fixed_w, st) : launch_rows<1>(A, W, C, M, N, K, rows, fixed_w, st);
+int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, int splits, float* ws, bool fixed_w, cudaStream_t st) {
+  auto launch = [&](auto halves, auto parts) {
+    return launch_rows<decltype(halves)::value, decltype(parts)::value>(A, W, C, M, N, K, rows, splits, ws, fixed_w, st);
+  };
+  const std::integral_constant<int, 1> one;
+  const std::integral_constant<int, 2> two;
+  if (splits > 1) return rows > 256 ? launch(two, std::true_type{}) : launch(one, std::true_type{});
+  return rows > 256 ? launch(two, std::false_type{}) : launch(one, std::false_type{});
 }
 
 }  // namespace b200q

@@ -338,18 +338,33 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
 }
 
-// out[m][n] = bf16(sum_s ws[s][m][n]), partials added in split order (deterministic)
+// out[m][n] = bf16(sum_s ws[s][m][n]), partials added in split order (deterministic), four parts asked for at once
 __global__ void __launch_bounds__(256)
     splitk_reduce_kernel(const float4* __restrict__ ws, uint4* __restrict__ out, long long mn8,
                          int splits) {
   follow_previous(ws, out);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < mn8;
        i += (long long)gridDim.x * blockDim.x) {
-    float4 a = ws[2 * i], b = ws[2 * i + 1];
-    for (int s = 1; s < splits; ++s) {
-      const float4 c = ws[2 * (i + (long long)s * mn8)], d = ws[2 * (i + (long long)s * mn8) + 1];
-      a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
-      b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+    float4 a, b;
+    for (int s0 = 0; s0 < splits; s0 += 4) {
+      float4 c[4], d[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (s0 + x < splits) {
+          c[x] = ws[2 * (i + (s0 + x) * mn8)];
+          d[x] = ws[2 * (i + (s0 + x) * mn8) + 1];
+        }
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (s0 + x < splits) {
+          if (s0 + x == 0) {
+            a = c[x];
+            b = d[x];
+          } else {
+            a.x += c[x].x; a.y += c[x].y; a.z += c[x].z; a.w += c[x].w;
+            b.x += d[x].x; b.y += d[x].y; b.z += d[x].z; b.w += d[x].w;
+          }
+        }
     }
     uint4 o;
     o.x = pack_bf16x2(a.x, a.y);
@@ -846,6 +861,26 @@ static int splitk_scratch(int splits, int M, int N, cudaStream_t st, float** out
   return B200Q_OK;
 }
 
+// (no other thread's product on the same stream between a product and the sum of its parts, whichever kernels they take)
+static std::mutex g_split_pair;
+// product leaves its parts in ws; they are summed into C, or by whoever reads C where partials_out asks for them
+template <typename F>
+static int split_product(float* ws, void* C, int M, int N, int splits, cudaStream_t st, const float** partials_out, F&& product) {
+  std::unique_lock<std::mutex> together(g_split_pair, std::defer_lock);
+  if (!partials_out) together.lock();
+  const int rc = product();
+  if (rc) return rc;
+  if (partials_out) {
+    *partials_out = ws;
+    return B200Q_OK;
+  }
+  const long long mn8 = (long long)M * N / 8;
+  const int grid = (int)((mn8 + 255) / 256 < 148 * 8 ? (mn8 + 255) / 256 : 148 * 8);
+  B200Q_CUDA(launch_early(splitk_reduce_kernel, grid, 256, 0, st, 1, (const float4*)ws, (uint4*)C, mn8, splits));
+  count_launch();
+  return B200Q_OK;
+}
+
 template <int BN, int kAct = ACT_NONE>
 static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int K,
                        cudaStream_t st, int splits = 1, const float** partials_out = nullptr, long long ldc = 0,
@@ -867,24 +902,14 @@ static int launch_gemm(const void* A, const void* W, void* C, int M, int N, int 
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (N / BN) * splits;
   const int grid = tiles < num_sms() ? tiles : num_sms();
   float* ws = nullptr;
-  static std::mutex pair;  // (no other thread's product on the same stream between a product and the sum of its parts)
-  std::unique_lock<std::mutex> together(pair, std::defer_lock);
-  if (splits > 1) {
-    if (!partials_out) together.lock();
-    rc = splitk_scratch(splits, M, N, st, &ws);
-    if (rc) return rc;
-  }
-  B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K, splits, ws, a_rows * GEMM_BK * 2,
-                          ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate, (int)fixed_w));
-  count_launch();
-  if (partials_out) *partials_out = ws;  // the caller fuses the reduction into the consumer of C
-  if (splits > 1 && !partials_out) {
-    const long long mn8 = (long long)M * N / 8;
-    const int rgrid = (int)((mn8 + 255) / 256 < 148 * 8 ? (mn8 + 255) / 256 : 148 * 8);
-    B200Q_CUDA(launch_early(splitk_reduce_kernel, rgrid, 256, 0, st, 1, (const float4*)ws, (uint4*)C, mn8, splits));
+  if (splits > 1 && (rc = splitk_scratch(splits, M, N, st, &ws))) return rc;
+  auto product = [&]() -> int {
+    B200Q_CUDA(launch_early(kern, grid, GEMM_THREADS, Cfg::SMEM_TOTAL, st, 1, ta, tb, (bf16*)C, M, N, K, splits, ws, a_rows * GEMM_BK * 2,
+                            ldc > 0 ? ldc : (kAct != ACT_NONE ? N / 2 : N), gate, (int)fixed_w));
     count_launch();
-  }
-  return B200Q_OK;
+    return B200Q_OK;
+  };
+  return splits > 1 ? split_product(ws, C, M, N, splits, st, partials_out, product) : product();
 }
 
 static int g_gemm2_pairs = 0;  // co-resident CTA pairs reported by the occupancy query
@@ -984,23 +1009,43 @@ static double tile_rounds(int M, int N, const TileChoice& t) {
 // 3584 x 4096 24 / 21; 1600 x 4096 x 14336 148 / 130; 4608 x 3584 x 14336 373 / 331.  Up to 128 rows only for vocabulary sizes, whose tiles
 // of 256 columns leave the last round half empty (what has fewer columns goes to gemm_skinny.cu).  Gated products gain nothing here: a
 // gate and an up tile per CTA leave fewer tiles than the rounds want.
-static int rows_tile(int M, int N, int K, const TileChoice& other) {
-  if (M <= 64 || (M <= GEMM_BM && N < 148 * 256) || N % 128 != 0) return 0;
+//
+// Parts of K (up to 8, of 4 k-blocks or more, M x parts up to 1536: 800 rows in two are 4 % slower, 750 10 % faster, and a model's scratch
+// holds 2048) are what fills the rounds of a product of few columns.  A round is then bound by its products or, with few pairs at work, by
+// the weights they fetch; the parts are written and summed in 0.3 us a MB, 0.2 us each and 1.1 us (the two kernels overlap), another round
+// costs 2 us; 3 % have to be gained.  17 shapes x 20 row counts from 129 to 1000, sums included: the rule takes 0.937 of the time without
+// parts on average and 1.002 at worst, where always knowing the best would take 0.92.  us, without / with: 150 x 3584 x 14336 38.2 / 29.3,
+// 200 x 4096 x 14336 39.0 / 34.5; 256 x 2560 x 10240 32.4 / 20.5; 300 x 2048 x 8192 27.3 / 17.5, 512 rows 28.0 / 20.9, 750 rows 28.8 / 26.3;
+// 400 x 4096 x 14336 49.1 / 46.0.  (129 to 256 rows were split over tiles of 128 x 128 before: slower at all of 9 such shapes.)
+struct RowsTile {
+  int rows, splits;
+};
+static RowsTile rows_tile(int M, int N, int K, const TileChoice& other, bool may_split) {
+  if (M <= 64 || (M <= GEMM_BM && N < 148 * 256) || N % 128 != 0) return {0, 1};
   const struct {
     int rows;
     double cost;
   } all[8] = {{64, 0.43}, {96, 0.45}, {128, 0.49}, {160, 0.575}, {192, 0.645}, {224, 0.70}, {256, 0.83}, {320, 1.12}};
-  const double unit = 0.3817 * (K / GEMM_BK);
-  double least = 0.95 * unit * tile_rounds(M, N, other);
-  int best = 0;
-  for (const auto& c : all) {
-    const long long tiles = (long long)((N / 128 + 1) / 2) * ((M + c.rows - 1) / c.rows), pairs = num_sms() / 2;
-    const double t = (double)((tiles + pairs - 1) / pairs) * c.cost * unit + 2.0;
-    if (t < least) {
-      least = t;
-      best = c.rows;
+  const int pairs = num_sms() / 2, kb = K / GEMM_BK, most = may_split && N <= 8192 ? 8 : 1;
+  const double k_block = 0.3817;
+  double least = 0.95 * k_block * kb * tile_rounds(M, N, other);
+  RowsTile best{0, 1};
+  for (const auto& c : all)
+    for (int s = 1; s <= most && (s == 1 || (kb / s >= 4 && s * M <= 1536)); ++s) {
+      const long long tiles = (long long)((N / 128 + 1) / 2) * ((M + c.rows - 1) / c.rows) * s;
+      const double rounds = (double)((tiles + pairs - 1) / pairs);
+      double t = rounds * c.cost * k_block * ((kb + s - 1) / s);
+      if (s > 1) {
+        const double weights = 0.124e-6 * 2.0 * N * K * pairs / (tiles < pairs ? tiles : pairs);
+        t = 1.03 * ((t > weights ? t : weights) + 2.0 * rounds + 1.1 + s * (0.2 + 0.3e-6 * 4.0 * M * N));
+      } else {
+        t += 2.0;
+      }
+      if (t < least) {
+        least = t;
+        best = {c.rows, s};
+      }
     }
-  }
   return best;
 }
 
@@ -1019,9 +1064,7 @@ bool batch_invariant() {
 // output tiles to put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
 static int choose_splits(int M, int N, int K, bool invariant, int forced_bn) {
   const int want = invariant ? 1 : g_gemm_splitk;  // 0 = auto, 1 = off, >1 = forced (tests)
-  if (want == 1 || forced_bn != 0 || M > 256 || N % 128 != 0 || N > 8192) return 1;
-  // (129 to 256 rows: with 2048 <= K < 4096 the partial tiles cost more than the idle SMs: 256 x 3072 x 2048 14.0 us split, 10.4 not)
-  if (want == 0 && M > GEMM_BM && K >= 2048 && K < 4096) return 1;
+  if (want == 1 || forced_bn != 0 || M > (want ? 256 : GEMM_BM) || N % 128 != 0 || N > 8192) return 1;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (N / 128);
   const int kb = K / GEMM_BK;
   int splits = want > 1 ? want : 1;
@@ -1040,6 +1083,19 @@ int g_gemm_mode = 0;      // 0 = auto, 1 = force 1-CTA kernels, 2 = force the 2-
 // rows (its splits depend on it, and the kernels here that larger steps use add in another order).
 static bool use_skinny(int M, int N, int K, bool gated) {
   return g_gemm_mode == 0 && g_gemm_force_bn == 0 && g_gemm_splitk == 0 && !batch_invariant() && gemm_skinny_ok(M, N, K, gated);
+}
+
+// the tile of gemm_rows.cu that a product takes, none where a hook asks for other kernels; parts only where the sums may depend on the rows
+static RowsTile rows_tile_of(int M, int N, int K) {
+  if (g_gemm_mode != 0 || g_gemm_force_bn != 0) return {0, 1};
+  return rows_tile(M, N, K, choose_tile(M, N, false, true), g_gemm_splitk == 0 && !batch_invariant());
+}
+// the same for a product on st, with the memory for its parts, and without parts where there is none
+static RowsTile rows_tile_of(int M, int N, int K, cudaStream_t st, float** ws) {
+  const RowsTile r = rows_tile_of(M, N, K);
+  if (r.splits <= 1 || splitk_scratch(r.splits, M, N, st, ws) == B200Q_OK) return r;
+  cudaGetLastError();
+  return rows_tile(M, N, K, choose_tile(M, N, false, true), false);
 }
 
 
@@ -1276,6 +1332,12 @@ static int gemm_gated(const char* what, const void* A, const void* W, void* C, i
 
 namespace b200q {
 
+static int rows_product(const void* A, const void* W, void* C, int M, int N, int K, RowsTile r, float* ws, bool fixed_w, cudaStream_t st,
+                        const float** partials_out) {
+  return split_product(ws, C, M, N, r.splits, st, partials_out,
+                       [&]() { return gemm_rows(A, W, nullptr, M, N, K, r.rows, r.splits, ws, fixed_w, st); });
+}
+
 int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st) {
   B200Q_CHECK_ARG(M >= 0 && N > 0 && K > 0 && K % GEMM_BK == 0 && N % 64 == 0,
                   "gemm: unsupported shape M=%d N=%d K=%d (need K%%64==0, N%%64==0)", M, N, K);
@@ -1300,9 +1362,11 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
     if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
   }
   if (bn == 0) {
+    float* ws = nullptr;
+    const RowsTile r = rows_tile_of(M, N, K, st, &ws);
+    if (r.splits > 1) return rows_product(A, W, C, M, N, K, r, ws, fixed_w, st, nullptr);
+    if (r.rows > 0) return gemm_rows(A, W, C, M, N, K, r.rows, 1, nullptr, fixed_w, st);
     const TileChoice t = choose_tile(M, N, false, g_gemm_mode == 0);
-    if (g_gemm_mode == 0)
-      if (const int rows = rows_tile(M, N, K, t)) return gemm_rows(A, W, C, M, N, K, rows, fixed_w, st);
     auto pair = [&](auto width) {
       return launch_gemm2<decltype(width)::value>(A, W, C, M, N, K, st, 0, GateArgs{nullptr, 0.f}, fixed_w);
     };
@@ -1341,7 +1405,14 @@ int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w
     return B200Q_OK;
   }
   const int splits = choose_splits(M, N, K, batch_invariant(), 0);
-  if (splits <= 1) return B200Q_OK;
+  if (splits <= 1) {
+    float* ws = nullptr;
+    const RowsTile r = rows_tile_of(M, N, K, st, &ws);
+    if (r.splits <= 1) return B200Q_OK;
+    int rc = rows_product(A, W, nullptr, M, N, K, r, ws, fixed_w, st, partials_out);
+    if (!rc) *splits_out = r.splits;
+    return rc;
+  }
   int rc = launch_gemm<128>(A, W, nullptr, M, N, K, st, splits, partials_out, 0, GateArgs{nullptr, 0.f}, fixed_w);
   if (rc) return rc;
   *splits_out = splits;
@@ -1416,8 +1487,14 @@ int b200q_gemm_resident_pairs(void) { return g_gemm2_pairs; }
 
 // test hook: rows of A in the tiles of gemm_rows.cu that a product takes (0: none of them)
 int b200q_gemm_rows_tile(int M, int N, int K) {
-  if (g_gemm_mode || g_gemm_force_bn || use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 0;
-  return rows_tile(M, N, K, choose_tile(M, N, false, true));
+  if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 0;
+  return rows_tile_of(M, N, K).rows;
+}
+
+// test hook: the parts of K of such a product (1: not split)
+int b200q_gemm_rows_splits(int M, int N, int K) {
+  if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 1;
+  return rows_tile_of(M, N, K).splits;
 }
 
 // test hook: columns of the tiles of a product of more than 128 rows whose reduction is not split

@@ -260,6 +260,7 @@ int gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, int 
                 float* parts, bool fixed_w, cudaStream_t st);
 
 // tiles of 256 weight rows and `rows` rows of A (gemm_rows.cu): a multiple of 32 up to 256, of 64 beyond; N a multiple of 128
-int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, bool fixed_w, cudaStream_t st);
+// with splits > 1 (of the K / 64 blocks, at least one each) the sums of its parts go to ws[split][M][N] and C is not looked at
+int gemm_rows(const void* A, const void* W, void* C, int M, int N, int K, int rows, int splits, float* ws, bool fixed_w, cudaStream_t st);
 
 }  // namespace b200q

@@ -362,6 +362,7 @@ EXTRA_SIGNATURES = {
     "b200q_gemm_resident_pairs": (_i, []),
     "b200q_gemm_tile_n": (_i, [_i, _i]),
     "b200q_gemm_rows_tile": (_i, [_i, _i, _i]),
+    "b200q_gemm_rows_splits": (_i, [_i, _i, _i]),
     "b200q_decode_attn_set_variant": (_i, [_i]),
     "b200q_gemm_set_splitk": (_i, [_i]),
     "b200q_gemm_set_give_up": (_i, [_i]),
