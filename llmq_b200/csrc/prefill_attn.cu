@@ -1047,10 +1047,7 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
           if (by_tma) {
             fence_async_shared();
             __syncwarp();
-            if (lane == 0) {
-              tma_store_3d(&out_map, c, r.kvh * a.G, r.row0 + (int)((uint32_t)first_row * a.inv_g >> 16), patch);
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
+            if (lane == 0) tma_store_3d(&out_map, c, r.kvh * a.G, r.row0 + (int)((uint32_t)first_row * a.inv_g >> 16), patch);
           } else {
             __syncwarp();
 #pragma unroll 1
@@ -1074,6 +1071,8 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
             }
             __syncwarp();
           }
+          // (a group for every use of a patch, an empty one where nothing was copied: the wait above counts groups)
+          if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
       tc_fence_before();
