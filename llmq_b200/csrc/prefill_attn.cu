@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
   uint8_t* v_s = k_s + STG * C::T_BYTES;
   constexpr int SLOTS = NQ == 1 ? 4 : 2;  // blocks of scores in tensor memory (D = 256: of consecutive steps; else one per query tile)
   __shared__ __align__(8) uint64_t k_full[STG], k_empty[STG], v_full[STG], v_empty[STG], q_ready[2], q_empty[2], s_full[SLOTS], p_ready[SLOTS],
-      o_full[2], pv_done[4], o_read, m_ready[SW], l_ready[SW], work_full[FA_RING], work_empty[FA_RING];
+      o_full[2], pv_done[4], o_read, m_ready[SW], l_ready[2 * SW], work_full[FA_RING], work_empty[FA_RING];
   __shared__ FaWork ring[FA_RING];
   uint8_t* patches = v_s + STG * C::T_BYTES;
   __shared__ float row_max[NQ == 1 ? 128 : 1], part[2][GROUPS][NQ == 1 ? 128 : 1];  // D = 256: running maxima; sums of every warpgroup's steps, in turns
@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
     for (int i = 0; i < SW; ++i) {
       mbar_init(m_ready + i, 1);
       mbar_init(l_ready + i, 1);
+      mbar_init(l_ready + SW + i, 1);
     }
     for (int i = 0; i < FA_RING; ++i) {
       mbar_init(work_full + i, 1);
@@ -995,11 +996,13 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
         }
         part[x & 1][wg][row] = l;
         __syncwarp();
-        if (lane == 0) mbar_arrive(l_ready + wg * 4 + quarter);
+        // (barriers of every other run: a warpgroup may give the next run's sum before another one has looked for this run's, but not the one
+        // behind it, for which that one has to have given the next)
+        if (lane == 0) mbar_arrive(l_ready + (x & 1) * SW + wg * 4 + quarter);
         l = 0.f;
 #pragma unroll
         for (int i = 0; i < GROUPS; ++i) {
-          wait(l_ready + i * 4 + quarter, (uint32_t)x & 1u);
+          wait(l_ready + (x & 1) * SW + i * 4 + quarter, (uint32_t)x / 2 & 1u);
           l += part[x & 1][i][row];
         }
         __syncwarp();
