@@ -474,15 +474,13 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, D == 64 ? 4 : 2)
 }
 
 // ------------------------------------------------------------------------------------------
-// K7 decode, streaming variant for large batches.  Every warp of a persistent grid owns whole
-// (sequence, kv-head) items and walks them back to back: the 3-stage TMA page ring never
-// drains between items (the pages of the next item are already in flight while the current
-// one finishes), there is no cross-warp merge and no CTA turnover, and the next item's Q
-// fragments / context length are prefetched one item ahead.  With ~12 pages per item
-// (128-in/128-out) the v1 kernel above spends as long in its prologue (ctx -> block ids -> first
-// TMA, ~1-2 us of dependent latency) as in streaming; this one pays that once per warp.
-// Used when there are enough items to give every resident warp several of them; v1 keeps the
-// small-batch / long-context cases (it splits one item across 4 warps).
+// K7 decode, streaming variant for large batches: a warp owns whole (sequence, kv-head) items, there is no merge across warps.
+// Of short tables a resident warp walks several items back to back: its page ring runs on across them (the pages of the next item
+// are in flight while the current one ends), and the next item's Q fragments and context length are fetched one item ahead, so that
+// the start (context -> block ids -> first page, 1-2 us of dependent latency) is paid once per warp.  Of longer tables a warp has
+// one item, and the start of a CTA lies beside the pages of the other one on its SM.
+// Used when there are enough items to give every resident warp several of them; which form, and which items go to the kernel above
+// (it splits one item across 4 warps) all the same: launch_decode_stream and decode_attn.
 // ------------------------------------------------------------------------------------------
 template <int D, int BS>
 struct Dec2Smem {
@@ -1055,8 +1053,10 @@ static int launch_decode_stream(const void* q, int q_stride, void* out, const vo
   const int total = n_seqs * n_kv;
   // An item to a warp, so that CTAs begin as others end: dealt out evenly over two CTAs per SM, ragged items leave most of them waiting for
   // the longest share (8 kv heads, D = 128: 4608 sequences of 129 to 256 tokens 582 -> 529 us, 1000 of 10 to 500 189 -> 164, 400 of 200
-  // 55.9 / 56.1; D = 64 323 -> 271, 115 -> 92, 34.7 / 36.5).  Items of up to 8 pages are dealt out: a CTA's start is longer than they are
-  // (1500 of 40 to 60 59 us, 66 with an item to a warp).  variant 3 (tests) squeezes everything through 4 CTAs so that every warp walks many.
+  // 55.9 / 56.1; D = 64 323 -> 271, 115 -> 92, 34.6 / 35.7).  Items of one length lose by it what their CTAs' starts cost, up to 8 % of
+  // tables of 9 to 16 pages (D = 256, 800 of 200 tokens 191 / 201; of 1 to 208 132 / 111).  Items of up to 8 pages are dealt out: a CTA's
+  // start is longer than they are (1500 of 40 to 60 59 us, 66 with an item to a warp).  variant 3 (tests) squeezes everything through 4
+  // CTAs so that every warp walks many.
   const int want = (total + DEC_WARPS - 1) / DEC_WARPS;
   const int max_ctas = g_decode_variant == 3 ? 4 : bt_stride > 8 ? want : 2 * attn_num_sms();
   const int grid = want < max_ctas ? want : max_ctas;
@@ -1130,12 +1130,16 @@ int decode_attn(const void* q, int q_stride, void* out, const void* kv_layer, co
                   block_size);
   if (n_seqs == 0) return B200Q_OK;
   // The streaming kernel once every resident warp (2 CTAs x 4 warps per SM) gets >= 2 items (one warp walks a sequence's pages, not four:
-  // another order of sums); but up to 5000 items of which some have 40 pages and more are shared by a CTA's warps all the same, whose ends
-  // lie closer together (us, streamed / shared: 8 kv heads, D = 128, 400 sequences of 20 to 900 tokens 130 / 116, 600 of 1 to 1500
-  // 294 / 268; D = 64 76 / 61, 166 / 139; but 1000 of 10 to 500 164 / 169, D = 256 320 / 385).
+  // another order of sums); but up to 5000 items of tables of 24 pages and more (D = 128: 40, 256: 96) are shared by a CTA's warps all the
+  // same, whose ends lie closer together.  The larger D, the fewer CTAs lie beside each other, and the more a CTA's start costs.  us, an item
+  // to a warp / shared, 8 kv heads: D = 64 400 sequences of 400 tokens 62.8 / 55.1, of 20 to 900 74.3 / 60.6; D = 128 126 / 115 (of 20 to
+  // 900), 48.3 / 46.2 (of 100, one of 640); D = 256 193 / 230 (360 of 20 to 900), 67.2 / 85.3 (400 of 100, one of 640), 138 / 101 (one of
+  // 2000).  2137 sizes (2368 to 40000 items, equal, spread and with one long context; 2, 4 and 8 kv heads): 0.88 of the time of dealing
+  // everything out over the resident warps, 1.02 of always knowing the best.
   const long long items = (long long)n_seqs * n_kv;
+  const int long_table = D == 64 ? 24 : D == 128 ? 40 : 96;
   const bool stream_variant =
-      g_decode_variant >= 2 || (g_decode_variant == 0 && !batch_invariant() && items >= 16LL * attn_num_sms() && !(items <= 5000 && bt_stride >= 40));
+      g_decode_variant >= 2 || (g_decode_variant == 0 && !batch_invariant() && items >= 16LL * attn_num_sms() && !(items <= 5000 && bt_stride >= long_table));
   if (stream_variant)
     B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
                         ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);

@@ -33,7 +33,8 @@ def test_shared_pages(cuda, D, n_q, n_kv, ctxs, cap, window):
 
 
 @pytest.mark.parametrize("D,n_q,n_kv", [(64, 16, 8), (128, 8, 8), (256, 16, 8)])
-@pytest.mark.parametrize("columns", [8, 9, 39, 40])     # dealt out over the resident warps; a warp to an item (twice); an item to a CTA
+# dealt out over the resident warps; a warp to an item; an item to a CTA from 24 (D = 64), 40 (128) and 96 (256) columns on
+@pytest.mark.parametrize("columns", [8, 9, 23, 24, 39, 40, 95, 96])
 def test_many_sequences(cuda, D, n_q, n_kv, columns):
     """296 sequences and a few more: items enough for the streaming kernel, contexts of one token up to the whole table"""
     from llmq_b200 import lib
