@@ -319,8 +319,8 @@ struct SkinnyPlan {
 //   3072 x 2048             5.2 /  6.3   6.8 /  8.0   8.0 /  9.6   8.5 / 10.5
 //   4096 x 4096             8.6 /  9.2  10.4 / 10.6  11.2 / 11.7  11.8 / 13.1
 //   4096 x 14336           21.3 / 22.4  23.8 / 24.7  24.3 / 26.7  25.2 / 28.9
-//   16384 x 2048 gated     12.9 / 43.2  14.4 / 43.7  17.3 / 44.1  18.1 / 25.1
-//   28672 x 4096 gated     38.7 / 66.4  41.1 / 68.3  45.7 / 68.8  47.7 / 50.2
+//   16384 x 2048 gated     13.9 / 25.8  15.3 / 25.9  18.4 / 26.2  19.4 / 26.2
+//   28672 x 4096 gated     38.5 / 49.1  41.6 / 49.7  46.3 / 50.8  49.1 / 52.1
 // Splits: up to 64 rows two CTAs per SM with three or more stages each are best; with more rows a stage grows and one CTA per SM
 // with the whole memory as its ring is (28.7 against 29.7 us at 4096 x 14336, 100 rows), unless the tiles alone would leave half
 // of the SMs idle.  All clusters have to be resident at once: a cluster lies within a processing cluster of the chip, and one
@@ -388,16 +388,18 @@ static bool wide_tiles(int N) { return N % 256 == 0 && N / 256 >= 148; }
 //   * plain, more tiles, a CTA to each: the longer the reduction, the less the start and the end of a tile count, which the persistent
 //     kernels hide.  Share of the time there, 12288 columns: K = 2048 0.99 at 16 rows, 1.07 at 48, 1.31 at 128; K = 4096 0.98 at 80, 1.06
 //     at 128; K = 8192 1.02 at 100; two CTAs per SM hide some of it: 24576 x 2048 0.97 at 64 rows, 1.08 at 128.
-//   * plain, tiles of 256 (vocabulary sizes): up to 32 rows (128256 x 2048 86 / 88); up to 112 where K >= 4096 and the tiles fill rounds
-//     of two CTAs per SM (128256 x 4096 177 / 179 at 100 rows, 1.7 rounds; but 50176 x 5120 98 / 89, 0.66).
-//   * gated: always (16384 x 2048 13 / 43 at one row, 18 / 25 at 128; 28672 x 4096 46 / 69 at 112, 47.7 / 50.2 at 128; 2048 x 512 5 / 32,
-//     9.8 / 13.7); the kernels there spend 15 to 20 us on the division of rows that do not exist.
+//   * plain, tiles of 256 (vocabulary sizes): up to 32 rows (128256 x 2048 84 / 87); where K >= 4096 and the tiles fill rounds of two CTAs
+//     per SM (128256 x 4096 178 / 183 at 64 rows, 1.7 rounds; but 50176 x 5120 98 / 89, 0.66) up to 64, or 112 if there is one round.  From
+//     65 rows on there are the tiles of gemm_rows.cu: 128256 x 4096 181 / 172 at 65, 193 / 176 at 100, 197 / 179 at 112; 151552 x 4096 208 /
+//     205, 206 / 202, 211 / 202; one round: 60672 x 4096 83.1 / 87.5, 87.1 / 87.1, 89.1 / 88.5, 65536 x 8192 185 / 193, 189 / 191, 193 / 192.
+//   * gated: always (16384 x 2048 13.9 / 25.8 at one row, 19.4 / 26.2 at 128; 28672 x 4096 47.7 / 51.6 at 112, 49.1 / 52.1 at 128; 2048 x 512
+//     5.4 / 14.3, 10.5 / 14.6; 9 shapes x 11 row counts: 0.32 to 0.94 of the time there).
 bool gemm_skinny_ok(int M, int N, int K, bool gated) {
   if (M < 1 || M > 128 || K % SK_BK != 0 || N % (gated ? 256 : 128) != 0 || N / 128 > 65535) return false;
   if (gated) return true;
   if (wide_tiles(N)) {
     const int tiles = N / 256, rounds = (tiles + 295) / 296;
-    return M <= 32 || (M <= 112 && K >= 4096 && 5 * tiles >= 4 * 296 * rounds);
+    return M <= 32 || (M <= (rounds == 1 ? 112 : 64) && K >= 4096 && 5 * tiles >= 4 * 296 * rounds);
   }
   const int tiles = N / 128;
   if (K < 1024) return M <= (tiles > 148 ? 32 : K >= 768 ? 16 : 0);

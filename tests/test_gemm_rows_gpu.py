@@ -24,11 +24,13 @@ def whole_sums():
     lib.check(lib.load().b200q_gemm_set_splitk(0))
 
 
-# (M, N, K, tile): one round and several of 64 to 384 rows, a last part of one row and of all, an odd number of blocks of 128 columns
+# (M, N, K, tile): one round and several of 64 to 320 rows, a last part of one row and of all, an odd number of blocks of 128 columns, the first
+# row count of large vocabularies
 @pytest.mark.parametrize("M,N,K,tile", [(300, 2304, 9216, 64), (257, 4096, 14336, 96), (513, 3584, 8192, 128), (513, 4096, 14336, 160),
                                         (300, 8192, 3584, 160), (129, 38016, 2048, 160), (352, 8192, 3584, 192), (900, 3584, 8192, 192),
                                         (1024, 3584, 14336, 224), (450, 8832, 2048, 256), (300, 15104, 2048, 320), (1600, 3584, 14336, 320),
-                                        (1700, 3712, 9216, 192), (65, 38400, 2048, 96), (128, 38016, 2048, 128), (1537, 4096, 14336, 192)])
+                                        (1700, 3712, 9216, 192), (65, 38400, 2048, 96), (128, 38016, 2048, 128), (65, 128256, 4096, 96),
+                                        (1537, 4096, 14336, 192)])
 def test_plain(cuda, M, N, K, tile, whole_sums):
     from llmq_b200 import lib
     assert lib.load().b200q_gemm_rows_tile(M, N, K) == tile and lib.load().b200q_gemm_rows_splits(M, N, K) == 1
