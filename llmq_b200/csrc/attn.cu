@@ -878,17 +878,6 @@ static inline ScoreConsts score_consts(float scale, float softcap) {
 
 int g_decode_variant = 0;  // test hook: 0 = auto, 1 = split kernel (v1), 2 = streaming kernel
 
-static int attn_num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 template <int D, int BS, bool kCap, bool kShared, int PAGES>
 static int prepare_decode() {
   static bool attr_set = false;
@@ -932,10 +921,10 @@ static int decode_resident(int splits) {
               ? cudaErrorUnknown
               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, decode_attn_kernel<D, BS, kCap, false, PAGES>,
                                                               DEC_WARPS * 32, DecSmem<D, BS, PAGES>::TOTAL);
-      v *= attn_num_sms();
+      v *= num_sms();
     } else {
       cudaLaunchAttribute attr;
-      const cudaLaunchConfig_t cfg = decode_config<D, BS, true, PAGES>(splits, attn_num_sms(), 1, &attr, nullptr);
+      const cudaLaunchConfig_t cfg = decode_config<D, BS, true, PAGES>(splits, num_sms(), 1, &attr, nullptr);
       e = prepare_decode<D, BS, kCap, true, PAGES>() ? cudaErrorUnknown
                                               : cudaOccupancyMaxActiveClusters(&v, decode_attn_kernel<D, BS, kCap, true, PAGES>, &cfg);
     }
@@ -970,7 +959,7 @@ struct DecodeCosts {
 template <int D, int BS, bool kCap, int PAGES>
 static void decode_plan_of(int n_seqs, int n_kv, int bt_stride, int window, DecodeCosts c, DecodePlan* best, double* least) {
   const long long n = (long long)n_seqs * n_kv;
-  const int sms = attn_num_sms(), per_sm = decode_resident<D, BS, kCap, PAGES>(1) / sms;
+  const int sms = num_sms(), per_sm = decode_resident<D, BS, kCap, PAGES>(1) / sms;
   const int pages = window > 0 && (window + 15) / 16 + 1 < bt_stride ? (window + 15) / 16 + 1 : bt_stride;
   for (int s = 1; s <= 8 && (s == 1 || pages >= 4 * DEC_WARPS * s); ++s) {
     const long long resident = decode_resident<D, BS, kCap, PAGES>(s), rounds = (n + resident - 1) / resident, deep = (n * s + sms - 1) / sms;
@@ -1058,7 +1047,7 @@ static int launch_decode_stream(const void* q, int q_stride, void* out, const vo
   // start is longer than they are (1500 of 40 to 60 59 us, 66 with an item to a warp).  variant 3 (tests) squeezes everything through 4
   // CTAs so that every warp walks many.
   const int want = (total + DEC_WARPS - 1) / DEC_WARPS;
-  const int max_ctas = g_decode_variant == 3 ? 4 : bt_stride > 8 ? want : 2 * attn_num_sms();
+  const int max_ctas = g_decode_variant == 3 ? 4 : bt_stride > 8 ? want : 2 * num_sms();
   const int grid = want < max_ctas ? want : max_ctas;
   const ScoreConsts sc = score_consts(scale, softcap);
   B200Q_CUDA(launch_early(kern, grid, DEC_WARPS * 32, S_::TOTAL, st, 1, (const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt,
@@ -1089,7 +1078,7 @@ static int launch_prefill(const void* q, int q_stride, void* out, const void* kv
   // 3 of 60 to 120, 144 CTAs 6.4 / 7.3, but 32 of 16, 256 CTAs 5.1 / 4.9 and one of 128, 64 CTAs 7.1 / 6.6; D = 64, of which an SM holds
   // more: 32 of 16, 256 CTAs 3.95 / 4.32, one of 512, 256 CTAs 18.6 / 21.6, 12 of 40 to 80, 432 CTAs 6.3 / 6.7, but 104 CTAs 4.4 / 4.3 and
   // 20 of 10 to 100, 620 CTAs 8.9 / 8.3).
-  const long long ctas = (long long)n_tiles * n_kv, sms = attn_num_sms();
+  const long long ctas = (long long)n_tiles * n_kv, sms = num_sms();
   const bool uneven = D == 64 ? ctas > sms - 20 && ctas <= 13 * sms / 4 : 2 * ctas > sms && ctas <= sms;
   if (uneven) {
     kern<<<grid, (G + 1) * 32, S_::TOTAL, st>>>((const bf16*)q, q_stride, (bf16*)out, (const uint8_t*)kv, bt, bt_stride, (const int4*)tiles,
@@ -1139,7 +1128,7 @@ int decode_attn(const void* q, int q_stride, void* out, const void* kv_layer, co
   const long long items = (long long)n_seqs * n_kv;
   const int long_table = D == 64 ? 24 : D == 128 ? 40 : 96;
   const bool stream_variant =
-      g_decode_variant >= 2 || (g_decode_variant == 0 && !batch_invariant() && items >= 16LL * attn_num_sms() && !(items <= 5000 && bt_stride >= long_table));
+      g_decode_variant >= 2 || (g_decode_variant == 0 && !batch_invariant() && items >= 16LL * num_sms() && !(items <= 5000 && bt_stride >= long_table));
   if (stream_variant)
     B200Q_ATTN_DISPATCH(launch_decode_stream, q, q_stride, out, kv_layer, block_table, bt_stride,
                         ctx_lens, n_seqs, n_q, n_kv, scale, softcap, window, st);

@@ -317,7 +317,7 @@ static int launch_rows(const void* A, const void* W, void* C, int M, int N, int 
   if (pairs == 0) {
     B200Q_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(148);
+    cfg.gridDim = dim3(num_sms() & ~1);
     cfg.blockDim = dim3(GR_THREADS);
     cfg.dynamicSmemBytes = GR_SMEM;
     cudaLaunchAttribute attr;
@@ -329,9 +329,9 @@ static int launch_rows(const void* A, const void* W, void* C, int M, int N, int 
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
-      n = 74;
+      n = num_sms() / 2;
     }
-    pairs = n < 74 ? n : 74;
+    pairs = n < num_sms() / 2 ? n : num_sms() / 2;
   }
   const int tiles = (a.n_blocks + 1) / 2 * a.parts * splits;
   B200Q_CUDA(launch_early(kern, 2 * (tiles < pairs ? tiles : pairs), GR_THREADS, GR_SMEM, st, 1, tw, ta, tc, a));

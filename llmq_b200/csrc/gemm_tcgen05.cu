@@ -759,7 +759,7 @@ int get_head_rows_tmap(const void* p, int n_q, int D, long long stride, int head
   return B200Q_OK;
 }
 
-static int num_sms() {
+int num_sms() {
   static int n = 0;
   if (n == 0) {
     int dev = 0;
@@ -875,7 +875,7 @@ static int split_product(float* ws, void* C, int M, int N, int splits, cudaStrea
     return B200Q_OK;
   }
   const long long mn8 = (long long)M * N / 8;
-  const int grid = (int)((mn8 + 255) / 256 < 148 * 8 ? (mn8 + 255) / 256 : 148 * 8);
+  const int most = 8 * num_sms(), grid = (int)((mn8 + 255) / 256 < most ? (mn8 + 255) / 256 : most);
   B200Q_CUDA(launch_early(splitk_reduce_kernel, grid, 256, 0, st, 1, (const float4*)ws, (uint4*)C, mn8, splits));
   count_launch();
   return B200Q_OK;
@@ -1021,7 +1021,7 @@ struct RowsTile {
   int rows, splits;
 };
 static RowsTile rows_tile(int M, int N, int K, const TileChoice& other, bool may_split) {
-  if (M <= 64 || (M <= GEMM_BM && N < 148 * 256) || N % 128 != 0) return {0, 1};
+  if (M <= 64 || (M <= GEMM_BM && N < num_sms() * 256) || N % 128 != 0) return {0, 1};
   const struct {
     int rows;
     double cost;

@@ -253,6 +253,7 @@ int get_head_rows_tmap(const void* p, int n_q, int D, long long stride, int head
 int prefill_tiles(const void* q, int q_stride, void* out, const void* kv, const int32_t* bt, int bt_stride, const int32_t* tiles,
                   int n_tiles, int n_q, int n_kv, int D, float scale, float softcap, int window, int long_keys, cudaStream_t st);
 
+int num_sms();  // of the device (gemm_tcgen05.cu)
 // products of up to 128 rows (gemm_skinny.cu)
 bool gemm_skinny_ok(int M, int N, int K, bool gated);
 int gemm_skinny_splits(int M, int N, int K);
