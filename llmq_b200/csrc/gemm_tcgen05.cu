@@ -971,6 +971,7 @@ static int launch_gemm2(const void* A, const void* W, void* C, int M, int N, int
 struct TileChoice {
   bool pair;
   int bn;
+  double rounds;  // rounds x a round's time, in rounds of 128 x 256 tiles
 };
 static TileChoice choose_tile(int M, int N, bool gated, bool pairs) {
   const struct {
@@ -979,29 +980,18 @@ static TileChoice choose_tile(int M, int N, bool gated, bool pairs) {
     double cost;
   } all[7] = {{true, 256, 0.84},  {false, 256, 1.0},   {true, 192, 0.70},  {true, 160, 0.65},
               {true, 128, 0.595}, {false, 128, 0.645}, {false, 64, 0.585}};
-  TileChoice best{false, N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64};
-  double least = 1e30;
+  TileChoice best{false, N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64, 1e30};
   for (const auto& c : all) {
     const bool ragged = c.bn == 160 || c.bn == 192;
     if ((ragged ? N < c.bn : N % c.bn != 0) || (gated && c.bn != 256) || (c.pair && (!pairs || M <= GEMM_BM))) continue;
     const long long rows = c.pair ? 256 : GEMM_BM, slots = c.pair ? num_sms() / 2 : num_sms();
     const long long tiles = (M + rows - 1) / rows * ((N + c.bn - 1) / c.bn);
     const double t = (double)((tiles + slots - 1) / slots) * c.cost;
-    if (t < least - 1e-9) {
-      least = t;
-      best = {c.pair, c.bn};
-    }
+    if (t < best.rounds - 1e-9) best = {c.pair, c.bn, t};
   }
   return best;
 }
 
-// the least (rounds x round's time) of the tiles above, in 128 x 256 tiles
-static double tile_rounds(int M, int N, const TileChoice& t) {
-  const long long rows = t.pair ? 256 : GEMM_BM, slots = t.pair ? num_sms() / 2 : num_sms();
-  const double cost = t.pair ? (t.bn == 256 ? 0.84 : t.bn == 192 ? 0.70 : t.bn == 160 ? 0.65 : 0.595) : t.bn == 256 ? 1.0 : t.bn == 128 ? 0.645 : 0.585;
-  const long long tiles = (M + rows - 1) / rows * ((N + t.bn - 1) / t.bn);
-  return (double)((tiles + slots - 1) / slots) * cost;
-}
 // Rows of A in a tile of gemm_rows.cu, 0 where the tiles above are faster.  A round there costs, in the same measure (0.38 us a k-block of
 // 64), what stands here, its start and end 2 us more.  Measured with 13 shapes of the built-in models x 25 row counts from 80 to 4608 and
 // every tile: the rule takes 0.956 of the time without these tiles on average, at worst 1.008, where always knowing the best would take
@@ -1028,7 +1018,7 @@ static RowsTile rows_tile(int M, int N, int K, const TileChoice& other, bool may
   } all[8] = {{64, 0.43}, {96, 0.45}, {128, 0.49}, {160, 0.575}, {192, 0.645}, {224, 0.70}, {256, 0.83}, {320, 1.12}};
   const int pairs = num_sms() / 2, kb = K / GEMM_BK, most = may_split && N <= 8192 ? 8 : 1;
   const double k_block = 0.3817;
-  double least = 0.95 * k_block * kb * tile_rounds(M, N, other);
+  double least = 0.95 * k_block * kb * other.rounds;
   RowsTile best{0, 1};
   for (const auto& c : all)
     for (int s = 1; s <= most && (s == 1 || (kb / s >= 4 && s * M <= 1536)); ++s) {
@@ -1089,6 +1079,11 @@ static bool use_skinny(int M, int N, int K, bool gated) {
 static RowsTile rows_tile_of(int M, int N, int K) {
   if (g_gemm_mode != 0 || g_gemm_force_bn != 0) return {0, 1};
   return rows_tile(M, N, K, choose_tile(M, N, false, true), g_gemm_splitk == 0 && !batch_invariant());
+}
+// the same for a product that may go to the kernels that `linear` looks at first
+static RowsTile rows_tile_behind(int M, int N, int K) {
+  if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), g_gemm_force_bn) > 1) return {0, 1};
+  return rows_tile_of(M, N, K);
 }
 // the same for a product on st, with the memory for its parts, and without parts where there is none
 static RowsTile rows_tile_of(int M, int N, int K, cudaStream_t st, float** ws) {
@@ -1485,17 +1480,9 @@ int b200q_gemm_set_tile_n(int bn) {
 // diagnostics: co-resident CTA pairs the 2-CTA kernel's grid is sized to (0 until first use)
 int b200q_gemm_resident_pairs(void) { return g_gemm2_pairs; }
 
-// test hook: rows of A in the tiles of gemm_rows.cu that a product takes (0: none of them)
-int b200q_gemm_rows_tile(int M, int N, int K) {
-  if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 0;
-  return rows_tile_of(M, N, K).rows;
-}
-
-// test hook: the parts of K of such a product (1: not split)
-int b200q_gemm_rows_splits(int M, int N, int K) {
-  if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), 0) > 1) return 1;
-  return rows_tile_of(M, N, K).splits;
-}
+// test hooks: rows of A in the tiles of gemm_rows.cu that a product takes (0: none of them), and the parts of K (1: not split)
+int b200q_gemm_rows_tile(int M, int N, int K) { return rows_tile_behind(M, N, K).rows; }
+int b200q_gemm_rows_splits(int M, int N, int K) { return rows_tile_behind(M, N, K).splits; }
 
 // test hook: columns of the tiles of a product of more than 128 rows whose reduction is not split
 int b200q_gemm_tile_n(int M, int N) { return g_gemm_force_bn ? g_gemm_force_bn : choose_tile(M, N, false, g_gemm_mode == 0).bn; }
