@@ -97,13 +97,14 @@ int b200q_prefill_attn(const void* q_dev, int q_stride, void* out_dev, const voi
 
 /* K3/K8/K9/K11/K12  C[M,N] = A[M,K] * W[N,K]^T, bf16 in, fp32 accumulate in TMEM (tcgen05),
  *     bf16 out.  A, W, C row-major and contiguous; K % 64 == 0, N % 64 == 0.  Waits inside the kernel are bounded
- *     (b200q_wait_failures).
+ *     (b200q_wait_failures).  129 to 768 rows of N <= 8192 may be summed in parts of K, which lie in scratch that the
+ *     stream keeps (up to 64 MiB, allocated when first needed); where there is no memory for it they are not.
  *     (replaces F.linear -> cuBLASLt, vllm/model_executor/layers/utils.py:92-98) */
 int b200q_gemm_bf16(const void* A_dev, const void* W_dev, void* C_dev,
                     int M, int N, int K, void* stream);
 
-/* Decode-sized batches: the split-K form of b200q_gemm_bf16 WITHOUT its reduce pass.  If the library
- *     would split the reduction for this shape, the fp32 partial tiles are left in its scratch
+/* Up to 768 rows: the split-K form of b200q_gemm_bf16 WITHOUT its reduce pass.  If the library
+ *     would split the reduction for this shape (up to 8 parts, N <= 8192), the fp32 partial tiles are left in its scratch
  *     (*partials = [splits][M][N], the stream's or, during capture, the graph's; valid until the next split product there) and *splits > 1;
  *     the caller folds sum-in-split-order + bf16 rounding into the consumer (the two *_splitk ops
  *     below).  *splits == 1: nothing was launched, call b200q_gemm_bf16.  Results are bit-identical

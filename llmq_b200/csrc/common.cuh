@@ -33,7 +33,7 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
 int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w, cudaStream_t st, const float** partials_out,
                  int* splits_out);
 int linear_gated(bool gelu, const void* A, const void* W, void* C, int M, int N, int K, bool fixed_w, cudaStream_t st);
-// parts of one split reduction: up to 8 splits x 256 rows x 8192 columns, 64 MiB
+// parts of one split reduction: up to 2048 rows x parts of 8192 columns (256 rows in 6, 768 in 2, 128 in 8), 64 MiB
 constexpr size_t SPLIT_BYTES = (size_t)8 * 256 * 8192 * sizeof(float);
 // While one of these lives, split products that the calling thread asks for leave their parts there: a pass runs under its model's
 class SplitScratchOf {

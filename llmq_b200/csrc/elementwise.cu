@@ -131,7 +131,7 @@ __device__ __forceinline__ void sum_partials_bf16(const float* ws, const long lo
 }
 
 // kPartials: x is not read from x_in but reduced on the fly from the fp32 partials of a split-K GEMM
-// (decode-sized batches): the projection's reduce pass, the residual add and the norm become ONE
+// (up to 768 rows): the projection's reduce pass, the residual add and the norm become ONE
 // launch instead of two, and the bf16 GEMM output never makes a round trip through memory.
 template <int CH, bool kAdd, bool kPartials = false>
 __global__ void __launch_bounds__(NORM_THREADS)
@@ -385,7 +385,7 @@ __device__ __forceinline__ void rope_chunk_pair(uint4& x1, uint4& x2, const uint
 }
 
 // kPartials: the qkv row is reduced on the fly from the fp32 partials of the split-K qkv projection
-// (decode-sized batches) instead of being read back as bf16 — reduce + RoPE + KV write in one launch
+// (up to 768 rows) instead of being read back as bf16 — reduce + RoPE + KV write in one launch
 template <bool kPartials>
 __global__ void __launch_bounds__(kPartials ? 128 : 256)
     rope_kvwrite_kernel(uint4* __restrict__ qkv, const uint4* __restrict__ cos_sin,

@@ -1050,8 +1050,9 @@ bool batch_invariant() {
   return v || g_gemm_splitk == 1;  // (the hook without splits stands for the variable)
 }
 
-// split-K factor for a decode-sized projection (1 = do not split): when it has too few 128-wide
-// output tiles to put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs
+// split-K factor for a decode-sized projection that gemm_skinny.cu leaves (1 = do not split): when it has too few 128-wide
+// output tiles to put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs.  129 to 256 rows are
+// split here only where a test asks for a count: rows_tile has their parts.
 static int choose_splits(int M, int N, int K, bool invariant, int forced_bn) {
   const int want = invariant ? 1 : g_gemm_splitk;  // 0 = auto, 1 = off, >1 = forced (tests)
   if (want == 1 || forced_bn != 0 || M > (want ? 256 : GEMM_BM) || N % 128 != 0 || N > 8192) return 1;

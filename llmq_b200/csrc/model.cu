@@ -293,7 +293,7 @@ int b200q_model_forward(b200q_model_t m, const b200q_batch* b, void* stream) {
   B200Q_TRY(B200Q_PROF_ELEMENTWISE, 2.0 * T * H * 2,
             b200q_embed_ex(b->token_ids, b->prev_out_ids, m->embed, m->residual, T, H,
                            gemma ? c.embed_scale : 0.f, stream));
-  // Decode-sized batches (llama arch): a projection that the GEMM splits along K leaves its fp32
+  // Up to 768 rows (llama arch): a projection that the GEMM splits along K leaves its fp32
   // partials in the library's scratch and the NEXT kernel of the chain reduces them on the fly —
   // qkv -> RoPE/KV write, o -> add+RMSNorm, down -> the next add+RMSNorm — instead of a separate
   // reduce pass per projection (96 launches per 32-layer step).  Bit-identical to the unfused chain.

@@ -12,7 +12,7 @@
 //     (keys K-major, values N-major).
 //   * Scores and outputs live in tensor memory; probabilities go back there as bf16 and are the A operand of the second product.
 //     D = 64, 128: two query tiles per CTA (four warps of softmax each), one's exponentials behind the other's products; 128 keys at a
-//     time.  D = 256: one query tile (its outputs take 256 columns), 64 keys at a time, four blocks of scores; the two warpgroups take the
+//     time.  D = 256: one query tile (its outputs take 256 columns), 64 keys at a time, four blocks of scores; three warpgroups take the
 //     steps in turns.
 //   * The running maximum moves only when a row's grows by more than 2^8 (exponents stay far from overflow; at D = 256 the first 512
 //     keys follow it exactly, so that short contexts round as the plain form does); the outputs in tensor memory are scaled in place.
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(FaCfg<D>::THREADS, 1) prefill_attn_kernel(cons
     const int wg = warp >> 2, i_tile = NQ == 2 ? wg : 0;
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    uint32_t s_count = 0, o_par = 0;  // steps so far (D = 256: of both warpgroups)
+    uint32_t s_count = 0, o_par = 0;  // steps so far (D = 256: of all warpgroups)
     const float c0e = 2.8853900817779268f * a.c0;  // 2 log2 e c0
     auto capped = [&](float v) {  // c1 tanh(c0 v) = c1 - 2 c1 / (1 + e^(2 c0 v))
       return fmaf(-2.f * a.c1, fa_rcp(fa_ex2(v * c0e) + 1.f), a.c1);

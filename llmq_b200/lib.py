@@ -533,7 +533,7 @@ def gemm_bf16(a, w, c, stream=None):
 
 
 def gemm_bf16_splitk(a, w, stream=None):
-    """decode-sized batches: split-K GEMM without its reduce pass.  Returns (partials_ptr, splits);
+    """up to 768 rows: split-K GEMM without its reduce pass.  Returns (partials_ptr, splits);
     splits == 1 means nothing was launched (the library would not split this shape)"""
     M, K = a.shape
     N = w.shape[0]
