@@ -1006,7 +1006,10 @@ static TileChoice choose_tile(int M, int N, bool gated, bool pairs) {
 // costs 2 us; 3 % have to be gained.  17 shapes x 20 row counts from 129 to 1000, sums included: the rule takes 0.937 of the time without
 // parts on average and 1.002 at worst, where always knowing the best would take 0.92.  us, without / with: 150 x 3584 x 14336 38.2 / 29.3,
 // 200 x 4096 x 14336 39.0 / 34.5; 256 x 2560 x 10240 32.4 / 20.5; 300 x 2048 x 8192 27.3 / 17.5, 512 rows 28.0 / 20.9, 750 rows 28.8 / 26.3;
-// 400 x 4096 x 14336 49.1 / 46.0.  (129 to 256 rows were split over tiles of 128 x 128 before: slower at all of 9 such shapes.)
+// 400 x 4096 x 14336 49.1 / 46.0.  From K = 2560 to 3584 parts have to gain 0.8 us more: another 1469 sizes (128 to 8192 columns, K 512 to 14336,
+// 129 to 768 rows, every tile and number of parts) showed 2 to 9 % lost there (513 x 1536 x 3072 14.6 in two parts, 13.4 whole; 256 x 3072 x 3072
+// 14.6 / 13.6).  With that and the parts that choose_splits still has, the rule takes 1.008 of the best's time there and 0.857 of the
+// time without these tiles, at worst 1.044 (20 sizes above 1.02).
 struct RowsTile {
   int rows, splits;
 };
@@ -1027,7 +1030,7 @@ static RowsTile rows_tile(int M, int N, int K, const TileChoice& other, bool may
       double t = rounds * c.cost * k_block * ((kb + s - 1) / s);
       if (s > 1) {
         const double weights = 0.124e-6 * 2.0 * N * K * pairs / (tiles < pairs ? tiles : pairs);
-        t = 1.03 * ((t > weights ? t : weights) + 2.0 * rounds + 1.1 + s * (0.2 + 0.3e-6 * 4.0 * M * N));
+        t = 1.03 * ((t > weights ? t : weights) + 2.0 * rounds + 1.1 + s * (0.2 + 0.3e-6 * 4.0 * M * N)) + (kb >= 40 && kb <= 56 ? 0.8 : 0.0);
       } else {
         t += 2.0;
       }
@@ -1051,13 +1054,22 @@ bool batch_invariant() {
 }
 
 // split-K factor for a decode-sized projection that gemm_skinny.cu leaves (1 = do not split): when it has too few 128-wide
-// output tiles to put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs.  129 to 256 rows are
-// split here only where a test asks for a count: rows_tile has their parts.
+// output tiles to put every SM on the weight stream, split the reduction so that tiles x splits ~ #SMs.
+// 193 to 256 rows whose tiles and parts are 128 CTAs (1024 columns in 8 parts, 2048 in 4), parts of 10 to 28 k-blocks: faster than the
+// parts of gemm_rows.cu, whose tiles of 256 columns leave a poor choice there (us, here / there: 256 x 1024 x 5120 11.1 / 12.6, x 12288
+// 14.9 / 16.2; 256 x 2048 x 3072 11.6 / 13.5, x 4096 12.9 / 14.6, x 7168 15.7 / 16.3; but x 12288 20.5 / 20.4, 2048 x 2048 10.4 / 10.0 in
+// whole tiles; 112, 120 or 144 CTAs lose 2 to 10 %, fewer rows are even).  Others of 129 to 256 rows are split here only where a test
+// asks for a count.
 static int choose_splits(int M, int N, int K, bool invariant, int forced_bn) {
   const int want = invariant ? 1 : g_gemm_splitk;  // 0 = auto, 1 = off, >1 = forced (tests)
-  if (want == 1 || forced_bn != 0 || M > (want ? 256 : GEMM_BM) || N % 128 != 0 || N > 8192) return 1;
+  if (want == 1 || forced_bn != 0 || M > 256 || N % 128 != 0 || N > 8192) return 1;
   const int tiles = ((M + GEMM_BM - 1) / GEMM_BM) * (N / 128);
   const int kb = K / GEMM_BK;
+  if (want == 0 && M > GEMM_BM) {
+    for (int s = 8; s >= 4; s /= 2)
+      if (M > 192 && tiles * s == 128 && kb % s == 0 && kb / s >= 10 && kb / s <= 28) return s;
+    return 1;
+  }
   int splits = want > 1 ? want : 1;
   if (want == 0 && tiles * 2 <= num_sms()) {
     for (int sN = 8; sN >= 2; --sN)

@@ -85,3 +85,23 @@ def test_what_the_rule_leaves_alone(cuda):
         assert rows(300, 8192, 3584) == 0
     finally:
         lib.gemm_set_mode(0)
+
+
+@pytest.mark.parametrize("M,N,K,parts", [(193, 1024, 5120, 8), (256, 1024, 14336, 8), (256, 2048, 2560, 4), (200, 2048, 7168, 4)])
+def test_parts_that_stay_with_tiles_of_128_rows(cuda, M, N, K, parts):
+    """128 CTAs of tiles and parts: the first and last row count, the shortest and longest parts; their neighbours go to the tiles above"""
+    from llmq_b200 import lib
+    L = lib.load()
+    assert L.b200q_gemm_rows_tile(M, N, K) == 0
+    assert L.b200q_gemm_rows_tile(192, N, K) > 0 and L.b200q_gemm_rows_tile(200, 2048, 64 * 4 * 29) > 0
+    a, w = inputs(cuda, M, N, K)
+    whole = torch.full((M + 1, N), float("nan"), dtype=BF, device=cuda)
+    lib.gemm_bf16(a, w, whole[:M])
+    # (as in test_parts)
+    bf16_close(whole[:M].cpu(), (a.double() @ w.double().t()).to(BF).cpu(), ulps=1.0, atol=2e-5 + K / 16 * 2.0 ** -24, what=f"{M} x {N} x {K}")
+    assert torch.isnan(whole[M]).all() and L.b200q_wait_failures() == 0
+    part, n = lib.gemm_bf16_splitk(a, w)
+    assert n == parts
+    y, res = torch.empty(M, N, dtype=BF, device=cuda), torch.zeros(M, N, dtype=BF, device=cuda)
+    lib.add_rmsnorm_splitk(y, res, torch.ones(N, dtype=BF, device=cuda), part, n, 1e-5)
+    assert torch.equal(res, whole[:M])
