@@ -39,6 +39,8 @@ template <int D>
 struct DecCfg {
   static constexpr int STAGES = D > 128 ? 2 : 3;
 };
+// (results below 2^-126 are 0: beside a row's largest probability, 1, a value would have to be 2^100 times the others to show one.  exp2f,
+// which keeps them, takes 6 sequences of 3000 to 8100 tokens, D = 64, 12.2 -> 13.0 us; 1.5, 0.7, 0.5 % at D = 64, 128, 256 over 17 sizes)
 __device__ __forceinline__ float dec_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
