@@ -1126,7 +1126,8 @@ static int launch_prefill(FaArgs a, cudaStream_t st) {
     return B200Q_ECUDA;
   }
   CUtensorMap q_map{}, out_map{};
-  a.whole_tokens = a.vec && a.q_flip == 0 && 32 % a.G == 0;
+  // (a tensor map takes rows of queries that lie one behind the other; others are read as they were before there was one)
+  a.whole_tokens = a.vec && a.q_flip == 0 && 32 % a.G == 0 && a.q_stride >= a.n_q * D;
   if (a.whole_tokens) {
     rc = get_head_rows_tmap(a.out, a.n_q, D, (long long)a.n_q * D, a.G, 32 / a.G, 32, &out_map);
     if (!rc) rc = get_head_rows_tmap(a.q, a.n_q, D, a.q_stride, a.G, 128 / a.G, 64, &q_map);

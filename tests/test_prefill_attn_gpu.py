@@ -221,3 +221,32 @@ def test_only_short_and_only_long_portions_of_a_wide_table(cuda):
     for D in (64, 128, 256):
         check(cuda, D, 8, 4, [(0, n) for n in (5, 16, 31, 40)] * 6, more_rows=300, seed=2, routes=(-1, 2))
         check(cuda, D, 8, 4, [(0, 600), (1000, 40), (0, 900)], more_rows=300, seed=3, routes=(-1, 2))
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 8, 1), (128, 8, 2), (256, 8, 2)])
+@pytest.mark.parametrize("stride", ["8 more", "24 more", "0", "back"])
+def test_query_strides(cuda, D, n_q, n_kv, stride):
+    """rows of queries that are 16-byte aligned, at any distance: no multiple of a head, the same row for every token, from the last one back"""
+    from llmq_b200 import lib
+    row, n = n_q * D, 200
+    kv, bt, rows = make_cache([n], n_kv, D, 1, True)
+    q = torch.randn(n, row + {"8 more": 8, "24 more": 24}.get(stride, 0), generator=torch.Generator().manual_seed(3)).to(BF)
+    dev, used = q.to(cuda), q[:, :row]
+    at, step = dev.data_ptr(), q.shape[1]
+    if stride == "0":
+        step, used = 0, q[:1, :row].expand(n, row)
+    elif stride == "back":
+        at, step, used = at + 2 * (n - 1) * step, -step, q.flip(0)
+    tiles = torch.tensor([[0, j, min(16, n - j), j] for j in range(0, n, 16)], dtype=torch.int32, device=cuda)
+    ref = reference(used.view(n, n_q, D), *rows[0], torch.arange(n), D ** -0.5, 0.0, 0).to(BF)
+    kv, bt = kv.to(cuda), bt.to(cuda)
+    for route in (0, 1):
+        out = torch.empty(n, row, dtype=BF, device=cuda)
+        lib.check(lib.load().b200q_prefill_attn_set_route(route))
+        try:
+            lib.check(lib.load().b200q_prefill_attn_seqs(at, step, out.data_ptr(), kv.data_ptr(), bt.data_ptr(), bt.shape[1], 1, tiles.data_ptr(),
+                                                         tiles.shape[0], n_q, n_kv, D, BS, D ** -0.5, 0.0, 0, lib._stream()))
+        finally:
+            lib.check(lib.load().b200q_prefill_attn_set_route(-1))
+        # (as in check)
+        bf16_close(out.cpu().view(n, n_q, D), ref, ulps=2.0, atol=5e-3, max_mismatch_frac=0.6, what=f"stride {stride} route {route}")
