@@ -1098,7 +1098,15 @@ static RowsTile rows_tile_behind(int M, int N, int K) {
   if (use_skinny(M, N, K, false) || choose_splits(M, N, K, batch_invariant(), g_gemm_force_bn) > 1) return {0, 1};
   return rows_tile_of(M, N, K);
 }
-// the same for a product on st, with the memory for its parts, and without parts where there is none
+// choose_splits for a product on st; more than 128 rows go on without parts where there is no memory for them
+static int choose_splits(int M, int N, int K, int forced_bn, cudaStream_t st) {
+  const int splits = choose_splits(M, N, K, batch_invariant(), forced_bn);
+  float* ws = nullptr;
+  if (splits <= 1 || M <= GEMM_BM || splitk_scratch(splits, M, N, st, &ws) == B200Q_OK) return splits;
+  cudaGetLastError();
+  return 1;
+}
+// the same for the tiles of gemm_rows.cu
 static RowsTile rows_tile_of(int M, int N, int K, cudaStream_t st, float** ws) {
   const RowsTile r = rows_tile_of(M, N, K);
   if (r.splits <= 1 || splitk_scratch(r.splits, M, N, st, ws) == B200Q_OK) return r;
@@ -1366,7 +1374,7 @@ int linear(const void* A, const void* W, void* C, int M, int N, int K, bool fixe
     // B200Q_BATCH_INVARIANT=1 (read once): never split K, so every output element is reduced in
     // one sequential pass (the attention kernels do likewise) and a request's tokens cannot depend on its batch-mates (like
     // VLLM_BATCH_INVARIANT); costs decode-sized GEMMs up to 2x
-    const int splits = choose_splits(M, N, K, batch_invariant(), bn);
+    const int splits = choose_splits(M, N, K, bn, st);
     if (splits > 1) return launch_gemm<128>(A, W, C, M, N, K, st, splits, nullptr, 0, GateArgs{nullptr, 0.f}, fixed_w);
   }
   if (bn == 0) {
@@ -1412,7 +1420,7 @@ int linear_parts(const void* A, const void* W, int M, int N, int K, bool fixed_w
     *splits_out = n;
     return B200Q_OK;
   }
-  const int splits = choose_splits(M, N, K, batch_invariant(), 0);
+  const int splits = choose_splits(M, N, K, 0, st);
   if (splits <= 1) {
     float* ws = nullptr;
     const RowsTile r = rows_tile_of(M, N, K, st, &ws);
